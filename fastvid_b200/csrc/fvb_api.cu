@@ -162,7 +162,7 @@ void build_desc(const fvb_frame& fr, FrameDesc& d, int use_med) {
   d.tile_h = static_cast<int32_t>(fr.tile_h);
   d.tiles_y = static_cast<int32_t>(ceil_div(fr.height, fr.tile_h));
   d.last_h = static_cast<int32_t>(fr.height - static_cast<int64_t>(d.tiles_y - 1) * fr.tile_h);
-  int64_t tile = 0, shard = 0, sample = 0;
+  int64_t tile = 0, shard = 0, sample = 0, fold = 0;
   for (int p = 0; p < d.planes; ++p) {
     const bool sub = fr.layout == 1 && p != 0;
     const int64_t pw = sub ? (fr.width + 1) / 2 : fr.width;
@@ -173,12 +173,16 @@ void build_desc(const fvb_frame& fr, FrameDesc& d, int use_med) {
     d.tiles_x[p] = static_cast<int32_t>(txs);
     d.tile0[p] = tile;
     d.shard0[p] = shard;
-    d.sample0[p] = sample;
+    d.fold0[p] = fold;
     const int64_t wl = pw - (txs - 1) * ptw;
     for (int r = 0; r < 2; ++r) {
       const int64_t h = r ? d.last_h : fr.tile_h;
       d.shards_int[p][r] = static_cast<int32_t>(ceil_div(ptw * h, kShardSymbols));
       d.shards_last[p][r] = static_cast<int32_t>(ceil_div(wl * h, kShardSymbols));
+      d.fold_int[p][r] = static_cast<int32_t>(fold_padded(ptw * h));
+      const int64_t row = (txs - 1) * fold_padded(ptw * h) + fold_padded(wl * h);
+      if (!r) d.fold_row[p] = row;
+      fold += r ? row : (d.tiles_y - 1) * row;
     }
     d.shards_row[p] = (txs - 1) * d.shards_int[p][0] + d.shards_last[p][0];
     const int64_t plane_shards = (d.tiles_y - 1) * d.shards_row[p] + (txs - 1) * d.shards_int[p][1] + d.shards_last[p][1];
@@ -188,10 +192,10 @@ void build_desc(const fvb_frame& fr, FrameDesc& d, int use_med) {
   }
   d.tile0[d.planes] = tile;
   d.shard0[d.planes] = shard;
-  d.sample0[d.planes] = sample;
   d.ntiles = tile;
   d.nshards = shard;
   d.nsamples = sample;
+  d.nfold = fold;
   d.max_sample = (1 << fr.bit_depth) - 1;
   d.step0 = fr.step;
   d.force_order0 = fr.layout == 2 && (fr.bit_depth != 10 || fr.width < 3840);
@@ -319,6 +323,13 @@ struct Totals {
   int64_t samples_p[kMaxPasses] = {0, 0, 0}, prefix_p[kMaxPasses] = {0, 0, 0};
 };
 
+// Folded samples of a frame: its samples with every tile padded.
+int64_t folded_samples(const fvb_frame& fr) {
+  FrameDesc d;
+  build_desc(fr, d, 0);
+  return d.nfold;
+}
+
 Totals totals_of(const fvb_frame* frames, int n) {
   Totals t;
   t.frames = n;
@@ -326,7 +337,8 @@ Totals totals_of(const fvb_frame* frames, int n) {
     const fvb_frame& f = frames[i];
     t.tiles += f.tiles;
     t.shards += f.shards;
-    t.samples += f.samples;
+    const int64_t folded = folded_samples(f);
+    t.samples += folded;
     t.prefix += f.prefix_bytes;
     const int64_t ptw0 = f.tile_w;
     if (ptw0 > kFastMaxW) t.wide = true;
@@ -337,7 +349,7 @@ Totals totals_of(const fvb_frame* frames, int n) {
       ++t.frames_p[p];
       t.tiles_p[p] += f.tiles;
       t.shards_p[p] += f.shards;
-      t.samples_p[p] += f.samples;
+      t.samples_p[p] += folded;
       t.prefix_p[p] += f.prefix_bytes;
     }
   }
@@ -653,6 +665,11 @@ int rans_pipe_for(int knob, int grid) {
 }
 std::atomic<int> g_tile_warps{kDefaultTileWarps};
 
+// Whether a wavefront launch has too few tiles to hide its step chain behind
+// other warps.
+constexpr int kFewTilesPerSm = 8;
+bool few_tiles(int64_t tiles) { return tiles <= static_cast<int64_t>(device_sms()) * kFewTilesPerSm; }
+
 int ctas(int kernel) {
   const int v = g_ctas[kernel].load(std::memory_order_relaxed);
   return v > 0 ? v : kDefaultCtas[kernel];
@@ -890,7 +907,7 @@ int encode_prepare(const Totals& cap, const fvb_frame* frames, int n, const uint
     d.prefix_base = pb;
     tb += d.ntiles;
     sb += d.nshards;
-    nb += d.nsamples;
+    nb += d.nfold;
     pb += d.prefix_bytes;
   }
   char* ws = static_cast<char*>(workspace);
@@ -1250,7 +1267,7 @@ int fill_decode_descs(const fvb_frame* frames, int n, const uint8_t* const* stre
     d.sample_base = nb;
     tb += d.ntiles;
     sb += d.nshards;
-    nb += d.nsamples;
+    nb += d.nfold;
   }
   return FVB_OK;
 }
@@ -1311,8 +1328,8 @@ int decode_enqueue(const Totals& t, int wavefront, void* workspace, int64_t work
   RansTable* tables = reinterpret_cast<RansTable*>(ws + L.tables);
   {
     LaunchScope scope_(K_DEC_SHARDS, stream);
-    dec_rans_tables_kernel<<<grid_for(t.shards, 128, ctas(K_DEC_SHARDS)), 128, 0, stream>>>(frames_d, state, shards, lists, items,
-                                                                           tables);
+    dec_rans_tables_kernel<<<grid_for(t.shards, 128, ctas(K_DEC_SHARDS)), 128, 0, stream>>>(
+        frames_d, state, shards, lists, items, tables, f16 ? 1 : 0);
   }
   FVB_LAUNCHED("dec_rans_tables_kernel");
   SideStream* side = nullptr;
@@ -1347,9 +1364,11 @@ int decode_enqueue(const Totals& t, int wavefront, void* workspace, int64_t work
     {
       LaunchScope scope_(K_DEC_RECON, stream);
       const int tw = g_tile_warps.load(std::memory_order_relaxed);
-      dec_reconstruct_launch(g_wavefront_block.load(std::memory_order_relaxed), tw, f16,
-                             grid_for(t.tiles * tw, kWarpsPerCta, ctas(K_DEC_RECON)), stream, frames_d, state, dims,
-                             folded, queue);
+      // u16: one CTA per tile until the cap, so that few tiles spread over
+      // the SMs; the warps take tiles from the queue
+      const int grid = grid_for(f16 ? t.tiles : t.tiles * tw, f16 ? 1 : kWarpsPerCta, ctas(K_DEC_RECON));
+      dec_reconstruct_launch(g_wavefront_block.load(std::memory_order_relaxed), tw, f16, few_tiles(t.tiles), grid,
+                             stream, frames_d, state, dims, folded, queue);
     }
     FVB_LAUNCHED("dec_reconstruct_kernel");
     if (t.wide) {

@@ -27,6 +27,13 @@ constexpr uint32_t kRansL = 1u << 23;
 constexpr int kPredictTag = 6;
 constexpr int kMaxTiles = 1 << 20;
 
+// Every tile's folded samples start at a multiple of this many (16 bytes of
+// u16): tiles are read and written in 16-byte chunks whatever their size.
+constexpr int kFoldAlign = 8;
+__host__ __device__ constexpr int64_t fold_padded(int64_t samples) {
+  return (samples + kFoldAlign - 1) / kFoldAlign * kFoldAlign;
+}
+
 // Largest shard record: the competition never picks a body above the block
 // pack cost (<= 32 width bytes + 4096*17/8), forced rANS stays below that too.
 constexpr int kMaxRecordBytes = 3 + 32 + (kShardSymbols * 17 + 7) / 8;
@@ -63,11 +70,14 @@ struct FrameDesc {
   int32_t use_med0;     // predictor of the first encode pass / of the decode
   int64_t tile0[4];     // first tile of each plane; tile0[planes] = ntiles
   int64_t shard0[4];    // first shard of each plane
-  int64_t sample0[4];   // first sample of each plane
+  int64_t fold0[3];       // folded index of each plane's first sample
+  int64_t fold_row[3];    // folded samples of one full-height tile row
+  int32_t fold_int[3][2]; // folded samples of an interior tile [plane][last row?]
   int64_t shards_row[3];      // shards in one full-height tile row
   int32_t shards_int[3][2];   // shards of an interior tile [plane][last row?]
   int32_t shards_last[3][2];  // shards of a last-column tile
   int64_t ntiles, nshards, nsamples;
+  int64_t nfold;          // folded samples of the frame, tile padding included
   int64_t tile_base, shard_base, sample_base;  // placement in the batch arrays
   int64_t prefix_base;   // byte offset of this frame's header+directory in prefix scratch
   int64_t prefix_bytes;  // 32 + 32 * ntiles
@@ -137,7 +147,7 @@ struct ShardInfo {
 // encode.cu:739-767).
 struct TileGeo {
   int32_t plane, x, y, w, h;
-  int64_t sample_base;   // frame-local folded index of the tile's first sample
+  int64_t sample_base;   // frame-local folded index of the tile's first sample (a multiple of kFoldAlign)
   int64_t first_shard;   // frame-local
   int32_t shard_count;
 };
@@ -156,8 +166,8 @@ __host__ __device__ inline TileGeo tile_geo(const FrameDesc& f, int64_t t) {
   g.y = ty * f.tile_h;
   g.w = last_col ? f.plane_w[p] - g.x : f.ptile_w[p];
   g.h = last_row ? f.last_h : f.tile_h;
-  g.sample_base = f.sample0[p] + static_cast<int64_t>(ty) * f.tile_h * f.plane_w[p] +
-                  static_cast<int64_t>(tx) * f.ptile_w[p] * g.h;
+  g.sample_base = f.fold0[p] + static_cast<int64_t>(ty) * f.fold_row[p] +
+                  static_cast<int64_t>(tx) * f.fold_int[p][last_row];
   g.first_shard = f.shard0[p] + static_cast<int64_t>(ty) * f.shards_row[p] +
                   static_cast<int64_t>(tx) * f.shards_int[p][last_row];
   g.shard_count = last_col ? f.shards_last[p][last_row] : f.shards_int[p][last_row];

@@ -12,6 +12,7 @@
 // read shard records that were not written.
 #include "fvb_common.cuh"
 #include "fvb_kernels.cuh"
+#include "fvb_wave.cuh"
 
 namespace fvb {
 
@@ -170,7 +171,7 @@ struct RansTable {
   int32_t nsym, valid;
   int32_t pad[2];
   uint32_t freqcum[256];  // cum | freq << 12 (freq up to 4096: 13 bits)
-  uint32_t value[256];    // the symbol's value as u16 (decode.cu:484)
+  uint32_t value[256];    // what the symbol stores: its value as u16 (decode.cu:484), or fold_value of it
 };
 
 size_t dec_rans_table_bytes() { return sizeof(RansTable); }
@@ -315,7 +316,7 @@ struct LaneRing {
 
 // Order-0 table of one shard, parsed by one thread (decode.cu:456-517).
 __device__ bool rans_parse_serial(const uint8_t* __restrict__ body, int64_t blen, uint32_t maxf,
-                                  RansTable& t) {
+                                  const FoldMap& fm, RansTable& t) {
   ByteWindow r;
   r.init(body, blen);
   int64_t cursor = 0;
@@ -355,7 +356,7 @@ __device__ bool rans_parse_serial(const uint8_t* __restrict__ body, int64_t blen
         (i + 1 != n && fr == (1u << kRansTableLog) - assigned))
       return false;
     t.freqcum[i] = assigned | (fr << 12);
-    t.value[i] = value & 0xffffu;
+    t.value[i] = fm.lim ? fold_value<uint16_t>(value, fm) : value & 0xffffu;
     assigned += fr;
     prev = value;
   }
@@ -398,7 +399,7 @@ __device__ bool rans_parse_serial(const uint8_t* __restrict__ body, int64_t blen
 __global__ void __launch_bounds__(128)
 dec_rans_tables_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
                        const ShardInfo* __restrict__ shards, const DecodeLists* __restrict__ lists,
-                       const int32_t* __restrict__ list_items, RansTable* __restrict__ tables) {
+                       const int32_t* __restrict__ list_items, RansTable* __restrict__ tables, int fold16) {
   const int count = lists->count[0];
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x) {
     const ShardInfo& si = shards[list_items[p]];
@@ -407,7 +408,8 @@ dec_rans_tables_kernel(const FrameDesc* __restrict__ frames, FrameState* __restr
     bool ok = false;
     if (st.status == 0) {  // a failed parse may have left shard records unwritten
       const FrameDesc& f = frames[si.frame];
-      ok = rans_parse_serial(f.stream + si.offset, si.body, static_cast<uint32_t>(f.max_sample) * 2u, t);
+      ok = rans_parse_serial(f.stream + si.offset, si.body, static_cast<uint32_t>(f.max_sample) * 2u,
+                             fold_map(f, fold16), t);
       if (!ok) set_status(&st.status, 5);
     }
     t.valid = ok;
@@ -481,7 +483,7 @@ __device__ __forceinline__ void rans_decode_lane(const uint32_t* __restrict__ bc
     // starts at offsets 1..r of the bucket survive the shift by 31 - r
     const uint32_t sym = (bw >> 16) + __popc(bw << ((slot & ((1u << kBucketShift) - 1u)) ^ 31u));
     const uint32_t fc = fc_col[sym << LOG_S];
-    out[idx] = static_cast<FoldT>(val_col[sym << LOG_S]);  // symbols below 511
+    out[idx] = static_cast<FoldT>(val_col[sym << LOG_S]);
     x = (fc >> 12) * (x >> kRansTableLog) + slot - (fc & ((1u << kRansTableLog) - 1u));
     const int nb = (x < kRansL) + (x < (kRansL >> 8));
     const uint32_t sh = 8u * static_cast<uint32_t>(nb);  // 0, 8 or 16
@@ -664,7 +666,7 @@ __device__ __forceinline__ void zero_fill(FoldT* p, int64_t cnt) {
 // it with the same arguments.  Returns whether the shard is valid.
 template <typename FoldT>
 __device__ bool zero_run_warp(const uint8_t* __restrict__ body, int64_t blen, int n, uint32_t maxf,
-                              FoldT* __restrict__ out, int lane) {
+                              const FoldMap& fm, FoldT* __restrict__ out, int lane) {
   for (int i = lane; i < n; i += 32) out[i] = 0;
   __syncwarp();
   int produced = 0;        // symbols of the steps so far (warp-uniform)
@@ -715,7 +717,7 @@ __device__ bool zero_run_warp(const uint8_t* __restrict__ body, int64_t blen, in
     const uint32_t start = static_cast<uint32_t>(produced) + inc - cnt;
     if (is_end) {
       if (start + cnt > static_cast<uint32_t>(n)) tb = true;  // a run past the end, or a token after it
-      if (!tb && (tok & 1u)) out[start] = fold_store<FoldT>((tok + 1u) >> 1);
+      if (!tb && (tok & 1u)) out[start] = fold_value<FoldT>((tok + 1u) >> 1, fm);
     }
     bad = __any_sync(kFull, is_end && tb);
     produced += static_cast<int>(__shfl_sync(kFull, inc, 31));
@@ -790,6 +792,7 @@ dec_other_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ 
     const uint8_t* body = nullptr;
     FoldT* out = nullptr;
     uint32_t maxf = 0;
+    FoldMap fm{0, 0};
     if (s_mine >= 0) {
       const ShardInfo& si = shards[s_mine];
       fi = si.frame;
@@ -800,6 +803,7 @@ dec_other_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ 
       body = frames[fi].stream + si.offset;
       out = folded + si.sample_base;
       maxf = static_cast<uint32_t>(frames[fi].max_sample) * 2u;
+      fm = fold_map(frames[fi], sizeof(FoldT) == 2);
     }
     if (list == 1) {
       // ---- Rice ---------------------------------------------------------------
@@ -841,7 +845,7 @@ dec_other_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ 
                     ok = false;
                     break;
                   }
-                  out[idx] = fold_store<FoldT>(static_cast<uint32_t>(v));
+                  out[idx] = fold_value<FoldT>(static_cast<uint32_t>(v), fm);
                   idx += lc;
                   lo = static_cast<uint32_t>(rr.bits);
                   z0 = __ffs(lo) - 1;
@@ -886,7 +890,7 @@ dec_other_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ 
                 ok = false;
                 break;
               }
-              out[idx] = fold_store<FoldT>(static_cast<uint32_t>(v));
+              out[idx] = fold_value<FoldT>(static_cast<uint32_t>(v), fm);
               idx += lc;
             }
             cp_async_wait<0>();  // no copy into the ring outlives the lane
@@ -916,7 +920,8 @@ dec_other_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ 
         const uint8_t* bodyk =
             reinterpret_cast<const uint8_t*>(__shfl_sync(kFull, reinterpret_cast<uintptr_t>(body), 4 * k));
         FoldT* outk = reinterpret_cast<FoldT*>(__shfl_sync(kFull, reinterpret_cast<uintptr_t>(out), 4 * k));
-        if (!zero_run_warp(bodyk, bk, nk, mk, outk, lane) && lane == 0) set_status(&state[fk].status, 1);
+        const FoldMap fmk{__shfl_sync(kFull, fm.step, 4 * k), __shfl_sync(kFull, fm.lim, 4 * k)};
+        if (!zero_run_warp(bodyk, bk, nk, mk, fmk, outk, lane) && lane == 0) set_status(&state[fk].status, 1);
       }
     } else {
       // ---- block pack: the warp takes the shards one after another ------------
@@ -931,6 +936,7 @@ dec_other_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ 
         const uint32_t mk = __shfl_sync(kFull, maxf, 4 * k);
         const uint8_t* bodyk = reinterpret_cast<const uint8_t*>(__shfl_sync(kFull, reinterpret_cast<uintptr_t>(body), 4 * k));
         FoldT* outk = reinterpret_cast<FoldT*>(__shfl_sync(kFull, reinterpret_cast<uintptr_t>(out), 4 * k));
+        const FoldMap fmk{__shfl_sync(kFull, fm.step, 4 * k), __shfl_sync(kFull, fm.lim, 4 * k)};
         const int nblk = (nk + kBlockSymbols - 1) / kBlockSymbols;
         const int maxw = 32 - __clz(mk);
         if (lane == 0) {
@@ -986,7 +992,7 @@ dec_other_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ 
                 v = static_cast<uint32_t>((acc >> (bit & 7)) & ((1ull << w) - 1));
               }
               if (v > mk) bad = 1;
-              outk[static_cast<int64_t>(b) * kBlockSymbols + i] = fold_store<FoldT>(v);
+              outk[static_cast<int64_t>(b) * kBlockSymbols + i] = fold_value<FoldT>(v, fmk);
             }
           }
           if (__any_sync(kFull, bad) && lane == 0) set_status(&state[fk].status, 3);
@@ -1016,7 +1022,7 @@ struct RecWarpSmem {
 };
 
 size_t dec_reconstruct_smem(bool fold16) {
-  return (fold16 ? sizeof(RecWarpSmem<uint16_t>) : sizeof(RecWarpSmem<uint32_t>)) * kWarpsPerCta;
+  return (fold16 ? sizeof(WaveSm) : sizeof(RecWarpSmem<uint32_t>)) * kWarpsPerCta;
 }
 
 template <bool MED, bool STEP1, bool EDGE, int UNROLL, bool SPLIT, typename FoldT>
@@ -1232,8 +1238,154 @@ dec_reconstruct_kernel(const FrameDesc* __restrict__ frames, const FrameState* _
   }
 }
 
-// The wavefront block of dec_reconstruct is a launch-time choice, as for
-// enc_predict (4, 8, 16 or 32 steps unrolled; identical planes).
+// ---------------------------------------------------------------------------
+// dec_reconstruct on u16 symbols (every batch without a lossless 16-bit
+// frame): the two-rows-per-lane wavefront of fvb_wave.cuh.  Up to depth 12
+// the entropy decoders have already turned symbols into residuals times the
+// step (fold_value), so a step is one packed add-clamp after the prediction;
+// depth 16 unfolds and scales its symbols here, in 32 bits a row.
+
+// Eight steps of a window block.
+template <bool MED, int SK, bool O0, bool O1>
+__device__ __forceinline__ void rec_wave_steps(WavePacked<SK>& st, WaveBlock<SK, O0, O1>& blk, int g,
+                                               const WaveWords<O0>& x, const WaveWords<O1>& y, const WaveCarry& c,
+                                               int32_t maxs, int32_t) {
+  const uint32_t maxs2 = pair2(maxs);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t dq = wave_pack(x, y, j);
+    const uint32_t a = st.neighbours(c.up[j >> 1], j & 1, blk.lane);
+    const uint32_t rn = __viaddmin_s16x2_relu(st.template predict<MED>(a, maxs2), dq, maxs2);
+    blk.put(g, j, st.rec, rn, st.rec, rn);
+    st.above = a;
+    st.rec = rn;
+  }
+}
+
+template <bool MED, int SK, bool O0, bool O1>
+__device__ __forceinline__ void rec_wave_steps(WaveWide<SK>& st, WaveBlock<SK, O0, O1>& blk, int g,
+                                               const WaveWords<O0>& x, const WaveWords<O1>& y, const WaveCarry& c,
+                                               int32_t maxs, int32_t step) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    int32_t a0, a1;
+    st.neighbours(c.up[j >> 1], j & 1, blk.lane, a0, a1);
+    const uint32_t was = st.packed();
+    const int32_t p0 = st.template predict<MED>(st.rec0, a0, st.above0, maxs);
+    const int32_t p1 = st.template predict<MED>(st.rec1, a1, st.above1, maxs);
+    st.rec0 = __viaddmin_s32_relu(p0, unzigzag(x.sample(j)) * step, maxs);
+    st.rec1 = __viaddmin_s32_relu(p1, unzigzag(y.sample(j)) * step, maxs);
+    st.above0 = a0;
+    st.above1 = a1;
+    const uint32_t rn = st.packed();
+    blk.put(g, j, was, rn, was, rn);
+  }
+}
+
+// One window block: 32 steps in four groups of eight, the next group's words
+// loaded before this group's results are stored over theirs.
+template <bool MED, int SK, bool O0, bool O1, typename St>
+__device__ __forceinline__ void rec_wave_block(St& st, WaveBlock<SK, O0, O1> blk, int32_t maxs, int32_t step) {
+  WaveWords<O0> x, xn;
+  WaveWords<O1> y, yn;
+  WaveCarry c, cn;
+  x.first(blk.p0);
+  y.first(blk.p1);
+  x.load(blk.p0, 0);
+  y.load(blk.p1, 0);
+  c.load(blk.crow, 0);
+#pragma unroll 1
+  for (int g = 0; g < 4; g += 2) {
+    xn.after(x);
+    yn.after(y);
+    xn.load(blk.p0, g + 1);
+    yn.load(blk.p1, g + 1);
+    cn.load(blk.crow, g + 1);
+    rec_wave_steps<MED>(st, blk, g, x, y, c, maxs, step);
+    x.after(xn);
+    y.after(yn);
+    if (g == 0) {
+      x.load(blk.p0, 2);
+      y.load(blk.p1, 2);
+      c.load(blk.crow, 2);
+    }
+    rec_wave_steps<MED>(st, blk, g + 1, xn, yn, cn, maxs, step);
+  }
+  blk.finish(st.packed(), st.packed());
+}
+
+// ODD_W: the tile's rows start on even and odd samples in turn
+template <bool MED, bool WIDE, int SK, bool ODD_W>
+__device__ void rec_wave_tile(const FrameDesc& f, const TileGeo& g, const uint16_t* __restrict__ ftile, WaveSm& sm,
+                              int lane) {
+  for (int i = lane; i < kCarryCols / 8; i += 32) reinterpret_cast<uint4*>(sm.carry)[i] = make_uint4(0, 0, 0, 0);
+  __syncwarp();
+  WaveIo<SK, false> io(sm, lane, g.w, ftile, g.w, f.dst[g.plane] + static_cast<int64_t>(g.y) * f.dst_pitch[g.plane] + g.x,
+                       f.dst_pitch[g.plane], nullptr, nullptr);
+  for (int y = 0; y < g.h; y += kBandRows, io.next_band()) {
+    io.band(g.h - y);
+    io.fetch(0);
+    std::conditional_t<WIDE, WaveWide<SK>, WavePacked<SK>> st;
+    for (int b = 0; b < io.nblk; ++b) {
+      if (b) {
+        io.flush(b - 1);
+        io.move_head(b);
+        __syncwarp();
+      }
+      if (b + 1 < io.nblk) io.fetch(b + 1);
+      else cp_async_commit();
+      io.wait();
+      io.template fix_edge<false>(b);
+      rec_wave_block<MED, SK, false, !ODD_W>(st, WaveBlock<SK, false, !ODD_W>(sm, b, lane, io.off0, io.off1),
+                                             f.max_sample, f.step0);
+      __syncwarp();
+    }
+    io.flush_last();
+    __syncwarp();
+  }
+}
+
+template <int SK>
+__global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
+dec_reconstruct_wave_kernel(const FrameDesc* __restrict__ frames, const FrameState* __restrict__ state,
+                            const BatchDims* __restrict__ dims, const uint16_t* __restrict__ folded,
+                            int* __restrict__ queue) {
+  const int nframes = dims->frames_p[0];
+  const int64_t total_tiles = dims->tiles_p[0];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  WaveSm& sm = reinterpret_cast<WaveSm*>(smem_raw)[warp];
+  // a warp's first tile goes by its place -- the first warps of all CTAs
+  // before the second ones, so few tiles spread over all SMs -- and the rest
+  // come from the queue
+  const int64_t warps_total = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
+  for (int64_t t = static_cast<int64_t>(warp) * gridDim.x + blockIdx.x; t < total_tiles;) {
+    const int64_t mine = t;
+    if (lane == 0) t = warps_total + atomicAdd(queue, 1);
+    t = __shfl_sync(kFull, t, 0);
+    const int fi = frame_of_tile(frames, nframes, mine);
+    const FrameDesc& f = frames[fi];
+    if (state[fi].status != 0) continue;
+    const TileGeo g = tile_geo(f, mine - f.tile_base);
+    if (g.w > kFastMaxW) continue;
+    const uint16_t* ftile = folded + f.sample_base + g.sample_base;
+    const bool odd = g.w & 1, wide = f.bit_depth > 12;
+    if (f.use_med0) {
+      if (!wide) odd ? rec_wave_tile<true, false, SK, true>(f, g, ftile, sm, lane)
+                     : rec_wave_tile<true, false, SK, false>(f, g, ftile, sm, lane);
+      else odd ? rec_wave_tile<true, true, SK, true>(f, g, ftile, sm, lane)
+               : rec_wave_tile<true, true, SK, false>(f, g, ftile, sm, lane);
+    } else {
+      if (!wide) odd ? rec_wave_tile<false, false, SK, true>(f, g, ftile, sm, lane)
+                     : rec_wave_tile<false, false, SK, false>(f, g, ftile, sm, lane);
+      else odd ? rec_wave_tile<false, true, SK, true>(f, g, ftile, sm, lane)
+               : rec_wave_tile<false, true, SK, false>(f, g, ftile, sm, lane);
+    }
+  }
+}
+
+// The wavefront block of the u32 dec_reconstruct is a launch-time choice (4,
+// 8, 16 or 32 steps unrolled; identical planes), as are its warps per tile.
 cudaError_t dec_reconstruct_set_smem() {
   const int b32 = static_cast<int>(dec_reconstruct_smem(false)), b16 = static_cast<int>(dec_reconstruct_smem(true));
   for (auto k : {dec_reconstruct_kernel<4, false, uint32_t>, dec_reconstruct_kernel<8, false, uint32_t>,
@@ -1242,34 +1394,30 @@ cudaError_t dec_reconstruct_set_smem() {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, b32);
     if (e != cudaSuccess) return e;
   }
-  for (auto k : {dec_reconstruct_kernel<4, false, uint16_t>, dec_reconstruct_kernel<8, false, uint16_t>,
-                 dec_reconstruct_kernel<16, false, uint16_t>, dec_reconstruct_kernel<32, false, uint16_t>,
-                 dec_reconstruct_kernel<8, true, uint16_t>}) {
+  for (auto k : {dec_reconstruct_wave_kernel<2>, dec_reconstruct_wave_kernel<4>}) {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, b16);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
 
-template <typename FoldT>
-static void dec_reconstruct_launch_t(int unroll, int tile_warps, int grid, cudaStream_t stream,
-                                     const FrameDesc* frames, const FrameState* state, const BatchDims* dims,
-                                     const void* folded, int* queue) {
-  // warp pairs run with the default wavefront block
-  auto k = tile_warps == 2 ? dec_reconstruct_kernel<8, true, FoldT>
-           : unroll == 4   ? dec_reconstruct_kernel<4, false, FoldT>
-           : unroll == 16  ? dec_reconstruct_kernel<16, false, FoldT>
-           : unroll == 32  ? dec_reconstruct_kernel<32, false, FoldT>
-                           : dec_reconstruct_kernel<8, false, FoldT>;
-  k<<<grid, kWarpsPerCta * 32, dec_reconstruct_smem(sizeof(FoldT) == 2), stream>>>(
-      frames, state, dims, static_cast<const FoldT*>(folded), queue);
-}
-
-void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, int grid, cudaStream_t stream,
+void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, bool few, int grid, cudaStream_t stream,
                             const FrameDesc* frames, const FrameState* state, const BatchDims* dims,
                             const void* folded, int* queue) {
-  if (fold16) dec_reconstruct_launch_t<uint16_t>(unroll, tile_warps, grid, stream, frames, state, dims, folded, queue);
-  else dec_reconstruct_launch_t<uint32_t>(unroll, tile_warps, grid, stream, frames, state, dims, folded, queue);
+  if (fold16) {
+    auto k = few ? dec_reconstruct_wave_kernel<4> : dec_reconstruct_wave_kernel<2>;
+    k<<<grid, kWarpsPerCta * 32, dec_reconstruct_smem(true), stream>>>(
+        frames, state, dims, static_cast<const uint16_t*>(folded), queue);
+    return;
+  }
+  // warp pairs run with the default wavefront block
+  auto k = tile_warps == 2 ? dec_reconstruct_kernel<8, true, uint32_t>
+           : unroll == 4   ? dec_reconstruct_kernel<4, false, uint32_t>
+           : unroll == 16  ? dec_reconstruct_kernel<16, false, uint32_t>
+           : unroll == 32  ? dec_reconstruct_kernel<32, false, uint32_t>
+                           : dec_reconstruct_kernel<8, false, uint32_t>;
+  k<<<grid, kWarpsPerCta * 32, dec_reconstruct_smem(false), stream>>>(
+      frames, state, dims, static_cast<const uint32_t*>(folded), queue);
 }
 
 void dec_rans_launch(bool fold16, int grid, size_t smem, cudaStream_t stream, const FrameDesc* frames,
@@ -1316,7 +1464,7 @@ __global__ void dec_reconstruct_wide_kernel(const FrameDesc* __restrict__ frames
     uint16_t* plane = f.dst[g.plane];
     const int64_t pitch = f.dst_pitch[g.plane];
     const int64_t fbase = f.sample_base + g.sample_base;
-    const int32_t maxs = f.max_sample, step = f.step0;
+    const int32_t maxs = f.max_sample;
     for (int d = 0; d < g.w + g.h - 1; ++d) {
       const int y0 = max(0, d - g.w + 1), y1 = min(d, g.h - 1);
       for (int y = y0 + threadIdx.x; y <= y1; y += blockDim.x) {
@@ -1326,8 +1474,8 @@ __global__ void dec_reconstruct_wide_kernel(const FrameDesc* __restrict__ frames
         const int32_t a = y > 0 ? o[-pitch] : 0;
         const int32_t ul = (x > 0 && y > 0) ? o[-pitch - 1] : 0;
         const int32_t pred = f.use_med0 ? predict_med(l, a, ul) : predict_grad(l, a, ul, maxs);
-        const uint32_t fv = fold_at(folded, fold16, fbase + static_cast<int64_t>(y) * g.w + x);
-        *o = static_cast<uint16_t>(max(0, min(maxs, pred + unzigzag(fv) * step)));
+        const int32_t dq = delta_at(f, folded, fold16, fbase + static_cast<int64_t>(y) * g.w + x);
+        *o = static_cast<uint16_t>(max(0, min(maxs, pred + dq)));
       }
       __syncthreads();
     }
@@ -1349,7 +1497,7 @@ __global__ void dec_reconstruct_serial_kernel(const FrameDesc* __restrict__ fram
   uint16_t* plane = f.dst[g.plane];
   const int64_t pitch = f.dst_pitch[g.plane];
   const int64_t fbase = f.sample_base + g.sample_base;
-  const int32_t maxs = f.max_sample, step = f.step0;
+  const int32_t maxs = f.max_sample;
   const bool med = f.use_med0 != 0;
   for (int y = 0; y < g.h; ++y) {
     int32_t left = 0, ul = 0;
@@ -1358,7 +1506,7 @@ __global__ void dec_reconstruct_serial_kernel(const FrameDesc* __restrict__ fram
     for (int x = 0; x < g.w; ++x) {
       const int32_t a = y > 0 ? orow[x - pitch] : 0;
       const int32_t pred = med ? predict_med(left, a, ul) : predict_grad(left, a, ul, maxs);
-      const int32_t r = max(0, min(maxs, pred + unzigzag(fold_at(folded, fold16, frow + x)) * step));
+      const int32_t r = max(0, min(maxs, pred + delta_at(f, folded, fold16, frow + x)));
       orow[x] = static_cast<uint16_t>(r);
       ul = a;
       left = r;

@@ -30,7 +30,7 @@ __host__ __device__ inline bool pair_splits(int w, int h) { return ((h + 31) >> 
 // 16-bit frame below quality 100 has a step of at least 12.  The decoder
 // accepts symbols up to 2 * max_sample (decode.cu bounds), which at depth 16
 // can exceed 16 bits in a valid stream; such a symbol is stored as 65534 or
-// 65535 by parity (fold_store), i.e. a residual of +32767 or -32768 steps,
+// 65535 by parity (fold_value), i.e. a residual of +32767 or -32768 steps,
 // which clamps to the same sample as the original since the step is >= 12.
 template <typename T>
 constexpr int fold_stride() {
@@ -43,14 +43,37 @@ template <typename T>
 __device__ __forceinline__ uint32_t ldf(const T* p) {
   return static_cast<uint32_t>(__ldg(p));
 }
+//
+// The decoder's u16 intermediate of a frame of depth 12 or less holds, in
+// place of the symbol, what the reconstruction adds to the prediction: the
+// unfolded residual times the step, as a signed 16-bit value.  The residual
+// is first clamped to +-ceil(max_sample / step), beyond which the sample
+// saturates whatever the prediction is, so the product stays below
+// 2 * max_sample.  The rANS decoder does this once per table entry.
+struct FoldMap {
+  int32_t step, lim;  // lim 0: symbols are stored as they are
+};
+__device__ __forceinline__ FoldMap fold_map(const FrameDesc& f, bool fold16) {
+  if (!fold16 || f.bit_depth > 12) return FoldMap{1, 0};
+  return FoldMap{f.step0, (f.max_sample + f.step0 - 1) / f.step0};
+}
 template <typename T>
-__device__ __forceinline__ T fold_store(uint32_t v) {
-  if constexpr (sizeof(T) == 2) return static_cast<T>(min(v, 65534u | (v & 1u)));
-  else return v;
+__device__ __forceinline__ T fold_value(uint32_t v, const FoldMap& m) {
+  if constexpr (sizeof(T) == 2) {
+    if (m.lim) return static_cast<T>(max(-m.lim, min(m.lim, unzigzag(v))) * m.step);
+    return static_cast<T>(min(v, 65534u | (v & 1u)));
+  } else {
+    return v;
+  }
 }
 __device__ __forceinline__ uint32_t fold_at(const void* folded, int fold16, int64_t i) {
   return fold16 ? static_cast<uint32_t>(static_cast<const uint16_t*>(folded)[i])
                 : static_cast<const uint32_t*>(folded)[i];
+}
+// The residual times the step of sample i of a decoded frame.
+__device__ __forceinline__ int32_t delta_at(const FrameDesc& f, const void* folded, int fold16, int64_t i) {
+  if (fold16 && f.bit_depth <= 12) return static_cast<const int16_t*>(folded)[i];
+  return unzigzag(fold_at(folded, fold16, i)) * f.step0;
 }
 __device__ __forceinline__ void unpack_piece(const uint4& p, uint32_t (&x)[4]) {
   x[0] = p.x;
@@ -115,7 +138,8 @@ struct RansTable;
 __global__ void dec_parse_kernel(const FrameDesc* frames, FrameState* state, const BatchDims* dims,
                                  ShardInfo* shards, DecodeLists* lists, int32_t* list_items);
 __global__ void dec_rans_tables_kernel(const FrameDesc* frames, FrameState* state, const ShardInfo* shards,
-                                       const DecodeLists* lists, const int32_t* list_items, RansTable* tables);
+                                       const DecodeLists* lists, const int32_t* list_items, RansTable* tables,
+                                       int fold16);
 void dec_rans_launch(bool fold16, int grid, size_t smem, cudaStream_t stream, const FrameDesc* frames,
                      FrameState* state, const ShardInfo* shards, DecodeLists* lists, const int32_t* list_items,
                      const RansTable* tables, void* folded);
@@ -123,7 +147,9 @@ cudaError_t dec_rans_set_attr(cudaFuncAttribute attr, int value);
 void dec_other_launch(bool fold16, int grid, cudaStream_t stream, const FrameDesc* frames, FrameState* state,
                       const ShardInfo* shards, const BatchDims* dims, DecodeLists* lists, const int32_t* list_items,
                       void* folded);
-void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, int grid, cudaStream_t stream,
+// u16 symbols: `few` tiles for the GPU's warps take the shorter-chain sweep;
+// u32 symbols: `unroll` and `tile_warps` as for enc_predict
+void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, bool few, int grid, cudaStream_t stream,
                             const FrameDesc* frames, const FrameState* state, const BatchDims* dims,
                             const void* folded, int* queue);
 cudaError_t dec_reconstruct_set_smem();
