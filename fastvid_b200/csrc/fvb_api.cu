@@ -282,6 +282,7 @@ int ensure_smem_attrs() {
   FVB_CUDA(enc_predict_set_smem());
   FVB_CUDA(enc_emit_set_smem(static_cast<int>(enc_emit_smem())));
   FVB_CUDA(dec_reconstruct_set_smem());
+  FVB_CUDA(dec_other_set_smem());
   FVB_CUDA(dec_rans_set_attr(cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dec_rans_smem())));
   // the whole unified L1/shared array as shared memory: four dec_rans CTAs
   // (56 KB each) per SM
@@ -1350,7 +1351,7 @@ int decode_enqueue(const Totals& t, int wavefront, void* workspace, int64_t work
     if (side) FVB_CUDA(cudaStreamWaitEvent(other, side->fork, 0));
     {
       LaunchScope scope_(K_DEC_OTHER, other);
-      dec_other_launch(f16, grid_for(ceil_div(t.shards, kGroupShards), 4, ctas(K_DEC_OTHER)), other, frames_d, state,
+      dec_other_launch(f16, grid_for(t.shards, 1, ctas(K_DEC_OTHER)), other, frames_d, state,
                        shards, dims, lists, items, folded);
     }
     const cudaError_t launched = cudaGetLastError();

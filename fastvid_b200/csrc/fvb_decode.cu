@@ -159,7 +159,6 @@ __global__ void dec_parse_kernel(const FrameDesc* __restrict__ frames, FrameStat
 //                    zero-run shard g on lane 4g (decode.cu:237-295), block
 //                    shards one after another warp-wide (decode.cu:342-396)
 
-constexpr int kGroup = 8;         // shards per warp
 constexpr int kBucketShift = 4;   // a bucket covers 16 slots
 constexpr int kBuckets = (1 << kRansTableLog) >> kBucketShift;
 
@@ -567,89 +566,197 @@ dec_rans_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
   }
 }
 
-// A Rice lane's bits, first bit lowest, through a private ring of 16 words
-// in shared memory fed by cp.async (the LaneRing scheme): 12 words are copied
-// before the first code; take() moves the next word into the 64-bit buffer
-// whenever the buffer holds 32 bits or fewer -- branch-free, once per refill
-// (the decoder then takes every code the buffer holds) -- and copies one more
-// word for each word it takes, so the copies stay at least 11 words ahead of
-// the word taken (10 ahead of the one read early).  (Loading words straight into a queue of
-// registers made every refill wait for a load: moving a register whose load
-// is in flight waits for it, and the four lanes of a shard refill at
-// different codes, so a warp met a load latency at nearly every code.)  Words
-// past the lane's last byte are not copied; bits read there are garbage, and
-// every position is checked against the lane's bit count instead.
-struct RiceRing {
-  static constexpr int kWords = 16;
-  static constexpr int kFill = 12;
-  static constexpr int kInFlight = 10;  // a word is read at least 10 copy groups after its copy
-  uint32_t* ring;         // slot 0 of this lane (slots 32 words apart)
-  const uint32_t* words;  // aligned base of the lane's bytes
-  int last;               // last word holding a lane byte (-1: none)
-  int fetched;            // next word to copy
-  int next;               // next word to take into the buffer
-  uint64_t bits;          // buffered bits, next bit lowest (zeros above nbits)
-  int nbits;
-  uint32_t ahead;         // word `next`, read one take early so no code waits on the ring load
+// Rice shards (decode.cu:297-340): a CTA of four warps per shard, 32 threads
+// on each of its four Rice lanes.  A lane's codes can only be found one after
+// another, so each thread takes a 32nd of the lane's bits and guesses where
+// its first code starts: it reads codes from a little before its part, and
+// such a reading falls in step with the true one after a few codes
+// (Weissenberger & Schmidt, "Massively parallel Huffman decoding on GPUs",
+// ICPP 2018).  Each thread then counts the codes of its part and hands the
+// end of its last one to the next thread; where that differs from the guess,
+// the part is read again from there.  Thread 0 starts at the true place, so
+// after at most 32 rounds -- almost always one -- every start is the true one,
+// and the codes are read once more for their values, now that their places
+// are known from the counts.  The body is staged in shared memory, and the
+// symbols leave from there in 16-byte stores.  Bound by the chain of one code
+// (about 30 instructions and 180 cycles in a lone warp): one thread a lane
+// read 1,024 of them in series, 100 us for the smallest frame with Rice
+// shards; eight threads a lane (a warp per shard) took 28 us, 32 take 12 us.
+constexpr int kRiceThreads = 32;    // per Rice lane
+constexpr int kOtherWarps = 4;
+constexpr int kRiceStage = 8800;    // bytes of a body held in shared memory: above any that the encoder writes
+constexpr int kRiceNone = 0x7fffffff;
 
-  __device__ void issue(int w) {
-    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(ring + (w & (kWords - 1)) * 32));
-    const int ok = w <= last;
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %2, 0;\n @p cp.async.ca.shared.global [%0], [%1], 4;\n}\n" ::"r"(sa),
-        "l"(words + w), "r"(ok)
-        : "memory");
-  }
-  __device__ void init(uint32_t* ring_smem, const uint8_t* p, int64_t len) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-    const int head = static_cast<int>(a & 3);
-    words = reinterpret_cast<const uint32_t*>(a - head);
-    ring = ring_smem;
-    last = len > 0 ? static_cast<int>((head + len - 1) >> 2) : -1;
-#pragma unroll
-    for (int i = 0; i < kFill; ++i) issue(i);
-    fetched = kFill;
-    cp_async_commit();
-    cp_async_wait<0>();
-    bits = ring[0] >> (8 * head);  // the first word's bytes before the lane are dropped
-    nbits = 32 - 8 * head;
-    next = 1;
-    ahead = ring[32];
-  }
-  // Takes the next word when 32 bits or fewer are buffered (afterwards at
-  // least 33 are, or the buffer was already fuller).
-  // The word taken was read from the ring by the take before (or by init);
-  // the next one is read here, after the wait, for the take after: word w
-  // is copied by the take that takes word w - 11 and read by the one that
-  // takes word w - 1, ten copy groups later, so a wait leaving ten groups
-  // pending covers it.
-  __device__ void take() {
-    const bool need = nbits <= 32;
-    bits |= need ? static_cast<uint64_t>(ahead) << nbits : 0ull;
-    nbits += need ? 32 : 0;
-    next += need;
-    if (need) issue(fetched);
-    fetched += need;
-    cp_async_commit();
-    cp_async_wait<kInFlight>();
-    const uint32_t w = ring[(next & (kWords - 1)) * 32];
-    ahead = need ? w : ahead;
+template <typename FoldT>
+struct alignas(16) RiceSm {
+  uint32_t body[(kRiceStage + 48) / 4];
+  FoldT out[kShardSymbols];
+  int32_t stop[4 * kRiceThreads];
+  int32_t total[kOtherWarps][4];
+};
+
+// Words of a body, in shared memory or (a longer one) in global memory, where
+// only words that hold a byte of it are read; words past the end are zero.
+struct RiceBody {
+  const uint32_t* words;
+  int last;  // last word holding a byte of the body (global)
+  bool staged;
+  __device__ uint32_t operator[](int i) const {
+    if (staged) return words[i];
+    return i <= last ? __ldg(words + i) : 0u;
   }
 };
 
-// cnt zero symbols from p: element stores up to a 16-byte boundary, then
-// 16-byte stores, then the tail (a zero run of a shard is up to 4,096
-// symbols, written by one thread).
+// Reads codes from bit `pos` while they start before `lim`, in a lane that
+// ends at bit `end`: emit(quotient, remainder, index) for each.  Returns the
+// bit after the last code, or kRiceNone when no further code was found (`rest`
+// is then where the search began; `bad` is set when the lane ends within a
+// code).  The number of codes is added to n.
+template <typename Emit>
+__device__ __forceinline__ int rice_read(const RiceBody& body, int pos, int lim, int end, int k, int& n, int& rest,
+                                         bool& bad, Emit emit) {
+  const uint32_t mask = (1u << k) - 1u;
+  const uint32_t ones = 0xffffffffu >> (k + 1);  // a one bit here ends a code of at most 31 bits
+  while (pos < lim) {
+    const int w = pos >> 5;
+    const uint32_t a = body[w], b = body[w + 1], c = body[w + 2];
+    uint32_t lo = __funnelshift_r(a, b, pos), hi = __funnelshift_r(b, c, pos);  // shift taken modulo 32
+    // codes of at most 31 bits wholly inside these 64 bits and the lane
+    const int avail = min(64, end - pos);
+    const int enough = avail - (lim - pos);  // bits left when the part is done
+    int left = avail;
+    uint32_t hit;
+    while ((hit = lo & ones) != 0) {
+      const int z = __clz(__brev(hit)), tot = z + 1 + k;
+      if (tot > left) break;
+      emit(static_cast<uint32_t>(z), (lo >> z >> 1) & mask, n);
+      ++n;
+      lo = __funnelshift_r(lo, hi, tot);
+      hi >>= tot;
+      left -= tot;
+      if (left <= enough) break;
+    }
+    pos += avail - left;
+    if (left < avail) continue;
+    // a longer code, or the end of the lane
+    int p = pos;
+    uint32_t x = lo;
+    while (x == 0 && p < end) {
+      p += 32;
+      x = __funnelshift_r(body[p >> 5], body[(p >> 5) + 1], p);
+    }
+    p += x ? __ffs(x) - 1 : 0;
+    if (p + 1 + k > end) {  // no further one bit in the lane, or one whose code would run past it
+      rest = pos;
+      bad = p < end;
+      return kRiceNone;
+    }
+    const int r = p + 1;
+    emit(static_cast<uint32_t>(p - pos), __funnelshift_r(body[r >> 5], body[(r >> 5) + 1], r) & mask, n);
+    ++n;
+    pos = r + k;
+  }
+  return pos;
+}
+
+// A Rice shard by the whole CTA; returns whether it is valid (every thread
+// the same).
 template <typename FoldT>
-__device__ __forceinline__ void zero_fill(FoldT* p, int64_t cnt) {
+__device__ bool rice_shard(const uint8_t* __restrict__ body, int blen, int n, int k, uint32_t maxf, const FoldMap& fm,
+                           FoldT* __restrict__ out, RiceSm<FoldT>& sm) {
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int lc = min(4, n);
+  const int table = (lc - 1) * 4;
+  if (table > blen) return false;
+  // the body, from a 16-byte boundary at or before it (the stream's header
+  // lies before every body)
+  const int head = static_cast<int>(reinterpret_cast<uintptr_t>(body) & 15);
+  const uint8_t* from = body - head;
+  const int bytes = head + blen;
+  RiceBody rb;
+  rb.staged = bytes <= kRiceStage;
+  rb.last = (bytes - 1) >> 2;
+  if (rb.staged) {
+    for (int i = 16 * t; i < bytes + 32; i += 16 * 32 * kOtherWarps) {
+      const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(sm.body)) + i;
+      const int have = max(0, min(16, bytes - i));  // the rest of the 16 bytes is zeroed
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(have ? from + i : from), "r"(have)
+                   : "memory");
+    }
+    cp_async_commit();
+    rb.words = sm.body;
+  } else {
+    rb.words = reinterpret_cast<const uint32_t*>(from);
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  // thread: Rice lane rl, part `part` of its bits (bit positions from `from`)
+  const int rl = t & 3, part = t >> 2;
+  const bool live = rl < lc;
+  bool bad = false;
+  int64_t off = table, len = 0;
+  for (int i = 0; i < lc - 1; ++i) {
+    const int64_t v = rd32(body + 4 * i);
+    if (i < rl) off += v;
+    else if (i == rl) len = v;
+  }
+  if (rl == lc - 1) len = blen - off;
+  if (off > blen || len < 0 || len > blen - off) bad = live;
+  if (__syncthreads_or(bad)) return false;
+  const int nl = live ? (n - rl + lc - 1) / lc : 0;  // codes of the lane
+  const int begin = 8 * (head + static_cast<int>(off)), end = live ? begin + 8 * static_cast<int>(len) : begin;
+  const int size = end - begin;
+  const int lo = begin + static_cast<int>(static_cast<int64_t>(size) * part / kRiceThreads);
+  const int lim = begin + static_cast<int>(static_cast<int64_t>(size) * (part + 1) / kRiceThreads);
+  auto skip = [](uint32_t, uint32_t, int) {};
+  int start = begin, stop, count = 0, rest = begin;
+  if (part) {
+    start = rice_read(rb, max(begin, lo - (8 + k) * (k + 2)), lo, end, k, count, rest, bad, skip);
+    if (start == kRiceNone) start = lo;
+  }
+  bool reread = true;
+  for (int round = 0; round < kRiceThreads; ++round) {
+    if (reread) {
+      count = 0;
+      bad = false;
+      stop = start;
+      if (start != kRiceNone) stop = rice_read(rb, start, lim, end, k, count, rest, bad, skip);
+    }
+    sm.stop[t] = stop;
+    __syncthreads();
+    const int before = part ? sm.stop[t - 4] : start;
+    reread = before != start;
+    start = before;
+    if (!__syncthreads_or(reread)) break;
+  }
+  int at = count;  // codes of the parts up to this one
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(kFull, at, o);
+    if (lane >= o) at += v;
+  }
+  if (lane >= 28) sm.total[warp][rl] = at;
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) at += sm.total[w][rl];
+  // exactly the lane's codes, and fewer than eight bits left, all zero
+  if (start != kRiceNone && stop == kRiceNone) bad |= end - rest > 7;
+  if (part == kRiceThreads - 1) bad |= at != nl;
+  at -= count;
+  if (__syncthreads_or(bad)) return false;
+  if (start != kRiceNone) {
+    int m = 0;
+    rice_read(rb, start, lim, end, k, m, rest, bad, [&](uint32_t q, uint32_t r, int i) {
+      const uint64_t v = (static_cast<uint64_t>(q) << k) + r;
+      bad |= v > maxf;
+      sm.out[(at + i) * lc + rl] = fold_value<FoldT>(static_cast<uint32_t>(v), fm);
+    });
+  }
+  if (__syncthreads_or(bad)) return false;
   constexpr int kPer = 16 / sizeof(FoldT);
-  int64_t i = 0;
-  const int head = static_cast<int>(((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / sizeof(FoldT));
-  for (; i < head && i < cnt; ++i) p[i] = 0;
-  uint4* v = reinterpret_cast<uint4*>(p + i);
-  const int64_t nv = (cnt - i) / kPer;
-  for (int64_t j = 0; j < nv; ++j) v[j] = make_uint4(0, 0, 0, 0);
-  for (i += nv * kPer; i < cnt; ++i) p[i] = 0;
+  uint4* o4 = reinterpret_cast<uint4*>(out);  // shards start on 16-byte boundaries
+  for (int i = t; i < n / kPer; i += 32 * kOtherWarps) o4[i] = reinterpret_cast<const uint4*>(sm.out)[i];
+  for (int i = n / kPer * kPer + t; i < n; i += 32 * kOtherWarps) out[i] = sm.out[i];
+  return true;
 }
 
 // A zero-run shard (decode.cu:237-295) decoded by the whole warp, 32 body
@@ -755,254 +862,121 @@ struct OtherGroupSm {
 };
 
 template <typename FoldT>
-__global__ void __launch_bounds__(128)
+struct OtherSm {
+  RiceSm<FoldT> rice;
+  OtherGroupSm block[kOtherWarps];
+  int claimed;
+};
+
+size_t dec_other_smem(bool fold16) { return fold16 ? sizeof(OtherSm<uint16_t>) : sizeof(OtherSm<uint32_t>); }
+
+// A CTA takes a Rice shard, or four zero-run or block shards (one a warp).
+template <typename FoldT>
+__global__ void __launch_bounds__(32 * kOtherWarps)
 dec_other_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
                  const ShardInfo* __restrict__ shards, const BatchDims* __restrict__ dims,
                  DecodeLists* __restrict__ lists, const int32_t* __restrict__ list_items,
                  FoldT* __restrict__ folded) {
   const int64_t total_shards = dims->shards_p[0];
-  __shared__ OtherGroupSm sm_all[4];
-  __shared__ uint32_t rice_rings[4][RiceRing::kWords * 32];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  OtherGroupSm& sm = sm_all[warp];
-  const int my_g = lane >> 2, my_l = lane & 3;
-  int ngroups[3], total_groups = 0;
-  for (int l = 0; l < 3; ++l) {
-    ngroups[l] = (lists->count[l + 1] + kGroup - 1) / kGroup;
-    total_groups += ngroups[l];
-  }
+  OtherSm<FoldT>& osm = *reinterpret_cast<OtherSm<FoldT>*>(smem_raw);
+  OtherGroupSm& sm = osm.block[warp];
+  const int count1 = lists->count[1], count2 = lists->count[2], count3 = lists->count[3];
+  const int fours2 = (count2 + kOtherWarps - 1) / kOtherWarps, fours3 = (count3 + kOtherWarps - 1) / kOtherWarps;
   for (;;) {
-    int g = 0;
-    if (lane == 0) g = atomicAdd(&lists->next_group, 1);
-    g = __shfl_sync(kFull, g, 0);
-    if (g >= total_groups) break;
-    int list = 0;
-    while (g >= ngroups[list]) {
-      g -= ngroups[list];
-      ++list;
-    }
-    ++list;  // 1 Rice, 2 zero-run, 3 block pack
-    const int first = g * kGroup;
-    const int count = lists->count[list];
-    const int32_t* items = list_items + static_cast<int64_t>(list) * total_shards;
-    const int64_t s_mine = (first + my_g < count) ? items[first + my_g] : -1;
-    bool live = false;
-    int fi = 0, mode = 0, n = 0;
-    int64_t blen = 0;
-    const uint8_t* body = nullptr;
-    FoldT* out = nullptr;
-    uint32_t maxf = 0;
-    FoldMap fm{0, 0};
-    if (s_mine >= 0) {
-      const ShardInfo& si = shards[s_mine];
-      fi = si.frame;
-      live = state[fi].status == 0;  // a failed parse may have left shard records unwritten
-      mode = si.mode;
-      n = si.count;
-      blen = si.body;
-      body = frames[fi].stream + si.offset;
-      out = folded + si.sample_base;
-      maxf = static_cast<uint32_t>(frames[fi].max_sample) * 2u;
-      fm = fold_map(frames[fi], sizeof(FoldT) == 2);
-    }
+    __syncthreads();  // the CTA's last shard is done, its claim read
+    if (threadIdx.x == 0) osm.claimed = atomicAdd(&lists->next_group, 1);
+    __syncthreads();
+    int g = osm.claimed;
+    if (g >= count1 + fours2 + fours3) break;
+    const int list = g < count1 ? 1 : g < count1 + fours2 ? 2 : 3;  // Rice, zero-run, block pack
+    if (list == 2) g = (g - count1) * kOtherWarps + warp;
+    if (list == 3) g = (g - count1 - fours2) * kOtherWarps + warp;
+    if (g >= lists->count[list]) continue;
+    const ShardInfo& si = shards[list_items[static_cast<int64_t>(list) * total_shards + g]];
+    const int fi = si.frame;
+    // a failed parse may have left shard records unwritten.  (Only the parse
+    // writes status 10 and 11; one set meanwhile by another shard must not
+    // split the CTA, so the CTA decides together.)
+    const int failed = state[fi].status != 0;
+    if (list == 1 ? __syncthreads_or(failed) : failed) continue;
+    const FrameDesc& f = frames[fi];
+    const int mode = si.mode, n = si.count, blen = si.body;
+    const uint8_t* body = f.stream + si.offset;
+    FoldT* out = folded + si.sample_base;
+    const uint32_t maxf = static_cast<uint32_t>(f.max_sample) * 2u;
+    const FoldMap fm = fold_map(f, sizeof(FoldT) == 2);
     if (list == 1) {
-      // ---- Rice ---------------------------------------------------------------
-      if (s_mine >= 0 && live) {
-        const int lc = n < 4 ? n : 4;
-        const int64_t table = static_cast<int64_t>(lc - 1) * 4;
-        if (table > blen) {
-          if (my_l == 0) set_status(&state[fi].status, 2);
-        } else if (my_l < lc) {
-          int64_t loff = table;
-          for (int i = 0; i < my_l; ++i) loff += rd32(body + i * 4);
-          const int64_t llen = my_l + 1 < lc ? static_cast<int64_t>(rd32(body + my_l * 4)) : blen - loff;
-          bool ok = !(loff > blen || llen < 0 || llen > blen - loff);
-          if (ok) {
-            const int k = mode - 1;
-            const uint32_t rmask = k ? (1u << k) - 1u : 0u;
-            const int64_t total = 8 * llen;  // bits of this lane
-            RiceRing rr;
-            rr.init(&rice_rings[warp][lane], body + loff, llen);
-            int64_t pos = 0;
-            int idx = my_l;
-            while (idx < n && ok) {
-              // unary quotient: zeros up to the next one bit, then k
-              // remainder bits (decode.cu:63-125)
-              rr.take();
-              uint32_t lo = static_cast<uint32_t>(rr.bits);
-              int z0 = __ffs(lo) - 1;  // -1: no one bit in the low word
-              if (z0 >= 0 && z0 + 1 + k <= rr.nbits) {
-                // codes wholly buffered, each with a quotient below 32: one
-                // pass over each, as many as the buffer holds
-                do {
-                  const int tot = z0 + 1 + k;  // at most 48
-                  const uint32_t r = __funnelshift_rc(lo, static_cast<uint32_t>(rr.bits >> 32), z0 + 1) & rmask;
-                  rr.bits >>= tot;
-                  rr.nbits -= tot;
-                  pos += tot;
-                  const uint64_t v = (static_cast<uint64_t>(z0) << k) + r;
-                  if (pos > total || v > maxf) {  // the code runs past the lane, or its value is too large
-                    ok = false;
-                    break;
-                  }
-                  out[idx] = fold_value<FoldT>(static_cast<uint32_t>(v), fm);
-                  idx += lc;
-                  lo = static_cast<uint32_t>(rr.bits);
-                  z0 = __ffs(lo) - 1;
-                } while (idx < n && z0 >= 0 && z0 + 1 + k <= rr.nbits);
-                continue;
-              }
-              uint64_t v;
-              {
-                uint32_t q = 0;
-                while (rr.bits == 0) {  // every buffered bit is zero: a long quotient
-                  q += rr.nbits;
-                  pos += rr.nbits;
-                  rr.nbits = 0;
-                  if (pos >= total || q > maxf) {
-                    ok = false;
-                    break;
-                  }
-                  rr.take();
-                }
-                if (!ok) break;
-                const int z = __ffsll(static_cast<long long>(rr.bits)) - 1;
-                q += z;
-                rr.bits = z == 63 ? 0ull : rr.bits >> (z + 1);
-                rr.nbits -= z + 1;
-                pos += z + 1;
-                if (pos > total || q > maxf) {  // the one bit lies past the lane, or the quotient is too large
-                  ok = false;
-                  break;
-                }
-                if (rr.nbits < k) rr.take();
-                const uint32_t r = static_cast<uint32_t>(rr.bits) & rmask;
-                rr.bits >>= k;
-                rr.nbits -= k;
-                pos += k;
-                v = (static_cast<uint64_t>(q) << k) + r;
-                if (pos > total) {
-                  ok = false;
-                  break;
-                }
-              }
-              if (v > maxf) {
-                ok = false;
-                break;
-              }
-              out[idx] = fold_value<FoldT>(static_cast<uint32_t>(v), fm);
-              idx += lc;
-            }
-            cp_async_wait<0>();  // no copy into the ring outlives the lane
-            if (ok) {
-              const int64_t used = (pos + 7) / 8;
-              if (used != llen) ok = false;
-              else if ((pos & 7) != 0) {
-                const uint8_t mask = static_cast<uint8_t>(~((1u << (pos & 7)) - 1u));
-                if (body[loff + used - 1] & mask) ok = false;
-              }
-            }
-          }
-          if (!ok) set_status(&state[fi].status, 2);
-        }
-      }
+      if (!rice_shard(body, blen, n, mode - 1, maxf, fm, out, osm.rice) && threadIdx.x == 0)
+        set_status(&state[fi].status, 2);
     } else if (list == 2) {
-      // ---- zero-run: the warp takes the shards one after another --------------
-      for (int k = 0; k < kGroup; ++k) {
-        const int64_t sk = __shfl_sync(kFull, s_mine, 4 * k);
-        if (sk < 0) continue;
-        const bool lk = __shfl_sync(kFull, live, 4 * k);
-        if (!lk) continue;
-        const int nk = __shfl_sync(kFull, n, 4 * k);
-        const int64_t bk = __shfl_sync(kFull, blen, 4 * k);
-        const int fk = __shfl_sync(kFull, fi, 4 * k);
-        const uint32_t mk = __shfl_sync(kFull, maxf, 4 * k);
-        const uint8_t* bodyk =
-            reinterpret_cast<const uint8_t*>(__shfl_sync(kFull, reinterpret_cast<uintptr_t>(body), 4 * k));
-        FoldT* outk = reinterpret_cast<FoldT*>(__shfl_sync(kFull, reinterpret_cast<uintptr_t>(out), 4 * k));
-        const FoldMap fmk{__shfl_sync(kFull, fm.step, 4 * k), __shfl_sync(kFull, fm.lim, 4 * k)};
-        if (!zero_run_warp(bodyk, bk, nk, mk, fmk, outk, lane) && lane == 0) set_status(&state[fk].status, 1);
-      }
+      if (!zero_run_warp(body, blen, n, maxf, fm, out, lane) && lane == 0) set_status(&state[fi].status, 1);
     } else {
-      // ---- block pack: the warp takes the shards one after another ------------
-      for (int k = 0; k < kGroup; ++k) {
-        const int64_t sk = __shfl_sync(kFull, s_mine, 4 * k);
-        if (sk < 0) continue;
-        const bool lk = __shfl_sync(kFull, live, 4 * k);
-        if (!lk) continue;
-        const int nk = __shfl_sync(kFull, n, 4 * k);
-        const int64_t bk = __shfl_sync(kFull, blen, 4 * k);
-        const int fk = __shfl_sync(kFull, fi, 4 * k);
-        const uint32_t mk = __shfl_sync(kFull, maxf, 4 * k);
-        const uint8_t* bodyk = reinterpret_cast<const uint8_t*>(__shfl_sync(kFull, reinterpret_cast<uintptr_t>(body), 4 * k));
-        FoldT* outk = reinterpret_cast<FoldT*>(__shfl_sync(kFull, reinterpret_cast<uintptr_t>(out), 4 * k));
-        const FoldMap fmk{__shfl_sync(kFull, fm.step, 4 * k), __shfl_sync(kFull, fm.lim, 4 * k)};
-        const int nblk = (nk + kBlockSymbols - 1) / kBlockSymbols;
-        const int maxw = 32 - __clz(mk);
-        if (lane == 0) {
-          int64_t cursor = 0;
-          int ok = 1;
-          for (int b = 0; b < nblk; ++b) {
-            if (cursor >= bk) {
-              ok = 0;
-              break;
-            }
-            const int w = bodyk[cursor++];
-            if (w > maxw) {
-              ok = 0;
-              break;
-            }
-            const int64_t nb = min(static_cast<int64_t>(kBlockSymbols), static_cast<int64_t>(nk) - static_cast<int64_t>(b) * kBlockSymbols);
-            const int64_t pay = (nb * w + 7) / 8;
-            if (pay > bk - cursor) {
-              ok = 0;
-              break;
-            }
-            sm.boff[b] = static_cast<int32_t>(cursor);
-            sm.bwidth[b] = w;
-            const int64_t bits = nb * w;
-            if ((bits & 7) != 0) {
-              const uint8_t mask = static_cast<uint8_t>(~((1u << (bits & 7)) - 1u));
-              if (bodyk[cursor + pay - 1] & mask) {
-                ok = 0;
-                break;
-              }
-            }
-            cursor += pay;
+      const int nblk = (n + kBlockSymbols - 1) / kBlockSymbols;
+      const int maxw = 32 - __clz(maxf);
+      if (lane == 0) {
+        int64_t cursor = 0;
+        int ok = 1;
+        for (int b = 0; b < nblk; ++b) {
+          if (cursor >= blen) {
+            ok = 0;
+            break;
           }
-          if (ok && cursor != bk) ok = 0;
-          sm.valid = ok;
-          if (!ok) set_status(&state[fk].status, 3);
-        }
-        __syncwarp();
-        if (sm.valid) {
-          int bad = 0;
-          for (int b = 0; b < nblk; ++b) {
-            const int w = sm.bwidth[b];
-            const uint8_t* pay = bodyk + sm.boff[b];
-            const int nb = min(kBlockSymbols, nk - b * kBlockSymbols);
-            for (int i = lane; i < nb; i += 32) {
-              uint32_t v = 0;
-              if (w) {
-                const int64_t bit = static_cast<int64_t>(i) * w;
-                const int64_t byte0 = bit >> 3;
-                const int64_t lastb = (bit + w - 1) >> 3;
-                uint64_t acc = 0;
-                for (int64_t j = byte0; j <= lastb; ++j) acc |= static_cast<uint64_t>(pay[j]) << (8 * (j - byte0));
-                v = static_cast<uint32_t>((acc >> (bit & 7)) & ((1ull << w) - 1));
-              }
-              if (v > mk) bad = 1;
-              outk[static_cast<int64_t>(b) * kBlockSymbols + i] = fold_value<FoldT>(v, fmk);
+          const int w = body[cursor++];
+          if (w > maxw) {
+            ok = 0;
+            break;
+          }
+          const int64_t nb = min(static_cast<int64_t>(kBlockSymbols), static_cast<int64_t>(n) - static_cast<int64_t>(b) * kBlockSymbols);
+          const int64_t pay = (nb * w + 7) / 8;
+          if (pay > blen - cursor) {
+            ok = 0;
+            break;
+          }
+          sm.boff[b] = static_cast<int32_t>(cursor);
+          sm.bwidth[b] = w;
+          const int64_t bits = nb * w;
+          if ((bits & 7) != 0) {
+            const uint8_t mask = static_cast<uint8_t>(~((1u << (bits & 7)) - 1u));
+            if (body[cursor + pay - 1] & mask) {
+              ok = 0;
+              break;
             }
           }
-          if (__any_sync(kFull, bad) && lane == 0) set_status(&state[fk].status, 3);
+          cursor += pay;
         }
-        __syncwarp();
+        if (ok && cursor != blen) ok = 0;
+        sm.valid = ok;
+        if (!ok) set_status(&state[fi].status, 3);
       }
+      __syncwarp();
+      if (sm.valid) {
+        int bad = 0;
+        for (int b = 0; b < nblk; ++b) {
+          const int w = sm.bwidth[b];
+          const uint8_t* pay = body + sm.boff[b];
+          const int nb = min(kBlockSymbols, n - b * kBlockSymbols);
+          for (int i = lane; i < nb; i += 32) {
+            uint32_t v = 0;
+            if (w) {
+              const int64_t bit = static_cast<int64_t>(i) * w;
+              const int64_t byte0 = bit >> 3;
+              const int64_t lastb = (bit + w - 1) >> 3;
+              uint64_t acc = 0;
+              for (int64_t j = byte0; j <= lastb; ++j) acc |= static_cast<uint64_t>(pay[j]) << (8 * (j - byte0));
+              v = static_cast<uint32_t>((acc >> (bit & 7)) & ((1ull << w) - 1));
+            }
+            if (v > maxf) bad = 1;
+            out[static_cast<int64_t>(b) * kBlockSymbols + i] = fold_value<FoldT>(v, fm);
+          }
+        }
+        if (__any_sync(kFull, bad) && lane == 0) set_status(&state[fi].status, 3);
+      }
+      __syncwarp();
     }
   }
 }
-
 
 // ---------------------------------------------------------------------------
 // dec_reconstruct: warp per tile, lane = row of a 32-row band, column c of
@@ -1437,14 +1411,22 @@ cudaError_t dec_rans_set_attr(cudaFuncAttribute attr, int value) {
   return cudaFuncSetAttribute(dec_rans_kernel<uint32_t>, attr, value);
 }
 
+cudaError_t dec_other_set_smem() {
+  const cudaError_t e = cudaFuncSetAttribute(dec_other_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(dec_other_smem(true)));
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(dec_other_kernel<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              static_cast<int>(dec_other_smem(false)));
+}
+
 void dec_other_launch(bool fold16, int grid, cudaStream_t stream, const FrameDesc* frames, FrameState* state,
                       const ShardInfo* shards, const BatchDims* dims, DecodeLists* lists, const int32_t* list_items,
                       void* folded) {
   if (fold16)
-    dec_other_kernel<uint16_t><<<grid, 128, 0, stream>>>(frames, state, shards, dims, lists, list_items,
+    dec_other_kernel<uint16_t><<<grid, 32 * kOtherWarps, dec_other_smem(true), stream>>>(frames, state, shards, dims, lists, list_items,
                                                          static_cast<uint16_t*>(folded));
   else
-    dec_other_kernel<uint32_t><<<grid, 128, 0, stream>>>(frames, state, shards, dims, lists, list_items,
+    dec_other_kernel<uint32_t><<<grid, 32 * kOtherWarps, dec_other_smem(false), stream>>>(frames, state, shards, dims, lists, list_items,
                                                          static_cast<uint32_t*>(folded));
 }
 

@@ -152,6 +152,7 @@ void dec_other_launch(bool fold16, int grid, cudaStream_t stream, const FrameDes
 void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, bool few, int grid, cudaStream_t stream,
                             const FrameDesc* frames, const FrameState* state, const BatchDims* dims,
                             const void* folded, int* queue);
+cudaError_t dec_other_set_smem();
 cudaError_t dec_reconstruct_set_smem();
 __global__ void dec_reconstruct_wide_kernel(const FrameDesc* frames, const FrameState* state, const BatchDims* dims,
                                             const void* folded, int fold16);
