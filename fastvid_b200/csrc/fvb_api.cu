@@ -268,11 +268,13 @@ int side_stream(SideStream** out) {
   return FVB_OK;
 }
 
-// batches of at least this many shards (about 256 thousand samples: a 720p
-// gray frame has 240) decode their non-rANS shards on the side stream, beside
-// the rANS shards; both kernels are latency-bound for a single frame, so
-// overlapping them shortens its decode
-constexpr int64_t kSideStreamShards = 64;
+// Batches of at least this many shards decode their non-rANS shards on the
+// side stream, beside the rANS shards: a mixed batch of 13,800 shards takes
+// 700 us so and 739 us with dec_other after dec_rans on one stream.  Below it
+// dec_other is a matter of 3 to 15 us, and the fork, the join and its CTAs on
+// dec_rans's SMs cost more (a 1080p rgb10 frame, 1,539 shards: 307 us beside,
+// 273 us after).
+constexpr int64_t kSideStreamShards = 4096;
 
 int ensure_smem_attrs() {
   static bool done[64] = {false};
