@@ -285,10 +285,7 @@ int ensure_smem_attrs() {
   FVB_CUDA(enc_emit_set_smem(static_cast<int>(enc_emit_smem())));
   FVB_CUDA(dec_reconstruct_set_smem());
   FVB_CUDA(dec_other_set_smem());
-  FVB_CUDA(dec_rans_set_attr(cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dec_rans_smem())));
-  // the whole unified L1/shared array as shared memory: four dec_rans CTAs
-  // (56 KB each) per SM
-  FVB_CUDA(dec_rans_set_attr(cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  FVB_CUDA(dec_rans_set_smem());
   if (dev >= 0 && dev < 64) done[dev] = true;
   return FVB_OK;
 }
@@ -667,6 +664,13 @@ int rans_pipe_for(int knob, int grid) {
   return grid <= device_sms() * kRansAutoCtasPerSm ? 8 : 0;
 }
 std::atomic<int> g_tile_warps{kDefaultTileWarps};
+
+// Whether dec_rans runs on tables of all slots: as long as all shards are
+// resident at once that way (six CTAs of two shards on an SM, 94 us for the
+// chain of a shard against 125 us with bucket tables, which take ten times as
+// many shards at once).
+constexpr int kSlotCtasPerSm = 6;
+bool few_rans_shards(int64_t shards) { return shards <= static_cast<int64_t>(device_sms()) * kSlotCtasPerSm * 2; }
 
 // Whether a wavefront launch has too few tiles to hide its step chain behind
 // other warps.
@@ -1331,7 +1335,7 @@ int decode_enqueue(const Totals& t, int wavefront, void* workspace, int64_t work
   RansTable* tables = reinterpret_cast<RansTable*>(ws + L.tables);
   {
     LaunchScope scope_(K_DEC_SHARDS, stream);
-    dec_rans_tables_kernel<<<grid_for(t.shards, 128, ctas(K_DEC_SHARDS)), 128, 0, stream>>>(
+    dec_rans_tables_kernel<<<grid_for(t.shards, 4, ctas(K_DEC_SHARDS)), 128, 0, stream>>>(
         frames_d, state, shards, lists, items, tables, f16 ? 1 : 0);
   }
   FVB_LAUNCHED("dec_rans_tables_kernel");
@@ -1343,8 +1347,10 @@ int decode_enqueue(const Totals& t, int wavefront, void* workspace, int64_t work
   if (side) FVB_CUDA(cudaEventRecord(side->fork, stream));
   {
     LaunchScope scope_(K_DEC_RANS, stream);
-    dec_rans_launch(f16, grid_for(ceil_div(t.shards, kGroupShards), kWarpsPerCta, ctas(K_DEC_RANS)), dec_rans_smem(),
-                    stream, frames_d, state, shards, lists, items, tables, folded);
+    const bool few = few_rans_shards(t.shards);
+    const int grid = few ? grid_for(t.shards, 2, kSlotCtasPerSm)
+                         : grid_for(ceil_div(t.shards, kGroupShards), kWarpsPerCta, ctas(K_DEC_RANS));
+    dec_rans_launch(f16, few, grid, stream, frames_d, state, shards, lists, items, tables, folded);
   }
   FVB_LAUNCHED("dec_rans_kernel");
   {

@@ -148,370 +148,544 @@ __global__ void dec_parse_kernel(const FrameDesc* __restrict__ frames, FrameStat
 
 // ---------------------------------------------------------------------------
 // Entropy decode (decode.cu:222-550).  dec_parse bins shards by mode; then
-//   dec_rans_tables  one thread per rANS shard parses its order-0 table
-//                    serially (decode.cu:456-517) into a table record
-//   dec_rans         a 4-lane group streams rANS shards: it copies a shard's
-//                    table into shared memory, builds a bucket table of
-//                    symbol starts, and lane l decodes lane l of the shard
-//                    (decode.cu:530-549)
-//   dec_other        a warp takes eight Rice, zero-run or block shards: Rice
-//                    lane l of shard g on lane 4g+l (decode.cu:297-340),
-//                    zero-run shard g on lane 4g (decode.cu:237-295), block
-//                    shards one after another warp-wide (decode.cu:342-396)
+//   dec_rans_tables  a warp per rANS shard parses its order-0 table
+//                    (decode.cu:456-517) into a table record
+//   dec_rans         four threads per rANS shard, one on each of its lanes
+//                    (decode.cu:530-549), through the record's bucket table or
+//                    (few shards) a table of all slots
+//   dec_other        a CTA per Rice shard (decode.cu:297-340), a warp per
+//                    zero-run (decode.cu:237-295) or block shard
+//                    (decode.cu:342-396)
 
 constexpr int kBucketShift = 4;   // a bucket covers 16 slots
 constexpr int kBuckets = (1 << kRansTableLog) >> kBucketShift;
 
 // One parsed order-0 table (decode.cu:456-517).  Symbol i covers slots
-// cum_i .. cum_i + freq_i - 1 of the 4096-slot ring.
+// cum_i .. cum_i + freq_i - 1 of the 4096-slot ring.  data holds
+//  * per symbol, an entry: freq - 1 in bits 31..20, cum in bits 19..8, and in
+//    bits 7..0 what the symbol stores (its value as u16, or fold_value of it)
+//    when every symbol's, as a signed number, fits eight bits (narrow), else
+//    the symbol's index;
+//  * per symbol, what it stores, as u16;
+//  * for up to kBucketSymbols symbols, a bucket table: word u = (four times
+//    the symbol holding slot 16u) << 16, with bit i set for every symbol that
+//    starts at slot 16u + i (i = 1..15).  The symbol holding a slot is then
+//    the bucket's first plus the starts at or below the slot inside the
+//    bucket: one load and a population count, no search.
+constexpr int kBucketSymbols = 170;
 struct RansTable {
   int32_t lane_start[4], lane_len[4];
   uint32_t state[4];
-  int32_t nsym, valid;
-  int32_t pad[2];
-  uint32_t freqcum[256];  // cum | freq << 12 (freq up to 4096: 13 bits)
-  uint32_t value[256];    // what the symbol stores: its value as u16 (decode.cu:484), or fold_value of it
+  int32_t nsym, valid, narrow;
+  int32_t pad;
+  uint32_t data[512];
+  __host__ __device__ static int entries_at(int nsym) { return nsym <= kBucketSymbols ? kBuckets : 0; }
+  __host__ __device__ static int values_at(int nsym) { return entries_at(nsym) + nsym; }
 };
+static_assert(kBuckets + kBucketSymbols + (kBucketSymbols + 1) / 2 <= 512 && 255 + 128 <= 512, "table record");
+static_assert(sizeof(RansTable) == 2112, "the scratch limit of the allocation-free decode counts on it");
 
 size_t dec_rans_table_bytes() { return sizeof(RansTable); }
 
-// Sequential reader of a byte range through aligned 32-bit loads.  Only words
-// holding at least one byte of the range are loaded; four are kept in flight
-// ahead of the bit buffer.  Bytes past the range read as zero.
-struct ByteWindow {
-  const uint32_t* words;
-  int64_t next, last;
-  int tail_bytes;
-  uint64_t bits;
-  int nbits;
-  uint32_t q0, q1, q2, q3;
-  int c0, c1, c2, c3;
-
-  // Issues the load of the next word and returns it unmasked; nothing here
-  // waits for the data (bytes past the range are masked off when merged).
-  __device__ uint32_t load_word(int* nb) {
-    const int64_t at = next < last ? next : (last > 0 ? last : 0);
-    const int valid = next < last ? 4 : (next == last ? tail_bytes : 0);
-    const uint32_t w = last >= 0 ? __ldg(words + at) : 0u;
-    ++next;
-    *nb = 8 * valid;
-    return w;
-  }
-  __device__ void init(const uint8_t* p, int64_t len) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-    const int head = static_cast<int>(a & 3);
-    words = reinterpret_cast<const uint32_t*>(a - head);
-    next = 0;
-    last = len > 0 ? (head + len - 1) >> 2 : -1;
-    tail_bytes = len > 0 ? static_cast<int>((head + len - 1) & 3) + 1 : 0;
-    int nb;
-    const uint32_t w = load_word(&nb);
-    q0 = load_word(&c0);
-    q1 = load_word(&c1);
-    q2 = load_word(&c2);
-    q3 = load_word(&c3);
-    const uint32_t w0 = nb >= 32 ? w : (w & ((1u << nb) - 1u));
-    bits = nb ? (w0 >> (8 * head)) : 0u;
-    nbits = nb ? nb - 8 * head : 0;
-    refill();
-  }
-  __device__ void shift_in() {
-    const uint32_t m0 = c0 >= 32 ? q0 : (q0 & ((1u << c0) - 1u));
-    bits |= static_cast<uint64_t>(m0) << nbits;
-    nbits += c0;
-    q0 = q1;
-    c0 = c1;
-    q1 = q2;
-    c1 = c2;
-    q2 = q3;
-    c2 = c3;
-    q3 = load_word(&c3);
-  }
-  __device__ void refill_once() {
-    if (nbits <= 32) shift_in();
-  }
-  __device__ void refill() {
-    while (nbits <= 32 && c0) shift_in();
-  }
-  __device__ uint32_t byte() {  // next byte (zero past the range)
-    if (nbits < 8) refill();
-    const uint32_t b = static_cast<uint32_t>(bits) & 0xffu;
-    bits >>= 8;
-    nbits -= 8;
-    return b;
-  }
-};
-
-
-// A lane's byte stream through a private ring of 16 words in shared memory,
-// fed by cp.async: 12 words before the first read, then two words with every
-// eight-byte read -- as many as four decoding steps can consume -- so the
-// ring stays at least 12 words ahead of the read position (the gap shrinks by
-// at most the two words a read consumes and grows by the two it issues, up
-// to the ring size).  A read may leave the newest four copy groups in flight;
-// the words it touches (w .. w+2, at most ten words below the copy front,
-// which advances at most two words per read) were issued five or more reads
-// earlier, so their groups are complete.  There is no refill branch: every
-// read issues its two copies under predicates.  Word w of the aligned range
-// lives in slot w % 16; slot s of lane l is word s * 32 + l of the warp's ring
-// block, so every lane reads and fills its own bank whatever its position.
-// Only words holding a byte of the lane are copied (others keep stale bytes,
-// and reading them is an overrun that the byte count check reports).  A
-// 16-word ring (2 KB per warp, 32 before) lets four dec_rans CTAs share an
-// SM.
-struct LaneRing {
-  static constexpr int kWords = 16;    // slots per lane
-  static constexpr int kFill = 12;     // words copied before the first read
-  static constexpr int kInFlight = 4;  // copy groups a read may leave pending
-  static_assert(kFill >= 10 && kFill <= kWords, "read words must be five copy groups old");
-  uint32_t* ring;          // slot 0 of this lane (slots 32 words apart)
-  const uint32_t* words;   // aligned base of the lane's bytes
-  int head;                // lane byte 0 = byte `head` of word 0
-  int last;                // last word holding a lane byte (-1: none)
-  int fetched;             // next word to copy
-
-  // Copy word w into its slot if it holds a lane byte and its slot is free
-  // (the word 32 below it is behind the read position `low`).
-  __device__ void issue(int w, int low) {
-    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(ring + (w & (kWords - 1)) * 32));
-    const int ok = (w <= last) & (w <= low + kWords - 1);
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %2, 0;\n @p cp.async.ca.shared.global [%0], [%1], 4;\n}\n" ::"r"(s),
-        "l"(words + w), "r"(ok)
-        : "memory");
-  }
-  __device__ void init(uint32_t* ring_smem, const uint8_t* p, int len) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-    head = static_cast<int>(a & 3);
-    words = reinterpret_cast<const uint32_t*>(a - head);
-    ring = ring_smem;
-    last = len > 0 ? (head + len - 1) >> 2 : -1;
+// Varint tokens of a byte string, 32 bytes a step, by a warp.  A byte without
+// the 0x80 bit ends a token (ballot); the lane holding a token's last byte
+// gathers the token's bytes from the lanes before it by shuffles, with the
+// bytes of a token begun in an earlier step carried over.  `bad` covers the
+// varint rules: at most five bytes, the fifth at most 0x0f, canonical length.
+struct TokenReader {
+  uint32_t pend_val = 0;  // value bits of a token begun in an earlier step
+  int pend_used = 0;      // its bytes so far (capped at 6)
+  bool pend_bad = false;  // its fifth byte was above 0x0f, or it is too long
+  uint32_t endm;          // this step: lanes holding a token's last byte
+  __device__ uint32_t step(uint32_t byte, bool vld, int nvalid, int lane, bool& bad) {
+    endm = __ballot_sync(kFull, vld && !(byte & 0x80u));
+    const uint32_t below = endm & ((1u << lane) - 1u);
+    const int prev = below ? 31 - __clz(below) : -1;  // the previous token's end in this step
+    const bool carried = prev < 0;                    // the token began in an earlier step
+    const int here = lane - prev;                     // its bytes in this step
+    const int cu = carried ? pend_used : 0;
+    uint32_t tok = carried ? pend_val : 0u;
+    bad = carried && pend_bad;
 #pragma unroll
-    for (int i = 0; i < kFill; ++i) issue(i, 0);
-    fetched = kFill;
-    cp_async_commit();
-  }
-  __device__ void ready() { cp_async_wait<0>(); }
-  // The eight bytes at lane positions cur..cur+7, first byte in the top
-  // bits of hi, the next four in lo; cur advances by at most eight between
-  // calls.
-  __device__ void window(int cur, uint32_t& hi_out, uint32_t& lo_out) {
-    const int pos = head + cur;
-    const int w = pos >> 2;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      issue(fetched, w);
-      fetched += fetched <= w + kWords - 1;
-    }
-    cp_async_commit();
-    cp_async_wait<kInFlight>();
-    const uint32_t a = ring[(w & (kWords - 1)) * 32], b = ring[((w + 1) & (kWords - 1)) * 32],
-                   c = ring[((w + 2) & (kWords - 1)) * 32];
-    const int sh = 8 * (pos & 3);
-    hi_out = __byte_perm(__funnelshift_r(a, b, sh), 0, 0x0123);
-    lo_out = __byte_perm(__funnelshift_r(b, c, sh), 0, 0x0123);
-  }
-};
-
-// Order-0 table of one shard, parsed by one thread (decode.cu:456-517).
-__device__ bool rans_parse_serial(const uint8_t* __restrict__ body, int64_t blen, uint32_t maxf,
-                                  const FoldMap& fm, RansTable& t) {
-  ByteWindow r;
-  r.init(body, blen);
-  int64_t cursor = 0;
-  auto varint = [&](uint32_t* value) -> bool {
-    uint32_t result = 0;
-    int shift = 0;
-    for (int used = 0; used < 5; ++used) {
-      if (cursor >= blen) return false;
-      const uint32_t b = r.byte();
-      ++cursor;
-      if (used == 4 && b > 0x0f) return false;
-      result |= (b & 0x7f) << shift;
-      if ((b & 0x80) == 0) {
-        if (varint_len(result) != used + 1) return false;
-        *value = result;
-        return true;
+    for (int t = 0; t < 5; ++t) {
+      const uint32_t bt = __shfl_sync(kFull, byte, max(lane - t, 0));
+      const int p = cu + here - 1 - t;  // position of byte lane - t in the token
+      if (t < here && p < 5) {
+        tok |= (bt & 0x7fu) << (7 * p);
+        if (p == 4 && bt > 0x0fu) bad = true;
       }
-      shift += 7;
     }
-    return false;
-  };
-  if (blen < 1) return false;
-  ++cursor;
-  if (r.byte() != kRansTableLog) return false;
-  uint32_t n = 0;
-  if (!varint(&n) || n == 0 || n > 255) return false;
-  uint32_t prev = 0, assigned = 0;
-  for (uint32_t i = 0; i < n; ++i) {
-    uint32_t delta = 0;
-    if (!varint(&delta) || (i != 0 && delta == 0) || prev + delta > maxf) return false;
-    const uint32_t value = prev + delta;
-    uint32_t fr = (1u << kRansTableLog) - assigned;
-    if (i + 1 != n && !varint(&fr)) return false;
-    // no 32-bit wrap-around: a frequency above 4096 - assigned is rejected
-    // (decode.cu:479-480 would wrap and then overrun its slot table)
-    if (fr == 0 || fr > (1u << kRansTableLog) - assigned ||
-        (i + 1 != n && fr == (1u << kRansTableLog) - assigned))
-      return false;
-    t.freqcum[i] = assigned | (fr << 12);
-    t.value[i] = fm.lim ? fold_value<uint16_t>(value, fm) : value & 0xffffu;
-    assigned += fr;
-    prev = value;
+    if (cu + here > 5) bad = true;
+    if (!bad && cu + here != varint_len(tok)) bad = true;
+    // bytes after the step's last token end begin (or continue) a token
+    const int last_end = endm ? 31 - __clz(endm) : -1;
+    const int tail = nvalid - 1 - last_end;
+    if (tail > 0) {
+      const int c0 = endm ? 0 : pend_used;
+      uint32_t v = endm ? 0u : pend_val;
+      bool pb = endm ? false : pend_bad;
+#pragma unroll
+      for (int t = 0; t < 5; ++t) {
+        const uint32_t bt = __shfl_sync(kFull, byte, min(last_end + 1 + t, 31));
+        const int p = c0 + t;
+        if (t < tail && p < 5) {
+          v |= (bt & 0x7fu) << (7 * p);
+          if (p == 4 && bt > 0x0fu) pb = true;
+        }
+      }
+      pend_val = v;
+      pend_used = min(c0 + tail, 6);
+      pend_bad = pb || c0 + tail > 5;
+    } else {
+      pend_val = 0;
+      pend_used = 0;
+      pend_bad = false;
+    }
+    return tok;
   }
-  if (assigned != (1u << kRansTableLog)) return false;
-  // three lane lengths (int in the reference: >= 2^31 ends in status 5
-  // there too), four states, the fourth length implied
-  int64_t total = 0;
-  for (int l = 0; l < 3; ++l) {
-    if (cursor + 4 > blen) return false;
-    uint32_t v = r.byte();
-    v |= r.byte() << 8;
-    v |= r.byte() << 16;
-    v |= r.byte() << 24;
-    cursor += 4;
-    if (v >= (1u << 31)) return false;
-    t.lane_len[l] = static_cast<int32_t>(v);
-    total += v;
+};
+
+__device__ __forceinline__ uint32_t scan_add(uint32_t v, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(kFull, v, o);
+    if (lane >= o) v += t;
   }
-  if (cursor + 16 > blen) return false;
-  for (int l = 0; l < 4; ++l) {
-    uint32_t v = r.byte();
-    v |= r.byte() << 8;
-    v |= r.byte() << 16;
-    v |= r.byte() << 24;
-    if (v < kRansL) return false;
-    t.state[l] = v;
-  }
-  cursor += 16;
-  const int64_t l3 = blen - cursor - total;
-  if (l3 < 0) return false;
-  t.lane_len[3] = static_cast<int32_t>(l3);
-  for (int l = 0; l < 4; ++l) {
-    t.lane_start[l] = static_cast<int32_t>(cursor);
-    cursor += t.lane_len[l];
-  }
-  t.nsym = static_cast<int32_t>(n);
-  return cursor == blen;
+  return v;
 }
 
+struct TableSm {
+  uint16_t starts[kBuckets];  // bit i of word u: a symbol starts at slot 16u + i
+  uint32_t entry[256];
+  uint16_t value[256];
+};
+
+// Order-0 table of one shard, parsed by a warp (decode.cu:456-517).  Tokens:
+// the symbol count n, then per symbol the value's delta and its frequency
+// (none for the last).  Values and cumulative frequencies are warp prefix sums
+// over the tokens of a step, in 32-bit arithmetic like the serial parser's
+// running sums; a table is rejected exactly when one of the serial parser's
+// checks fails at some symbol.
+__device__ bool rans_parse_warp(const uint8_t* __restrict__ body, int blen, uint32_t maxf, const FoldMap& fm,
+                                bool fold16, RansTable& t, TableSm& sm, int lane) {
+#pragma unroll
+  for (int i = 0; i < kBuckets / 64; ++i) reinterpret_cast<uint32_t*>(sm.starts)[32 * i + lane] = 0;
+  __syncwarp();
+  if (blen < 1 || body[0] != kRansTableLog) return false;
+  TokenReader tr;
+  int tokens = 0, n = 0;  // tokens of the steps so far; symbols, once known
+  uint32_t val0 = 0, cum0 = 0;
+  int cursor = 1;
+  bool wide = false;
+  for (;;) {
+    if (cursor >= blen) return false;
+    const bool vld = cursor + lane < blen;
+    const uint32_t byte = vld ? body[cursor + lane] : 0u;
+    bool bad;
+    const uint32_t tok = tr.step(byte, vld, min(32, blen - cursor), lane, bad);
+    const bool is_end = (tr.endm >> lane) & 1u;
+    const int at = tokens + __popc(tr.endm & ((1u << lane) - 1u));  // this token's number
+    if (tokens == 0 && tr.endm) {
+      const int first = __ffs(tr.endm) - 1;
+      const uint32_t count = __shfl_sync(kFull, tok, first);
+      if (__shfl_sync(kFull, bad, first) || count == 0 || count > 255) return false;
+      n = static_cast<int>(count);
+    }
+    const int i = (at - 1) >> 1;
+    const bool is_sym = is_end && at > 0 && i < n;
+    const bool is_freq = is_sym && !(at & 1);   // even numbers from 2: frequencies
+    const bool is_delta = is_sym && (at & 1);
+    const bool last = i == n - 1;
+    const bool use = is_delta || (is_freq && !last);
+    const uint32_t vals = scan_add(is_delta ? tok : 0u, lane) + val0;
+    const uint32_t cums = scan_add(is_freq && !last ? tok : 0u, lane) + cum0;
+    bool no = use && bad;
+    if (is_delta) no |= (i != 0 && tok == 0) || vals > maxf;
+    const bool whole = (is_freq && !last) || (is_delta && last);  // the symbol's frequency is known
+    const uint32_t fr = last ? (1u << kRansTableLog) - cums : tok;
+    const uint32_t cum = last ? cums : cums - tok;
+    if (is_freq && !last) no |= fr == 0 || fr >= (1u << kRansTableLog) - cum;
+    if (__any_sync(kFull, no)) return false;
+    if (whole) {
+      const uint32_t store = fm.lim ? fold_value<uint16_t>(vals, fm) : vals & 0xffffu;
+      sm.value[i] = static_cast<uint16_t>(store);
+      // (u32 symbols are not sign-extended to 16 bits but to 32)
+      wide |= static_cast<int16_t>(store) != static_cast<int8_t>(store) || (!fold16 && store > 127u);
+      sm.entry[i] = ((fr - 1u) << 20) | (cum << 8);
+      // two buckets a word
+      atomicOr(reinterpret_cast<uint32_t*>(sm.starts) + (cum >> 5), 1u << (cum & 31u));
+    }
+    const int count_here = __popc(tr.endm);
+    if (n && tokens + count_here >= 2 * n) {  // the last delta is in this step
+      const uint32_t lastm = __ballot_sync(kFull, is_delta && last);
+      cursor += __ffs(lastm);
+      break;
+    }
+    tokens += count_here;
+    val0 = __shfl_sync(kFull, vals, 31);
+    cum0 = __shfl_sync(kFull, cums, 31);
+    cursor += 32;
+  }
+  // three lane lengths, four states (each at least kRansL); the fourth lane
+  // takes the rest
+  if (cursor + 28 > blen) return false;
+  const uint32_t w = lane < 7 ? rd32(body + cursor + 4 * lane) : 0u;
+  cursor += 28;
+  const bool no = (lane < 3 && w >= (1u << 31)) || (lane >= 3 && lane < 7 && w < kRansL);
+  if (__any_sync(kFull, no)) return false;
+  int64_t start = cursor;
+  int64_t len[4];
+  for (int l = 0; l < 3; ++l) len[l] = __shfl_sync(kFull, w, l);
+  len[3] = blen - start - len[0] - len[1] - len[2];
+  if (len[3] < 0) return false;
+  wide = __any_sync(kFull, wide);
+  __syncwarp();
+  if (lane < 4) {
+    for (int l = 0; l < lane; ++l) start += len[l];
+    t.lane_start[lane] = static_cast<int32_t>(start);
+    t.lane_len[lane] = static_cast<int32_t>(len[lane]);
+  }
+  if (lane >= 3 && lane < 7) t.state[lane - 3] = w;
+  if (lane == 0) {
+    t.nsym = n;
+    t.narrow = !wide;
+  }
+  uint32_t* entries = t.data + RansTable::entries_at(n);
+  uint16_t* values = reinterpret_cast<uint16_t*>(t.data + RansTable::values_at(n));
+  for (int i = lane; i < n; i += 32) {
+    entries[i] = sm.entry[i] | (wide ? static_cast<uint32_t>(i) : sm.value[i] & 0xffu);
+    values[i] = sm.value[i];
+  }
+  if (n <= kBucketSymbols) {
+    // lane l: buckets 8l .. 8l + 7
+    const uint4 m = reinterpret_cast<const uint4*>(sm.starts)[lane];
+    const uint32_t w4[4] = {m.x, m.y, m.z, m.w};
+    const uint32_t mine = __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
+    uint32_t before = scan_add(mine, lane) - mine;  // symbols that start in earlier buckets
+    uint32_t b[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t m16 = (k & 1) ? w4[k >> 1] >> 16 : w4[k >> 1] & 0xffffu;
+      b[k] = ((before + (m16 & 1u) - 1u) << 18) | (m16 & 0xfffeu);
+      before += __popc(m16);
+    }
+    uint4* o = reinterpret_cast<uint4*>(t.data) + 2 * lane;
+    o[0] = make_uint4(b[0], b[1], b[2], b[3]);
+    o[1] = make_uint4(b[4], b[5], b[6], b[7]);
+  }
+  return true;
+}
+
+// A warp per rANS shard.  (A thread per shard, its serial parser waiting for
+// every token, took 18 us for a 1080p frame, this takes 4 us; 16 4K rgb frames
+// take 90 us, 13 more than that parser, but with the bucket tables that every
+// dec_rans group used to build for itself.)
 __global__ void __launch_bounds__(128)
 dec_rans_tables_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
                        const ShardInfo* __restrict__ shards, const DecodeLists* __restrict__ lists,
                        const int32_t* __restrict__ list_items, RansTable* __restrict__ tables, int fold16) {
+  __shared__ __align__(16) TableSm sm_all[4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int count = lists->count[0];
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x) {
+  for (int p = blockIdx.x * 4 + warp; p < count; p += gridDim.x * 4) {
     const ShardInfo& si = shards[list_items[p]];
     FrameState& st = state[si.frame];
     RansTable& t = tables[p];
     bool ok = false;
-    if (st.status == 0) {  // a failed parse may have left shard records unwritten
+    if (__any_sync(kFull, st.status == 0)) {  // a failed parse may have left shard records unwritten
       const FrameDesc& f = frames[si.frame];
-      ok = rans_parse_serial(f.stream + si.offset, si.body, static_cast<uint32_t>(f.max_sample) * 2u,
-                             fold_map(f, fold16), t);
-      if (!ok) set_status(&st.status, 5);
+      ok = rans_parse_warp(f.stream + si.offset, si.body, static_cast<uint32_t>(f.max_sample) * 2u,
+                           fold_map(f, fold16), fold16 != 0, t, sm_all[warp], lane);
+      if (!ok && lane == 0) set_status(&st.status, 5);
     }
-    t.valid = ok;
+    if (lane == 0) t.valid = ok;
+    __syncwarp();
   }
 }
 
-// Shared memory of one dec_rans warp: one column per 4-lane group, the
-// columns interleaved word by word (word k of group j at pool[k * 8 + j]) so
-// that the groups' lookups fall in different banks; and the lanes' byte
-// rings.  A column holds the shard's bucket table and, for tables of up to
-// 64 symbols (a predicted shard holds a few dozen), its freq|cum and value
-// words; larger tables are read from global memory.
-constexpr int kColumns = 8;  // 4-lane groups per warp
-constexpr int kColumnSymbols = 64;
-constexpr int kColumnWords = kBuckets + 2 * kColumnSymbols;
+// A lane's byte stream through a private ring of four 16-byte chunks in shared
+// memory, fed by cp.async: all four before the first read, then one with
+// every second eight-byte read (feed()).  Eight steps take at most 13 bytes, so
+// the read position enters at most one new chunk between two feeds and the ring
+// stays full whatever the data.  A feed may leave the newest two copies in
+// flight: a chunk is copied when the read position is three chunks before it
+// and read when it is one chunk before, at least two feeds later.  Of the
+// lane's last chunk only the bytes up to the lane's end are copied (reading past
+// them is an overrun that the byte count check reports).
+template <int LANES>
+struct LaneRing {
+  static constexpr int kChunks = 4;
+  uint32_t ring;          // shared address of slot 0 of this lane (slots LANES chunks apart)
+  const uint8_t* next;    // global address of the next chunk to copy
+  int at;                 // bit position of the next unread byte, from the first chunk's start
+  int last, last_bytes;   // last chunk holding a lane byte (-1: none), and its bytes
+  int fetched;            // number of the next chunk to copy
 
-struct RansWarpSm {
-  uint32_t pool[kColumns * kColumnWords];
-  // per-lane byte rings, slot-major: rings[s][lane]
-  uint32_t rings[LaneRing::kWords][32];
+  __device__ void issue(int upto) {
+    const uint32_t s = ring + (fetched & (kChunks - 1)) * (LANES * 16);
+    const int ok = fetched <= min(last, upto);
+    const int n = fetched == last ? last_bytes : 16;
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %3, 0;\n @p cp.async.cg.shared.global [%0], [%1], 16, %2;\n}\n" ::"r"(s),
+        "l"(next), "r"(n), "r"(ok)
+        : "memory");
+    fetched += ok;
+    next += ok ? 16 : 0;
+  }
+  __device__ void init(uint4* ring_smem, const uint8_t* p, int len) {
+    const int head = static_cast<int>(reinterpret_cast<uintptr_t>(p) & 15);
+    next = p - head;
+    at = 8 * head;
+    ring = static_cast<uint32_t>(__cvta_generic_to_shared(ring_smem));
+    last = len > 0 ? (head + len - 1) >> 4 : -1;
+    last_bytes = ((head + len - 1) & 15) + 1;
+    fetched = 0;
+#pragma unroll
+    for (int i = 0; i < kChunks; ++i) issue(kChunks - 1);
+    cp_async_commit();
+  }
+  __device__ __forceinline__ void feed() {
+    issue((at >> 7) + kChunks - 1);
+    cp_async_commit();
+    cp_async_wait<2>();
+  }
+  // The next eight bytes, first byte in the top bits of hi, the last four in lo.
+  __device__ __forceinline__ void window(uint32_t& hi, uint32_t& lo) const {
+    const uint32_t q = static_cast<uint32_t>(at) >> 6;  // pair of words holding the first byte
+    auto pair = [&](uint32_t i) { return ring + ((i >> 1) & (kChunks - 1)) * (LANES * 16) + (i & 1) * 8; };
+    uint32_t w0, w1, w2, w3;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w0), "=r"(w1) : "r"(pair(q)));
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w2), "=r"(w3) : "r"(pair(q + 1)));
+    const bool upper = at & 32;
+    const uint32_t a = upper ? w1 : w0, b = upper ? w2 : w1, c = upper ? w3 : w2;
+    const uint32_t sel = 0x0123u + 0x1111u * ((static_cast<uint32_t>(at) >> 3) & 3u);
+    hi = __byte_perm(a, b, sel);
+    lo = __byte_perm(b, c, sel);
+  }
+};
+
+// Shared memory of one dec_rans warp: eight shards' tables (bucket words, then
+// the entries of up to kLocalSymbols symbols; a shard with more reads its
+// entries from its table record) and the lanes' byte rings.
+constexpr int kGroups = 8;  // shards per warp, four lanes each
+constexpr int kLocalSymbols = 64;
+constexpr int kTableWords = kBuckets + kLocalSymbols;
+
+struct alignas(16) RansWarpSm {
+  uint32_t table[kGroups][kTableWords];
+  uint4 rings[LaneRing<32>::kChunks][32];
 };
 
 size_t dec_rans_smem() { return sizeof(RansWarpSm) * kWarpsPerCta; }
 
-// Bucket table of one shard: word u = (symbol holding slot 16u) << 16, with
-// bit i set for every symbol whose range starts at slot 16u + i (i = 1..15).
-// The symbol holding slot s is then the bucket's first symbol plus the
-// starts at or below s inside the bucket -- one shared load and a population
-// count, no search.  `fc` is the freq|cum list at a stride of 2^fc_shift
-// words; lane l of the group writes buckets 64l .. 64l + 63.
-__device__ __forceinline__ void build_buckets(uint32_t* bcol, const uint32_t* fc, int fc_shift, int nsym,
-                                              int my_l) {
+// Bucket table of a shard of more than kBucketSymbols symbols, by its four
+// lanes: lane l writes buckets 64l .. 64l + 63.
+__device__ __forceinline__ void build_buckets(uint32_t* b, const uint32_t* entries, int nsym, int my_l) {
   constexpr uint32_t kSlots = 1u << kRansTableLog;
-  auto start = [&](int i) { return i < nsym ? (fc[i << fc_shift] & (kSlots - 1u)) : kSlots; };
+  auto start = [&](int i) { return i < nsym ? ((entries[i] >> 8) & (kSlots - 1u)) : kSlots; };
   int s = 0;
   uint32_t next = start(1);  // first slot of symbol s + 1
   for (int k = 0; k < kBuckets / 4; ++k) {
     const uint32_t u = static_cast<uint32_t>(my_l * (kBuckets / 4) + k);
     const uint32_t lo = u << kBucketShift;
     while (next <= lo) next = start(++s + 1);
-    uint32_t w = static_cast<uint32_t>(s) << 16;
+    uint32_t w = static_cast<uint32_t>(s) << 18;
     for (int i = s + 1; next < lo + (1u << kBucketShift);) {
       w |= 1u << (next - lo);
       next = start(++i);
     }
     next = start(s + 1);
-    bcol[u * kColumns] = w;
+    b[u] = w;
   }
 }
 
-// Decode lane `my_l` of one shard: n symbols from this lane's byte ring,
-// initial state x; the bucket table at a stride of 8 words,
-// the freq|cum and value words at a stride of 2^LOG_S.  Returns the bytes
-// consumed and the final state.
-template <int LOG_S, typename FoldT>
-__device__ __forceinline__ void rans_decode_lane(const uint32_t* __restrict__ bcol, const uint32_t* __restrict__ fc_col,
-                                                 const uint32_t* __restrict__ val_col, LaneRing& ring,
-                                                 FoldT* __restrict__ out, int n, int my_l, uint32_t& x, int& cur) {
-  cur = 0;
-  ring.ready();
-  // Branch-free step: after x = freq*(x>>12) + slot - cum, x >= 2^11, so
-  // renormalisation shifts in one byte when x < 2^23 and a second when
-  // x < 2^15 (decode.cu:540-545), taken from the top of an eight-byte window
-  // read ahead of the state chain; four steps use at most eight bytes.
-  // Reading past the lane is an error, found by the byte count.  The window
-  // is two 32-bit words (whi, wlo), shifted by funnel shifts: a 64-bit
-  // variable shift costs several instructions on the state chain.
-  auto step = [&](uint32_t& whi, uint32_t& wlo, int idx) {
-    const uint32_t slot = x & ((1u << kRansTableLog) - 1u);
-    const uint32_t bw = bcol[(slot >> kBucketShift) * kColumns];
+// The entry of the state's slot, through a shard's bucket table.
+struct BucketLookup {
+  const uint32_t* buckets;
+  const uint32_t* entries;
+  // x' = freq * (x >> 12) + slot - cum
+  __device__ __forceinline__ uint32_t operator()(uint32_t& x) const {
+    const uint32_t slot = x & ((1u << kRansTableLog) - 1u), xh = x >> kRansTableLog;
+    const uint32_t bw = buckets[slot >> kBucketShift];
     // starts at offsets 1..r of the bucket survive the shift by 31 - r
-    const uint32_t sym = (bw >> 16) + __popc(bw << ((slot & ((1u << kBucketShift) - 1u)) ^ 31u));
-    const uint32_t fc = fc_col[sym << LOG_S];
-    out[idx] = static_cast<FoldT>(val_col[sym << LOG_S]);
-    x = (fc >> 12) * (x >> kRansTableLog) + slot - (fc & ((1u << kRansTableLog) - 1u));
-    const int nb = (x < kRansL) + (x < (kRansL >> 8));
-    const uint32_t sh = 8u * static_cast<uint32_t>(nb);  // 0, 8 or 16
-    x = __funnelshift_l(whi, x, sh);
-    whi = __funnelshift_l(wlo, whi, sh);
-    wlo <<= sh;
-    cur += nb;
-  };
-  int idx = my_l;
-  for (; idx + 12 < n; idx += 16) {
-    uint32_t whi, wlo;
-    ring.window(cur, whi, wlo);
-    step(whi, wlo, idx);
-    step(whi, wlo, idx + 4);
-    step(whi, wlo, idx + 8);
-    step(whi, wlo, idx + 12);
+    const uint32_t more = __popc(bw << ((slot & ((1u << kBucketShift) - 1u)) ^ 31u));
+    const uint32_t e = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(entries) + (bw >> 16) + 4 * more);
+    x = (e >> 20) * xh + (xh + slot - ((e >> 8) & 0xfffu));
+    return e;
   }
-  if (idx < n) {
-    uint32_t whi, wlo;
-    ring.window(cur, whi, wlo);
-    for (; idx < n; idx += 4) step(whi, wlo, idx);  // at most three steps
+};
+
+// Through a table of all 4096 slots: entries with slot - cum in place of cum.
+struct SlotLookup {
+  const uint32_t* slots;
+  __device__ __forceinline__ uint32_t operator()(uint32_t& x) const {
+    const uint32_t xh = x >> kRansTableLog;
+    const uint32_t e = slots[x & ((1u << kRansTableLog) - 1u)];
+    x = (e >> 20) * xh + (xh + ((e >> 8) & 0xfffu));
+    return e;
+  }
+};
+
+// Bytes of b by prmt selector; a selector digit with its top bit set repeats
+// the byte's sign (__byte_perm ignores that bit).
+template <int SEL>
+__device__ __forceinline__ uint32_t sign_bytes(uint32_t b) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(b), "n"(SEL));
+  return r;
+}
+
+template <typename FoldT>
+__device__ __forceinline__ FoldT rans_value(uint32_t byte, bool narrow, const uint16_t* values) {
+  const uint32_t v = narrow ? static_cast<uint32_t>(static_cast<int8_t>(byte)) : values[byte];
+  return static_cast<FoldT>(v);
+}
+
+// The state map's renormalisation: after it x >= 2^11, so one byte comes in
+// when x < 2^23 and a second when x < 2^15 (decode.cu:540-545).
+__device__ __forceinline__ uint32_t rans_shift(uint32_t x) {
+  const uint32_t sh = x < kRansL ? 8u : 0u;
+  return x < (kRansL >> 8) ? 16u : sh;
+}
+
+// Four steps of a lane; byte k of the result is the low byte of step k's
+// entry.  The bytes come from the top of an eight-byte window, as many as four
+// steps can use; reading past the lane is an error, found by the byte count.
+// `aside0`, `aside1` and `aside2` run between the steps, where the warp would
+// wait for its lookups.
+template <int LANES, typename Lookup, typename A0, typename A1, typename A2>
+__device__ __forceinline__ uint32_t rans_four(const Lookup lookup, LaneRing<LANES>& ring, uint32_t& x, A0 aside0,
+                                              A1 aside1, A2 aside2) {
+  uint32_t hi, lo;
+  ring.window(hi, lo);
+  aside0();
+  const uint32_t e0 = lookup(x);
+  const uint32_t s0 = rans_shift(x);
+  x = __funnelshift_l(hi, x, s0);
+  aside1();
+  const uint32_t e1 = lookup(x);
+  const uint32_t s1 = rans_shift(x);
+  x = __funnelshift_l(__funnelshift_l(lo, hi, s0), x, s1);
+  const uint32_t half = s0 + s1;  // at most 32
+  hi = __funnelshift_lc(lo, hi, half);
+  lo = half < 32 ? lo << half : 0u;
+  aside2();
+  const uint32_t e2 = lookup(x);
+  const uint32_t s2 = rans_shift(x);
+  x = __funnelshift_l(hi, x, s2);
+  const uint32_t e3 = lookup(x);
+  const uint32_t s3 = rans_shift(x);
+  x = __funnelshift_l(__funnelshift_l(lo, hi, s2), x, s3);
+  ring.at += half + s2 + s3;
+  return __byte_perm(__byte_perm(e0, e1, 0x0040), __byte_perm(e2, e3, 0x0040), 0x5410);
+}
+
+// Decode lane `my_l` of one shard: n symbols from this lane's byte ring,
+// initial state x; lane l decodes symbols l, l + 4, ...  Returns the final
+// state; the ring's position tells the bytes consumed.  Four steps' symbols of
+// the four lanes, one byte each, are transposed among the lanes by two
+// shuffles, so each lane stores four consecutive symbols at once.
+template <typename FoldT, int LANES, typename Lookup>
+__device__ __forceinline__ void rans_decode_lane(const Lookup lookup, bool narrow, const uint16_t* __restrict__ values,
+                                                 LaneRing<LANES>& ring, FoldT* __restrict__ out, int n, int my_l,
+                                                 unsigned group, uint32_t& x) {
+  const uint32_t sel1 = my_l < 2 ? 0x5410u : 0x3276u, sel2 = (my_l & 1) ? 0x3715u : 0x6240u;
+  out += 4 * my_l;
+  // b: byte k is the byte of step my_l of lane k, i.e. of symbol 4 my_l + k of
+  // sixteen
+  auto put = [&](FoldT* o, uint32_t b) {
+    if constexpr (sizeof(FoldT) == 2) {
+      uint2 v;
+      if (narrow) {
+        v = make_uint2(sign_bytes<0x9180>(b), sign_bytes<0xb3a2>(b));
+      } else {
+        v.x = values[b & 0xffu] | (static_cast<uint32_t>(values[(b >> 8) & 0xffu]) << 16);
+        v.y = values[(b >> 16) & 0xffu] | (static_cast<uint32_t>(values[b >> 24]) << 16);
+      }
+      *reinterpret_cast<uint2*>(o) = v;
+    } else {
+      uint4 v;
+      if (narrow) {
+        v = make_uint4(sign_bytes<0x8880>(b), sign_bytes<0x9991>(b), sign_bytes<0xaaa2>(b), sign_bytes<0xbbb3>(b));
+      } else {
+        v = make_uint4(values[b & 0xffu], values[(b >> 8) & 0xffu], values[(b >> 16) & 0xffu], values[b >> 24]);
+      }
+      *reinterpret_cast<uint4*>(o) = v;
+    }
+  };
+  auto none = [] {};
+  int left = n;
+  // the bytes of the last 32 symbols (byte k: this lane's step k) are
+  // transposed and stored while the next ones are decoded
+  uint32_t b0 = 0, b1 = 0, t0 = 0, t1 = 0;
+  auto swap2 = [&] {
+    t0 = __shfl_xor_sync(group, b0, 2);
+    t1 = __shfl_xor_sync(group, b1, 2);
+  };
+  auto swap1 = [&] {
+    b0 = __byte_perm(b0, t0, sel1);
+    b1 = __byte_perm(b1, t1, sel1);
+    t0 = __shfl_xor_sync(group, b0, 1);
+    t1 = __shfl_xor_sync(group, b1, 1);
+  };
+  auto store = [&] {
+    put(out - 32, __byte_perm(b0, t0, sel2));
+    put(out - 16, __byte_perm(b1, t1, sel2));
+  };
+  if (left >= 32) {
+    ring.feed();
+    b0 = rans_four<LANES>(lookup, ring, x, none, none, none);
+    b1 = rans_four<LANES>(lookup, ring, x, none, none, none);
+    left -= 32;
+    out += 32;
+    for (; left >= 32; left -= 32, out += 32) {
+      ring.feed();
+      const uint32_t n0 = rans_four<LANES>(lookup, ring, x, swap2, swap1, store);
+      const uint32_t n1 = rans_four<LANES>(lookup, ring, x, none, none, none);
+      b0 = n0;
+      b1 = n1;
+    }
+    swap2();
+    swap1();
+    store();
+  }
+  if (left >= 16) {
+    ring.feed();
+    b0 = rans_four<LANES>(lookup, ring, x, none, none, none);
+    swap2();
+    swap1();
+    put(out, __byte_perm(b0, t0, sel2));
+    left -= 16;
+    out += 16;
+  }
+  if (left > 0) {  // at most 15 symbols: at most four steps a lane
+    ring.feed();
+    uint32_t hi, lo;
+    ring.window(hi, lo);
+    out -= 4 * my_l;
+    for (int i = my_l; i < left; i += 4) {
+      out[i] = rans_value<FoldT>(lookup(x) & 0xffu, narrow, values);
+      const uint32_t sh = rans_shift(x);
+      x = __funnelshift_l(hi, x, sh);
+      hi = __funnelshift_l(lo, hi, sh);
+      lo <<= sh;
+      ring.at += sh;
+    }
   }
   cp_async_wait<0>();
 }
 
-// Each 4-lane group streams rANS shards: it claims the next shard from the
-// list, builds the shard's tables in its column and decodes its four lanes,
-// then claims another -- so every lane stays busy until the list is done,
-// whatever the mix of shards.
+// A warp takes eight rANS shards at a time (all shards but the last of a tile
+// have 1,024 steps a lane), copies their tables into shared memory and decodes
+// their 32 lanes.
+//
+// Bound by the chain of a step -- two dependent shared-memory lookups and a
+// population count -- and, with 16 warps an SM, by the shared-memory pipe
+// (12 cycles a step: the lookups hit about three banks twice) and issue (42
+// instructions).  16 4K rgb10 frames: 1117 us with a lookup and a store of two
+// bytes for every symbol's value and tables built by four lanes while the rest
+// of the warp waited; 861 us with the value in the entry, 16-byte transposed
+// stores and tables made once by dec_rans_tables.
 template <typename FoldT>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 dec_rans_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
@@ -524,45 +698,120 @@ dec_rans_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
   const int j = lane >> 2, my_l = lane & 3;
   const unsigned group = 0xfu << (4 * j);
   const int count = lists->count[0];
-  uint32_t* bcol = sm.pool + j;
-  uint32_t* fc_col = sm.pool + kBuckets * kColumns + j;
-  uint32_t* val_col = sm.pool + (kBuckets + kColumnSymbols) * kColumns + j;
   for (;;) {
-    int p = 0;
-    if (my_l == 0) p = atomicAdd(&lists->next_group_rans, 1);
-    p = __shfl_sync(group, p, 4 * j);
-    if (p >= count) break;
-    const RansTable& t = tables[p];
-    if (!t.valid) continue;
-    const ShardInfo& si = shards[list_items[p]];
-    const FrameDesc& f = frames[si.frame];
-    const uint8_t* body = f.stream + si.offset;
-    FoldT* out = folded + si.sample_base;
-    uint32_t x = t.state[my_l];
-    const int llen = t.lane_len[my_l];
-    const uint8_t* lb = body + t.lane_start[my_l];
-    const int nsym = t.nsym;
-    const bool local = nsym <= kColumnSymbols;
-    int cur = 0;
-    LaneRing ring;
-    ring.init(&sm.rings[0][lane], lb, llen);  // the first copies land while the tables are built
-    __syncwarp(group);  // the group's previous shard is decoded
-    if (local) {
-      for (int i = my_l; i < nsym; i += 4) {
-        fc_col[i * kColumns] = t.freqcum[i];
-        val_col[i * kColumns] = t.value[i];
-      }
-      __syncwarp(group);
-      build_buckets(bcol, fc_col, 3, nsym, my_l);
-    } else {
-      build_buckets(bcol, t.freqcum, 0, nsym, my_l);
+    int p0 = 0;
+    if (lane == 0) p0 = atomicAdd(&lists->next_group_rans, kGroups);
+    p0 = __shfl_sync(kFull, p0, 0);
+    if (p0 >= count) break;
+    const int p = p0 + j;
+    const bool live = p < count && tables[p].valid;
+    const RansTable& t = tables[live ? p : p0];
+    const int nsym = live ? t.nsym : 0;
+    const bool local = nsym <= kLocalSymbols;
+    LaneRing<32> ring;
+    const ShardInfo* si = nullptr;
+    const FrameDesc* f = nullptr;
+    if (live) {
+      si = &shards[list_items[p]];
+      f = &frames[si->frame];
+      ring.init(&sm.rings[0][lane], f->stream + si->offset + t.lane_start[my_l], t.lane_len[my_l]);
     }
-    __syncwarp(group);
-    if (local)
-      rans_decode_lane<3>(bcol, fc_col, val_col, ring, out, si.count, my_l, x, cur);
-    else
-      rans_decode_lane<0>(bcol, t.freqcum, t.value, ring, out, si.count, my_l, x, cur);
-    if (cur != llen || x != kRansL) set_status(&state[si.frame].status, 5);
+    // the bucket words and the local entries, 16 bytes a copy
+    const uint32_t* entries = t.data + RansTable::entries_at(nsym);
+    if (live) {
+      uint32_t* to = sm.table[j];
+      if (nsym <= kBucketSymbols) {
+        const int chunks = (kBuckets + (local ? nsym : 0) + 3) / 4;  // the entries follow the buckets
+        for (int i = my_l; i < chunks; i += 4) cp_async16(to + 4 * i, t.data + 4 * i);
+      } else {
+        build_buckets(to, entries, nsym, my_l);
+      }
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncwarp();
+    if (live) {
+      const uint16_t* values = reinterpret_cast<const uint16_t*>(t.data + RansTable::values_at(nsym));
+      FoldT* out = folded + si->sample_base;
+      uint32_t x = t.state[my_l];
+      const int from = ring.at;
+      if (local)
+        rans_decode_lane<FoldT, 32>(BucketLookup{sm.table[j], sm.table[j] + kBuckets}, t.narrow, values, ring, out,
+                                    si->count, my_l, group, x);
+      else
+        rans_decode_lane<FoldT, 32>(BucketLookup{sm.table[j], entries}, t.narrow, values, ring, out, si->count, my_l,
+                                    group, x);
+      if (ring.at - from != 8 * t.lane_len[my_l] || x != kRansL) set_status(&state[si->frame].status, 5);
+    }
+    __syncwarp();
+  }
+}
+
+// Few shards: the chain of a step decides, not the number of lanes in flight.
+// A warp of its own takes two shards and spreads their tables over all 4096
+// slots (16 KB each), which leaves one lookup a step: a 1080p rgb10 frame of
+// 1,539 shards takes 94 us here, 125 us in dec_rans_kernel.
+constexpr int kSlotGroups = 2;
+struct alignas(16) RansSlotSm {
+  uint32_t slots[kSlotGroups][1 << kRansTableLog];
+  uint4 rings[LaneRing<4 * kSlotGroups>::kChunks][4 * kSlotGroups];
+  uint32_t entry[256];
+  uint32_t bucket[kBuckets];
+};
+size_t dec_rans_slots_smem() { return sizeof(RansSlotSm); }
+
+template <typename FoldT>
+__global__ void __launch_bounds__(32)
+dec_rans_slots_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
+                      const ShardInfo* __restrict__ shards, DecodeLists* __restrict__ lists,
+                      const int32_t* __restrict__ list_items, const RansTable* __restrict__ tables,
+                      FoldT* __restrict__ folded) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  RansSlotSm& sm = *reinterpret_cast<RansSlotSm*>(smem_raw);
+  const int lane = threadIdx.x;
+  const int j = lane >> 2, my_l = lane & 3;
+  const int count = lists->count[0];
+  for (int p0 = blockIdx.x * kSlotGroups; p0 < count; p0 += gridDim.x * kSlotGroups) {
+    const int p = p0 + j;
+    const bool live = j < kSlotGroups && p < count && tables[p].valid;
+    const RansTable& mine = tables[live ? p : p0];
+    LaneRing<4 * kSlotGroups> ring;
+    const ShardInfo* si = nullptr;
+    if (live) {
+      si = &shards[list_items[p]];
+      ring.init(&sm.rings[0][lane], frames[si->frame].stream + si->offset + mine.lane_start[my_l],
+                mine.lane_len[my_l]);
+    }
+    for (int g = 0; g < kSlotGroups && p0 + g < count; ++g) {
+      const RansTable& t = tables[p0 + g];
+      if (!t.valid) continue;
+      const int nsym = t.nsym;
+      const uint32_t* entries = t.data + RansTable::entries_at(nsym);
+      __syncwarp();
+      for (int i = lane; i < nsym; i += 32) sm.entry[i] = entries[i];
+      if (nsym <= kBucketSymbols)
+        for (int i = lane; i < kBuckets; i += 32) sm.bucket[i] = t.data[i];
+      else if (lane < 4)
+        build_buckets(sm.bucket, entries, nsym, lane);
+      __syncwarp();
+#pragma unroll 4
+      for (int i = lane; i < (1 << kRansTableLog); i += 32) {
+        const uint32_t bw = sm.bucket[i >> kBucketShift];
+        const uint32_t e = sm.entry[(bw >> 18) + __popc(bw << ((i & ((1 << kBucketShift) - 1)) ^ 31))];
+        sm.slots[g][i] = (e & 0xfff000ffu) | ((static_cast<uint32_t>(i) - ((e >> 8) & 0xfffu)) << 8);
+      }
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+    if (live) {
+      const uint16_t* values = reinterpret_cast<const uint16_t*>(mine.data + RansTable::values_at(mine.nsym));
+      uint32_t x = mine.state[my_l];
+      const int from = ring.at;
+      rans_decode_lane<FoldT, 4 * kSlotGroups>(SlotLookup{sm.slots[j]}, mine.narrow, values, ring,
+                                               folded + si->sample_base, si->count, my_l, 0xfu << (4 * j), x);
+      if (ring.at - from != 8 * mine.lane_len[my_l] || x != kRansL) set_status(&state[si->frame].status, 5);
+    }
+    __syncwarp();
   }
 }
 
@@ -760,51 +1009,28 @@ __device__ bool rice_shard(const uint8_t* __restrict__ body, int blen, int n, in
 }
 
 // A zero-run shard (decode.cu:237-295) decoded by the whole warp, 32 body
-// bytes per step, one per lane.  A byte without the 0x80 bit ends a token
-// (ballot); the lane holding a token's last byte gathers the token's bytes
-// from the lanes before it by shuffles, with the bytes of a token begun in an
-// earlier step carried over; the symbols of the step's tokens are placed by
-// a warp prefix sum.  Every check of the serial parser is made -- at most
-// five bytes, the fifth at most 0x0f, canonical length, a run no longer than
-// the symbols left, a value in 1..maxf, no token after the last symbol, no
-// partial token and no missing symbol at the end -- so a stream is accepted
-// exactly when the serial parser accepts it.  The shard's symbols are zeroed
-// first; value tokens then write theirs.  Warp-collective: every lane calls
-// it with the same arguments.  Returns whether the shard is valid.
+// bytes per step, one per lane: the step's tokens (TokenReader) are placed by
+// a warp prefix sum of the symbols they stand for.  Every check of the serial
+// parser is made -- the varint rules, a run no longer than the symbols left, a
+// value in 1..maxf, no token after the last symbol, no partial token and no
+// missing symbol at the end -- so a stream is accepted exactly when the serial
+// parser accepts it.  The shard's symbols are zeroed first; value tokens then
+// write theirs.  Warp-collective: every lane calls it with the same arguments.
+// Returns whether the shard is valid.
 template <typename FoldT>
 __device__ bool zero_run_warp(const uint8_t* __restrict__ body, int64_t blen, int n, uint32_t maxf,
                               const FoldMap& fm, FoldT* __restrict__ out, int lane) {
   for (int i = lane; i < n; i += 32) out[i] = 0;
   __syncwarp();
-  int produced = 0;        // symbols of the steps so far (warp-uniform)
-  uint32_t pend_val = 0;   // value bits of a token begun in an earlier step
-  int pend_used = 0;       // its bytes so far (capped at 6)
-  bool pend_bad = false;   // its fifth byte was above 0x0f, or it is too long
+  int produced = 0;  // symbols of the steps so far (warp-uniform)
+  TokenReader tr;
   bool bad = false;
   for (int64_t base = 0; base < blen && !bad; base += 32) {
     const bool vld = base + lane < blen;
     const uint32_t byte = vld ? body[base + lane] : 0u;
-    const uint32_t endm = __ballot_sync(kFull, vld && !(byte & 0x80u));
-    const int nvalid = static_cast<int>(min(static_cast<int64_t>(32), blen - base));
-    const bool is_end = (endm >> lane) & 1u;
-    const uint32_t below = endm & ((1u << lane) - 1u);
-    const int prev = below ? 31 - __clz(below) : -1;  // the previous token's end in this step
-    const bool carried = prev < 0;                    // the token began in an earlier step
-    const int here = lane - prev;                     // its bytes in this step
-    const int cu = carried ? pend_used : 0;
-    uint32_t tok = carried ? pend_val : 0u;
-    bool tb = carried && pend_bad;
-#pragma unroll
-    for (int t = 0; t < 5; ++t) {
-      const uint32_t bt = __shfl_sync(kFull, byte, max(lane - t, 0));
-      const int p = cu + here - 1 - t;  // position of byte lane - t in the token
-      if (t < here && p < 5) {
-        tok |= (bt & 0x7fu) << (7 * p);
-        if (p == 4 && bt > 0x0fu) tb = true;
-      }
-    }
-    if (cu + here > 5) tb = true;
-    if (!tb && cu + here != varint_len(tok)) tb = true;
+    bool tb;
+    const uint32_t tok = tr.step(byte, vld, static_cast<int>(min(static_cast<int64_t>(32), blen - base)), lane, tb);
+    const bool is_end = (tr.endm >> lane) & 1u;
     uint32_t cnt = 0;
     if (is_end) {
       if (tok & 1u) {
@@ -815,12 +1041,7 @@ __device__ bool zero_run_warp(const uint8_t* __restrict__ body, int64_t blen, in
         cnt = min((tok >> 1) + 1u, static_cast<uint32_t>(n) + 1u);  // a run; longer than n fails below
       }
     }
-    uint32_t inc = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(kFull, inc, o);
-      if (lane >= o) inc += v;
-    }
+    const uint32_t inc = scan_add(cnt, lane);
     const uint32_t start = static_cast<uint32_t>(produced) + inc - cnt;
     if (is_end) {
       if (start + cnt > static_cast<uint32_t>(n)) tb = true;  // a run past the end, or a token after it
@@ -828,32 +1049,8 @@ __device__ bool zero_run_warp(const uint8_t* __restrict__ body, int64_t blen, in
     }
     bad = __any_sync(kFull, is_end && tb);
     produced += static_cast<int>(__shfl_sync(kFull, inc, 31));
-    // bytes after the step's last token end begin (or continue) a token
-    const int last_end = endm ? 31 - __clz(endm) : -1;
-    const int tail = nvalid - 1 - last_end;
-    if (tail > 0) {
-      const int c0 = endm ? 0 : pend_used;
-      uint32_t v = endm ? 0u : pend_val;
-      bool pb = endm ? false : pend_bad;
-#pragma unroll
-      for (int t = 0; t < 5; ++t) {
-        const uint32_t bt = __shfl_sync(kFull, byte, min(last_end + 1 + t, 31));
-        const int p = c0 + t;
-        if (t < tail && p < 5) {
-          v |= (bt & 0x7fu) << (7 * p);
-          if (p == 4 && bt > 0x0fu) pb = true;
-        }
-      }
-      pend_val = v;
-      pend_used = min(c0 + tail, 6);
-      pend_bad = pb || c0 + tail > 5;
-    } else {
-      pend_val = 0;
-      pend_used = 0;
-      pend_bad = false;
-    }
   }
-  return !bad && pend_used == 0 && produced == n;
+  return !bad && tr.pend_used == 0 && produced == n;
 }
 
 struct OtherGroupSm {
@@ -1396,21 +1593,35 @@ void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, bool few, i
       frames, state, dims, static_cast<const uint32_t*>(folded), queue);
 }
 
-void dec_rans_launch(bool fold16, int grid, size_t smem, cudaStream_t stream, const FrameDesc* frames,
+void dec_rans_launch(bool fold16, bool few, int grid, cudaStream_t stream, const FrameDesc* frames,
                      FrameState* state, const ShardInfo* shards, DecodeLists* lists, const int32_t* list_items,
                      const RansTable* tables, void* folded) {
-  if (fold16)
-    dec_rans_kernel<uint16_t><<<grid, kWarpsPerCta * 32, smem, stream>>>(frames, state, shards, lists, list_items,
-                                                                         tables, static_cast<uint16_t*>(folded));
-  else
-    dec_rans_kernel<uint32_t><<<grid, kWarpsPerCta * 32, smem, stream>>>(frames, state, shards, lists, list_items,
-                                                                         tables, static_cast<uint32_t*>(folded));
+  const int threads = few ? 32 : kWarpsPerCta * 32;
+  const size_t smem = few ? dec_rans_slots_smem() : dec_rans_smem();
+  if (fold16) {
+    auto k = few ? dec_rans_slots_kernel<uint16_t> : dec_rans_kernel<uint16_t>;
+    k<<<grid, threads, smem, stream>>>(frames, state, shards, lists, list_items, tables,
+                                       static_cast<uint16_t*>(folded));
+  } else {
+    auto k = few ? dec_rans_slots_kernel<uint32_t> : dec_rans_kernel<uint32_t>;
+    k<<<grid, threads, smem, stream>>>(frames, state, shards, lists, list_items, tables,
+                                       static_cast<uint32_t*>(folded));
+  }
 }
 
-cudaError_t dec_rans_set_attr(cudaFuncAttribute attr, int value) {
-  const cudaError_t e = cudaFuncSetAttribute(dec_rans_kernel<uint16_t>, attr, value);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(dec_rans_kernel<uint32_t>, attr, value);
+cudaError_t dec_rans_set_smem() {
+  const int b = static_cast<int>(dec_rans_smem()), bs = static_cast<int>(dec_rans_slots_smem());
+  auto set = [](auto k, int bytes) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                                   cudaSharedmemCarveoutMaxShared);
+  };
+  cudaError_t e = set(dec_rans_kernel<uint16_t>, b);
+  if (e == cudaSuccess) e = set(dec_rans_kernel<uint32_t>, b);
+  if (e == cudaSuccess) e = set(dec_rans_slots_kernel<uint16_t>, bs);
+  if (e == cudaSuccess) e = set(dec_rans_slots_kernel<uint32_t>, bs);
+  return e;
 }
 
 // Every kernel of the decode asks for the same split of the L1/shared array as

@@ -140,10 +140,11 @@ __global__ void dec_parse_kernel(const FrameDesc* frames, FrameState* state, con
 __global__ void dec_rans_tables_kernel(const FrameDesc* frames, FrameState* state, const ShardInfo* shards,
                                        const DecodeLists* lists, const int32_t* list_items, RansTable* tables,
                                        int fold16);
-void dec_rans_launch(bool fold16, int grid, size_t smem, cudaStream_t stream, const FrameDesc* frames,
+// `few` shards: one warp for two shards, tables of all slots
+void dec_rans_launch(bool fold16, bool few, int grid, cudaStream_t stream, const FrameDesc* frames,
                      FrameState* state, const ShardInfo* shards, DecodeLists* lists, const int32_t* list_items,
                      const RansTable* tables, void* folded);
-cudaError_t dec_rans_set_attr(cudaFuncAttribute attr, int value);
+cudaError_t dec_rans_set_smem();
 void dec_other_launch(bool fold16, int grid, cudaStream_t stream, const FrameDesc* frames, FrameState* state,
                       const ShardInfo* shards, const BatchDims* dims, DecodeLists* lists, const int32_t* list_items,
                       void* folded);
@@ -162,7 +163,6 @@ __global__ void dec_reconstruct_serial_kernel(const FrameDesc* frames, const Fra
 size_t enc_predict_smem(bool fold16);
 size_t enc_emit_smem();
 size_t dec_reconstruct_smem(bool fold16);
-size_t dec_rans_smem();
 size_t dec_rans_table_bytes();
 
 }  // namespace fvb
