@@ -53,12 +53,12 @@ int cuda_fail(cudaError_t e, const char* where) {
 enum KernelId {
   K_ENC_INIT, K_ENC_PREDICT, K_ENC_PREDICT_WIDE, K_ENC_ANALYZE, K_ENC_RANS, K_ENC_SCAN, K_ENC_PREFIX,
   K_ENC_EMIT, K_DEC_PARSE, K_DEC_SHARDS, K_DEC_RECON, K_DEC_RECON_WIDE, K_DEC_RECON_SERIAL, K_RESULTS,
-  K_DEC_RANS, K_DEC_OTHER, K_COUNT
+  K_DEC_RANS, K_DEC_OTHER, K_ENC_LOSSLESS, K_COUNT
 };
 const char* const kKernelNames[K_COUNT] = {
     "enc_init", "enc_predict", "enc_predict_wide", "enc_analyze", "enc_rans", "enc_scan", "enc_prefix",
     "enc_emit", "dec_parse", "dec_rans_tables", "dec_reconstruct", "dec_reconstruct_wide",
-    "dec_reconstruct_serial", "results", "dec_rans", "dec_other"};
+    "dec_reconstruct_serial", "results", "dec_rans", "dec_other", "enc_lossless"};
 constexpr int kGroupShards = 8;
 
 std::atomic<int64_t> g_launches{0};
@@ -315,6 +315,7 @@ struct Totals {
   int64_t tiles = 0, shards = 0, samples = 0, prefix = 0;
   bool wide = false;
   bool fold16 = true;  // folded symbols held as u16 (every frame below depth 16 or quality 100)
+  bool lossless = false, lossy = false;  // has frames of step 1, of larger steps (a bucket: may have)
   int passes = 1;
   // frames, tiles and shards that take part in pass p; the encoder lays the
   // batch out with frames of more passes first, so these are prefixes
@@ -343,6 +344,7 @@ Totals totals_of(const fvb_frame* frames, int n) {
     const int64_t ptw0 = f.tile_w;
     if (ptw0 > kFastMaxW) t.wide = true;
     if (f.bit_depth >= 16 && f.quality >= 100) t.fold16 = false;
+    (f.step == 1 ? t.lossless : t.lossy) = true;
     const int passes = frame_passes(f);
     if (passes > t.passes) t.passes = passes;
     for (int p = 0; p < passes; ++p) {
@@ -466,6 +468,7 @@ int from_bucket(const fvb_bucket* b, Totals* t) {
   t->passes = b->passes;
   t->wide = b->wide != 0;
   t->fold16 = b->fold16 != 0;
+  t->lossless = t->lossy = true;
   return FVB_OK;
 }
 
@@ -646,7 +649,7 @@ constexpr int kDefaultCtas[K_COUNT] = {
     /*enc_init*/ 0, /*enc_predict*/ 4, /*enc_predict_wide*/ 8, /*enc_analyze*/ 6, /*enc_rans*/ 0,
     /*enc_scan*/ 0, /*enc_prefix*/ 0, /*enc_emit*/ 8, /*dec_parse*/ 8, /*dec_rans_tables*/ 16,
     /*dec_reconstruct*/ 4, /*dec_reconstruct_wide*/ 8, /*dec_reconstruct_serial*/ 0, /*results*/ 0,
-    /*dec_rans*/ 16, /*dec_other*/ 16};
+    /*dec_rans*/ 16, /*dec_other*/ 16, /*enc_lossless*/ 0};
 std::atomic<int> g_ctas[K_COUNT];
 std::atomic<int> g_wavefront_block{kDefaultWavefrontBlock};
 std::atomic<int> g_decode_overlap{1};
@@ -671,11 +674,6 @@ std::atomic<int> g_tile_warps{kDefaultTileWarps};
 // many shards at once).
 constexpr int kSlotCtasPerSm = 6;
 bool few_rans_shards(int64_t shards) { return shards <= static_cast<int64_t>(device_sms()) * kSlotCtasPerSm * 2; }
-
-// Whether a wavefront launch has too few tiles to hide its step chain behind
-// other warps.
-constexpr int kFewTilesPerSm = 8;
-bool few_tiles(int64_t tiles) { return tiles <= static_cast<int64_t>(device_sms()) * kFewTilesPerSm; }
 
 int ctas(int kernel) {
   const int v = g_ctas[kernel].load(std::memory_order_relaxed);
@@ -951,16 +949,26 @@ int encode_enqueue(const Totals& cap, void* workspace, int64_t workspace_bytes, 
     void* folded = ws + (pass ? L.folded_b : L.folded);
     uint8_t* rans = reinterpret_cast<uint8_t*>(ws + (pass ? L.rans_b : L.rans));
     uint8_t* prefix = reinterpret_cast<uint8_t*>(ws + (pass ? L.prefix_b : L.prefix));
-    FVB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), stream));
-    {
-      LaunchScope scope_(K_ENC_PREDICT, stream);
-      const int tw = g_tile_warps.load(std::memory_order_relaxed);
-      enc_predict_launch(g_wavefront_block.load(std::memory_order_relaxed), tw, f16,
-                         grid_for(tiles * tw, kWarpsPerCta, ctas(K_ENC_PREDICT)), stream, frames_d, state, dims, pass,
-                         shards, folded, queue);
+    if (pass == 0 && cap.lossless) {
+      {
+        LaunchScope scope_(K_ENC_LOSSLESS, stream);
+        enc_lossless_launch(f16, tiles, device_sms() * 12, stream, frames_d, state, dims, shards, folded);
+      }
+      FVB_LAUNCHED("enc_lossless_kernel");
     }
-    FVB_LAUNCHED("enc_predict_kernel");
-    if (cap.wide) {
+    if (cap.lossy) {
+      FVB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), stream));
+      {
+        LaunchScope scope_(K_ENC_PREDICT, stream);
+        const int tw = g_tile_warps.load(std::memory_order_relaxed);
+        // u16: one CTA per tile until the cap, as dec_reconstruct
+        const int grid = grid_for(f16 ? tiles : tiles * tw, f16 ? 1 : kWarpsPerCta, ctas(K_ENC_PREDICT));
+        enc_predict_launch(g_wavefront_block.load(std::memory_order_relaxed), tw, f16, grid, stream,
+                           frames_d, state, dims, pass, shards, folded, queue);
+      }
+      FVB_LAUNCHED("enc_predict_kernel");
+    }
+    if (cap.wide && cap.lossy) {
       {
         LaunchScope scope_(K_ENC_PREDICT_WIDE, stream);
         enc_predict_wide_kernel<<<grid_for(tiles, 1, ctas(K_ENC_PREDICT_WIDE)), 256, 0, stream>>>(
@@ -1376,8 +1384,8 @@ int decode_enqueue(const Totals& t, int wavefront, void* workspace, int64_t work
       // u16: one CTA per tile until the cap, so that few tiles spread over
       // the SMs; the warps take tiles from the queue
       const int grid = grid_for(f16 ? t.tiles : t.tiles * tw, f16 ? 1 : kWarpsPerCta, ctas(K_DEC_RECON));
-      dec_reconstruct_launch(g_wavefront_block.load(std::memory_order_relaxed), tw, f16, few_tiles(t.tiles), grid,
-                             stream, frames_d, state, dims, folded, queue);
+      dec_reconstruct_launch(g_wavefront_block.load(std::memory_order_relaxed), tw, f16, grid, stream,
+                             frames_d, state, dims, folded, queue);
     }
     FVB_LAUNCHED("dec_reconstruct_kernel");
     if (t.wide) {

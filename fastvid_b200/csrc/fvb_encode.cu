@@ -15,6 +15,7 @@
 // Nothing here traps; every failure is a status word.
 #include "fvb_common.cuh"
 #include "fvb_kernels.cuh"
+#include "fvb_wave.cuh"
 
 namespace fvb {
 
@@ -61,7 +62,7 @@ struct EncWarpSmem {
   uint16_t carry[kFastMaxW + 128];  // row above the band, column c at index c + 32
 };
 
-template <bool MED, bool STEP1, bool EDGE, int UNROLL, bool SPLIT, typename FoldT>
+template <bool MED, bool EDGE, int UNROLL, bool SPLIT, typename FoldT>
 __device__ __forceinline__ void enc_block(EncWarpSmem<FoldT>& sm, const uint16_t* carry_in, uint16_t* carry_out, int lane,
                                           int t0, int W, int32_t maxs, int32_t step, int32_t half, uint32_t magic,
                                           bool band0, int32_t& rec, int32_t& a_prev) {
@@ -78,15 +79,9 @@ __device__ __forceinline__ void enc_block(EncWarpSmem<FoldT>& sm, const uint16_t
     if (lane == 0) a = band0 ? 0 : above0;
     const int32_t pred = MED ? predict_med(rec, a, a_prev) : predict_grad(rec, a, a_prev, maxs);
     const int32_t res = s - pred;
-    int32_t q, rn;
-    if (STEP1) {
-      q = res;
-      rn = min(s, maxs);
-    } else {
-      const int32_t mag = static_cast<int32_t>(__umulhi(static_cast<uint32_t>(abs(res) + half), magic));
-      q = res < 0 ? -mag : mag;
-      rn = max(0, min(maxs, pred + q * step));
-    }
+    const int32_t mag = static_cast<int32_t>(__umulhi(static_cast<uint32_t>(abs(res) + half), magic));
+    const int32_t q = res < 0 ? -mag : mag;
+    int32_t rn = max(0, min(maxs, pred + q * step));
     if (EDGE) {
       const int c = t0 + u - lane;
       if (c < 0) rn = 0;  // left of the tile: zero left/upper-left for column 0
@@ -105,7 +100,7 @@ __device__ __forceinline__ void enc_block(EncWarpSmem<FoldT>& sm, const uint16_t
 // source chunks, block(k) runs wavefront block k (staging the chunk ahead
 // and flushing the folded residuals two chunks behind), end() flushes the
 // rest.  vmax tracks the largest source sample read (the depth check).
-template <bool MED, bool STEP1, int UNROLL, bool SPLIT, typename FoldT>
+template <bool MED, int UNROLL, bool SPLIT, typename FoldT>
 struct EncBand {
   static constexpr int kFS = EncWarpSmem<FoldT>::kFS;
   EncWarpSmem<FoldT>& sm;
@@ -190,10 +185,10 @@ struct EncBand {
     }
     const int t0 = blk * 32;
     if (t0 < 31 || t0 + 31 >= W)
-      enc_block<MED, STEP1, true, UNROLL, SPLIT, FoldT>(sm, carry_in, carry_out, lane, t0, W, maxs, step, half, magic, band0, rec,
+      enc_block<MED, true, UNROLL, SPLIT, FoldT>(sm, carry_in, carry_out, lane, t0, W, maxs, step, half, magic, band0, rec,
                                           a_prev);
     else
-      enc_block<MED, STEP1, false, UNROLL, SPLIT, FoldT>(sm, carry_in, carry_out, lane, t0, W, maxs, step, half, magic, band0, rec,
+      enc_block<MED, false, UNROLL, SPLIT, FoldT>(sm, carry_in, carry_out, lane, t0, W, maxs, step, half, magic, band0, rec,
                                            a_prev);
   }
   __device__ void end() {
@@ -206,7 +201,7 @@ struct EncBand {
 // A tile by one warp: bands in order, one carry row (read by lane 0 before
 // lane 31 overwrites it).  Kept apart from EncBand: written as one loop nest
 // it needs no register spills.
-template <bool MED, bool STEP1, int UNROLL, typename FoldT>
+template <bool MED, int UNROLL, typename FoldT>
 __device__ void enc_tile_fast(const FrameDesc& f, const TileGeo& g, int32_t step, uint32_t magic,
                               FoldT* __restrict__ folded_tile, EncWarpSmem<FoldT>& sm, int lane, int32_t& bad) {
   constexpr int kFS = EncWarpSmem<FoldT>::kFS;
@@ -272,10 +267,10 @@ __device__ void enc_tile_fast(const FrameDesc& f, const TileGeo& g, int32_t step
       const int t0 = blk * 32;
       const bool edge = t0 < 31 || t0 + 31 >= W;
       if (edge)
-        enc_block<MED, STEP1, true, UNROLL, false, FoldT>(sm, sm.carry, sm.carry, lane, t0, W, maxs, step, half, magic, band0,
+        enc_block<MED, true, UNROLL, false, FoldT>(sm, sm.carry, sm.carry, lane, t0, W, maxs, step, half, magic, band0,
                                                    rec, a_prev);
       else
-        enc_block<MED, STEP1, false, UNROLL, false, FoldT>(sm, sm.carry, sm.carry, lane, t0, W, maxs, step, half, magic,
+        enc_block<MED, false, UNROLL, false, FoldT>(sm, sm.carry, sm.carry, lane, t0, W, maxs, step, half, magic,
                                                     band0, rec, a_prev);
     }
     __syncwarp();
@@ -290,7 +285,7 @@ __device__ __forceinline__ void enc_pair_sync(int pair) {
   asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
 }
 
-template <bool MED, bool STEP1, int UNROLL, bool PAIRS, typename FoldT>
+template <bool MED, int UNROLL, bool PAIRS, typename FoldT>
 __device__ void enc_tile(const FrameDesc& f, const TileGeo& g, int32_t step, uint32_t magic,
                          FoldT* __restrict__ folded_tile, EncWarpSmem<FoldT>* smw, int warp, int lane,
                          int32_t& bad) {
@@ -301,7 +296,7 @@ __device__ void enc_tile(const FrameDesc& f, const TileGeo& g, int32_t step, uin
       // schedule of dec_reconstruct)
       const int pw = warp & 1;
       EncWarpSmem<FoldT>& sm = smw[warp];
-      EncBand<MED, STEP1, UNROLL, true, FoldT> eb(f, g, step, magic, folded_tile, sm, lane);
+      EncBand<MED, UNROLL, true, FoldT> eb(f, g, step, magic, folded_tile, sm, lane);
       const int n = eb.nblocks, nbands = (g.h + 31) >> 5;
       const int own = pw ? (nbands / 2) * n : ((nbands + 1) / 2) * n;
       const int slots = max(((nbands + 1) / 2) * n, (nbands / 2) * n + 2);
@@ -320,8 +315,26 @@ __device__ void enc_tile(const FrameDesc& f, const TileGeo& g, int32_t step, uin
     }
     if (warp & 1) return;  // too small to split: the pair's first warp alone
   }
-  enc_tile_fast<MED, STEP1, UNROLL, FoldT>(f, g, step, magic, folded_tile, smw[warp], lane, bad);
+  enc_tile_fast<MED, UNROLL, FoldT>(f, g, step, magic, folded_tile, smw[warp], lane, bad);
 }
+
+// Shard records of a tile (encode.cu:753-759), written for every frame of the
+// pass, active or not: the later passes write a region of their own, and the
+// analysis kernels read every record of the pass (frame index first) before
+// they skip inactive frames.
+__device__ __forceinline__ void write_shard_records(const FrameDesc& f, const TileGeo& g, int fi,
+                                                    ShardInfo* __restrict__ shards, int lane) {
+  for (int j = lane; j < g.shard_count; j += 32) {
+    ShardInfo& si = shards[f.shard_base + g.first_shard + j];
+    const int64_t local = static_cast<int64_t>(j) * kShardSymbols;
+    si.sample_base = f.sample_base + g.sample_base + local;
+    si.count = static_cast<int32_t>(min(static_cast<int64_t>(kShardSymbols), static_cast<int64_t>(g.w) * g.h - local));
+    si.frame = fi;
+  }
+}
+
+// A frame with a quality step of 1 is lossless in its only pass.
+__device__ __forceinline__ bool frame_lossless(const FrameDesc& f) { return f.step0 == 1; }
 
 // Tiles come from a queue; with warp pairs the pair's first warp claims a
 // tile and both read it after the pair barrier (two alternating slots), and
@@ -354,20 +367,9 @@ enc_predict_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict_
     const FrameDesc& f = frames[fi];
     FrameState& st = state[fi];
     const TileGeo g = tile_geo(f, t - f.tile_base);
-    // shard records of this tile (encode.cu:753-759), written for every
-    // frame of the pass, active or not: the later passes write a region of
-    // their own, and the analysis kernels read every record of the pass
-    // (frame index first) before they skip inactive frames; with pairs the
-    // first warp writes them
-    if (!pairs || (warp & 1) == 0) {
-      for (int j = lane; j < g.shard_count; j += 32) {
-        ShardInfo& si = shards[f.shard_base + g.first_shard + j];
-        const int64_t local = static_cast<int64_t>(j) * kShardSymbols;
-        si.sample_base = f.sample_base + g.sample_base + local;
-        si.count = static_cast<int32_t>(min(static_cast<int64_t>(kShardSymbols), static_cast<int64_t>(g.w) * g.h - local));
-        si.frame = fi;
-      }
-    }
+    // with pairs the first warp writes the records
+    if (frame_lossless(f)) continue;  // enc_lossless_kernel's
+    if (!pairs || (warp & 1) == 0) write_shard_records(f, g, fi, shards, lane);
     if (!st.active) continue;
     if (g.w > kFastMaxW) continue;  // wide tiles go through enc_predict_wide_kernel
     const int32_t step = st.step;
@@ -375,20 +377,405 @@ enc_predict_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict_
     FoldT* ftile = folded + f.sample_base + g.sample_base;
     int32_t bad = 0;
     const bool med = st.use_med != 0;
-    if (med) {
-      if (step == 1) enc_tile<true, true, UNROLL, PAIRS, FoldT>(f, g, step, magic, ftile, smw, warp, lane, bad);
-      else enc_tile<true, false, UNROLL, PAIRS, FoldT>(f, g, step, magic, ftile, smw, warp, lane, bad);
+    if (med) enc_tile<true, UNROLL, PAIRS, FoldT>(f, g, step, magic, ftile, smw, warp, lane, bad);
+    else enc_tile<false, UNROLL, PAIRS, FoldT>(f, g, step, magic, ftile, smw, warp, lane, bad);
+    if (__any_sync(kFull, bad) && lane == 0) set_status(&st.status, 1);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// enc_predict on u16 symbols (every batch without a lossless 16-bit frame):
+// the two-rows-per-lane wavefront of fvb_wave.cuh, symbols written over the
+// samples they came from.
+//
+// Up to depth 12 a step works on both rows at once in packed 16-bit halves.
+// The quantizer's q = sign(res) floor((|res| + half) / step) becomes one
+// floored division of a non-negative number: with K so large that
+// n = res + half + K step is positive, floor(n / step) = q + K for every res of
+// an odd step; of an even step's ties, half-way cases round away from zero, so
+// negative residuals take one less (bit 13 of res + 8192 tells the sign).  The
+// division of the low half is div_step; that of the high half is the upper half
+// of umulhi(n, magic) on the packed word: the low half adds less than a quarter
+// to the dividend and the reciprocal's excess less than 2^-18 to the quotient,
+// which cannot carry it past the next multiple of the step.
+//
+// Bound by issue, 41 instructions for a step of 64 samples (the 32-bit sweep of
+// 32-row bands took about 30 for 32), and with few tiles by the chain of a step
+// in a lone warp: 24 4K yuv422-10 frames 830 -> 593 us, a 1080p rgb8 frame
+// 85 -> 60 us, a 4K gray16 frame's two passes 103 -> 76 us.
+struct PackedQuant {
+  uint32_t magic, step, even, add, back, twice, maxs2;
+  __device__ PackedQuant(int32_t maxs, int32_t st, uint32_t magic_) : magic(magic_), step(st) {
+    const int32_t half = st >> 1, k = (8193 + st) / st;  // half + K step >= 8193
+    even = (st & 1) ? 0u : 0x00010001u;
+    add = pair2(half + k * st - 8192 - (st & 1 ? 0 : 1));
+    back = pair2(-k * st);
+    twice = pair2(-2 * k);
+    maxs2 = pair2(maxs);
+  }
+  // samples s, prediction p: reconstruction and zigzag-folded symbol
+  __device__ __forceinline__ void operator()(uint32_t s, uint32_t p, uint32_t& rec, uint32_t& sym) const {
+    const uint32_t r = s + 0x20002000u - p;  // residual + 8192
+    const uint32_t n = r + ((r >> 13) & even) + add;
+    const uint32_t q = __byte_perm(__umulhi(n & 0xffffu, magic), __umulhi(n, magic), 0x7610);  // q + K
+    rec = __viaddmin_s16x2_relu(q * step + p, back, maxs2);
+    const uint32_t t = __vadd2(q + q, twice);
+    sym = __vmaxs2(t, ~t);  // max(2 q, -2 q - 1)
+  }
+};
+
+template <bool MED, bool O1>
+__device__ __forceinline__ void enc_wave_steps(WavePacked& st, uint32_t& sym, uint32_t& vmax,
+                                               WaveBlock<O1>& blk, int g, const WaveWords<false>& x,
+                                               const WaveWords<O1>& y, const WaveCarry& c, const PackedQuant& quant) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t s = wave_pack(x, y, j);
+    vmax = __vmaxu2(vmax, s);
+    const uint32_t a = st.neighbours(c.up[j >> 1], j & 1, blk.lane);
+    const uint32_t p = st.template predict<MED>(a, quant.maxs2);
+    uint32_t rn, z;
+    quant(s, p, rn, z);
+    blk.put(g, j, sym, z, st.rec, rn);
+    sym = z;
+    st.above = a;
+    st.rec = rn;
+  }
+}
+
+struct WideQuant {
+  int32_t maxs, step, half;
+  uint32_t magic;
+  __device__ WideQuant(int32_t maxs_, int32_t st, uint32_t magic_)
+      : maxs(maxs_), step(st), half(st >> 1), magic(magic_) {}
+  __device__ __forceinline__ void operator()(int32_t s, int32_t p, int32_t& rec, uint32_t& sym) const {
+    const int32_t res = s - p;
+    const int32_t mag = div_step(static_cast<uint32_t>(abs(res) + half), magic);
+    const int32_t q = res < 0 ? -mag : mag;
+    rec = __viaddmin_s32_relu(p, q * step, maxs);
+    sym = zigzag(q);
+  }
+};
+
+template <bool MED, bool O1>
+__device__ __forceinline__ void enc_wave_steps(WaveWide& st, uint32_t& sym, uint32_t&, WaveBlock<O1>& blk,
+                                               int g, const WaveWords<false>& x, const WaveWords<O1>& y,
+                                               const WaveCarry& c, const WideQuant& quant) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    int32_t a0, a1;
+    st.neighbours(c.up[j >> 1], j & 1, blk.lane, a0, a1);
+    const uint32_t was = st.packed();
+    const int32_t p0 = st.template predict<MED>(st.rec0, a0, st.above0, quant.maxs);
+    const int32_t p1 = st.template predict<MED>(st.rec1, a1, st.above1, quant.maxs);
+    uint32_t z0, z1;
+    quant(static_cast<int32_t>(x.sample(j)), p0, st.rec0, z0);
+    quant(static_cast<int32_t>(y.sample(j)), p1, st.rec1, z1);
+    st.above0 = a0;
+    st.above1 = a1;
+    const uint32_t z = __byte_perm(z0, z1, 0x5410);
+    blk.put(g, j, sym, z, was, st.packed());
+    sym = z;
+  }
+}
+
+// One window block (as rec_wave_block).
+template <bool MED, bool O1, typename St, typename Quant>
+__device__ __forceinline__ void enc_wave_block(St& st, uint32_t& sym, uint32_t& vmax, WaveBlock<O1> blk,
+                                               const Quant& quant) {
+  WaveWords<false> x, xn;
+  WaveWords<O1> y, yn;
+  WaveCarry c, cn;
+  x.first(blk.p0);
+  y.first(blk.p1);
+  x.load(blk.p0, 0);
+  y.load(blk.p1, 0);
+  c.load(blk.crow, 0);
+#pragma unroll 1
+  for (int g = 0; g < 4; g += 2) {
+    xn.after(x);
+    yn.after(y);
+    xn.load(blk.p0, g + 1);
+    yn.load(blk.p1, g + 1);
+    cn.load(blk.crow, g + 1);
+    enc_wave_steps<MED>(st, sym, vmax, blk, g, x, y, c, quant);
+    x.after(xn);
+    y.after(yn);
+    if (g == 0) {
+      x.load(blk.p0, 2);
+      y.load(blk.p1, 2);
+      c.load(blk.crow, 2);
+    }
+    enc_wave_steps<MED>(st, sym, vmax, blk, g + 1, xn, yn, cn, quant);
+  }
+  blk.finish(sym, st.packed());
+}
+
+template <bool MED, bool WIDE, bool O1>
+__device__ void enc_wave_tile(const FrameDesc& f, const TileGeo& g, int32_t step, uint32_t magic,
+                              uint16_t* __restrict__ ftile, WaveSm& sm, int lane, int32_t& bad) {
+  for (int i = lane; i < kCarryCols / 8; i += 32) reinterpret_cast<uint4*>(sm.carry)[i] = make_uint4(0, 0, 0, 0);
+  __syncwarp();
+  const uint16_t* plane = f.src[g.plane];
+  const int64_t pitch = f.src_pitch[g.plane];
+  const std::conditional_t<WIDE, WideQuant, PackedQuant> quant(f.max_sample, step, magic);
+  WaveIo<true> io(sm, lane, g.w, plane + static_cast<int64_t>(g.y) * pitch + g.x, pitch, ftile, g.w, plane,
+                      plane + static_cast<int64_t>(f.height - 1) * pitch + f.plane_w[g.plane]);
+  uint32_t vmax = 0;
+  for (int y = 0; y < g.h; y += kBandRows, io.next_band()) {
+    io.band(g.h - y);
+    io.fetch(0);
+    std::conditional_t<WIDE, WaveWide, WavePacked> st;
+    uint32_t sym = 0;
+    for (int b = 0; b < io.nblk; ++b) {
+      if (b) {
+        io.flush(b - 1);
+        io.move_head(b);
+        __syncwarp();
+      }
+      if (b + 1 < io.nblk) io.fetch(b + 1);
+      else cp_async_commit();
+      io.wait();
+      io.template fix_edge<true>(b);
+      enc_wave_block<MED, O1>(st, sym, vmax, WaveBlock<O1>(sm, b, lane, io.off0, io.off1), quant);
+      __syncwarp();
+    }
+    io.flush_last();
+    __syncwarp();
+  }
+  if (!WIDE && max(vmax & 0xffffu, vmax >> 16) > static_cast<uint32_t>(f.max_sample)) bad = 1;
+}
+
+template <bool MED, bool WIDE>
+__device__ void enc_wave_any(const FrameDesc& f, const TileGeo& g, int32_t step, uint32_t magic,
+                             uint16_t* __restrict__ ftile, WaveSm& sm, int lane, int32_t& bad) {
+  if (f.src_pitch[g.plane] & 1) enc_wave_tile<MED, WIDE, false>(f, g, step, magic, ftile, sm, lane, bad);
+  else enc_wave_tile<MED, WIDE, true>(f, g, step, magic, ftile, sm, lane, bad);
+}
+
+__global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
+enc_predict_wave_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
+                        const BatchDims* __restrict__ dims, int pass, ShardInfo* __restrict__ shards,
+                        uint16_t* __restrict__ folded, int* __restrict__ queue) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int nframes = dims->frames_p[pass];
+  const int64_t total_tiles = dims->tiles_p[pass];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  WaveSm& sm = reinterpret_cast<WaveSm*>(smem_raw)[warp];
+  // tiles by place first, then from the queue (as dec_reconstruct_wave_kernel)
+  const int64_t warps_total = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
+  for (int64_t t = static_cast<int64_t>(warp) * gridDim.x + blockIdx.x; t < total_tiles;) {
+    const int64_t mine = t;
+    if (lane == 0) t = warps_total + atomicAdd(queue, 1);
+    t = __shfl_sync(kFull, t, 0);
+    const int fi = frame_of_tile(frames, nframes, mine);
+    const FrameDesc& f = frames[fi];
+    FrameState& st = state[fi];
+    if (frame_lossless(f)) continue;  // enc_lossless_kernel's
+    const TileGeo g = tile_geo(f, mine - f.tile_base);
+    write_shard_records(f, g, fi, shards, lane);
+    if (!st.active || g.w > kFastMaxW) continue;  // wide tiles go through enc_predict_wide_kernel
+    const int32_t step = st.step;
+    const uint32_t magic = static_cast<uint32_t>((0x100000000ull + step - 1) / step);
+    uint16_t* ftile = folded + f.sample_base + g.sample_base;
+    int32_t bad = 0;
+    const bool wide = f.bit_depth > 12;
+    if (st.use_med) {
+      if (wide) enc_wave_any<true, true>(f, g, step, magic, ftile, sm, lane, bad);
+      else enc_wave_any<true, false>(f, g, step, magic, ftile, sm, lane, bad);
     } else {
-      if (step == 1) enc_tile<false, true, UNROLL, PAIRS, FoldT>(f, g, step, magic, ftile, smw, warp, lane, bad);
-      else enc_tile<false, false, UNROLL, PAIRS, FoldT>(f, g, step, magic, ftile, smw, warp, lane, bad);
+      if (wide) enc_wave_any<false, true>(f, g, step, magic, ftile, sm, lane, bad);
+      else enc_wave_any<false, false>(f, g, step, magic, ftile, sm, lane, bad);
     }
     if (__any_sync(kFull, bad) && lane == 0) set_status(&st.status, 1);
   }
 }
 
-// The wavefront block of enc_predict -- steps of each 32-step block unrolled
-// -- is a launch-time choice (4, 8, 16 or 32; the autotuner's knob): every
-// choice computes the same bytes.
+// ---------------------------------------------------------------------------
+// enc_lossless: frames with a step of 1.  Their reconstruction is the source,
+// so every residual can be computed from the samples around it and there is no
+// wavefront: a warp takes 16 rows of a tile, eight columns a lane (rows of
+// fewer than 256 columns side by side), and walks down with the row above in
+// registers.  A 320x180 gray8 frame, four tiles, took 62 us in the wavefront
+// (one warp a tile) and takes 6 us; a 720p frame 15 us and 4 us.
+constexpr int kSlabRows = 16;
+
+// Eight samples of a row, packed, zero outside [0, n).
+__device__ __forceinline__ uint4 load8(const uint16_t* __restrict__ p, int n) {
+  if (n >= 8 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) return __ldg(reinterpret_cast<const uint4*>(p));
+  uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    if (e < n) w[e >> 1] |= static_cast<uint32_t>(__ldg(p + e)) << (16 * (e & 1));
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+template <typename FoldT>
+__device__ __forceinline__ void store8(FoldT* __restrict__ p, const uint32_t (&z)[8], int n) {
+  if (n >= 8 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+    uint4* o = reinterpret_cast<uint4*>(p);
+    if constexpr (sizeof(FoldT) == 2) {
+      o[0] = make_uint4(z[0] | (z[1] << 16), z[2] | (z[3] << 16), z[4] | (z[5] << 16), z[6] | (z[7] << 16));
+    } else {
+      o[0] = make_uint4(z[0], z[1], z[2], z[3]);
+      o[1] = make_uint4(z[4], z[5], z[6], z[7]);
+    }
+    return;
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    if (e < n) p[e] = static_cast<FoldT>(z[e]);
+}
+
+// left: the sample before the eight (high half), above / corner: the row above
+// and the sample before it (high half)
+template <bool MED, bool WIDE>
+__device__ __forceinline__ void fold8(const uint4& v, uint32_t left, const uint4& above, uint32_t corner, int32_t maxs,
+                                      uint32_t (&z)[8]) {
+  const uint32_t s[4] = {v.x, v.y, v.z, v.w}, a[4] = {above.x, above.y, above.z, above.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t l = __byte_perm(i ? s[i - 1] : left, s[i], 0x5432);
+    const uint32_t ul = __byte_perm(i ? a[i - 1] : corner, a[i], 0x5432);
+    if constexpr (WIDE) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int32_t lv = h ? l >> 16 : l & 0xffffu, av = h ? a[i] >> 16 : a[i] & 0xffffu;
+        const int32_t uv = h ? ul >> 16 : ul & 0xffffu, sv = h ? s[i] >> 16 : s[i] & 0xffffu;
+        z[2 * i + h] = zigzag(sv - (MED ? predict_med(lv, av, uv) : predict_grad(lv, av, uv, maxs)));
+      }
+    } else {
+      const uint32_t d = sub2(a[i], ul);
+      const uint32_t p = MED ? __vmaxs2(__vmins2(l, a[i]), __viaddmin_s16x2(l, d, __vmaxs2(l, a[i])))
+                             : __viaddmin_s16x2_relu(l, d, pair2(maxs));
+      const uint32_t r = sub2(s[i], p), t = __vadd2(r, r);
+      const uint32_t w = __vmaxs2(t, ~t);  // max(2 r, -2 r - 1)
+      z[2 * i] = w & 0xffffu;
+      z[2 * i + 1] = w >> 16;
+    }
+  }
+}
+
+template <bool MED, bool WIDE, typename FoldT>
+__device__ void lossless_slab(const FrameDesc& f, const TileGeo& g, int y0, FoldT* __restrict__ ftile, int lane,
+                              int32_t& bad) {
+  const uint16_t* __restrict__ plane = f.src[g.plane];
+  const int64_t pitch = f.src_pitch[g.plane];
+  const uint16_t* __restrict__ tile = plane + static_cast<int64_t>(g.y) * pitch + g.x;
+  const int W = g.w, rows = min(kSlabRows, g.h - y0);
+  int per = 32;  // lanes of a row
+  while (per > 1 && 4 * per >= W) per >>= 1;
+  const int strips = 32 / per, cl = lane & (per - 1);
+  const int height = (rows + strips - 1) / strips;  // rows of a strip
+  const int ya = y0 + lane / per * height, yb = min(ya + height, y0 + rows);
+  uint32_t vmax = 0;
+  for (int c0 = 0; c0 < W; c0 += 8 * per) {
+    const int c = c0 + 8 * cl, n = W - c;
+    auto row = [&](int y) { return load8(tile + y * pitch + c, y < yb ? n : 0); };
+    // the sample before a row's eight: from the lane before, the first lane's
+    // from memory
+    auto before = [&](const uint4& v, int y) {
+      uint32_t l = __shfl_up_sync(kFull, v.w, 1, per);
+      if (cl == 0) l = (c > 0 && y >= 0 && y < yb) ? static_cast<uint32_t>(__ldg(tile + y * pitch + c - 1)) << 16 : 0u;
+      return l;
+    };
+    const bool first = ya >= yb || ya == 0;
+    uint4 above = load8(tile + (ya - (first ? 0 : 1)) * pitch + c, first ? 0 : n);
+    uint32_t corner = before(above, first ? -1 : ya - 1);
+    constexpr int kAhead = 4;
+    for (int y = 0; y < height; y += kAhead) {
+      uint4 v[kAhead];
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) v[i] = row(y + i < height ? ya + y + i : yb);
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        const int at = y + i < height ? ya + y + i : yb;
+        const uint32_t left = before(v[i], at);
+        uint32_t z[8];
+        fold8<MED, WIDE>(v[i], left, above, corner, f.max_sample, z);
+        if (at < yb) store8(ftile + static_cast<int64_t>(at) * W + c, z, n);
+        vmax = __vmaxu2(vmax, __vmaxu2(__vmaxu2(v[i].x, v[i].y), __vmaxu2(v[i].z, v[i].w)));
+        above = v[i];
+        corner = left;
+      }
+    }
+  }
+  if (max(vmax & 0xffffu, vmax >> 16) > static_cast<uint32_t>(f.max_sample)) bad = 1;
+}
+
+// Work items: eight slabs a tile (a taller tile's later slabs go round).
+constexpr int kSlabs = 8;
+
+template <typename FoldT>
+__global__ void __launch_bounds__(128)
+enc_lossless_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
+                    const BatchDims* __restrict__ dims, ShardInfo* __restrict__ shards,
+                    FoldT* __restrict__ folded) {
+  const int nframes = dims->frames_p[0];
+  const int64_t items = dims->tiles_p[0] * kSlabs;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the lossless frames (bit per frame, the first kMaskFrames frames; later
+  // ones count as lossless until their own step is read)
+  constexpr int kMaskFrames = 4096;
+  __shared__ uint32_t mask[kMaskFrames / 32];
+  const int words = min((nframes + 31) / 32, kMaskFrames / 32);
+  int any = nframes > kMaskFrames;
+  for (int w = warp; w < words; w += 4) {
+    const int k = w * 32 + lane;
+    const uint32_t m = __ballot_sync(kFull, k < nframes && frame_lossless(frames[k]));
+    if (lane == 0) mask[w] = m;
+    any |= m != 0;
+  }
+  if (!__syncthreads_or(any)) return;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * 4;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * 4 + warp; i < items; i += stride) {
+    const int64_t t = i / kSlabs;
+    const int fi = frame_of_tile(frames, nframes, t);
+    const FrameDesc& f = frames[fi];
+    if (!frame_lossless(f)) {  // on to this warp's first item in a lossless frame
+      int next = fi + 1;
+      if (next < kMaskFrames) {
+        int w = next >> 5;
+        uint32_t m = w < words ? mask[w] >> (next & 31) << (next & 31) : 0u;
+        while (!m && ++w < words) m = mask[w];
+        next = m ? 32 * w + __ffs(m) - 1 : kMaskFrames;
+      }
+      if (next >= nframes) break;
+      i += (frames[next].tile_base * kSlabs - i - 1) / stride * stride;
+      continue;
+    }
+    const TileGeo g = tile_geo(f, t - f.tile_base);
+    if (i == t * kSlabs) write_shard_records(f, g, fi, shards, lane);
+    FoldT* ftile = folded + f.sample_base + g.sample_base;
+    int32_t bad = 0;
+    for (int y0 = static_cast<int>(i - t * kSlabs) * kSlabRows; y0 < g.h; y0 += kSlabs * kSlabRows) {
+      if (f.bit_depth > 12) {
+        if (f.use_med0) lossless_slab<true, true>(f, g, y0, ftile, lane, bad);
+        else lossless_slab<false, true>(f, g, y0, ftile, lane, bad);
+      } else {
+        if (f.use_med0) lossless_slab<true, false>(f, g, y0, ftile, lane, bad);
+        else lossless_slab<false, false>(f, g, y0, ftile, lane, bad);
+      }
+    }
+    if (__any_sync(kFull, bad) && lane == 0) set_status(&state[fi].status, 1);
+  }
+}
+
+void enc_lossless_launch(bool fold16, int64_t tiles, int max_ctas, cudaStream_t stream, const FrameDesc* frames,
+                         FrameState* state, const BatchDims* dims, ShardInfo* shards, void* folded) {
+  const int64_t want = (tiles * kSlabs + 3) / 4;
+  const int grid = static_cast<int>(want < max_ctas ? (want > 0 ? want : 1) : max_ctas);
+  if (fold16)
+    enc_lossless_kernel<uint16_t><<<grid, 128, 0, stream>>>(frames, state, dims, shards,
+                                                            static_cast<uint16_t*>(folded));
+  else
+    enc_lossless_kernel<uint32_t><<<grid, 128, 0, stream>>>(frames, state, dims, shards,
+                                                            static_cast<uint32_t*>(folded));
+}
+
+// The wavefront block of the u32 enc_predict -- steps of each 32-step block
+// unrolled -- is a launch-time choice (4, 8, 16 or 32; the autotuner's knob),
+// as are its warps per tile: every choice computes the same bytes.
 cudaError_t enc_predict_set_smem() {
   const int b32 = static_cast<int>(enc_predict_smem(false)), b16 = static_cast<int>(enc_predict_smem(true));
   for (auto k : {enc_predict_kernel<4, false, uint32_t>, enc_predict_kernel<8, false, uint32_t>,
@@ -397,36 +784,25 @@ cudaError_t enc_predict_set_smem() {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, b32);
     if (e != cudaSuccess) return e;
   }
-  for (auto k : {enc_predict_kernel<4, false, uint16_t>, enc_predict_kernel<8, false, uint16_t>,
-                 enc_predict_kernel<16, false, uint16_t>, enc_predict_kernel<32, false, uint16_t>,
-                 enc_predict_kernel<8, true, uint16_t>}) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, b16);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
-
-template <typename FoldT>
-void enc_predict_launch_t(int unroll, int tile_warps, int grid, cudaStream_t stream, const FrameDesc* frames,
-                          FrameState* state, const BatchDims* dims, int pass, ShardInfo* shards, void* folded,
-                          int* queue) {
-  // warp pairs run with the default wavefront block
-  auto k = tile_warps == 2 ? enc_predict_kernel<8, true, FoldT>
-           : unroll == 4   ? enc_predict_kernel<4, false, FoldT>
-           : unroll == 16  ? enc_predict_kernel<16, false, FoldT>
-           : unroll == 32  ? enc_predict_kernel<32, false, FoldT>
-                           : enc_predict_kernel<8, false, FoldT>;
-  k<<<grid, kWarpsPerCta * 32, enc_predict_smem(sizeof(FoldT) == 2), stream>>>(
-      frames, state, dims, pass, shards, static_cast<FoldT*>(folded), queue);
+  return cudaFuncSetAttribute(enc_predict_wave_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, b16);
 }
 
 void enc_predict_launch(int unroll, int tile_warps, bool fold16, int grid, cudaStream_t stream,
                         const FrameDesc* frames, FrameState* state, const BatchDims* dims, int pass,
                         ShardInfo* shards, void* folded, int* queue) {
-  if (fold16)
-    enc_predict_launch_t<uint16_t>(unroll, tile_warps, grid, stream, frames, state, dims, pass, shards, folded, queue);
-  else
-    enc_predict_launch_t<uint32_t>(unroll, tile_warps, grid, stream, frames, state, dims, pass, shards, folded, queue);
+  if (fold16) {
+    enc_predict_wave_kernel<<<grid, kWarpsPerCta * 32, enc_predict_smem(true), stream>>>(
+        frames, state, dims, pass, shards, static_cast<uint16_t*>(folded), queue);
+    return;
+  }
+  // warp pairs run with the default wavefront block
+  auto k = tile_warps == 2 ? enc_predict_kernel<8, true, uint32_t>
+           : unroll == 4   ? enc_predict_kernel<4, false, uint32_t>
+           : unroll == 16  ? enc_predict_kernel<16, false, uint32_t>
+           : unroll == 32  ? enc_predict_kernel<32, false, uint32_t>
+                           : enc_predict_kernel<8, false, uint32_t>;
+  k<<<grid, kWarpsPerCta * 32, enc_predict_smem(false), stream>>>(frames, state, dims, pass, shards,
+                                                                  static_cast<uint32_t*>(folded), queue);
 }
 
 // Tiles wider than kFastMaxW: one CTA per tile walks the antidiagonals with
@@ -441,7 +817,7 @@ __global__ void enc_predict_wide_kernel(const FrameDesc* __restrict__ frames, Fr
     const int fi = frame_of_tile(frames, nframes, t);
     const FrameDesc& f = frames[fi];
     FrameState& st = state[fi];
-    if (!st.active) continue;
+    if (!st.active || frame_lossless(f)) continue;
     const TileGeo g = tile_geo(f, t - f.tile_base);
     if (g.w <= kFastMaxW) continue;
     const int32_t step = st.step, maxs = f.max_sample;
@@ -1395,7 +1771,7 @@ struct EmitWarpSmem {
 static_assert(sizeof(EmitWarpSmem) % 16 == 0, "record buffers must stay 16-byte aligned");
 
 size_t enc_predict_smem(bool fold16) {
-  return (fold16 ? sizeof(EncWarpSmem<uint16_t>) : sizeof(EncWarpSmem<uint32_t>)) * kWarpsPerCta;
+  return (fold16 ? sizeof(WaveSm) : sizeof(EncWarpSmem<uint32_t>)) * kWarpsPerCta;
 }
 size_t enc_emit_smem() { return sizeof(EmitWarpSmem) * kWarpsPerCta; }
 

@@ -95,8 +95,11 @@ __device__ __forceinline__ void cp_async_piece(uint2* smem, const uint2* gmem) {
 
 // encoder (counts of pass `pass` from dims); `folded` is u16 when fold16
 __global__ void enc_init_kernel(const FrameDesc* frames, FrameState* state, const BatchDims* dims);
-// enc_predict with a wavefront block of `unroll` steps (4, 8, 16, 32)
-// and `tile_warps` (1, or 2: a warp pair splits each tile's bands)
+// frames of step 1 (pass 0 only)
+void enc_lossless_launch(bool fold16, int64_t tiles, int max_ctas, cudaStream_t stream, const FrameDesc* frames,
+                         FrameState* state, const BatchDims* dims, ShardInfo* shards, void* folded);
+// the other frames; u32 symbols: a wavefront block of `unroll` steps (4, 8, 16,
+// 32) and `tile_warps` (1, or 2: a warp pair splits each tile's bands)
 void enc_predict_launch(int unroll, int tile_warps, bool fold16, int grid, cudaStream_t stream,
                         const FrameDesc* frames, FrameState* state, const BatchDims* dims, int pass,
                         ShardInfo* shards, void* folded, int* queue);
@@ -148,9 +151,8 @@ cudaError_t dec_rans_set_smem();
 void dec_other_launch(bool fold16, int grid, cudaStream_t stream, const FrameDesc* frames, FrameState* state,
                       const ShardInfo* shards, const BatchDims* dims, DecodeLists* lists, const int32_t* list_items,
                       void* folded);
-// u16 symbols: `few` tiles for the GPU's warps take the shorter-chain sweep;
 // u32 symbols: `unroll` and `tile_warps` as for enc_predict
-void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, bool few, int grid, cudaStream_t stream,
+void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, int grid, cudaStream_t stream,
                             const FrameDesc* frames, const FrameState* state, const BatchDims* dims,
                             const void* folded, int* queue);
 cudaError_t dec_other_set_smem();

@@ -42,14 +42,13 @@ struct alignas(16) WaveSm {
   uint16_t carry[kCarryCols];  // row above the band, column c at index c + kCarryPad
 };
 
-// Skew per lane: 2 puts every row one step behind the row above it, the
-// shortest sweep (W + 63 steps a band), with the shuffle on the chain from
-// step to step; 4 gives the value from the lane below two more steps to
-// arrive, which takes it off that chain, for 62 steps more a band.
-template <int SK>
-__host__ __device__ constexpr int wave_skew(int row) {
-  return SK * (row >> 1) + (row & 1);
-}
+// Row k runs one step behind the row above it: the shortest sweep (W + 63 steps
+// a band), with the shuffle on the chain from step to step.  (Four steps a lane
+// instead of two take the shuffle off the chain for 62 steps more a band: 2 us
+// less of 35 for the reconstruction of a 1080p frame, 2 to 4 us more for its
+// prediction, 6 to 20 % more for batches.)
+constexpr int kSkew = 2;  // per lane, two rows
+__host__ __device__ constexpr int wave_skew(int row) { return row; }
 constexpr int kWinHop = 8 * kWinChunks + 1;  // chunks from row k to row k + 8
 __device__ __forceinline__ int win_row(int row) { return kWinChunks * row + (row >> 3); }
 
@@ -68,16 +67,21 @@ __device__ __forceinline__ uint32_t bit_range(int lo, int hi) {
   return (hi < 0 ? 0u : 0xffffffffu >> (31 - min(hi, 31))) & (lo > 31 ? 0u : 0xffffffffu << max(lo, 0));
 }
 
+// a - b of packed halves in 0..32767, as signed halves: the low half cannot
+// borrow from the high one once its top bit is set.  (The packed subtraction is
+// a negation and an addition.)
+__device__ __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) { return (a + 0x8000u - b) ^ 0x8000u; }
+
 __device__ __forceinline__ uint32_t pair2(int32_t v) { return static_cast<uint32_t>(v & 0xffff) * 0x10001u; }
 
 // Loads and stores of one warp's windows over the bands of a tile.  Chunks of
 // global memory are copied as they lie, so a row's first chunk may hold up to
 // seven samples left of the tile, cleared by fix_edge().  CHECK: a chunk may
 // reach outside [lo, hi), the memory that may be read.
-template <int SK, bool CHECK>
+template <bool CHECK>
 struct WaveIo {
-  static constexpr int kShift = SK == 2 ? 3 : 4;  // rows eight apart: columns 1 << kShift apart
-  static_assert(4 * SK == 1 << kShift, "skew of eight rows");
+  static constexpr int kShift = 3;  // rows eight apart: columns 1 << kShift apart
+  static_assert(4 * kSkew == 1 << kShift, "skew of eight rows");
   WaveSm& sm;
   const int lane;
   const int W;
@@ -87,6 +91,7 @@ struct WaveIo {
   const int64_t out_pitch;
   const uint16_t* lo;
   const uint16_t* hi;
+  bool at_edge;  // the band touches the plane's first or last chunk
   int nrows, nblk, row_top;  // row_top: the last i with row lr + 8 i in the band
   int a_in, a_step;  // alignment (samples modulo 8) of row 0, and its change per row
   int store_mode;    // 0: single samples, 1: pairs, 2: 16-byte chunks
@@ -98,8 +103,11 @@ struct WaveIo {
   // own rows 2 lane, 2 lane + 1
   int off0, off1;
 
+  // a row start on an odd sample delays the whole sweep by a step, so that the
+  // even rows' window positions are even
+  __device__ int skew(int row) const { return wave_skew(row) + (a_in & 1); }
   __device__ int align_of(int row) const { return (a_in + row * a_step) & 7; }
-  __device__ int off_of(int row) const { return (align_of(row) - wave_skew<SK>(row)) & 7; }
+  __device__ int off_of(int row) const { return (align_of(row) - skew(row)) & 7; }
 
   __device__ WaveIo(WaveSm& sm_, int lane_, int W_, const uint16_t* in_, int64_t in_pitch_, uint16_t* out_,
                     int64_t out_pitch_, const uint16_t* lo_, const uint16_t* hi_)
@@ -115,16 +123,17 @@ struct WaveIo {
     ragged = ((a_in | a_step | W) & 7) != 0;
     lr = lane >> 2;
     lj = lane & 3;
-    c_first = -wave_skew<SK>(lr) - off_of(lr) + 8 * lj;
-    in_hop = 8 * in_pitch - 4 * SK;
-    out_hop = 8 * out_pitch - 4 * SK;
+    c_first = -skew(lr) - off_of(lr) + 8 * lj;
+    in_hop = 8 * in_pitch - 4 * kSkew;
+    out_hop = 8 * out_pitch - 4 * kSkew;
     off0 = off_of(2 * lane);
     off1 = off_of(2 * lane + 1);
   }
   __device__ void band(int rows_left) {
     nrows = min(kBandRows, rows_left);
+    at_edge = CHECK && (in - 7 < lo || in + (nrows - 1) * in_pitch + W + 7 > hi);
     row_top = ((nrows - lr + 7) >> 3) - 1;
-    nblk = (W + wave_skew<SK>(nrows - 1) + 31) >> 5;
+    nblk = (W + skew(nrows - 1) + 31) >> 5;
   }
   __device__ void next_band() {
     in += kBandRows * in_pitch;
@@ -132,9 +141,10 @@ struct WaveIo {
   }
 
   __device__ void fetch_chunk(uint4* dst, const uint16_t* src, int c, bool valid) {
-    if constexpr (CHECK) {
+    if (CHECK && at_edge) {
       if (valid && (src < lo || src + 8 > hi)) {  // the plane's first or last chunk
         uint16_t* d = reinterpret_cast<uint16_t*>(dst);
+#pragma unroll 1
         for (int e = 0; e < 8; ++e) d[e] = (c + e >= 0 && c + e < W) ? src[e] : 0;
         return;
       }
@@ -150,16 +160,22 @@ struct WaveIo {
     uint4* dst = w + kWinChunks * lr + 1 + lj;
     // rows whose chunk, at column c - (i << kShift), holds a column of the tile
     const uint32_t valid = bit_range((c - W + (1 << kShift)) >> kShift, min((c + 7) >> kShift, row_top));
+    if (CHECK && at_edge) {
+#pragma unroll 1
+      for (int i = 0; i < 8; ++i)
+        fetch_chunk(dst + kWinHop * i, src + i * in_hop, c - (i << kShift), valid & (1u << i));
+    } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      fetch_chunk(dst + kWinHop * i, src, c - (i << kShift), valid & (1u << i));
-      src += in_hop;
+      for (int i = 0; i < 8; ++i) {
+        cp_async16_or_zero(dst + kWinHop * i, src, !(valid & (1u << i)));
+        src += in_hop;
+      }
     }
     if (b == 0) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int row = 2 * lane + h;
-        const int c0 = -wave_skew<SK>(row) - (h ? off1 : off0);
+        const int c0 = -skew(row) - (h ? off1 : off0);
         fetch_chunk(w + win_row(row), in + row * in_pitch + c0, c0, row < nrows && c0 > -8);
       }
     }
@@ -179,7 +195,7 @@ struct WaveIo {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int row = 2 * lane + h;
-      const int a = align_of(row), sk = wave_skew<SK>(row), off = h ? off1 : off0;
+      const int a = align_of(row), sk = skew(row), off = h ? off1 : off0;
       const int base = 32 * b - sk - off;  // column of the window's first position
       uint16_t* w = reinterpret_cast<uint16_t*>(sm.win[b & 1] + win_row(row));
       // chunk 0 was cleared as chunk 4 of the window before, except in the first
@@ -257,7 +273,7 @@ struct WaveIo {
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
       const int row = 2 * lane + h;
-      const int c = 32 * b + 32 - wave_skew<SK>(row) - (h ? off1 : off0);
+      const int c = 32 * b + 32 - skew(row) - (h ? off1 : off0);
       if (row < nrows && c > -8 && c < W) {
         const uint4* src = sm.win[b & 1] + win_row(row) + 4;
         uint16_t* dst = out + row * out_pitch + c;
@@ -271,8 +287,8 @@ struct WaveIo {
 // Group of eight steps of one row's window words.  A row whose first position
 // is even has steps 2i and 2i+1 in word i; one whose first position is odd
 // has steps 2i-1 and 2i there, so the group spans five words, the first kept
-// from the group before.  The parities are the same for all lanes (rows 2r
-// start at skew SK * r, rows 2r + 1 one later).
+// from the group before.  Rows 2r start even; rows 2r + 1, one step later,
+// start odd, unless the row pitch is odd.
 template <bool ODD>
 struct WaveWords {
   uint32_t w[5];
@@ -288,15 +304,15 @@ struct WaveWords {
 };
 
 // Both rows' samples of step j in one register.
-template <bool O0, bool O1>
-__device__ __forceinline__ uint32_t wave_pack(const WaveWords<O0>& x, const WaveWords<O1>& y, int j) {
-  const uint32_t sel = (WaveWords<O0>::high(j) ? 0x32u : 0x10u) | (WaveWords<O1>::high(j) ? 0x7600u : 0x5400u);
+template <bool O1>
+__device__ __forceinline__ uint32_t wave_pack(const WaveWords<false>& x, const WaveWords<O1>& y, int j) {
+  const uint32_t sel = (WaveWords<false>::high(j) ? 0x32u : 0x10u) | (WaveWords<O1>::high(j) ? 0x7600u : 0x5400u);
   return __byte_perm(x.word(j), y.word(j), sel);
 }
 
 // Pointers of one window block of a lane, and the stores of its results: two
 // steps a word, over the samples they came from.
-template <int SK, bool O0, bool O1>
+template <bool O1>
 struct WaveBlock {
   uint32_t* p0;
   uint32_t* p1;
@@ -308,19 +324,18 @@ struct WaveBlock {
     p0 = reinterpret_cast<uint32_t*>(win) + (off0 >> 1);
     p1 = reinterpret_cast<uint32_t*>(win + kWinChunks) + (off1 >> 1);
     crow = sm.carry + kCarryPad + 32 * b;
-    cout = reinterpret_cast<uint32_t*>(sm.carry + kCarryPad + 32 * b - 1 - wave_skew<SK>(kBandRows - 1));
+    cout = reinterpret_cast<uint32_t*>(sm.carry + kCarryPad + 32 * b - 1 - wave_skew(kBandRows - 1));
   }
   // Results of step j of group g, packed (even row low), and those of the
   // step before; the carry row takes the reconstruction's.
   __device__ void put(int g, int j, uint32_t was, uint32_t now, uint32_t last_was, uint32_t last_now) {
     const int i = 4 * g + (j >> 1);
-    if (O0 == !(j & 1)) p0[i] = __byte_perm(was, now, 0x5410);
+    if (j & 1) p0[i] = __byte_perm(was, now, 0x5410);
     if (O1 == !(j & 1)) p1[i] = __byte_perm(was, now, 0x7632);
     if (!(j & 1) && lane == 31) cout[i] = __byte_perm(last_was, last_now, 0x7632);
   }
   // after step 31: the half word that the next block's first word completes
   __device__ void finish(uint32_t now, uint32_t last_now) {
-    if (O0) *reinterpret_cast<uint16_t*>(p0 + 16) = static_cast<uint16_t>(now);
     if (O1) *reinterpret_cast<uint16_t*>(p1 + 16) = static_cast<uint16_t>(now >> 16);
     if (lane == 31) *reinterpret_cast<uint16_t*>(cout + 16) = static_cast<uint16_t>(last_now >> 16);
   }
@@ -338,28 +353,20 @@ struct WaveCarry {
 };
 
 // What a lane keeps from step to step, packed (even row in the low half).
-template <int SK>
 struct WavePacked {
   uint32_t rec = 0, above = 0;
-  uint32_t late[2] = {0, 0};  // shuffled values on their way (skew 4)
   __device__ uint32_t packed() const { return rec; }
 
   // The upper neighbours of this step: the even row's from the lane below in
   // rank (lane 0: the carry row), the odd row's from the lane's last step.
   __device__ uint32_t neighbours(uint32_t carry, int odd_step, int lane) {
-    uint32_t up = __shfl_up_sync(0xffffffffu, rec, 1);
-    if (SK == 4) {
-      const uint32_t now = late[0];
-      late[0] = late[1];
-      late[1] = up;
-      up = now;
-    }
+    const uint32_t up = __shfl_up_sync(0xffffffffu, rec, 1);
     const uint32_t sel = (lane == 0 && !odd_step) ? 0x5410u : 0x5432u;
     return __byte_perm(lane == 0 ? carry : up, rec, sel);
   }
   template <bool MED>
   __device__ uint32_t predict(uint32_t a, uint32_t maxs2) {
-    const uint32_t d = __vsub2(a, above);
+    const uint32_t d = sub2(a, above);
     if (MED) {
       const uint32_t mn = __vmins2(rec, a), mx = __vmaxs2(rec, a);
       return __vmaxs2(mn, __viaddmin_s16x2(rec, d, mx));
@@ -369,20 +376,12 @@ struct WavePacked {
 };
 
 // The same in 32 bits a row (depth 16).
-template <int SK>
 struct WaveWide {
   int32_t rec0 = 0, rec1 = 0, above0 = 0, above1 = 0;
-  int32_t late[2] = {0, 0};
   __device__ uint32_t packed() const { return __byte_perm(rec0, rec1, 0x5410); }
 
   __device__ void neighbours(uint32_t carry, int odd_step, int lane, int32_t& a0, int32_t& a1) {
-    int32_t up = __shfl_up_sync(0xffffffffu, rec1, 1);
-    if (SK == 4) {
-      const int32_t now = late[0];
-      late[0] = late[1];
-      late[1] = up;
-      up = now;
-    }
+    const int32_t up = __shfl_up_sync(0xffffffffu, rec1, 1);
     a0 = lane == 0 ? static_cast<int32_t>(odd_step ? carry >> 16 : carry & 0xffffu) : up;
     a1 = rec0;
   }
