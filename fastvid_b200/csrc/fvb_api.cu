@@ -653,19 +653,10 @@ constexpr int kDefaultCtas[K_COUNT] = {
 std::atomic<int> g_ctas[K_COUNT];
 std::atomic<int> g_wavefront_block{kDefaultWavefrontBlock};
 std::atomic<int> g_decode_overlap{1};
-// rANS encoder fetch scheme per pass: 0, 8, 16, or -1 (automatic: the
-// software pipeline over blocks of 8 steps when the launch leaves the SMs
-// short of warps -- a single frame, the frame policy's later passes -- where
-// the state chain would otherwise wait on its loads; the one-stage fetch,
-// which holds fewer registers, when the launch fills the GPU)
+// rANS encoder fetch scheme per pass: accepted and kept for callers that set
+// it; enc_rans has one scheme
 std::atomic<int> g_rans_pipeline{-1};
 std::atomic<int> g_rans_pipeline_tail{-1};
-constexpr int kRansAutoCtasPerSm = 4;
-
-int rans_pipe_for(int knob, int grid) {
-  if (knob >= 0) return knob;
-  return grid <= device_sms() * kRansAutoCtasPerSm ? 8 : 0;
-}
 std::atomic<int> g_tile_warps{kDefaultTileWarps};
 
 // Whether dec_rans runs on tables of all slots: as long as all shards are
@@ -985,10 +976,7 @@ int encode_enqueue(const Totals& cap, void* workspace, int64_t workspace_bytes, 
     FVB_LAUNCHED("enc_analyze_kernel");
     {
       LaunchScope scope_(K_ENC_RANS, stream);
-      const int grid = static_cast<int>(ceil_div(nsh * 4 > 0 ? nsh * 4 : 1, 128));
-      enc_rans_launch(rans_pipe_for((pass == 0 ? g_rans_pipeline : g_rans_pipeline_tail).load(std::memory_order_relaxed),
-                                    grid),
-                      f16, grid, stream, state, dims, pass, shards, folded, rans);
+      enc_rans_launch(f16, nsh, stream, state, dims, pass, shards, folded, rans);
     }
     FVB_LAUNCHED("enc_rans_kernel");
     {

@@ -887,7 +887,9 @@ __device__ __forceinline__ uint32_t bit_or_zero(uint32_t s) {
 // for every x < 2^31, because m exceeds 2^(31+s)/f by less than one, which
 // moves x * m / 2^(31+s) by less than x / 2^(31+s) < 2^-s <= 1/f.  For f = 1
 // the multiplier 2^32-1 yields x - 1, and the bias carries the missing 4095.
-// Table entry: the multiplier, then bias | (4096 - f) << 13 | (s - 1) << 25.
+// Table entry: the multiplier, then f << 19 | bias << 5 | s - 1 (the upper 13
+// bits are the renormalisation threshold f * 2^19 as they stand, the lowest five
+// a shift amount).
 __device__ __forceinline__ uint32_t rans_multiplier(uint32_t f) {
   if (f < 2) return 0xffffffffu;
   const uint32_t s = 32 - __clz(f - 1);
@@ -901,7 +903,7 @@ __device__ __forceinline__ uint32_t rans_multiplier(uint32_t f) {
 __device__ __forceinline__ uint32_t rans_packed(uint32_t f, uint32_t cum) {
   const uint32_t bias = f < 2 ? cum + 4095u : cum;
   const uint32_t sh = f < 2 ? 0u : 31u - __clz(f - 1);  // s - 1
-  return bias | ((4096u - f) << 13) | (sh << 25);
+  return (f << 19) | (bias << 5) | sh;
 }
 
 // Zero-run token statistics of one 128-symbol block (encode.cu:232-240): a
@@ -1388,6 +1390,7 @@ enc_analyze_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict_
           ser[c++] = byte;
         } while (d);
         si.rans_table = static_cast<int32_t>(c_cursor);
+        si.param = static_cast<int32_t>(shard_max);  // for enc_rans; enc_scan sets the mode's
       }
       // Skip the trial encoding when it cannot win.  Each rANS step takes a
       // state x in [f 2^11, f 2^19) after renormalisation to one at least
@@ -1414,147 +1417,199 @@ enc_analyze_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict_
 // enc_rans: four interleaved lanes per shard, one thread per lane, eight
 // shards per warp.  Lane bytes are written back to front so they end up in
 // stream order (the reference reverses them at emission, encode.cu:609).
+//
+// A lane codes every fourth symbol.  The four lanes of a shard load sixteen
+// symbols at once, four consecutive ones each, and transpose them by two rounds
+// of shuffles; the table entries of values below kEncLocal are looked up in
+// shared memory, one group of four steps ahead of the state chain, the symbols
+// two groups ahead.
+//
+// Bound by issue, about 36 instructions a step, and in a lone warp by their
+// latency.  Loading single symbols (eight lines a load) and entries from global
+// memory (up to 32 lines), 53 instructions a step, 24 4K yuv422-10 frames took
+// 737 us, a 4K gray16 frame's two passes 167 us, a 1080p rgb8 frame 82 us; now
+// 645, 147 and 72 us.
+constexpr int kEncLocal = 128;
 
-template <int PIPE, typename FoldT>
+struct RansLane {
+  uint32_t x = kRansL;
+  // pending bytes, the upper `bits` of a 64-bit value in two words (hi:lo), the
+  // latest emitted on top: renormalising by sh bits is a right shift of x and,
+  // by the same amount, of the value with x's low bits coming in
+  uint32_t hi = 0, lo = 0;
+  int bits = 0;
+  uint32_t* out;  // next word is written below
+  // one encoding step (encode.cu:401-418): renormalise -- at most two bytes,
+  // since x < 2^31 and the threshold f * 2^19 >= 2^19 -- then the state map
+  __device__ __forceinline__ void step(uint2 e) {
+    const uint32_t thr = e.y & 0xfff80000u;  // ((L >> 12) << 8) * f
+    const uint32_t one = x >= thr ? 8u : 0u;
+    const uint32_t sh = (x >> 8) >= thr ? 16u : one;
+    lo = __funnelshift_r(lo, hi, sh);
+    hi = __funnelshift_r(hi, x, sh);
+    bits += sh;
+    x >>= sh;
+    const uint32_t q = __funnelshift_r(__umulhi(x, e.x), 0u, e.y);  // shift taken modulo 32
+    x = q * (4096u - (e.y >> 19)) + (x + ((e.y >> 5) & 0x1fffu));
+  }
+  // Writes the four earliest pending bytes, the first at the highest address,
+  // if there are as many: after a pair of steps (at most 3 + 4 = 7 bytes
+  // pending, at most 3 afterwards), or a single one.
+  __device__ __forceinline__ void flush() {
+    if (bits >= 32) {
+      *--out = __byte_perm(__funnelshift_rc(lo, hi, 64 - bits), 0, 0x0123);
+      bits -= 32;
+    }
+  }
+};
+
+// LOCAL: all values below kEncLocal.  ALL: the warp's eight shards run in step
+// (the usual case: as many symbols each), so the shuffles need no mask of
+// their own, which the compiler can only serve by a vote for each (2.5 % of a
+// 1080p frame's time).
+template <bool LOCAL, bool ALL, typename FoldT>
+__device__ __forceinline__ void rans_encode_lane(RansLane& st, const FoldT* __restrict__ f, int n,
+                                                 const uint2* __restrict__ tab, const uint2 (*local)[8], int j, int l) {
+  const unsigned group = ALL ? kFull : 0xfu << (4 * j);
+  auto entry = [&](uint32_t v) { return (LOCAL || v < kEncLocal) ? local[v][j] : __ldg(tab + v); };
+  auto near = [&](uint32_t v) { return local[v & (kEncLocal - 1)][j]; };
+  const int g0 = n & ~15;
+  for (int i = n - 1 - ((n - 1 - l) & 3); i >= g0; i -= 4) {  // symbols past the last whole sixteen
+    st.step(entry(ldf(f + i)));
+    st.flush();
+  }
+  // symbols 16 m + 4 l .. + 3 as 16-bit pairs
+  f += 4 * l;
+  auto load = [&](int m) {
+    uint2 r = make_uint2(0, 0);
+    if (m >= 0) {
+      const FoldT* p = f + 16 * m;
+      if constexpr (sizeof(FoldT) == 2) {
+        r = __ldg(reinterpret_cast<const uint2*>(p));
+      } else {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+        r = make_uint2(v.x | (v.y << 16), v.z | (v.w << 16));
+      }
+    }
+    return r;
+  };
+  const bool upper = l & 2, odd = l & 1;
+  struct Four {
+    uint2 e[4];
+  };
+  // the entries of symbols 16 m + 4 k + l, k = 0..3
+  auto fetch = [&](uint2 r) {
+    const uint32_t mine = upper ? r.y : r.x;
+    const uint32_t theirs = __shfl_xor_sync(group, upper ? r.x : r.y, 2);
+    const uint32_t lows = __byte_perm(mine, theirs, 0x5410), highs = __byte_perm(mine, theirs, 0x7632);
+    const uint32_t keep = odd ? highs : lows;
+    const uint32_t got = __shfl_xor_sync(group, odd ? lows : highs, 1);
+    // lanes 0 and 1 hold (even lane's, odd lane's) in this order, lanes 2 and 3
+    // the upper pair first
+    const uint32_t a = __byte_perm(keep, got, odd ? 0x1054u : 0x5410u), b = __byte_perm(keep, got, odd ? 0x3276u : 0x7632u);
+    const uint32_t w0 = upper ? b : a, w1 = upper ? a : b;
+    Four q;
+    q.e[0] = near(w0);
+    q.e[1] = near(w0 >> 16);
+    q.e[2] = near(w1);
+    q.e[3] = near(w1 >> 16);
+    constexpr uint32_t kFar = (0xffffu & ~(kEncLocal - 1u)) * 0x10001u;
+    if (!LOCAL && ((w0 | w1) & kFar)) {  // few symbols: outliers of a predicted frame
+      if (w0 & kFar & 0xffffu) q.e[0] = __ldg(tab + (w0 & 0xffffu));
+      if (w0 & kFar >> 16 << 16) q.e[1] = __ldg(tab + (w0 >> 16));
+      if (w1 & kFar & 0xffffu) q.e[2] = __ldg(tab + (w1 & 0xffffu));
+      if (w1 & kFar >> 16 << 16) q.e[3] = __ldg(tab + (w1 >> 16));
+    }
+    return q;
+  };
+  auto run = [&](const Four& q) {
+    st.step(q.e[3]);
+    st.step(q.e[2]);
+    st.flush();
+    st.step(q.e[1]);
+    st.step(q.e[0]);
+    st.flush();
+  };
+  int m = (g0 >> 4) - 1;
+  if (m < 0) return;
+  // symbols are loaded four to eight groups ahead (L2 latency), entries one
+  Four a = fetch(load(m)), b;
+  uint2 r[4], t[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) r[i] = load(m - 1 - i);
+  for (; m >= 4; m -= 4) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t[i] = load(m - 5 - i);
+    b = fetch(r[0]);
+    run(a);
+    a = fetch(r[1]);
+    run(b);
+    b = fetch(r[2]);
+    run(a);
+    a = fetch(r[3]);
+    run(b);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = t[i];
+  }
+  run(a);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if (m > i) run(fetch(r[i]));
+}
+
+template <typename FoldT>
 __global__ void __launch_bounds__(128)
 enc_rans_kernel(const FrameState* __restrict__ state, const BatchDims* __restrict__ dims, int pass,
                 ShardInfo* __restrict__ shards, const FoldT* __restrict__ folded,
                 uint8_t* __restrict__ rans_scratch) {
+  // entry of value v of shard j: local[v][j], so that the shards' lookups fall
+  // in different banks
+  __shared__ uint2 local_all[4][kEncLocal][8];
   const int64_t total_shards = dims->shards_p[pass];
-  const int64_t gid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t s = gid >> 2;
-  const int lane = static_cast<int>(gid & 3);
-  if (s >= total_shards) return;
-  ShardInfo& si = shards[s];
-  if (!state[si.frame].active || !si.rans_ok) return;
-  const int n = si.count;
-  const FoldT* __restrict__ f = folded + si.sample_base;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, j = lane >> 2, l = lane & 3;
+  const int64_t s = (static_cast<int64_t>(blockIdx.x) * 4 + warp) * 8 + j;
+  uint2 (*local)[8] = local_all[warp];
+  const bool live = s < total_shards && state[shards[s].frame].active && shards[s].rans_ok;
+  const int top = live ? shards[s].param : 0;  // the shard's largest value
   uint8_t* base = rans_scratch + s * static_cast<int64_t>(kRansScratchBytes);
   const uint2* __restrict__ tab = reinterpret_cast<const uint2*>(base);
-  uint32_t* out_end = reinterpret_cast<uint32_t*>(base + kRansTableWords * 4 + kRansSerialBytes +
-                                                  (lane + 1) * kRansLaneBytes);
-  uint32_t x = kRansL;
-  // pending bytes, earliest emitted in the highest position, as a 64-bit
-  // value in two words (ahi:alo) moved by funnel shifts: a 64-bit variable
-  // shift costs several instructions per step
-  uint32_t ahi = 0, alo = 0;
-  int nacc = 0, nwords = 0;
-  const int first = n - 1 - ((n - 1 - lane) & 3);
-  const int steps = first >= 0 ? first / 4 + 1 : 0;  // symbols first, first-4, ..., >= 0
-  // one encoding step (encode.cu:401-418): renormalise -- at most two bytes,
-  // since x < 2^31 and the threshold f * 2^19 >= 2^19 -- then the state map.
-  // Pending bytes are written out a word at a time by flush(): after a pair
-  // of steps (at most 3 + 4 = 7 pending, one word written leaves at most 3),
-  // or after every step of an odd tail.
-  auto step = [&](uint2 e) {
-    const uint32_t cmpl = (e.y >> 13) & 0xfffu;
-    const uint32_t thr = (4096u - cmpl) << 19;  // ((L >> 12) << 8) * f
-    const uint32_t b1 = x >= thr, b2 = (x >> 8) >= thr;
-    const int nb = static_cast<int>(b1 + b2);
-    const uint32_t bytes = b2 ? __byte_perm(x, 0, 0x4401) : (x & 0xffu);  // first byte on top
-    const uint32_t sh = 8u * static_cast<uint32_t>(nb);  // 0, 8 or 16
-    ahi = __funnelshift_l(alo, ahi, sh);
-    alo = (alo << sh) | (nb ? bytes : 0u);
-    nacc += nb;
-    x >>= sh;
-    const uint32_t q = __umulhi(x, e.x) >> (e.y >> 25);
-    x += (e.y & 0x1fffu) + q * cmpl;
-  };
-  auto flush = [&]() {
-    if (nacc >= 4) {
-      nacc -= 4;
-      out_end[-(++nwords)] = __funnelshift_r(alo, ahi, 8 * nacc);  // (ahi:alo) >> 8 nacc, nacc 0..3
+  if (live)
+    for (int v = l; v <= min(top, kEncLocal - 1); v += 4) {
+      const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(&local[v][j]));
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(a), "l"(tab + v) : "memory");
     }
-  };
-  int c = 0;
-  if (PIPE == 0) {
-    // symbols and table entries are loaded 16 steps ahead of the state chain
-    constexpr int kAhead = 16;
-    for (; c + kAhead <= steps; c += kAhead) {
-      uint32_t v[kAhead];
-      uint2 e[kAhead];
-#pragma unroll
-      for (int j = 0; j < kAhead; ++j) v[j] = ldf(f + first - 4 * (c + j));
-#pragma unroll
-      for (int j = 0; j < kAhead; ++j) e[j] = tab[v[j]];
-#pragma unroll
-      for (int j = 0; j < kAhead; j += 2) {
-        step(e[j]);
-        step(e[j + 1]);
-        flush();
-      }
-    }
+  cp_async_commit();
+  cp_async_wait<0>();
+  const bool all_local = !__any_sync(kFull, top >= kEncLocal);
+  const int count = live ? shards[s].count : -1;
+  const int count0 = __shfl_sync(kFull, count, 0);  // by all lanes: not inside the condition
+  const bool in_step = __all_sync(kFull, count >= 0 && count == count0);
+  if (!live) return;
+  ShardInfo& si = shards[s];
+  const FoldT* __restrict__ f = folded + si.sample_base;
+  uint32_t* end = reinterpret_cast<uint32_t*>(base + kRansTableWords * 4 + kRansSerialBytes + (l + 1) * kRansLaneBytes);
+  RansLane st;
+  st.out = end;
+  if (in_step) {
+    if (all_local) rans_encode_lane<true, true>(st, f, si.count, tab, local, j, l);
+    else rans_encode_lane<false, true>(st, f, si.count, tab, local, j, l);
   } else {
-    // Software pipeline over blocks of PIPE steps: while block b runs, the
-    // table entries of block b+1 (whose symbols arrived a block earlier) and
-    // the symbols of block b+2 are in flight, so neither the symbol load nor
-    // the dependent table load sits on the state chain.
-    constexpr int kB = PIPE > 0 ? PIPE : 2;  // even: steps go in pairs
-    const int nblk = steps / kB;
-    uint32_t vn[kB];      // symbols of block b+2
-    uint2 en[kB], ec[kB];  // table entries of blocks b+1 and b
-    auto load_v = [&](int b, uint32_t (&v)[kB]) {
-#pragma unroll
-      for (int j = 0; j < kB; ++j) v[j] = ldf(f + first - 4 * (b * kB + j));
-    };
-    if (nblk > 0) {
-      load_v(0, vn);
-#pragma unroll
-      for (int j = 0; j < kB; ++j) ec[j] = tab[vn[j]];
-    }
-    if (nblk > 1) {
-      load_v(1, vn);
-#pragma unroll
-      for (int j = 0; j < kB; ++j) en[j] = tab[vn[j]];
-    }
-    if (nblk > 2) load_v(2, vn);
-    for (int b = 0; b < nblk; ++b) {
-      uint2 cur[kB];
-#pragma unroll
-      for (int j = 0; j < kB; ++j) {
-        cur[j] = ec[j];
-        ec[j] = en[j];
-      }
-      if (b + 2 < nblk) {
-#pragma unroll
-        for (int j = 0; j < kB; ++j) en[j] = tab[vn[j]];
-      }
-      if (b + 3 < nblk) load_v(b + 3, vn);
-#pragma unroll
-      for (int j = 0; j < kB; j += 2) {
-        step(cur[j]);
-        step(cur[j + 1]);
-        flush();
-      }
-    }
-    c = nblk * kB;
+    rans_encode_lane<false, false>(st, f, si.count, tab, local, j, l);
   }
-  for (; c < steps; ++c) {
-    step(tab[ldf(f + first - 4 * c)]);
-    flush();
-  }
-  if (nacc) out_end[-(nwords + 1)] = alo << (8 * (4 - nacc));  // low bytes unused
-  si.rans_lane[lane] = 4 * nwords + nacc;
-  si.rans_state[lane] = x;
+  if (st.bits) *(st.out - 1) = __byte_perm(st.hi >> (32 - st.bits), 0, 0x0123);  // low bytes unused
+  si.rans_lane[l] = 4 * static_cast<int>(end - st.out) + (st.bits >> 3);
+  si.rans_state[l] = st.x;
 }
 
-// enc_rans with its loads either 16 steps ahead in one stage (PIPE 0) or
-// pipelined over blocks of 8 or 16 steps (the autotuner's knob; identical
-// bytes).
-template <typename FoldT>
-static void enc_rans_launch_t(int pipe, int grid, cudaStream_t stream, const FrameState* state,
-                              const BatchDims* dims, int pass, ShardInfo* shards, const void* folded,
-                              uint8_t* rans_scratch) {
-  auto k = pipe == 8    ? enc_rans_kernel<8, FoldT>
-           : pipe == 16 ? enc_rans_kernel<16, FoldT>
-                        : enc_rans_kernel<0, FoldT>;
-  k<<<grid, 128, 0, stream>>>(state, dims, pass, shards, static_cast<const FoldT*>(folded), rans_scratch);
-}
-
-void enc_rans_launch(int pipe, bool fold16, int grid, cudaStream_t stream, const FrameState* state,
-                     const BatchDims* dims, int pass, ShardInfo* shards, const void* folded, uint8_t* rans_scratch) {
-  if (fold16) enc_rans_launch_t<uint16_t>(pipe, grid, stream, state, dims, pass, shards, folded, rans_scratch);
-  else enc_rans_launch_t<uint32_t>(pipe, grid, stream, state, dims, pass, shards, folded, rans_scratch);
+void enc_rans_launch(bool fold16, int64_t nshards, cudaStream_t stream, const FrameState* state, const BatchDims* dims,
+                     int pass, ShardInfo* shards, const void* folded, uint8_t* rans_scratch) {
+  const int grid = static_cast<int>(nshards > 0 ? (nshards + 31) / 32 : 1);
+  if (fold16)
+    enc_rans_kernel<uint16_t><<<grid, 128, 0, stream>>>(state, dims, pass, shards,
+                                                        static_cast<const uint16_t*>(folded), rans_scratch);
+  else
+    enc_rans_kernel<uint32_t><<<grid, 128, 0, stream>>>(state, dims, pass, shards,
+                                                        static_cast<const uint32_t*>(folded), rans_scratch);
 }
 
 void enc_analyze_launch(bool fold16, int grid, cudaStream_t stream, const FrameDesc* frames, FrameState* state,

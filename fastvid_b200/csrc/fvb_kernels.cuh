@@ -109,10 +109,8 @@ __global__ void enc_predict_wide_kernel(const FrameDesc* frames, FrameState* sta
 void enc_analyze_launch(bool fold16, int grid, cudaStream_t stream, const FrameDesc* frames, FrameState* state,
                         const BatchDims* dims, int pass, ShardInfo* shards, const void* folded,
                         uint8_t* rans_scratch);
-// enc_rans with one-stage loads (pipe 0) or a software pipeline over blocks
-// of `pipe` (8 or 16) steps
-void enc_rans_launch(int pipe, bool fold16, int grid, cudaStream_t stream, const FrameState* state,
-                     const BatchDims* dims, int pass, ShardInfo* shards, const void* folded, uint8_t* rans_scratch);
+void enc_rans_launch(bool fold16, int64_t nshards, cudaStream_t stream, const FrameState* state, const BatchDims* dims,
+                     int pass, ShardInfo* shards, const void* folded, uint8_t* rans_scratch);
 __global__ void enc_scan_kernel(const FrameDesc* frames, FrameState* state, const BatchDims* dims, int pass,
                                 ShardInfo* shards, uint8_t* prefix);
 // Records of one encoder region: pass 0's, or the later pass's (region b,
