@@ -121,6 +121,11 @@ def encode_frame(planes, layout, bit_depth, quality, fps_numerator=24, fps_denom
 
 
 def header_of(encoded: torch.Tensor) -> bytes:
+    if encoded.is_cuda and encoded.dtype == torch.uint8 and encoded.dim() == 1 and encoded.numel() >= 32 \
+            and encoded.is_contiguous():
+        buf = ctypes.create_string_buffer(32)
+        _native.check(_native.load().fvb_read_header(encoded.data_ptr(), buf, _stream_handle(encoded.device)))
+        return buf.raw
     head = encoded[:32]
     if head.is_cuda:
         head = head.cpu()

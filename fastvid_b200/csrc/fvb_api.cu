@@ -476,7 +476,7 @@ int from_bucket(const fvb_bucket* b, Totals* t) {
 // the frames that take part in pass 1: a prefix of the batch, so the same
 // global shard and sample indices address both regions).
 struct EncLayout {
-  size_t dims, frames, state, outs, queue, results, shards, folded, rans, prefix, recon;
+  size_t dims, frames, state, queue, outs, results, shards, folded, rans, prefix, recon;
   size_t shards_b, folded_b, rans_b, prefix_b, total;
 };
 
@@ -492,8 +492,8 @@ EncLayout enc_layout(const Totals& t) {
   w.dims = take(sizeof(BatchDims));
   w.frames = take(sizeof(FrameDesc) * n);
   w.state = take(sizeof(FrameState) * n);
+  w.queue = take(kAlign);  // a counter per pass
   w.outs = take(sizeof(uint8_t*) * n);
-  w.queue = take(kAlign);
   w.results = take(16 * static_cast<size_t>(n));
   w.shards = take(sizeof(ShardInfo) * t.shards);
   w.folded = take((t.fold16 ? 2 : 4) * static_cast<size_t>(t.samples));
@@ -510,7 +510,7 @@ EncLayout enc_layout(const Totals& t) {
 }
 
 struct DecLayout {
-  size_t dims, frames, state, queue, results, shards, lists, items, tables, folded, total;
+  size_t dims, frames, state, queue, lists, results, shards, items, tables, folded, total;
 };
 
 DecLayout dec_layout(const Totals& t) {
@@ -526,9 +526,9 @@ DecLayout dec_layout(const Totals& t) {
   w.frames = take(sizeof(FrameDesc) * n);
   w.state = take(sizeof(FrameState) * n);
   w.queue = take(kAlign);
+  w.lists = take(sizeof(DecodeLists));
   w.results = take(16 * static_cast<size_t>(n));
   w.shards = take(sizeof(ShardInfo) * t.shards);
-  w.lists = take(sizeof(DecodeLists));
   w.items = take(4 * 4 * static_cast<size_t>(t.shards));
   w.tables = take(dec_rans_table_bytes() * static_cast<size_t>(t.shards));
   w.folded = take((t.fold16 ? 2 : 4) * static_cast<size_t>(t.samples));
@@ -557,14 +557,26 @@ __global__ void encode_headers_kernel(const FrameDesc* __restrict__ frames, cons
   out[f.slot * kHeaderBytes + b] = (state[k].final_b ? prefix_b : prefix_a)[f.prefix_base + b];
 }
 
-__global__ void results_kernel(const FrameDesc* __restrict__ frames, const FrameState* __restrict__ state,
-                               const BatchDims* __restrict__ dims, int64_t* __restrict__ out, int decode) {
-  const int n = dims->frames_p[0];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int slot = frames[i].slot;
-  out[2 * slot] = state[i].status;
-  out[2 * slot + 1] = decode ? 0 : state[i].stream_len;
+__global__ void read_header_kernel(const uint8_t* __restrict__ stream, uint8_t* __restrict__ out) {
+  out[threadIdx.x] = stream[threadIdx.x];
+}
+
+// 64 bytes of page-locked memory, one block per host thread, that the
+// single-frame entry points' kernels write their results to (see host_mapped
+// for why; a copy to pageable memory also costs a staging copy).  The entry
+// points wait for the result, so a block serves one call at a time.
+struct PinnedResult {
+  int64_t* host = nullptr;
+  ~PinnedResult() {
+    if (host) cudaFreeHost(host);
+  }
+};
+int pinned_result(int64_t** out) {
+  thread_local PinnedResult r;
+  if (!r.host)
+    FVB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&r.host), 64, cudaHostAllocPortable | cudaHostAllocMapped));
+  *out = r.host;
+  return FVB_OK;
 }
 
 // Restores the caller's current device when an entry point returns: the
@@ -869,8 +881,11 @@ namespace {
 // ---- encoder batch internals: `cap` sizes the workspace layout and the
 // launch grids; the actual counts go to the device in BatchDims ------------
 
+// `started`: the frames' initial state and the tile queues go up with the frame
+// table, for an enqueue that is told so (a single frame: three launches less).
 int encode_prepare(const Totals& cap, const fvb_frame* frames, int n, const uint16_t* const* planes,
-                   const int64_t* pitches, void* workspace, int64_t workspace_bytes, void* cuda_stream) {
+                   const int64_t* pitches, void* workspace, int64_t workspace_bytes, void* cuda_stream,
+                   bool started) {
   if (n <= 0 || !frames) return fail(FVB_ERR_ARGUMENT, "empty batch");
   const Totals t = totals_of(frames, n);
   if (!fits(t, cap)) return fail(FVB_ERR_ARGUMENT, "batch does not fit the bucket");
@@ -878,8 +893,8 @@ int encode_prepare(const Totals& cap, const fvb_frame* frames, int n, const uint
   int rc = check_ws(workspace, workspace_bytes, L.total);
   if (rc) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-  // one upload: the dims record, then the frame table
-  std::vector<unsigned char> table(L.frames + sizeof(FrameDesc) * n);
+  // one upload: the dims record, the frame table, then state and queues
+  std::vector<unsigned char> table(started ? L.queue + kAlign : L.frames + sizeof(FrameDesc) * n);
   const BatchDims dims = dims_of(t);
   std::memcpy(table.data() + L.dims, &dims, sizeof(dims));
   FrameDesc* descs = reinterpret_cast<FrameDesc*>(table.data() + L.frames);
@@ -901,6 +916,12 @@ int encode_prepare(const Totals& cap, const fvb_frame* frames, int n, const uint
     d.shard_base = sb;
     d.sample_base = nb;
     d.prefix_base = pb;
+    if (started) {  // as enc_init_kernel
+      FrameState& st = reinterpret_cast<FrameState*>(table.data() + L.state)[j];
+      st.step = d.step0;
+      st.use_med = d.use_med0;
+      st.active = 1;
+    }
     tb += d.ntiles;
     sb += d.nshards;
     nb += d.nfold;
@@ -911,7 +932,8 @@ int encode_prepare(const Totals& cap, const fvb_frame* frames, int n, const uint
   return FVB_OK;
 }
 
-int encode_enqueue(const Totals& cap, void* workspace, int64_t workspace_bytes, int64_t* results, void* cuda_stream) {
+int encode_enqueue(const Totals& cap, void* workspace, int64_t workspace_bytes, int64_t* results, void* cuda_stream,
+                   bool started) {
   const EncLayout L = enc_layout(cap);
   int rc = check_ws(workspace, workspace_bytes, L.total);
   if (rc) return rc;
@@ -926,11 +948,17 @@ int encode_enqueue(const Totals& cap, void* workspace, int64_t workspace_bytes, 
   const bool f16 = cap.fold16;  // u16 or u32 folded symbols
   uint16_t* recon = reinterpret_cast<uint16_t*>(ws + L.recon);
   const int n = cap.frames;
-  {
-    LaunchScope scope_(K_ENC_INIT, stream);
-    enc_init_kernel<<<(n + 127) / 128, 128, 0, stream>>>(frames_d, state, dims);
+  if (!started) {
+    FVB_CUDA(cudaMemsetAsync(queue, 0, kAlign, stream));
+    {
+      LaunchScope scope_(K_ENC_INIT, stream);
+      enc_init_kernel<<<(n + 127) / 128, 128, 0, stream>>>(frames_d, state, dims);
+    }
+    FVB_LAUNCHED("enc_init_kernel");
   }
-  FVB_LAUNCHED("enc_init_kernel");
+  int64_t* res_d = reinterpret_cast<int64_t*>(ws + L.results);
+  int64_t* direct = static_cast<int64_t*>(host_mapped(results));  // pinned: written by the kernels
+  if (direct) res_d = direct;
   // pass p covers the batch's first frames_p[p] frames (layout order); the
   // later passes write region b
   for (int pass = 0; pass < cap.passes; ++pass) {
@@ -948,14 +976,13 @@ int encode_enqueue(const Totals& cap, void* workspace, int64_t workspace_bytes, 
       FVB_LAUNCHED("enc_lossless_kernel");
     }
     if (cap.lossy) {
-      FVB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), stream));
       {
         LaunchScope scope_(K_ENC_PREDICT, stream);
         const int tw = g_tile_warps.load(std::memory_order_relaxed);
         // u16: one CTA per tile until the cap, as dec_reconstruct
         const int grid = grid_for(f16 ? tiles : tiles * tw, f16 ? 1 : kWarpsPerCta, ctas(K_ENC_PREDICT));
         enc_predict_launch(g_wavefront_block.load(std::memory_order_relaxed), tw, f16, grid, stream,
-                           frames_d, state, dims, pass, shards, folded, queue);
+                           frames_d, state, dims, pass, shards, folded, queue + pass);
       }
       FVB_LAUNCHED("enc_predict_kernel");
     }
@@ -981,17 +1008,11 @@ int encode_enqueue(const Totals& cap, void* workspace, int64_t workspace_bytes, 
     FVB_LAUNCHED("enc_rans_kernel");
     {
       LaunchScope scope_(K_ENC_SCAN, stream);
-      enc_scan_kernel<<<nf > 0 ? nf : 1, 1024, 0, stream>>>(frames_d, state, dims, pass, shards, prefix);
+      enc_scan_kernel<<<nf > 0 ? nf : 1, 1024, 0, stream>>>(frames_d, state, dims, pass, shards, prefix,
+                                                                res_d);
     }
     FVB_LAUNCHED("enc_scan_kernel");
   }
-  int64_t* res_d = reinterpret_cast<int64_t*>(ws + L.results);
-  int64_t* direct = static_cast<int64_t*>(host_mapped(results));  // pinned: written by the kernel
-  {
-    LaunchScope scope_(K_RESULTS, stream);
-    results_kernel<<<(n + 127) / 128, 128, 0, stream>>>(frames_d, state, dims, direct ? direct : res_d, 0);
-  }
-  FVB_LAUNCHED("results_kernel");
   if (results && !direct)
     FVB_CUDA(cudaMemcpyAsync(results, res_d, 16 * static_cast<size_t>(n), cudaMemcpyDeviceToHost, stream));
   return FVB_OK;
@@ -1012,21 +1033,16 @@ int encode_emit(const Totals& cap, const fvb_frame* frames, int n, void* workspa
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   char* ws = static_cast<char*>(workspace);
   uint8_t** outs_d = reinterpret_cast<uint8_t**>(ws + L.outs);
-  std::vector<uint8_t*> outs_laid(n);  // in batch layout order
-  const std::vector<int> order = encode_order(frames, n);
-  for (int j = 0; j < n; ++j) outs_laid[j] = outs[order[j]];
-  FVB_CUDA(cudaMemcpyAsync(outs_d, outs_laid.data(), sizeof(uint8_t*) * n, cudaMemcpyHostToDevice, stream));
-  const FrameDesc* frames_d = reinterpret_cast<const FrameDesc*>(ws + L.frames);
+  if (n > 1) {  // a single output goes with the launch
+    std::vector<uint8_t*> outs_laid(n);  // in batch layout order
+    const std::vector<int> order = encode_order(frames, n);
+    for (int j = 0; j < n; ++j) outs_laid[j] = outs[order[j]];
+    FVB_CUDA(cudaMemcpyAsync(outs_d, outs_laid.data(), sizeof(uint8_t*) * n, cudaMemcpyHostToDevice, stream));
+  }
   int64_t max_prefix = 0;
   for (int i = 0; i < n; ++i) max_prefix = frames[i].prefix_bytes > max_prefix ? frames[i].prefix_bytes : max_prefix;
-  dim3 gp(static_cast<unsigned>(ceil_div(max_prefix, 256 * 4) > 64 ? 64 : ceil_div(max_prefix, 256 * 4)), n);
+  const int64_t head_ctas = ceil_div(max_prefix, 32 * kWarpsPerCta * 8);
   const FrameState* state = reinterpret_cast<const FrameState*>(ws + L.state);
-  {
-    LaunchScope scope_(K_ENC_PREFIX, stream);
-    enc_prefix_kernel<<<gp, 256, 0, stream>>>(frames_d, state, n, reinterpret_cast<const uint8_t*>(ws + L.prefix),
-                                              reinterpret_cast<const uint8_t*>(ws + L.prefix_b), outs_d);
-  }
-  FVB_LAUNCHED("enc_prefix_kernel");
   {
     LaunchScope scope_(K_ENC_EMIT, stream);
     enc_emit_launch(cap.fold16, grid_for(t.shards, kWarpsPerCta, ctas(K_ENC_EMIT)), enc_emit_smem(), stream, state,
@@ -1034,7 +1050,12 @@ int encode_emit(const Totals& cap, const fvb_frame* frames, int n, void* workspa
                                reinterpret_cast<const uint8_t*>(ws + L.rans), t.shards},
                     EmitRegion{reinterpret_cast<const ShardInfo*>(ws + L.shards_b), ws + L.folded_b,
                                reinterpret_cast<const uint8_t*>(ws + L.rans_b), t.passes > 1 ? t.shards_p[1] : 0},
-                    t.shards, outs_d);
+                    t.shards,
+                    EmitHeads{reinterpret_cast<const FrameDesc*>(ws + L.frames),
+                              reinterpret_cast<const uint8_t*>(ws + L.prefix),
+                              reinterpret_cast<const uint8_t*>(ws + L.prefix_b), n,
+                              static_cast<int>(head_ctas > 16 ? 16 : head_ctas)},
+                    outs_d, n == 1 ? outs[0] : nullptr);
   }
   FVB_LAUNCHED("enc_emit_kernel");
   return FVB_OK;
@@ -1048,14 +1069,15 @@ int fvb_batch_encode_prepare(const fvb_frame* frames, int n, const uint16_t* con
                              void* workspace, int64_t workspace_bytes, void* cuda_stream) {
   DeviceGuard guard_;
   if (n <= 0 || !frames) return fail(FVB_ERR_ARGUMENT, "empty batch");
-  return encode_prepare(totals_of(frames, n), frames, n, planes, pitches, workspace, workspace_bytes, cuda_stream);
+  return encode_prepare(totals_of(frames, n), frames, n, planes, pitches, workspace, workspace_bytes, cuda_stream,
+                        false);
 }
 
 int fvb_batch_encode_enqueue(const fvb_frame* frames, int n, void* workspace, int64_t workspace_bytes,
                              int64_t* results, void* cuda_stream) {
   DeviceGuard guard_;
   if (n <= 0 || !frames) return fail(FVB_ERR_ARGUMENT, "empty batch");
-  return encode_enqueue(totals_of(frames, n), workspace, workspace_bytes, results, cuda_stream);
+  return encode_enqueue(totals_of(frames, n), workspace, workspace_bytes, results, cuda_stream, false);
 }
 
 int fvb_batch_encode_emit(const fvb_frame* frames, int n, void* workspace, int64_t workspace_bytes,
@@ -1071,7 +1093,7 @@ int fvb_bucket_encode_prepare(const fvb_bucket* bucket, const fvb_frame* frames,
   Totals cap;
   const int rc = from_bucket(bucket, &cap);
   if (rc) return rc;
-  return encode_prepare(cap, frames, n, planes, pitches, workspace, workspace_bytes, cuda_stream);
+  return encode_prepare(cap, frames, n, planes, pitches, workspace, workspace_bytes, cuda_stream, false);
 }
 
 int fvb_bucket_encode_enqueue(const fvb_bucket* bucket, void* workspace, int64_t workspace_bytes, int64_t* results,
@@ -1080,7 +1102,7 @@ int fvb_bucket_encode_enqueue(const fvb_bucket* bucket, void* workspace, int64_t
   Totals cap;
   const int rc = from_bucket(bucket, &cap);
   if (rc) return rc;
-  return encode_enqueue(cap, workspace, workspace_bytes, results, cuda_stream);
+  return encode_enqueue(cap, workspace, workspace_bytes, results, cuda_stream, false);
 }
 
 int fvb_bucket_encode_emit(const fvb_bucket* bucket, const fvb_frame* frames, int n, void* workspace,
@@ -1125,11 +1147,17 @@ int fvb_encode_analyze(const fvb_frame* frame, const uint16_t* const* planes, co
   if (rc) return rc;
   const uint16_t* p3[3] = {planes[0], frame->planes == 3 ? planes[1] : nullptr, frame->planes == 3 ? planes[2] : nullptr};
   const int64_t q3[3] = {pitches[0], frame->planes == 3 ? pitches[1] : 0, frame->planes == 3 ? pitches[2] : 0};
-  rc = fvb_batch_encode_prepare(frame, 1, p3, q3, workspace, workspace_bytes, cuda_stream);
+  const Totals t = totals_of(frame, 1);
+  rc = encode_prepare(t, frame, 1, p3, q3, workspace, workspace_bytes, cuda_stream, true);
   if (rc) return rc;
-  int64_t res[2] = {0, 0};
-  rc = fvb_batch_encode_enqueue(frame, 1, workspace, workspace_bytes, res, cuda_stream);
+  int64_t* res = nullptr;
+  rc = pinned_result(&res);
   if (rc) return rc;
+  rc = encode_enqueue(t, workspace, workspace_bytes, res, cuda_stream, true);
+  if (rc) {  // no kernel of this call may write the result block after it
+    cudaStreamSynchronize(static_cast<cudaStream_t>(cuda_stream));
+    return rc;
+  }
   FVB_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(cuda_stream)));
   if (res[0] != 0) return fail(static_cast<int>(res[0] < kStatusInternal ? res[0] : FVB_ERR_INTERNAL),
                                status_message_encode(res[0]));
@@ -1196,6 +1224,27 @@ int fvb_decode_plan(const uint8_t* b, int64_t header_len, int64_t size, fvb_fram
   int rc = fill_frame(frame);
   if (rc) return rc;
   if (workspace_bytes) *workspace_bytes = static_cast<int64_t>(dec_layout(totals_of(frame, 1)).total);
+  return FVB_OK;
+}
+
+int fvb_read_header(const uint8_t* stream_bytes, uint8_t* header, void* cuda_stream) {
+  DeviceGuard guard_;
+  if (!header) return fail(FVB_ERR_ARGUMENT, "null argument");
+  const int device = device_of(stream_bytes);
+  if (device < 0) return fail(FVB_ERR_ARGUMENT, "encoded stream must be device memory");
+  int cur = -1;
+  if (cudaGetDevice(&cur) != cudaSuccess || cur != device) FVB_CUDA(cudaSetDevice(device));
+  int64_t* res = nullptr;
+  const int rc = pinned_result(&res);
+  if (rc) return rc;
+  cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+  {
+    LaunchScope scope_(K_RESULTS, stream);
+    read_header_kernel<<<1, kHeaderBytes, 0, stream>>>(stream_bytes, static_cast<uint8_t*>(host_mapped(res)));
+  }
+  FVB_LAUNCHED("read_header_kernel");
+  FVB_CUDA(cudaStreamSynchronize(stream));
+  std::memcpy(header, res, kHeaderBytes);
   return FVB_OK;
 }
 
@@ -1276,9 +1325,10 @@ int fill_decode_descs(const fvb_frame* frames, int n, const uint8_t* const* stre
 }
 
 
+// `started`: as encode_prepare (state, queue and lists are zero at the start).
 int decode_prepare(const Totals& cap, const fvb_frame* frames, int n, const uint8_t* const* streams,
                    const int64_t* stream_lens, uint16_t* const* planes, const int64_t* pitches, void* workspace,
-                   int64_t workspace_bytes, void* cuda_stream) {
+                   int64_t workspace_bytes, void* cuda_stream, bool started) {
   if (n <= 0 || !frames) return fail(FVB_ERR_ARGUMENT, "empty batch");
   const Totals t = totals_of(frames, n);
   if (!fits(t, cap)) return fail(FVB_ERR_ARGUMENT, "batch does not fit the bucket");
@@ -1287,7 +1337,7 @@ int decode_prepare(const Totals& cap, const fvb_frame* frames, int n, const uint
   if (rc) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   // one upload: the dims record, then the frame table
-  std::vector<unsigned char> table(L.frames + sizeof(FrameDesc) * n);
+  std::vector<unsigned char> table(started ? L.lists + sizeof(DecodeLists) : L.frames + sizeof(FrameDesc) * n);
   const BatchDims dims = dims_of(t);
   std::memcpy(table.data() + L.dims, &dims, sizeof(dims));
   rc = fill_decode_descs(frames, n, streams, stream_lens, planes, pitches,
@@ -1301,7 +1351,7 @@ int decode_prepare(const Totals& cap, const fvb_frame* frames, int n, const uint
 // the calling thread's side stream (created on first use); the
 // allocation-free decode passes false, so it never creates a stream.
 int decode_enqueue(const Totals& t, int wavefront, void* workspace, int64_t workspace_bytes, int64_t* results,
-                   void* cuda_stream, bool side_ok) {
+                   void* cuda_stream, bool side_ok, bool started) {
   const int n = t.frames;
   const DecLayout L = dec_layout(t);
   int rc = check_ws(workspace, workspace_bytes, L.total);
@@ -1319,9 +1369,11 @@ int decode_enqueue(const Totals& t, int wavefront, void* workspace, int64_t work
   const bool f16 = t.fold16;
   DecodeLists* lists = reinterpret_cast<DecodeLists*>(ws + L.lists);
   int32_t* items = reinterpret_cast<int32_t*>(ws + L.items);
-  FVB_CUDA(cudaMemsetAsync(state, 0, sizeof(FrameState) * n, stream));
-  FVB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), stream));
-  FVB_CUDA(cudaMemsetAsync(lists, 0, sizeof(DecodeLists), stream));
+  // state, queue and lists lie one after another
+  if (!started) FVB_CUDA(cudaMemsetAsync(state, 0, L.lists + sizeof(DecodeLists) - L.state, stream));
+  int64_t* res_d = reinterpret_cast<int64_t*>(ws + L.results);
+  int64_t* direct = static_cast<int64_t*>(host_mapped(results));  // pinned: written by the kernels
+  if (direct) res_d = direct;
   {
     LaunchScope scope_(K_DEC_PARSE, stream);
     dec_parse_kernel<<<grid_for(t.tiles, 128, ctas(K_DEC_PARSE)), 128, 0, stream>>>(frames_d, state, dims, shards, lists,
@@ -1373,7 +1425,7 @@ int decode_enqueue(const Totals& t, int wavefront, void* workspace, int64_t work
       // the SMs; the warps take tiles from the queue
       const int grid = grid_for(f16 ? t.tiles : t.tiles * tw, f16 ? 1 : kWarpsPerCta, ctas(K_DEC_RECON));
       dec_reconstruct_launch(g_wavefront_block.load(std::memory_order_relaxed), tw, f16, grid, stream,
-                             frames_d, state, dims, folded, queue);
+                             frames_d, state, dims, folded, queue, res_d);
     }
     FVB_LAUNCHED("dec_reconstruct_kernel");
     if (t.wide) {
@@ -1388,17 +1440,10 @@ int decode_enqueue(const Totals& t, int wavefront, void* workspace, int64_t work
     {
       LaunchScope scope_(K_DEC_RECON_SERIAL, stream);
       dec_reconstruct_serial_kernel<<<static_cast<int>(ceil_div(t.tiles, 128)), 128, 0, stream>>>(
-          frames_d, state, dims, folded, f16 ? 1 : 0);
+          frames_d, state, dims, folded, f16 ? 1 : 0, res_d);
     }
     FVB_LAUNCHED("dec_reconstruct_serial_kernel");
   }
-  int64_t* res_d = reinterpret_cast<int64_t*>(ws + L.results);
-  int64_t* direct = static_cast<int64_t*>(host_mapped(results));  // pinned: written by the kernel
-  {
-    LaunchScope scope_(K_RESULTS, stream);
-    results_kernel<<<(n + 127) / 128, 128, 0, stream>>>(frames_d, state, dims, direct ? direct : res_d, 1);
-  }
-  FVB_LAUNCHED("results_kernel");
   if (results && !direct)
     FVB_CUDA(cudaMemcpyAsync(results, res_d, 16 * static_cast<size_t>(n), cudaMemcpyDeviceToHost, stream));
   return FVB_OK;
@@ -1415,14 +1460,14 @@ int fvb_batch_decode_prepare(const fvb_frame* frames, int n, const uint8_t* cons
   DeviceGuard guard_;
   if (n <= 0 || !frames) return fail(FVB_ERR_ARGUMENT, "empty batch");
   return decode_prepare(totals_of(frames, n), frames, n, streams, stream_lens, planes, pitches, workspace,
-                        workspace_bytes, cuda_stream);
+                        workspace_bytes, cuda_stream, false);
 }
 
 int fvb_batch_decode_enqueue(const fvb_frame* frames, int n, int wavefront, void* workspace, int64_t workspace_bytes,
                              int64_t* results, void* cuda_stream) {
   DeviceGuard guard_;
   if (n <= 0 || !frames) return fail(FVB_ERR_ARGUMENT, "empty batch");
-  return decode_enqueue(totals_of(frames, n), wavefront, workspace, workspace_bytes, results, cuda_stream, true);
+  return decode_enqueue(totals_of(frames, n), wavefront, workspace, workspace_bytes, results, cuda_stream, true, false);
 }
 
 int fvb_bucket_decode_prepare(const fvb_bucket* bucket, const fvb_frame* frames, int n, const uint8_t* const* streams,
@@ -1433,7 +1478,7 @@ int fvb_bucket_decode_prepare(const fvb_bucket* bucket, const fvb_frame* frames,
   const int rc = from_bucket(bucket, &cap);
   if (rc) return rc;
   return decode_prepare(cap, frames, n, streams, stream_lens, planes, pitches, workspace, workspace_bytes,
-                        cuda_stream);
+                        cuda_stream, false);
 }
 
 int fvb_bucket_decode_enqueue(const fvb_bucket* bucket, int wavefront, void* workspace, int64_t workspace_bytes,
@@ -1442,7 +1487,7 @@ int fvb_bucket_decode_enqueue(const fvb_bucket* bucket, int wavefront, void* wor
   Totals cap;
   const int rc = from_bucket(bucket, &cap);
   if (rc) return rc;
-  return decode_enqueue(cap, wavefront, workspace, workspace_bytes, results, cuda_stream, true);
+  return decode_enqueue(cap, wavefront, workspace, workspace_bytes, results, cuda_stream, true, false);
 }
 
 int fvb_decode(const fvb_frame* frame, const uint8_t* stream, int64_t stream_len, uint16_t* const* planes,
@@ -1455,11 +1500,17 @@ int fvb_decode(const fvb_frame* frame, const uint8_t* stream, int64_t stream_len
   const int64_t q3[3] = {pitches[0], frame->planes == 3 ? pitches[1] : 0, frame->planes == 3 ? pitches[2] : 0};
   const uint8_t* s1[1] = {stream};
   const int64_t l1[1] = {stream_len};
-  rc = fvb_batch_decode_prepare(frame, 1, s1, l1, p3, q3, workspace, workspace_bytes, cuda_stream);
+  const Totals t = totals_of(frame, 1);
+  rc = decode_prepare(t, frame, 1, s1, l1, p3, q3, workspace, workspace_bytes, cuda_stream, true);
   if (rc) return rc;
-  int64_t res[2] = {0, 0};
-  rc = fvb_batch_decode_enqueue(frame, 1, wavefront, workspace, workspace_bytes, res, cuda_stream);
+  int64_t* res = nullptr;
+  rc = pinned_result(&res);
   if (rc) return rc;
+  rc = decode_enqueue(t, wavefront, workspace, workspace_bytes, res, cuda_stream, true, true);
+  if (rc) {  // no kernel of this call may write the result block after it
+    cudaStreamSynchronize(static_cast<cudaStream_t>(cuda_stream));
+    return rc;
+  }
   FVB_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(cuda_stream)));
   if (res[0] != 0) {
     char buf[96];
@@ -1560,7 +1611,7 @@ int fvb_decode_noalloc(const fvb_frame* frame, const uint8_t* stream, int64_t st
   FVB_CUDA(cudaMemcpyAsync(static_cast<char*>(scratch) + L.frames, &desc, sizeof(FrameDesc), cudaMemcpyHostToDevice,
                            cs));
   // no side stream: dec_other runs on the caller's stream, so nothing is created
-  rc = decode_enqueue(t, wavefront, scratch, static_cast<int64_t>(kNoAllocScratchBytes), res, cuda_stream, false);
+  rc = decode_enqueue(t, wavefront, scratch, static_cast<int64_t>(kNoAllocScratchBytes), res, cuda_stream, false, false);
   if (rc) return rc;
   FVB_CUDA(cudaStreamSynchronize(cs));
   if (res[0] != 0) {

@@ -1365,6 +1365,18 @@ __device__ void rec_tile(const FrameDesc& f, const TileGeo& g, int32_t step, con
   }
 }
 
+// The frames' statuses, final once the entropy decoders are done, by the first
+// CTA of the reconstruction.
+__device__ __forceinline__ void write_results(const FrameDesc* frames, const FrameState* state, int nframes,
+                                              int64_t* results) {
+  if (blockIdx.x != 0) return;
+  for (int i = threadIdx.x; i < nframes; i += blockDim.x) {
+    const int slot = frames[i].slot;
+    results[2 * slot] = state[i].status;
+    results[2 * slot + 1] = 0;
+  }
+}
+
 // Tiles come from a queue.  With warp pairs, the pair's first warp claims a
 // tile and both read it after the pair barrier (two alternating slots, so a
 // claim never overwrites a tile the other warp has yet to read); both then
@@ -1373,10 +1385,11 @@ template <int UNROLL, bool PAIRS, typename FoldT>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, PAIRS ? 3 : 4)
 dec_reconstruct_kernel(const FrameDesc* __restrict__ frames, const FrameState* __restrict__ state,
                        const BatchDims* __restrict__ dims, const FoldT* __restrict__ folded,
-                       int* __restrict__ queue) {
+                       int* __restrict__ queue, int64_t* __restrict__ results) {
   static_assert(kWarpsPerCta % 2 == 0, "warp pairs");
   constexpr bool pairs = PAIRS;
   const int nframes = dims->frames_p[0];
+  write_results(frames, state, nframes, results);
   const int64_t total_tiles = dims->tiles_p[0];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int64_t claimed[kWarpsPerCta / 2][2];
@@ -1523,8 +1536,9 @@ __device__ void rec_wave_tile(const FrameDesc& f, const TileGeo& g, const uint16
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
 dec_reconstruct_wave_kernel(const FrameDesc* __restrict__ frames, const FrameState* __restrict__ state,
                             const BatchDims* __restrict__ dims, const uint16_t* __restrict__ folded,
-                            int* __restrict__ queue) {
+                            int* __restrict__ queue, int64_t* __restrict__ results) {
   const int nframes = dims->frames_p[0];
+  write_results(frames, state, nframes, results);
   const int64_t total_tiles = dims->tiles_p[0];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1577,10 +1591,10 @@ cudaError_t dec_reconstruct_set_smem() {
 
 void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, int grid, cudaStream_t stream,
                             const FrameDesc* frames, const FrameState* state, const BatchDims* dims,
-                            const void* folded, int* queue) {
+                            const void* folded, int* queue, int64_t* results) {
   if (fold16) {
     dec_reconstruct_wave_kernel<<<grid, kWarpsPerCta * 32, dec_reconstruct_smem(true), stream>>>(
-        frames, state, dims, static_cast<const uint16_t*>(folded), queue);
+        frames, state, dims, static_cast<const uint16_t*>(folded), queue, results);
     return;
   }
   // warp pairs run with the default wavefront block
@@ -1590,7 +1604,7 @@ void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, int grid, c
            : unroll == 32  ? dec_reconstruct_kernel<32, false, uint32_t>
                            : dec_reconstruct_kernel<8, false, uint32_t>;
   k<<<grid, kWarpsPerCta * 32, dec_reconstruct_smem(false), stream>>>(
-      frames, state, dims, static_cast<const uint32_t*>(folded), queue);
+      frames, state, dims, static_cast<const uint32_t*>(folded), queue, results);
 }
 
 void dec_rans_launch(bool fold16, bool few, int grid, cudaStream_t stream, const FrameDesc* frames,
@@ -1690,8 +1704,9 @@ __global__ void dec_reconstruct_wide_kernel(const FrameDesc* __restrict__ frames
 // predictor="serial": one thread per tile in raster order (decode.cu:608-656).
 __global__ void dec_reconstruct_serial_kernel(const FrameDesc* __restrict__ frames, const FrameState* __restrict__ state,
                                               const BatchDims* __restrict__ dims, const void* __restrict__ folded,
-                                              int fold16) {
+                                              int fold16, int64_t* __restrict__ results) {
   const int nframes = dims->frames_p[0];
+  write_results(frames, state, nframes, results);
   const int64_t total_tiles = dims->tiles_p[0];
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= total_tiles) return;

@@ -1638,7 +1638,7 @@ __device__ __forceinline__ void put32(uint8_t* p, uint32_t v) {
 __global__ void __launch_bounds__(1024)
 enc_scan_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
                 const BatchDims* __restrict__ dims, int pass, ShardInfo* __restrict__ shards,
-                uint8_t* __restrict__ prefix) {
+                uint8_t* __restrict__ prefix, int64_t* __restrict__ results) {
   const int nframes = dims->frames_p[pass];
   __shared__ int64_t warp_tot[32];
   __shared__ int64_t carry_s;
@@ -1789,6 +1789,9 @@ enc_scan_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
     // policy asked for it.
     if (st.status != 0) next = 0;
     st.active = next;
+    // the frame's status and stream length (a later pass overwrites them)
+    results[2 * f.slot] = st.status;
+    results[2 * f.slot + 1] = st.stream_len;
   }
 }
 
@@ -1965,15 +1968,29 @@ __device__ __forceinline__ void put_words(uint32_t* buf, int pos, uint32_t v, in
   if (sh && w + 1 < kEmitWords) atomicOr(&buf[w + 1], v >> (32 - sh));
 }
 
+// The first heads.ctas * heads.frames CTAs copy the frames' headers and
+// directories instead (from the region whose records the frame emits).
 template <typename FoldT>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 enc_emit_kernel(const FrameState* __restrict__ state, EmitRegion ra, EmitRegion rb, int64_t total_shards,
-                uint8_t* const* __restrict__ outs) {
+                EmitHeads heads, uint8_t* const* __restrict__ outs, uint8_t* __restrict__ only_out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int head_ctas = heads.ctas * heads.frames;
+  if (static_cast<int>(blockIdx.x) < head_ctas) {
+    const int fi = blockIdx.x / heads.ctas;
+    const FrameDesc& f = heads.descs[fi];
+    const uint8_t* src = (state[fi].final_b ? heads.prefix_b : heads.prefix) + f.prefix_base;
+    uint8_t* dst = only_out ? only_out : outs[fi];
+    for (int64_t i = static_cast<int64_t>(blockIdx.x % heads.ctas) * blockDim.x + threadIdx.x; i < f.prefix_bytes;
+         i += static_cast<int64_t>(heads.ctas) * blockDim.x)
+      dst[i] = src[i];
+    return;
+  }
   uint32_t* buf = reinterpret_cast<EmitWarpSmem*>(smem_raw)[warp].buf;
-  const int64_t warps_total = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
-  for (int64_t s = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + warp; s < total_shards; s += warps_total) {
+  const int64_t warps_total = static_cast<int64_t>(gridDim.x - head_ctas) * kWarpsPerCta;
+  for (int64_t s = static_cast<int64_t>(blockIdx.x - head_ctas) * kWarpsPerCta + warp; s < total_shards;
+       s += warps_total) {
     // the frame's records: pass 0's, or its later pass's (the shard record
     // of pass 0 names the frame either way).  Frames with a later pass come
     // first, so shards past region b's count skip the frame lookup.
@@ -1988,7 +2005,7 @@ enc_emit_kernel(const FrameState* __restrict__ state, EmitRegion ra, EmitRegion 
     const FoldT* __restrict__ folded = static_cast<const FoldT*>(from_b ? rb.folded : ra.folded);
     const uint8_t* __restrict__ rans_scratch = from_b ? rb.rans_scratch : ra.rans_scratch;
     const int mode = si.mode, k = si.param, body = si.body, n = si.count;
-    uint8_t* const dst_base = outs[si.frame];  // loaded now, used at the copy-out
+    uint8_t* const dst_base = only_out ? only_out : outs[si.frame];  // loaded now, used at the copy-out
     const int rec_len = min(body + 3, kMaxRecordBytes);
     const int nwords = (rec_len + 3) >> 2;
     // clear words 0 .. nwords (one past the record: the copy-out reads it)
@@ -2222,30 +2239,15 @@ enc_emit_kernel(const FrameState* __restrict__ state, EmitRegion ra, EmitRegion 
   }
 }
 
-// Header + directory bytes of every frame into its output buffer (from the
-// region whose records the frame emits).
-__global__ void enc_prefix_kernel(const FrameDesc* __restrict__ frames, const FrameState* __restrict__ state,
-                                  int nframes, const uint8_t* __restrict__ prefix, const uint8_t* __restrict__ prefix_b,
-                                  uint8_t* const* __restrict__ outs) {
-  const int fi = blockIdx.y;
-  if (fi >= nframes) return;
-  const FrameDesc& f = frames[fi];
-  const uint8_t* src = (state[fi].final_b ? prefix_b : prefix) + f.prefix_base;
-  uint8_t* dst = outs[fi];
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < f.prefix_bytes;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    dst[i] = src[i];
-}
-
-}  // namespace fvb
-
-namespace fvb {
-void enc_emit_launch(bool fold16, int grid, size_t smem, cudaStream_t stream, const FrameState* state,
-                     EmitRegion a, EmitRegion b, int64_t total_shards, uint8_t* const* outs) {
+void enc_emit_launch(bool fold16, int grid, size_t smem, cudaStream_t stream, const FrameState* state, EmitRegion a,
+                     EmitRegion b, int64_t total_shards, EmitHeads heads, uint8_t* const* outs, uint8_t* only_out) {
+  grid += heads.ctas * heads.frames;
   if (fold16)
-    enc_emit_kernel<uint16_t><<<grid, kWarpsPerCta * 32, smem, stream>>>(state, a, b, total_shards, outs);
+    enc_emit_kernel<uint16_t><<<grid, kWarpsPerCta * 32, smem, stream>>>(state, a, b, total_shards, heads, outs,
+                                                                         only_out);
   else
-    enc_emit_kernel<uint32_t><<<grid, kWarpsPerCta * 32, smem, stream>>>(state, a, b, total_shards, outs);
+    enc_emit_kernel<uint32_t><<<grid, kWarpsPerCta * 32, smem, stream>>>(state, a, b, total_shards, heads, outs,
+                                                                         only_out);
 }
 
 cudaError_t enc_emit_set_smem(int bytes) {

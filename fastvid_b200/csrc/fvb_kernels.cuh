@@ -112,7 +112,7 @@ void enc_analyze_launch(bool fold16, int grid, cudaStream_t stream, const FrameD
 void enc_rans_launch(bool fold16, int64_t nshards, cudaStream_t stream, const FrameState* state, const BatchDims* dims,
                      int pass, ShardInfo* shards, const void* folded, uint8_t* rans_scratch);
 __global__ void enc_scan_kernel(const FrameDesc* frames, FrameState* state, const BatchDims* dims, int pass,
-                                ShardInfo* shards, uint8_t* prefix);
+                                ShardInfo* shards, uint8_t* prefix, int64_t* results);
 // Records of one encoder region: pass 0's, or the later pass's (region b,
 // indexed like pass 0's for the frames that took part in it).
 struct EmitRegion {
@@ -121,12 +121,17 @@ struct EmitRegion {
   const uint8_t* rans_scratch;
   int64_t count;  // shards 0 .. count-1 have records in this region
 };
-void enc_emit_launch(bool fold16, int grid, size_t smem, cudaStream_t stream, const FrameState* state,
-                     EmitRegion a, EmitRegion b, int64_t total_shards, uint8_t* const* outs);
+// The frames' headers and directories, copied by `ctas` CTAs a frame.
+struct EmitHeads {
+  const FrameDesc* descs;
+  const uint8_t* prefix;
+  const uint8_t* prefix_b;
+  int frames, ctas;
+};
+// `only_out`: the output of a batch of one frame (null: the table `outs`)
+void enc_emit_launch(bool fold16, int grid, size_t smem, cudaStream_t stream, const FrameState* state, EmitRegion a,
+                     EmitRegion b, int64_t total_shards, EmitHeads heads, uint8_t* const* outs, uint8_t* only_out);
 cudaError_t enc_emit_set_smem(int bytes);
-__global__ void enc_prefix_kernel(const FrameDesc* frames, const FrameState* state, int nframes, const uint8_t* prefix,
-                                  const uint8_t* prefix_b, uint8_t* const* outs);
-
 // decoder: shards binned by mode (0 rANS, 1 Rice, 2 zero-run, 3 block pack);
 // counts from dims (entry 0)
 struct DecodeLists {
@@ -150,15 +155,17 @@ void dec_other_launch(bool fold16, int grid, cudaStream_t stream, const FrameDes
                       const ShardInfo* shards, const BatchDims* dims, DecodeLists* lists, const int32_t* list_items,
                       void* folded);
 // u32 symbols: `unroll` and `tile_warps` as for enc_predict
+// (every reconstruction kernel also writes the frames' statuses to `results`)
 void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, int grid, cudaStream_t stream,
                             const FrameDesc* frames, const FrameState* state, const BatchDims* dims,
-                            const void* folded, int* queue);
+                            const void* folded, int* queue, int64_t* results);
 cudaError_t dec_other_set_smem();
 cudaError_t dec_reconstruct_set_smem();
 __global__ void dec_reconstruct_wide_kernel(const FrameDesc* frames, const FrameState* state, const BatchDims* dims,
                                             const void* folded, int fold16);
 __global__ void dec_reconstruct_serial_kernel(const FrameDesc* frames, const FrameState* state,
-                                              const BatchDims* dims, const void* folded, int fold16);
+                                              const BatchDims* dims, const void* folded, int fold16,
+                                              int64_t* results);
 
 size_t enc_predict_smem(bool fold16);
 size_t enc_emit_smem();

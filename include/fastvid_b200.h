@@ -193,6 +193,10 @@ int fvb_batch_encode_enqueue(const fvb_frame* frames, int n, void* workspace, in
 int fvb_batch_encode_emit(const fvb_frame* frames, int n, void* workspace, int64_t workspace_bytes,
                           uint8_t* const* outs, void* cuda_stream);
 
+/* Copies the first 32 bytes of one device stream (of at least 32) into host
+ * `header`, in the order of `cuda_stream`, and waits for it. */
+int fvb_read_header(const uint8_t* stream, uint8_t* header, void* cuda_stream);
+
 /* Copies the 32-byte header of each device stream into host `headers`
  * (32 * n bytes) with one gather kernel (which writes page-locked
  * `headers` directly, other memory through one copy), and waits for it.
