@@ -476,8 +476,8 @@ int from_bucket(const fvb_bucket* b, Totals* t) {
 // the frames that take part in pass 1: a prefix of the batch, so the same
 // global shard and sample indices address both regions).
 struct EncLayout {
-  size_t dims, frames, state, queue, outs, results, shards, folded, rans, prefix, recon;
-  size_t shards_b, folded_b, rans_b, prefix_b, total;
+  size_t dims, frames, state, queue, outs, results, shards, sizes, folded, rans, prefix, recon;
+  size_t shards_b, sizes_b, folded_b, rans_b, prefix_b, total;
 };
 
 EncLayout enc_layout(const Totals& t) {
@@ -496,12 +496,14 @@ EncLayout enc_layout(const Totals& t) {
   w.outs = take(sizeof(uint8_t*) * n);
   w.results = take(16 * static_cast<size_t>(n));
   w.shards = take(sizeof(ShardInfo) * t.shards);
+  w.sizes = take(sizeof(int32_t) * t.shards);
   w.folded = take((t.fold16 ? 2 : 4) * static_cast<size_t>(t.samples));
   w.rans = take(static_cast<size_t>(kRansScratchBytes) * t.shards);
   w.prefix = take(static_cast<size_t>(t.prefix));
   w.recon = take(t.wide ? 2 * static_cast<size_t>(t.samples) : 0);
   const bool later = t.passes > 1;
   w.shards_b = take(later ? sizeof(ShardInfo) * t.shards_p[1] : 0);
+  w.sizes_b = take(later ? sizeof(int32_t) * t.shards_p[1] : 0);
   w.folded_b = take(later ? (t.fold16 ? 2 : 4) * static_cast<size_t>(t.samples_p[1]) : 0);
   w.rans_b = take(later ? static_cast<size_t>(kRansScratchBytes) * t.shards_p[1] : 0);
   w.prefix_b = take(later ? static_cast<size_t>(t.prefix_p[1]) : 0);
@@ -965,6 +967,7 @@ int encode_enqueue(const Totals& cap, void* workspace, int64_t workspace_bytes, 
     const int nf = cap.frames_p[pass];
     const int64_t tiles = cap.tiles_p[pass], nsh = cap.shards_p[pass];
     ShardInfo* shards = reinterpret_cast<ShardInfo*>(ws + (pass ? L.shards_b : L.shards));
+    int32_t* sizes = reinterpret_cast<int32_t*>(ws + (pass ? L.sizes_b : L.sizes));
     void* folded = ws + (pass ? L.folded_b : L.folded);
     uint8_t* rans = reinterpret_cast<uint8_t*>(ws + (pass ? L.rans_b : L.rans));
     uint8_t* prefix = reinterpret_cast<uint8_t*>(ws + (pass ? L.prefix_b : L.prefix));
@@ -1003,12 +1006,12 @@ int encode_enqueue(const Totals& cap, void* workspace, int64_t workspace_bytes, 
     FVB_LAUNCHED("enc_analyze_kernel");
     {
       LaunchScope scope_(K_ENC_RANS, stream);
-      enc_rans_launch(f16, nsh, stream, state, dims, pass, shards, folded, rans);
+      enc_rans_launch(f16, nsh, stream, frames_d, state, dims, pass, shards, sizes, folded, rans);
     }
     FVB_LAUNCHED("enc_rans_kernel");
     {
       LaunchScope scope_(K_ENC_SCAN, stream);
-      enc_scan_kernel<<<nf > 0 ? nf : 1, 1024, 0, stream>>>(frames_d, state, dims, pass, shards, prefix,
+      enc_scan_kernel<<<nf > 0 ? nf : 1, 1024, 0, stream>>>(frames_d, state, dims, pass, shards, sizes, prefix,
                                                                 res_d);
     }
     FVB_LAUNCHED("enc_scan_kernel");
@@ -1538,7 +1541,22 @@ int fvb_decode(const fvb_frame* frame, const uint8_t* stream, int64_t stream_len
 namespace {
 
 constexpr size_t kNoAllocScratchBytes = size_t{32} << 20;  // 32 MiB
-__device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
+// Frames are admitted by the charge below, which counts samples without the
+// padding of their tiles: at most 28 bytes a tile, and a tile is charged at
+// least the 2,232 bytes of a shard, so half a MiB covers the padding of any
+// admitted frame.
+constexpr size_t kNoAllocPadding = size_t{512} << 10;
+__device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes + kNoAllocPadding];
+
+// Scratch charged to a frame: 2,232 bytes a shard (its record, list entries and
+// table) and its samples' symbols, each array rounded up, and the frame's
+// fixed records.
+size_t noalloc_charge(const fvb_frame& f, bool fold16) {
+  constexpr size_t kFixed = 7 * kAlign;
+  const size_t shards = static_cast<size_t>(f.shards);
+  return kFixed + align_up(104 * shards) + align_up(16 * shards) + align_up(2112 * shards) +
+         align_up((fold16 ? 2 : 4) * static_cast<size_t>(f.samples));
+}
 
 std::mutex g_noalloc_mutex;
 void* g_noalloc_address[64] = {nullptr};
@@ -1579,12 +1597,13 @@ int fvb_decode_noalloc(const fvb_frame* frame, const uint8_t* stream, int64_t st
   if (!frame || !stream || !planes || !pitches) return fail(FVB_ERR_ARGUMENT, "null argument");
   const Totals t = totals_of(frame, 1);
   const DecLayout L = dec_layout(t);
-  if (L.total > kNoAllocScratchBytes) {
+  const size_t charge = noalloc_charge(*frame, t.fold16);
+  if (charge > kNoAllocScratchBytes || L.total > kNoAllocScratchBytes + kNoAllocPadding) {
     char buf[192];
     std::snprintf(buf, sizeof(buf),
                   "frame needs %zu bytes of decode scratch; the allocation-free decode has %zu "
                   "(frames up to about 7 million samples)",
-                  L.total, kNoAllocScratchBytes);
+                  charge, kNoAllocScratchBytes);
     return fail(FVB_ERR_WORKSPACE, buf);
   }
   int rc = check_decode_pointers(frame, stream, planes);
@@ -1601,7 +1620,7 @@ int fvb_decode_noalloc(const fvb_frame* frame, const uint8_t* stream, int64_t st
   cudaStream_t cs = static_cast<cudaStream_t>(cuda_stream);
   int64_t res[2] = {0, 0};
   FrameDesc desc;
-  rc = check_ws(scratch, static_cast<int64_t>(kNoAllocScratchBytes), L.total);
+  rc = check_ws(scratch, static_cast<int64_t>(kNoAllocScratchBytes + kNoAllocPadding), L.total);
   if (rc) return rc;
   rc = fill_decode_descs(frame, 1, s1, l1, p3, q3, &desc);
   if (rc) return rc;
@@ -1611,7 +1630,7 @@ int fvb_decode_noalloc(const fvb_frame* frame, const uint8_t* stream, int64_t st
   FVB_CUDA(cudaMemcpyAsync(static_cast<char*>(scratch) + L.frames, &desc, sizeof(FrameDesc), cudaMemcpyHostToDevice,
                            cs));
   // no side stream: dec_other runs on the caller's stream, so nothing is created
-  rc = decode_enqueue(t, wavefront, scratch, static_cast<int64_t>(kNoAllocScratchBytes), res, cuda_stream, false, false);
+  rc = decode_enqueue(t, wavefront, scratch, static_cast<int64_t>(kNoAllocScratchBytes + kNoAllocPadding), res, cuda_stream, false, false);
   if (rc) return rc;
   FVB_CUDA(cudaStreamSynchronize(cs));
   if (res[0] != 0) {

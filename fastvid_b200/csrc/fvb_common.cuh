@@ -138,7 +138,6 @@ struct ShardInfo {
   int32_t comp_lane[4];  // encode: Rice lane bytes of the competition winner
   int32_t rans_ok;       // encode: shard is rANS eligible
   int32_t rans_table;    // encode: serialised table bytes
-  int32_t rans_lane[4];  // encode: rANS lane bytes
   uint32_t rans_state[4];
 };
 

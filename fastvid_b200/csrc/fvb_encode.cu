@@ -1390,7 +1390,7 @@ enc_analyze_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict_
           ser[c++] = byte;
         } while (d);
         si.rans_table = static_cast<int32_t>(c_cursor);
-        si.param = static_cast<int32_t>(shard_max);  // for enc_rans; enc_scan sets the mode's
+        si.param = static_cast<int32_t>(shard_max);  // for enc_rans, which sets the mode's
       }
       // Skip the trial encoding when it cannot win.  Each rANS step takes a
       // state x in [f 2^11, f 2^19) after renormalisation to one at least
@@ -1557,11 +1557,16 @@ __device__ __forceinline__ void rans_encode_lane(RansLane& st, const FoldT* __re
     if (m > i) run(fetch(r[i]));
 }
 
+// The kernel also makes each shard's final choice of mode (encode.cu:420-430 and
+// the kernel order at :789-805) and writes its record's size to `sizes`, one
+// word a shard: enc_scan, one CTA a frame, then reads those instead of the
+// shard records (32 lines for every field of a warp's records: 13 us for the
+// 1,539 shards of a 1080p frame, SCAN_US now).
 template <typename FoldT>
 __global__ void __launch_bounds__(128)
-enc_rans_kernel(const FrameState* __restrict__ state, const BatchDims* __restrict__ dims, int pass,
-                ShardInfo* __restrict__ shards, const FoldT* __restrict__ folded,
-                uint8_t* __restrict__ rans_scratch) {
+enc_rans_kernel(const FrameDesc* __restrict__ frames, const FrameState* __restrict__ state,
+                const BatchDims* __restrict__ dims, int pass, ShardInfo* __restrict__ shards,
+                int32_t* __restrict__ sizes, const FoldT* __restrict__ folded, uint8_t* __restrict__ rans_scratch) {
   // entry of value v of shard j: local[v][j], so that the shards' lookups fall
   // in different banks
   __shared__ uint2 local_all[4][kEncLocal][8];
@@ -1569,7 +1574,8 @@ enc_rans_kernel(const FrameState* __restrict__ state, const BatchDims* __restric
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, j = lane >> 2, l = lane & 3;
   const int64_t s = (static_cast<int64_t>(blockIdx.x) * 4 + warp) * 8 + j;
   uint2 (*local)[8] = local_all[warp];
-  const bool live = s < total_shards && state[shards[s].frame].active && shards[s].rans_ok;
+  const bool mine = s < total_shards && state[shards[s].frame].active;
+  const bool live = mine && shards[s].rans_ok;
   const int top = live ? shards[s].param : 0;  // the shard's largest value
   uint8_t* base = rans_scratch + s * static_cast<int64_t>(kRansScratchBytes);
   const uint2* __restrict__ tab = reinterpret_cast<const uint2*>(base);
@@ -1584,31 +1590,54 @@ enc_rans_kernel(const FrameState* __restrict__ state, const BatchDims* __restric
   const int count = live ? shards[s].count : -1;
   const int count0 = __shfl_sync(kFull, count, 0);  // by all lanes: not inside the condition
   const bool in_step = __all_sync(kFull, count >= 0 && count == count0);
-  if (!live) return;
-  ShardInfo& si = shards[s];
-  const FoldT* __restrict__ f = folded + si.sample_base;
-  uint32_t* end = reinterpret_cast<uint32_t*>(base + kRansTableWords * 4 + kRansSerialBytes + (l + 1) * kRansLaneBytes);
-  RansLane st;
-  st.out = end;
-  if (in_step) {
-    if (all_local) rans_encode_lane<true, true>(st, f, si.count, tab, local, j, l);
-    else rans_encode_lane<false, true>(st, f, si.count, tab, local, j, l);
-  } else {
-    rans_encode_lane<false, false>(st, f, si.count, tab, local, j, l);
+  ShardInfo& si = shards[mine ? s : 0];
+  int lane_bytes = 0;
+  if (live) {
+    const FoldT* __restrict__ f = folded + si.sample_base;
+    uint32_t* end = reinterpret_cast<uint32_t*>(base + kRansTableWords * 4 + kRansSerialBytes + (l + 1) * kRansLaneBytes);
+    RansLane st;
+    st.out = end;
+    if (in_step) {
+      if (all_local) rans_encode_lane<true, true>(st, f, count, tab, local, j, l);
+      else rans_encode_lane<false, true>(st, f, count, tab, local, j, l);
+    } else {
+      rans_encode_lane<false, false>(st, f, count, tab, local, j, l);
+    }
+    if (st.bits) *(st.out - 1) = __byte_perm(st.hi >> (32 - st.bits), 0, 0x0123);  // low bytes unused
+    lane_bytes = 4 * static_cast<int>(end - st.out) + (st.bits >> 3);
+    si.rans_state[l] = st.x;
   }
-  if (st.bits) *(st.out - 1) = __byte_perm(st.hi >> (32 - st.bits), 0, 0x0123);  // low bytes unused
-  si.rans_lane[l] = 4 * static_cast<int>(end - st.out) + (st.bits >> 3);
-  si.rans_state[l] = st.x;
+  __syncwarp();
+  int bytes = lane_bytes + __shfl_xor_sync(kFull, lane_bytes, 1);
+  bytes += __shfl_xor_sync(kFull, bytes, 2);
+  if (!mine) return;
+  int mode = si.comp_mode, k = si.comp_k, body = si.comp_body;
+  if (live) {
+    const int rb = si.rans_table + 28 + bytes;
+    if (frames[si.frame].force_order0 || rb < body) {
+      mode = kModeOrder0;
+      k = kRansTableLog;
+      body = rb;
+      si.comp_lane[l] = lane_bytes;
+    }
+  }
+  if (l == 0) {
+    si.mode = mode;
+    si.param = k;
+    si.body = body;
+    sizes[s] = body + 3;
+  }
 }
 
-void enc_rans_launch(bool fold16, int64_t nshards, cudaStream_t stream, const FrameState* state, const BatchDims* dims,
-                     int pass, ShardInfo* shards, const void* folded, uint8_t* rans_scratch) {
+void enc_rans_launch(bool fold16, int64_t nshards, cudaStream_t stream, const FrameDesc* frames,
+                     const FrameState* state, const BatchDims* dims, int pass, ShardInfo* shards, int32_t* sizes,
+                     const void* folded, uint8_t* rans_scratch) {
   const int grid = static_cast<int>(nshards > 0 ? (nshards + 31) / 32 : 1);
   if (fold16)
-    enc_rans_kernel<uint16_t><<<grid, 128, 0, stream>>>(state, dims, pass, shards,
+    enc_rans_kernel<uint16_t><<<grid, 128, 0, stream>>>(frames, state, dims, pass, shards, sizes,
                                                         static_cast<const uint16_t*>(folded), rans_scratch);
   else
-    enc_rans_kernel<uint32_t><<<grid, 128, 0, stream>>>(state, dims, pass, shards,
+    enc_rans_kernel<uint32_t><<<grid, 128, 0, stream>>>(frames, state, dims, pass, shards, sizes,
                                                         static_cast<const uint32_t*>(folded), rans_scratch);
 }
 
@@ -1624,21 +1653,13 @@ void enc_analyze_launch(bool fold16, int grid, cudaStream_t stream, const FrameD
 }
 
 // ---------------------------------------------------------------------------
-// enc_scan: one CTA per frame.  Final mode choice (encode.cu:420-430 and the
-// kernel order at :789-805), exclusive scan of record sizes in shard order
-// (:858-867), directory and header bytes (:871-904), frame policy (:812-847).
-
-__device__ __forceinline__ void put32(uint8_t* p, uint32_t v) {
-  p[0] = static_cast<uint8_t>(v);
-  p[1] = static_cast<uint8_t>(v >> 8);
-  p[2] = static_cast<uint8_t>(v >> 16);
-  p[3] = static_cast<uint8_t>(v >> 24);
-}
+// enc_scan: one CTA per frame.  Exclusive scan of record sizes in shard order
+// (encode.cu:858-867), directory and header bytes (:871-904), frame policy (:812-847).
 
 __global__ void __launch_bounds__(1024)
 enc_scan_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
                 const BatchDims* __restrict__ dims, int pass, ShardInfo* __restrict__ shards,
-                uint8_t* __restrict__ prefix, int64_t* __restrict__ results) {
+                const int32_t* __restrict__ sizes, uint8_t* __restrict__ prefix, int64_t* __restrict__ results) {
   const int nframes = dims->frames_p[pass];
   __shared__ int64_t warp_tot[32];
   __shared__ int64_t carry_s;
@@ -1654,31 +1675,7 @@ enc_scan_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
   for (int64_t base = 0; base < f.nshards; base += blockDim.x) {
     const int64_t s = base + threadIdx.x;
     int64_t rec = 0;
-    if (s < f.nshards) {
-      ShardInfo& si = fs[s];
-      int mode = si.comp_mode, k = si.comp_k, body = si.comp_body;
-      int lanes[4] = {si.comp_lane[0], si.comp_lane[1], si.comp_lane[2], si.comp_lane[3]};
-      if (si.rans_ok) {
-        const int rb = si.rans_table + 28 + si.rans_lane[0] + si.rans_lane[1] + si.rans_lane[2] + si.rans_lane[3];
-        if (f.force_order0 || rb < body) {
-          mode = kModeOrder0;
-          k = kRansTableLog;
-          body = rb;
-          lanes[0] = si.rans_lane[0];
-          lanes[1] = si.rans_lane[1];
-          lanes[2] = si.rans_lane[2];
-          lanes[3] = si.rans_lane[3];
-        }
-      }
-      si.mode = mode;
-      si.param = k;
-      si.body = body;
-      si.comp_lane[0] = lanes[0];
-      si.comp_lane[1] = lanes[1];
-      si.comp_lane[2] = lanes[2];
-      si.comp_lane[3] = lanes[3];
-      rec = body + 3;
-    }
+    if (s < f.nshards) rec = sizes[f.shard_base + s];
     // block exclusive scan
     int64_t inc = rec;
 #pragma unroll
@@ -1713,18 +1710,13 @@ enc_scan_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
     const int64_t off = fs[g.first_shard].offset;
     const int64_t end = (g.first_shard + g.shard_count < f.nshards) ? fs[g.first_shard + g.shard_count].offset
                                                                      : f.prefix_bytes + payload;
-    uint8_t* e = pre + kHeaderBytes + t * kDirBytes;
-    e[0] = static_cast<uint8_t>(g.plane);
-    e[1] = kModeOrder0;
-    e[2] = kPredictTag;
-    e[3] = 0;
-    put32(e + 4, g.x);
-    put32(e + 8, g.y);
-    put32(e + 12, g.w);
-    put32(e + 16, g.h);
-    put32(e + 20, static_cast<uint32_t>(off));
-    put32(e + 24, static_cast<uint32_t>(static_cast<uint64_t>(off) >> 32));
-    put32(e + 28, static_cast<uint32_t>(end - off));
+    // little-endian fields in two 16-byte stores (entries lie on 32-byte
+    // boundaries)
+    uint4* e = reinterpret_cast<uint4*>(pre + kHeaderBytes + t * kDirBytes);
+    e[0] = make_uint4(static_cast<uint32_t>(g.plane) | (kModeOrder0 << 8) | (kPredictTag << 16),
+                      static_cast<uint32_t>(g.x), static_cast<uint32_t>(g.y), static_cast<uint32_t>(g.w));
+    e[1] = make_uint4(static_cast<uint32_t>(g.h), static_cast<uint32_t>(off),
+                      static_cast<uint32_t>(static_cast<uint64_t>(off) >> 32), static_cast<uint32_t>(end - off));
     if (end - off > 0xffffffffll) set_status(&st.status, kStatusInternal + 1);  // "tile payload is too large"
   }
   if (threadIdx.x == 0) {
@@ -1768,23 +1760,13 @@ enc_scan_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
     st.payload = keep_a ? st.baseline_payload : payload;
     st.stream_len = f.prefix_bytes + st.payload;
     // header (encode.cu:871-885) -- written every pass, the last one stands
-    pre[0] = 'F';
-    pre[1] = 'V';
-    pre[2] = 'I';
-    pre[3] = 'D';
-    pre[4] = 1;
-    pre[5] = static_cast<uint8_t>(f.layout);
-    pre[6] = static_cast<uint8_t>(f.quality);
-    pre[7] = static_cast<uint8_t>((f.bit_depth - 8) | (st.gray_med ? 0x40 : 0) | (st.refined ? 0x80 : 0));
-    put32(pre + 8, f.width);
-    put32(pre + 12, f.height);
-    pre[16] = static_cast<uint8_t>(f.tile_w);
-    pre[17] = static_cast<uint8_t>(f.tile_w >> 8);
-    pre[18] = static_cast<uint8_t>(f.tile_h);
-    pre[19] = static_cast<uint8_t>(f.tile_h >> 8);
-    put32(pre + 20, f.fps_num);
-    put32(pre + 24, f.fps_den);
-    put32(pre + 28, static_cast<uint32_t>(f.ntiles));
+    uint4* h = reinterpret_cast<uint4*>(pre);
+    const uint32_t flags = (f.bit_depth - 8) | (st.gray_med ? 0x40 : 0) | (st.refined ? 0x80 : 0);
+    h[0] = make_uint4('F' | ('V' << 8) | ('I' << 16) | ('D' << 24),
+                      1u | (static_cast<uint32_t>(f.layout) << 8) | (static_cast<uint32_t>(f.quality) << 16) | (flags << 24),
+                      static_cast<uint32_t>(f.width), static_cast<uint32_t>(f.height));
+    h[1] = make_uint4(static_cast<uint32_t>(f.tile_w & 0xffff) | (static_cast<uint32_t>(f.tile_h & 0xffff) << 16), f.fps_num,
+                      f.fps_den, static_cast<uint32_t>(f.ntiles));
     // A failed pass stops the frame; otherwise the next pass runs only if the
     // policy asked for it.
     if (st.status != 0) next = 0;

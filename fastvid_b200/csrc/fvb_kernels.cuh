@@ -109,10 +109,11 @@ __global__ void enc_predict_wide_kernel(const FrameDesc* frames, FrameState* sta
 void enc_analyze_launch(bool fold16, int grid, cudaStream_t stream, const FrameDesc* frames, FrameState* state,
                         const BatchDims* dims, int pass, ShardInfo* shards, const void* folded,
                         uint8_t* rans_scratch);
-void enc_rans_launch(bool fold16, int64_t nshards, cudaStream_t stream, const FrameState* state, const BatchDims* dims,
-                     int pass, ShardInfo* shards, const void* folded, uint8_t* rans_scratch);
+void enc_rans_launch(bool fold16, int64_t nshards, cudaStream_t stream, const FrameDesc* frames,
+                     const FrameState* state, const BatchDims* dims, int pass, ShardInfo* shards, int32_t* sizes,
+                     const void* folded, uint8_t* rans_scratch);
 __global__ void enc_scan_kernel(const FrameDesc* frames, FrameState* state, const BatchDims* dims, int pass,
-                                ShardInfo* shards, uint8_t* prefix, int64_t* results);
+                                ShardInfo* shards, const int32_t* sizes, uint8_t* prefix, int64_t* results);
 // Records of one encoder region: pass 0's, or the later pass's (region b,
 // indexed like pass 0's for the frames that took part in it).
 struct EmitRegion {
