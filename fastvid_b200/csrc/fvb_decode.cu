@@ -468,7 +468,7 @@ struct LaneRing {
 // the entries of up to kLocalSymbols symbols; a shard with more reads its
 // entries from its table record) and the lanes' byte rings.
 constexpr int kGroups = 8;  // shards per warp, four lanes each
-constexpr int kLocalSymbols = 64;
+constexpr int kLocalSymbols = 36;  // five CTAs on an SM: 758 us for 16 4K rgb10 frames, 854 us with 64 and four
 constexpr int kTableWords = kBuckets + kLocalSymbols;
 
 struct alignas(16) RansWarpSm {
@@ -680,12 +680,12 @@ __device__ __forceinline__ void rans_decode_lane(const Lookup lookup, bool narro
 // their 32 lanes.
 //
 // Bound by the chain of a step -- two dependent shared-memory lookups and a
-// population count -- and, with 16 warps an SM, by the shared-memory pipe
+// population count -- and, with 16 to 20 warps an SM, by the shared-memory pipe
 // (12 cycles a step: the lookups hit about three banks twice) and issue (42
 // instructions).  16 4K rgb10 frames: 1117 us with a lookup and a store of two
 // bytes for every symbol's value and tables built by four lanes while the rest
 // of the warp waited; 861 us with the value in the entry, 16-byte transposed
-// stores and tables made once by dec_rans_tables.
+// stores and tables made once by dec_rans_tables; 750 us with 20 warps an SM.
 template <typename FoldT>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 dec_rans_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
@@ -729,17 +729,18 @@ dec_rans_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
     }
     cp_async_commit();
     cp_async_wait<0>();
-    __syncwarp();
+    const bool all_local = __all_sync(kFull, local);
     if (live) {
       const uint16_t* values = reinterpret_cast<const uint16_t*>(t.data + RansTable::values_at(nsym));
       FoldT* out = folded + si->sample_base;
       uint32_t x = t.state[my_l];
       const int from = ring.at;
-      if (local)
+      const uint32_t* at = local ? sm.table[j] + kBuckets : entries;
+      if (all_local)
         rans_decode_lane<FoldT, 32>(BucketLookup{sm.table[j], sm.table[j] + kBuckets}, t.narrow, values, ring, out,
                                     si->count, my_l, group, x);
       else
-        rans_decode_lane<FoldT, 32>(BucketLookup{sm.table[j], entries}, t.narrow, values, ring, out, si->count, my_l,
+        rans_decode_lane<FoldT, 32>(BucketLookup{sm.table[j], at}, t.narrow, values, ring, out, si->count, my_l,
                                     group, x);
       if (ring.at - from != 8 * t.lane_len[my_l] || x != kRansL) set_status(&state[si->frame].status, 5);
     }
