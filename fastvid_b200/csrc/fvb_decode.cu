@@ -1506,11 +1506,11 @@ __device__ __forceinline__ void rec_wave_block(St& st, WaveBlock<O1> blk, int32_
 // ODD_W: the tile's rows start on even and odd samples in turn
 template <bool MED, bool WIDE, bool ODD_W>
 __device__ void rec_wave_tile(const FrameDesc& f, const TileGeo& g, const uint16_t* __restrict__ ftile, WaveSm& sm,
-                              int lane) {
+                              int lane, bool rowwise) {
   for (int i = lane; i < kCarryCols / 8; i += 32) reinterpret_cast<uint4*>(sm.carry)[i] = make_uint4(0, 0, 0, 0);
   __syncwarp();
   WaveIo<false> io(sm, lane, g.w, ftile, g.w, f.dst[g.plane] + static_cast<int64_t>(g.y) * f.dst_pitch[g.plane] + g.x,
-                       f.dst_pitch[g.plane], nullptr, nullptr);
+                       f.dst_pitch[g.plane], nullptr, nullptr, rowwise);
   for (int y = 0; y < g.h; y += kBandRows, io.next_band()) {
     io.band(g.h - y);
     io.fetch(0);
@@ -1548,6 +1548,7 @@ dec_reconstruct_wave_kernel(const FrameDesc* __restrict__ frames, const FrameSta
   // before the second ones, so few tiles spread over all SMs -- and the rest
   // come from the queue
   const int64_t warps_total = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
+  const bool rowwise = total_tiles > warps_total;
   for (int64_t t = static_cast<int64_t>(warp) * gridDim.x + blockIdx.x; t < total_tiles;) {
     const int64_t mine = t;
     if (lane == 0) t = warps_total + atomicAdd(queue, 1);
@@ -1560,15 +1561,15 @@ dec_reconstruct_wave_kernel(const FrameDesc* __restrict__ frames, const FrameSta
     const uint16_t* ftile = folded + f.sample_base + g.sample_base;
     const bool odd = g.w & 1, wide = f.bit_depth > 12;
     if (f.use_med0) {
-      if (!wide) odd ? rec_wave_tile<true, false, true>(f, g, ftile, sm, lane)
-                     : rec_wave_tile<true, false, false>(f, g, ftile, sm, lane);
-      else odd ? rec_wave_tile<true, true, true>(f, g, ftile, sm, lane)
-               : rec_wave_tile<true, true, false>(f, g, ftile, sm, lane);
+      if (!wide) odd ? rec_wave_tile<true, false, true>(f, g, ftile, sm, lane, rowwise)
+                     : rec_wave_tile<true, false, false>(f, g, ftile, sm, lane, rowwise);
+      else odd ? rec_wave_tile<true, true, true>(f, g, ftile, sm, lane, rowwise)
+               : rec_wave_tile<true, true, false>(f, g, ftile, sm, lane, rowwise);
     } else {
-      if (!wide) odd ? rec_wave_tile<false, false, true>(f, g, ftile, sm, lane)
-                     : rec_wave_tile<false, false, false>(f, g, ftile, sm, lane);
-      else odd ? rec_wave_tile<false, true, true>(f, g, ftile, sm, lane)
-               : rec_wave_tile<false, true, false>(f, g, ftile, sm, lane);
+      if (!wide) odd ? rec_wave_tile<false, false, true>(f, g, ftile, sm, lane, rowwise)
+                     : rec_wave_tile<false, false, false>(f, g, ftile, sm, lane, rowwise);
+      else odd ? rec_wave_tile<false, true, true>(f, g, ftile, sm, lane, rowwise)
+               : rec_wave_tile<false, true, false>(f, g, ftile, sm, lane, rowwise);
     }
   }
 }

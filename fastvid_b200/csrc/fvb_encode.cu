@@ -513,14 +513,14 @@ __device__ __forceinline__ void enc_wave_block(St& st, uint32_t& sym, uint32_t& 
 
 template <bool MED, bool WIDE, bool O1>
 __device__ void enc_wave_tile(const FrameDesc& f, const TileGeo& g, int32_t step, uint32_t magic,
-                              uint16_t* __restrict__ ftile, WaveSm& sm, int lane, int32_t& bad) {
+                              uint16_t* __restrict__ ftile, WaveSm& sm, int lane, bool rowwise, int32_t& bad) {
   for (int i = lane; i < kCarryCols / 8; i += 32) reinterpret_cast<uint4*>(sm.carry)[i] = make_uint4(0, 0, 0, 0);
   __syncwarp();
   const uint16_t* plane = f.src[g.plane];
   const int64_t pitch = f.src_pitch[g.plane];
   const std::conditional_t<WIDE, WideQuant, PackedQuant> quant(f.max_sample, step, magic);
   WaveIo<true> io(sm, lane, g.w, plane + static_cast<int64_t>(g.y) * pitch + g.x, pitch, ftile, g.w, plane,
-                      plane + static_cast<int64_t>(f.height - 1) * pitch + f.plane_w[g.plane]);
+                      plane + static_cast<int64_t>(f.height - 1) * pitch + f.plane_w[g.plane], rowwise);
   uint32_t vmax = 0;
   for (int y = 0; y < g.h; y += kBandRows, io.next_band()) {
     io.band(g.h - y);
@@ -548,9 +548,9 @@ __device__ void enc_wave_tile(const FrameDesc& f, const TileGeo& g, int32_t step
 
 template <bool MED, bool WIDE>
 __device__ void enc_wave_any(const FrameDesc& f, const TileGeo& g, int32_t step, uint32_t magic,
-                             uint16_t* __restrict__ ftile, WaveSm& sm, int lane, int32_t& bad) {
-  if (f.src_pitch[g.plane] & 1) enc_wave_tile<MED, WIDE, false>(f, g, step, magic, ftile, sm, lane, bad);
-  else enc_wave_tile<MED, WIDE, true>(f, g, step, magic, ftile, sm, lane, bad);
+                             uint16_t* __restrict__ ftile, WaveSm& sm, int lane, bool rowwise, int32_t& bad) {
+  if (f.src_pitch[g.plane] & 1) enc_wave_tile<MED, WIDE, false>(f, g, step, magic, ftile, sm, lane, rowwise, bad);
+  else enc_wave_tile<MED, WIDE, true>(f, g, step, magic, ftile, sm, lane, rowwise, bad);
 }
 
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
@@ -564,6 +564,7 @@ enc_predict_wave_kernel(const FrameDesc* __restrict__ frames, FrameState* __rest
   WaveSm& sm = reinterpret_cast<WaveSm*>(smem_raw)[warp];
   // tiles by place first, then from the queue (as dec_reconstruct_wave_kernel)
   const int64_t warps_total = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
+  const bool rowwise = total_tiles > warps_total;
   for (int64_t t = static_cast<int64_t>(warp) * gridDim.x + blockIdx.x; t < total_tiles;) {
     const int64_t mine = t;
     if (lane == 0) t = warps_total + atomicAdd(queue, 1);
@@ -581,11 +582,11 @@ enc_predict_wave_kernel(const FrameDesc* __restrict__ frames, FrameState* __rest
     int32_t bad = 0;
     const bool wide = f.bit_depth > 12;
     if (st.use_med) {
-      if (wide) enc_wave_any<true, true>(f, g, step, magic, ftile, sm, lane, bad);
-      else enc_wave_any<true, false>(f, g, step, magic, ftile, sm, lane, bad);
+      if (wide) enc_wave_any<true, true>(f, g, step, magic, ftile, sm, lane, rowwise, bad);
+      else enc_wave_any<true, false>(f, g, step, magic, ftile, sm, lane, rowwise, bad);
     } else {
-      if (wide) enc_wave_any<false, true>(f, g, step, magic, ftile, sm, lane, bad);
-      else enc_wave_any<false, false>(f, g, step, magic, ftile, sm, lane, bad);
+      if (wide) enc_wave_any<false, true>(f, g, step, magic, ftile, sm, lane, rowwise, bad);
+      else enc_wave_any<false, false>(f, g, step, magic, ftile, sm, lane, rowwise, bad);
     }
     if (__any_sync(kFull, bad) && lane == 0) set_status(&st.status, 1);
   }

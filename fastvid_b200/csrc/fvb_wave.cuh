@@ -96,6 +96,7 @@ struct WaveIo {
   int a_in, a_step;  // alignment (samples modulo 8) of row 0, and its change per row
   int store_mode;    // 0: single samples, 1: pairs, 2: 16-byte chunks
   bool ragged;       // rows have partial chunks
+  const bool rowwise;  // how modes 0 and 1 store (flush)
   // chunk role: chunk lj of rows lr, lr + 8, ...; c_first: the column of chunk
   // lj of row lr in window 0
   int lr, lj, c_first;
@@ -110,9 +111,9 @@ struct WaveIo {
   __device__ int off_of(int row) const { return (align_of(row) - skew(row)) & 7; }
 
   __device__ WaveIo(WaveSm& sm_, int lane_, int W_, const uint16_t* in_, int64_t in_pitch_, uint16_t* out_,
-                    int64_t out_pitch_, const uint16_t* lo_, const uint16_t* hi_)
+                    int64_t out_pitch_, const uint16_t* lo_, const uint16_t* hi_, bool rowwise_)
       : sm(sm_), lane(lane_), W(W_), in(in_), in_pitch(in_pitch_), out(out_), out_pitch(out_pitch_), lo(lo_),
-        hi(hi_) {
+        hi(hi_), rowwise(rowwise_) {
     a_in = static_cast<int>(reinterpret_cast<uintptr_t>(in) >> 1) & 7;
     a_step = static_cast<int>(in_pitch & 7);
     const int d_in = static_cast<int>(reinterpret_cast<uintptr_t>(out) >> 1) & 7;
@@ -222,7 +223,12 @@ struct WaveIo {
   }
 
   // A chunk whose columns c .. c + 7 all lie in the tile: one store where input
-  // and output rows are aligned alike, else four or eight.
+  // and output rows are aligned alike, else four or eight.  Those take a quarter
+  // of the instructions of storing row by row, but touch every 32-byte sector
+  // eight or sixteen times: the better way while a lone warp's instructions
+  // decide (a tile a warp at most: 43 us for an odd 1437x811 frame, 90 row by
+  // row), the worse one when the GPU is full (4 1921x1081 rgb10 frames in 64x64
+  // tiles, whole decode: 382 us, 326 us row by row).
   __device__ void store_whole(uint16_t* dst, const uint4 v) const {
     if (store_mode == 2) {
       *reinterpret_cast<uint4*>(dst) = v;
@@ -243,8 +249,36 @@ struct WaveIo {
     const uint16_t* s = reinterpret_cast<const uint16_t*>(src);
     for (int e = max(0, -c); e < min(8, W - c); ++e) dst[e] = s[e];
   }
+  // Positions 0..31 of window b, row by row: a warp's stores lie side by side.
+  template <typename T>
+  __device__ void flush_rows(int b) {
+    constexpr int kPer = sizeof(T) / 2;             // samples a lane
+    constexpr int kSide = kPer;                     // rows side by side, 64 / kSide apart
+    constexpr int kRows = 8 / kSide;                // of the eight rows k, k + 8, ...
+    const int side = kSide == 2 ? lane >> 4 : 0, p = kPer * (kSide == 2 ? lane & 15 : lane);
+#pragma unroll 1
+    for (int r = 0; r < 8; ++r) {
+      const int row = r + side * (kBandRows / 2);
+      int c = 32 * b + p - skew(row) - off_of(row);
+      uint16_t* dst = out + row * out_pitch + c;
+      const uint16_t* src = reinterpret_cast<const uint16_t*>(sm.win[b & 1] + win_row(row)) + p;
+#pragma unroll
+      for (int i = 0; i < kRows; ++i) {
+        if (row + 8 * i < nrows && static_cast<unsigned>(c) < static_cast<unsigned>(W))
+          *reinterpret_cast<T*>(dst) = *reinterpret_cast<const T*>(src);
+        dst += out_hop;
+        src += 8 * kWinHop;
+        c -= 1 << kShift;
+      }
+    }
+  }
   // Positions 0..31 of window b, all rows, to the output.
   __device__ void flush(int b) {
+    if (rowwise && store_mode != 2) {
+      if (store_mode == 1) flush_rows<uint32_t>(b);
+      else flush_rows<uint16_t>(b);
+      return;
+    }
     const int c = c_first + 32 * b;
     uint16_t* dst = out + lr * out_pitch + c;
     const uint4* src = sm.win[b & 1] + kWinChunks * lr + lj;
