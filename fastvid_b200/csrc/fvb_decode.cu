@@ -1504,36 +1504,42 @@ __device__ __forceinline__ void rec_wave_block(St& st, WaveBlock<O1> blk, int32_
 }
 
 // ODD_W: the tile's rows start on even and odd samples in turn
-template <bool MED, bool WIDE, bool ODD_W>
-__device__ void rec_wave_tile(const FrameDesc& f, const TileGeo& g, const uint16_t* __restrict__ ftile, WaveSm& sm,
-                              int lane, bool rowwise) {
+template <bool MED, bool WIDE, bool ODD_W, bool PAIR>
+__device__ void rec_wave_tile(const FrameDesc& f, const TileGeo& g, const uint16_t* __restrict__ ftile, WaveSm* sms,
+                              int warp, int lane, bool rowwise) {
+  WaveSm& sm = sms[warp];
   for (int i = lane; i < kCarryCols / 8; i += 32) reinterpret_cast<uint4*>(sm.carry)[i] = make_uint4(0, 0, 0, 0);
-  __syncwarp();
+  if (PAIR) wave_pair_sync(warp);
+  else __syncwarp();
+  const uint16_t* above = sms[PAIR ? warp ^ 1 : warp].carry;
   WaveIo<false> io(sm, lane, g.w, ftile, g.w, f.dst[g.plane] + static_cast<int64_t>(g.y) * f.dst_pitch[g.plane] + g.x,
                        f.dst_pitch[g.plane], nullptr, nullptr, rowwise);
-  for (int y = 0; y < g.h; y += kBandRows, io.next_band()) {
-    io.band(g.h - y);
+  std::conditional_t<WIDE, WaveWide, WavePacked> st;
+  auto begin = [&] {
+    st = {};
     io.fetch(0);
-    std::conditional_t<WIDE, WaveWide, WavePacked> st;
-    for (int b = 0; b < io.nblk; ++b) {
-      if (b) {
-        io.flush(b - 1);
-        io.move_head(b);
-        __syncwarp();
-      }
-      if (b + 1 < io.nblk) io.fetch(b + 1);
-      else cp_async_commit();
-      io.wait();
-      io.template fix_edge<false>(b);
-      rec_wave_block<MED, !ODD_W>(st, WaveBlock<!ODD_W>(sm, b, lane, io.off0, io.off1),
-                                             f.max_sample, f.step0);
+  };
+  auto block = [&](int b) {
+    if (b) {
+      io.flush(b - 1);
+      io.move_head(b);
       __syncwarp();
     }
+    if (b + 1 < io.nblk) io.fetch(b + 1);
+    else cp_async_commit();
+    io.wait();
+    io.template fix_edge<false>(b);
+    rec_wave_block<MED, !ODD_W>(st, WaveBlock<!ODD_W>(sm, above, b, lane, io.off0, io.off1), f.max_sample, f.step0);
+    __syncwarp();
+  };
+  auto end = [&] {
     io.flush_last();
     __syncwarp();
-  }
+  };
+  wave_sweep<PAIR>(io, g.h, warp, begin, block, end);
 }
 
+template <bool PAIR>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
 dec_reconstruct_wave_kernel(const FrameDesc* __restrict__ frames, const FrameState* __restrict__ state,
                             const BatchDims* __restrict__ dims, const uint16_t* __restrict__ folded,
@@ -1543,16 +1549,20 @@ dec_reconstruct_wave_kernel(const FrameDesc* __restrict__ frames, const FrameSta
   const int64_t total_tiles = dims->tiles_p[0];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  WaveSm& sm = reinterpret_cast<WaveSm*>(smem_raw)[warp];
-  // a warp's first tile goes by its place -- the first warps of all CTAs
-  // before the second ones, so few tiles spread over all SMs -- and the rest
-  // come from the queue
-  const int64_t warps_total = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
-  const bool rowwise = total_tiles > warps_total;
-  for (int64_t t = static_cast<int64_t>(warp) * gridDim.x + blockIdx.x; t < total_tiles;) {
+  WaveSm* sms = reinterpret_cast<WaveSm*>(smem_raw);
+  // a warp's (a pair's) first tile goes by its place -- the first warps of all
+  // CTAs before the second ones, so few tiles spread over all SMs -- and the
+  // rest come from the queue (for pairs there are none, or by place too)
+  const int64_t takers = static_cast<int64_t>(gridDim.x) * (PAIR ? kWarpsPerCta / 2 : kWarpsPerCta);
+  const bool rowwise = total_tiles > takers;
+  for (int64_t t = static_cast<int64_t>(PAIR ? warp >> 1 : warp) * gridDim.x + blockIdx.x; t < total_tiles;) {
     const int64_t mine = t;
-    if (lane == 0) t = warps_total + atomicAdd(queue, 1);
-    t = __shfl_sync(kFull, t, 0);
+    if (PAIR) {
+      t += takers;
+    } else {
+      if (lane == 0) t = takers + atomicAdd(queue, 1);
+      t = __shfl_sync(kFull, t, 0);
+    }
     const int fi = frame_of_tile(frames, nframes, mine);
     const FrameDesc& f = frames[fi];
     if (state[fi].status != 0) continue;
@@ -1561,15 +1571,15 @@ dec_reconstruct_wave_kernel(const FrameDesc* __restrict__ frames, const FrameSta
     const uint16_t* ftile = folded + f.sample_base + g.sample_base;
     const bool odd = g.w & 1, wide = f.bit_depth > 12;
     if (f.use_med0) {
-      if (!wide) odd ? rec_wave_tile<true, false, true>(f, g, ftile, sm, lane, rowwise)
-                     : rec_wave_tile<true, false, false>(f, g, ftile, sm, lane, rowwise);
-      else odd ? rec_wave_tile<true, true, true>(f, g, ftile, sm, lane, rowwise)
-               : rec_wave_tile<true, true, false>(f, g, ftile, sm, lane, rowwise);
+      if (!wide) odd ? rec_wave_tile<true, false, true, PAIR>(f, g, ftile, sms, warp, lane, rowwise)
+                     : rec_wave_tile<true, false, false, PAIR>(f, g, ftile, sms, warp, lane, rowwise);
+      else odd ? rec_wave_tile<true, true, true, PAIR>(f, g, ftile, sms, warp, lane, rowwise)
+               : rec_wave_tile<true, true, false, PAIR>(f, g, ftile, sms, warp, lane, rowwise);
     } else {
-      if (!wide) odd ? rec_wave_tile<false, false, true>(f, g, ftile, sm, lane, rowwise)
-                     : rec_wave_tile<false, false, false>(f, g, ftile, sm, lane, rowwise);
-      else odd ? rec_wave_tile<false, true, true>(f, g, ftile, sm, lane, rowwise)
-               : rec_wave_tile<false, true, false>(f, g, ftile, sm, lane, rowwise);
+      if (!wide) odd ? rec_wave_tile<false, false, true, PAIR>(f, g, ftile, sms, warp, lane, rowwise)
+                     : rec_wave_tile<false, false, false, PAIR>(f, g, ftile, sms, warp, lane, rowwise);
+      else odd ? rec_wave_tile<false, true, true, PAIR>(f, g, ftile, sms, warp, lane, rowwise)
+               : rec_wave_tile<false, true, false, PAIR>(f, g, ftile, sms, warp, lane, rowwise);
     }
   }
 }
@@ -1584,18 +1594,21 @@ cudaError_t dec_reconstruct_set_smem() {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, b32);
     if (e != cudaSuccess) return e;
   }
-  const cudaError_t e =
-      cudaFuncSetAttribute(dec_reconstruct_wave_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, b16);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(dec_reconstruct_wave_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                              cudaSharedmemCarveoutMaxShared);
+  for (auto k : {dec_reconstruct_wave_kernel<false>, dec_reconstruct_wave_kernel<true>}) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, b16);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
-void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, int grid, cudaStream_t stream,
+void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, bool pairs, int grid, cudaStream_t stream,
                             const FrameDesc* frames, const FrameState* state, const BatchDims* dims,
                             const void* folded, int* queue, int64_t* results) {
   if (fold16) {
-    dec_reconstruct_wave_kernel<<<grid, kWarpsPerCta * 32, dec_reconstruct_smem(true), stream>>>(
+    auto k = pairs ? dec_reconstruct_wave_kernel<true> : dec_reconstruct_wave_kernel<false>;
+    k<<<grid, kWarpsPerCta * 32, dec_reconstruct_smem(true), stream>>>(
         frames, state, dims, static_cast<const uint16_t*>(folded), queue, results);
     return;
   }

@@ -511,48 +511,59 @@ __device__ __forceinline__ void enc_wave_block(St& st, uint32_t& sym, uint32_t& 
   blk.finish(sym, st.packed());
 }
 
-template <bool MED, bool WIDE, bool O1>
+template <bool MED, bool WIDE, bool O1, bool PAIR>
 __device__ void enc_wave_tile(const FrameDesc& f, const TileGeo& g, int32_t step, uint32_t magic,
-                              uint16_t* __restrict__ ftile, WaveSm& sm, int lane, bool rowwise, int32_t& bad) {
+                              uint16_t* __restrict__ ftile, WaveSm* sms, int warp, int lane, bool rowwise,
+                              int32_t& bad) {
+  WaveSm& sm = sms[warp];
   for (int i = lane; i < kCarryCols / 8; i += 32) reinterpret_cast<uint4*>(sm.carry)[i] = make_uint4(0, 0, 0, 0);
-  __syncwarp();
+  if (PAIR) wave_pair_sync(warp);
+  else __syncwarp();
+  const uint16_t* above = sms[PAIR ? warp ^ 1 : warp].carry;
   const uint16_t* plane = f.src[g.plane];
   const int64_t pitch = f.src_pitch[g.plane];
   const std::conditional_t<WIDE, WideQuant, PackedQuant> quant(f.max_sample, step, magic);
   WaveIo<true> io(sm, lane, g.w, plane + static_cast<int64_t>(g.y) * pitch + g.x, pitch, ftile, g.w, plane,
-                      plane + static_cast<int64_t>(f.height - 1) * pitch + f.plane_w[g.plane], rowwise);
-  uint32_t vmax = 0;
-  for (int y = 0; y < g.h; y += kBandRows, io.next_band()) {
-    io.band(g.h - y);
+                  plane + static_cast<int64_t>(f.height - 1) * pitch + f.plane_w[g.plane], rowwise);
+  uint32_t vmax = 0, sym = 0;
+  std::conditional_t<WIDE, WaveWide, WavePacked> st;
+  auto begin = [&] {
+    st = {};
+    sym = 0;
     io.fetch(0);
-    std::conditional_t<WIDE, WaveWide, WavePacked> st;
-    uint32_t sym = 0;
-    for (int b = 0; b < io.nblk; ++b) {
-      if (b) {
-        io.flush(b - 1);
-        io.move_head(b);
-        __syncwarp();
-      }
-      if (b + 1 < io.nblk) io.fetch(b + 1);
-      else cp_async_commit();
-      io.wait();
-      io.template fix_edge<true>(b);
-      enc_wave_block<MED, O1>(st, sym, vmax, WaveBlock<O1>(sm, b, lane, io.off0, io.off1), quant);
+  };
+  auto block = [&](int b) {
+    if (b) {
+      io.flush(b - 1);
+      io.move_head(b);
       __syncwarp();
     }
+    if (b + 1 < io.nblk) io.fetch(b + 1);
+    else cp_async_commit();
+    io.wait();
+    io.template fix_edge<true>(b);
+    enc_wave_block<MED, O1>(st, sym, vmax, WaveBlock<O1>(sm, above, b, lane, io.off0, io.off1), quant);
+    __syncwarp();
+  };
+  auto end = [&] {
     io.flush_last();
     __syncwarp();
-  }
+  };
+  wave_sweep<PAIR>(io, g.h, warp, begin, block, end);
   if (!WIDE && max(vmax & 0xffffu, vmax >> 16) > static_cast<uint32_t>(f.max_sample)) bad = 1;
 }
 
-template <bool MED, bool WIDE>
+template <bool MED, bool WIDE, bool PAIR>
 __device__ void enc_wave_any(const FrameDesc& f, const TileGeo& g, int32_t step, uint32_t magic,
-                             uint16_t* __restrict__ ftile, WaveSm& sm, int lane, bool rowwise, int32_t& bad) {
-  if (f.src_pitch[g.plane] & 1) enc_wave_tile<MED, WIDE, false>(f, g, step, magic, ftile, sm, lane, rowwise, bad);
-  else enc_wave_tile<MED, WIDE, true>(f, g, step, magic, ftile, sm, lane, rowwise, bad);
+                             uint16_t* __restrict__ ftile, WaveSm* sms, int warp, int lane, bool rowwise,
+                             int32_t& bad) {
+  if (f.src_pitch[g.plane] & 1)
+    enc_wave_tile<MED, WIDE, false, PAIR>(f, g, step, magic, ftile, sms, warp, lane, rowwise, bad);
+  else
+    enc_wave_tile<MED, WIDE, true, PAIR>(f, g, step, magic, ftile, sms, warp, lane, rowwise, bad);
 }
 
+template <bool PAIR>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
 enc_predict_wave_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
                         const BatchDims* __restrict__ dims, int pass, ShardInfo* __restrict__ shards,
@@ -561,20 +572,24 @@ enc_predict_wave_kernel(const FrameDesc* __restrict__ frames, FrameState* __rest
   const int nframes = dims->frames_p[pass];
   const int64_t total_tiles = dims->tiles_p[pass];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  WaveSm& sm = reinterpret_cast<WaveSm*>(smem_raw)[warp];
+  WaveSm* sms = reinterpret_cast<WaveSm*>(smem_raw);
   // tiles by place first, then from the queue (as dec_reconstruct_wave_kernel)
-  const int64_t warps_total = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
-  const bool rowwise = total_tiles > warps_total;
-  for (int64_t t = static_cast<int64_t>(warp) * gridDim.x + blockIdx.x; t < total_tiles;) {
+  const int64_t takers = static_cast<int64_t>(gridDim.x) * (PAIR ? kWarpsPerCta / 2 : kWarpsPerCta);
+  const bool rowwise = total_tiles > takers;
+  for (int64_t t = static_cast<int64_t>(PAIR ? warp >> 1 : warp) * gridDim.x + blockIdx.x; t < total_tiles;) {
     const int64_t mine = t;
-    if (lane == 0) t = warps_total + atomicAdd(queue, 1);
-    t = __shfl_sync(kFull, t, 0);
+    if (PAIR) {
+      t += takers;
+    } else {
+      if (lane == 0) t = takers + atomicAdd(queue, 1);
+      t = __shfl_sync(kFull, t, 0);
+    }
     const int fi = frame_of_tile(frames, nframes, mine);
     const FrameDesc& f = frames[fi];
     FrameState& st = state[fi];
     if (frame_lossless(f)) continue;  // enc_lossless_kernel's
     const TileGeo g = tile_geo(f, mine - f.tile_base);
-    write_shard_records(f, g, fi, shards, lane);
+    if (!PAIR || !(warp & 1)) write_shard_records(f, g, fi, shards, lane);
     if (!st.active || g.w > kFastMaxW) continue;  // wide tiles go through enc_predict_wide_kernel
     const int32_t step = st.step;
     const uint32_t magic = static_cast<uint32_t>((0x100000000ull + step - 1) / step);
@@ -582,11 +597,11 @@ enc_predict_wave_kernel(const FrameDesc* __restrict__ frames, FrameState* __rest
     int32_t bad = 0;
     const bool wide = f.bit_depth > 12;
     if (st.use_med) {
-      if (wide) enc_wave_any<true, true>(f, g, step, magic, ftile, sm, lane, rowwise, bad);
-      else enc_wave_any<true, false>(f, g, step, magic, ftile, sm, lane, rowwise, bad);
+      if (wide) enc_wave_any<true, true, PAIR>(f, g, step, magic, ftile, sms, warp, lane, rowwise, bad);
+      else enc_wave_any<true, false, PAIR>(f, g, step, magic, ftile, sms, warp, lane, rowwise, bad);
     } else {
-      if (wide) enc_wave_any<false, true>(f, g, step, magic, ftile, sm, lane, rowwise, bad);
-      else enc_wave_any<false, false>(f, g, step, magic, ftile, sm, lane, rowwise, bad);
+      if (wide) enc_wave_any<false, true, PAIR>(f, g, step, magic, ftile, sms, warp, lane, rowwise, bad);
+      else enc_wave_any<false, false, PAIR>(f, g, step, magic, ftile, sms, warp, lane, rowwise, bad);
     }
     if (__any_sync(kFull, bad) && lane == 0) set_status(&st.status, 1);
   }
@@ -785,14 +800,19 @@ cudaError_t enc_predict_set_smem() {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, b32);
     if (e != cudaSuccess) return e;
   }
-  return cudaFuncSetAttribute(enc_predict_wave_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, b16);
+  for (auto k : {enc_predict_wave_kernel<false>, enc_predict_wave_kernel<true>}) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, b16);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
-void enc_predict_launch(int unroll, int tile_warps, bool fold16, int grid, cudaStream_t stream,
+void enc_predict_launch(int unroll, int tile_warps, bool fold16, bool pairs, int grid, cudaStream_t stream,
                         const FrameDesc* frames, FrameState* state, const BatchDims* dims, int pass,
                         ShardInfo* shards, void* folded, int* queue) {
   if (fold16) {
-    enc_predict_wave_kernel<<<grid, kWarpsPerCta * 32, enc_predict_smem(true), stream>>>(
+    auto k = pairs ? enc_predict_wave_kernel<true> : enc_predict_wave_kernel<false>;
+    k<<<grid, kWarpsPerCta * 32, enc_predict_smem(true), stream>>>(
         frames, state, dims, pass, shards, static_cast<uint16_t*>(folded), queue);
     return;
   }

@@ -98,9 +98,9 @@ __global__ void enc_init_kernel(const FrameDesc* frames, FrameState* state, cons
 // frames of step 1 (pass 0 only)
 void enc_lossless_launch(bool fold16, int64_t tiles, int max_ctas, cudaStream_t stream, const FrameDesc* frames,
                          FrameState* state, const BatchDims* dims, ShardInfo* shards, void* folded);
-// the other frames; u32 symbols: a wavefront block of `unroll` steps (4, 8, 16,
+// the other frames; u16 symbols: by warp pairs or single warps; u32 symbols: a wavefront block of `unroll` steps (4, 8, 16,
 // 32) and `tile_warps` (1, or 2: a warp pair splits each tile's bands)
-void enc_predict_launch(int unroll, int tile_warps, bool fold16, int grid, cudaStream_t stream,
+void enc_predict_launch(int unroll, int tile_warps, bool fold16, bool pairs, int grid, cudaStream_t stream,
                         const FrameDesc* frames, FrameState* state, const BatchDims* dims, int pass,
                         ShardInfo* shards, void* folded, int* queue);
 cudaError_t enc_predict_set_smem();
@@ -157,7 +157,7 @@ void dec_other_launch(bool fold16, int grid, cudaStream_t stream, const FrameDes
                       void* folded);
 // u32 symbols: `unroll` and `tile_warps` as for enc_predict
 // (every reconstruction kernel also writes the frames' statuses to `results`)
-void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, int grid, cudaStream_t stream,
+void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, bool pairs, int grid, cudaStream_t stream,
                             const FrameDesc* frames, const FrameState* state, const BatchDims* dims,
                             const void* folded, int* queue, int64_t* results);
 cudaError_t dec_other_set_smem();

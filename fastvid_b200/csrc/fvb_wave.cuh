@@ -353,11 +353,12 @@ struct WaveBlock {
   const uint16_t* crow;  // lane 0: the carry row, column of the block's first step
   uint32_t* cout;        // lane 31: where the last row of the band goes
   int lane;
-  __device__ WaveBlock(WaveSm& sm, int b, int lane_, int off0, int off1) : lane(lane_) {
+  // `above`: the carry row that the band above wrote (its own, or the partner's)
+  __device__ WaveBlock(WaveSm& sm, const uint16_t* above, int b, int lane_, int off0, int off1) : lane(lane_) {
     uint4* win = sm.win[b & 1] + win_row(2 * lane);
     p0 = reinterpret_cast<uint32_t*>(win) + (off0 >> 1);
     p1 = reinterpret_cast<uint32_t*>(win + kWinChunks) + (off1 >> 1);
-    crow = sm.carry + kCarryPad + 32 * b;
+    crow = above + kCarryPad + 32 * b;
     cout = reinterpret_cast<uint32_t*>(sm.carry + kCarryPad + 32 * b - 1 - wave_skew(kBandRows - 1));
   }
   // Results of step j of group g, packed (even row low), and those of the
@@ -374,6 +375,60 @@ struct WaveBlock {
     if (lane == 31) *reinterpret_cast<uint16_t*>(cout + 16) = static_cast<uint16_t>(last_now >> 16);
   }
 };
+
+// A warp pair's sweep of a tile, for launches with fewer tiles than half the
+// GPU's warps: band j runs on warp j % 2, three blocks behind band j - 1, whose
+// last row has then reached the columns that the block reads (row 63 is two
+// blocks behind row 0), in lock-step at the pair's barrier after every block.  A
+// carry row is overwritten by the band after next, at least three blocks behind
+// its reader.  Band j starts in slot wave_start(j, blocks).
+__device__ __forceinline__ int wave_start(int j, int blocks) {
+  return blocks >= 6 ? (j >> 1) * blocks + (j & 1) * 3 : 3 * j;
+}
+__device__ __forceinline__ void wave_pair_sync(int warp) {
+  asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp >> 1)) : "memory");
+}
+
+// Sweeps a tile: begin() at each of the warp's bands, block(b) for its blocks,
+// end() after the last, by one warp or a pair.
+template <bool PAIR, bool CHECK, typename Begin, typename Block, typename End>
+__device__ __forceinline__ void wave_sweep(WaveIo<CHECK>& io, int height, int warp, Begin begin, Block block, End end) {
+  if constexpr (!PAIR) {
+    for (int y = 0; y < height; y += kBandRows, io.next_band()) {
+      io.band(height - y);
+      begin();
+      for (int b = 0; b < io.nblk; ++b) block(b);
+      end();
+    }
+  } else {
+    const int bands = (height + kBandRows - 1) / kBandRows;
+    io.band(kBandRows);
+    const int full = io.nblk;
+    io.band(height - (bands - 1) * kBandRows);
+    const int slots = wave_start(bands - 1, full) + io.nblk;  // the last band ends last
+    int j = warp & 1;
+    if (j) io.next_band();
+    for (int slot = 0; slot < slots; ++slot) {
+      if (j < bands) {
+        const int b = slot - wave_start(j, full);
+        if (b == 0) {
+          io.band(height - j * kBandRows);
+          begin();
+        }
+        if (b >= 0) {
+          block(b);
+          if (b == io.nblk - 1) {
+            end();
+            j += 2;
+            io.next_band();
+            io.next_band();
+          }
+        }
+      }
+      wave_pair_sync(warp);
+    }
+  }
+}
 
 struct WaveCarry {
   uint32_t up[4];  // eight columns of the carry row

@@ -14,7 +14,7 @@ from fastvid_b200 import synth
 pytestmark = pytest.mark.gpu
 
 WIDTHS = (1, 2, 7, 8, 9, 31, 32, 33, 35, 62, 64, 65, 96, 127, 128, 130, 255, 256, 257, 511, 512)
-HEIGHTS = (1, 2, 63, 64, 65, 129)
+HEIGHTS = (1, 2, 63, 64, 65, 129, 250)
 FORMATS = (("gray", 8, 100), ("gray", 10, 90), ("gray", 12, 30), ("gray", 16, 87), ("yuv422", 10, 90),
            ("rgb444", 8, 66), ("rgb444", 12, 1), ("rgb444", 16, 50), ("gray", 16, 100))
 
