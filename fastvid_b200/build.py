@@ -26,6 +26,7 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC,-O3",
     "-Xptxas", "-O3",
     "--expt-relaxed-constexpr",
+    "--threads", "0",  # the source files side by side
 ]
 
 

@@ -1506,14 +1506,14 @@ __device__ __forceinline__ void rec_wave_block(St& st, WaveBlock<O1> blk, int32_
 // ODD_W: the tile's rows start on even and odd samples in turn
 template <bool MED, bool WIDE, bool ODD_W, bool PAIR>
 __device__ void rec_wave_tile(const FrameDesc& f, const TileGeo& g, const uint16_t* __restrict__ ftile, WaveSm* sms,
-                              int warp, int lane, bool rowwise) {
+                              int warp, int lane) {
   WaveSm& sm = sms[warp];
   for (int i = lane; i < kCarryCols / 8; i += 32) reinterpret_cast<uint4*>(sm.carry)[i] = make_uint4(0, 0, 0, 0);
   if (PAIR) wave_pair_sync(warp);
   else __syncwarp();
   const uint16_t* above = sms[PAIR ? warp ^ 1 : warp].carry;
-  WaveIo<false> io(sm, lane, g.w, ftile, g.w, f.dst[g.plane] + static_cast<int64_t>(g.y) * f.dst_pitch[g.plane] + g.x,
-                       f.dst_pitch[g.plane], nullptr, nullptr, rowwise);
+  WaveIo<false, !PAIR> io(sm, lane, g.w, ftile, g.w, f.dst[g.plane] + static_cast<int64_t>(g.y) * f.dst_pitch[g.plane] + g.x,
+                       f.dst_pitch[g.plane], nullptr, nullptr);
   std::conditional_t<WIDE, WaveWide, WavePacked> st;
   auto begin = [&] {
     st = {};
@@ -1554,7 +1554,6 @@ dec_reconstruct_wave_kernel(const FrameDesc* __restrict__ frames, const FrameSta
   // CTAs before the second ones, so few tiles spread over all SMs -- and the
   // rest come from the queue (for pairs there are none, or by place too)
   const int64_t takers = static_cast<int64_t>(gridDim.x) * (PAIR ? kWarpsPerCta / 2 : kWarpsPerCta);
-  const bool rowwise = total_tiles > takers;
   for (int64_t t = static_cast<int64_t>(PAIR ? warp >> 1 : warp) * gridDim.x + blockIdx.x; t < total_tiles;) {
     const int64_t mine = t;
     if (PAIR) {
@@ -1571,15 +1570,15 @@ dec_reconstruct_wave_kernel(const FrameDesc* __restrict__ frames, const FrameSta
     const uint16_t* ftile = folded + f.sample_base + g.sample_base;
     const bool odd = g.w & 1, wide = f.bit_depth > 12;
     if (f.use_med0) {
-      if (!wide) odd ? rec_wave_tile<true, false, true, PAIR>(f, g, ftile, sms, warp, lane, rowwise)
-                     : rec_wave_tile<true, false, false, PAIR>(f, g, ftile, sms, warp, lane, rowwise);
-      else odd ? rec_wave_tile<true, true, true, PAIR>(f, g, ftile, sms, warp, lane, rowwise)
-               : rec_wave_tile<true, true, false, PAIR>(f, g, ftile, sms, warp, lane, rowwise);
+      if (!wide) odd ? rec_wave_tile<true, false, true, PAIR>(f, g, ftile, sms, warp, lane)
+                     : rec_wave_tile<true, false, false, PAIR>(f, g, ftile, sms, warp, lane);
+      else odd ? rec_wave_tile<true, true, true, PAIR>(f, g, ftile, sms, warp, lane)
+               : rec_wave_tile<true, true, false, PAIR>(f, g, ftile, sms, warp, lane);
     } else {
-      if (!wide) odd ? rec_wave_tile<false, false, true, PAIR>(f, g, ftile, sms, warp, lane, rowwise)
-                     : rec_wave_tile<false, false, false, PAIR>(f, g, ftile, sms, warp, lane, rowwise);
-      else odd ? rec_wave_tile<false, true, true, PAIR>(f, g, ftile, sms, warp, lane, rowwise)
-               : rec_wave_tile<false, true, false, PAIR>(f, g, ftile, sms, warp, lane, rowwise);
+      if (!wide) odd ? rec_wave_tile<false, false, true, PAIR>(f, g, ftile, sms, warp, lane)
+                     : rec_wave_tile<false, false, false, PAIR>(f, g, ftile, sms, warp, lane);
+      else odd ? rec_wave_tile<false, true, true, PAIR>(f, g, ftile, sms, warp, lane)
+               : rec_wave_tile<false, true, false, PAIR>(f, g, ftile, sms, warp, lane);
     }
   }
 }

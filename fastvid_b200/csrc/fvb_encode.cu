@@ -513,8 +513,7 @@ __device__ __forceinline__ void enc_wave_block(St& st, uint32_t& sym, uint32_t& 
 
 template <bool MED, bool WIDE, bool O1, bool PAIR>
 __device__ void enc_wave_tile(const FrameDesc& f, const TileGeo& g, int32_t step, uint32_t magic,
-                              uint16_t* __restrict__ ftile, WaveSm* sms, int warp, int lane, bool rowwise,
-                              int32_t& bad) {
+                              uint16_t* __restrict__ ftile, WaveSm* sms, int warp, int lane, int32_t& bad) {
   WaveSm& sm = sms[warp];
   for (int i = lane; i < kCarryCols / 8; i += 32) reinterpret_cast<uint4*>(sm.carry)[i] = make_uint4(0, 0, 0, 0);
   if (PAIR) wave_pair_sync(warp);
@@ -523,8 +522,8 @@ __device__ void enc_wave_tile(const FrameDesc& f, const TileGeo& g, int32_t step
   const uint16_t* plane = f.src[g.plane];
   const int64_t pitch = f.src_pitch[g.plane];
   const std::conditional_t<WIDE, WideQuant, PackedQuant> quant(f.max_sample, step, magic);
-  WaveIo<true> io(sm, lane, g.w, plane + static_cast<int64_t>(g.y) * pitch + g.x, pitch, ftile, g.w, plane,
-                  plane + static_cast<int64_t>(f.height - 1) * pitch + f.plane_w[g.plane], rowwise);
+  WaveIo<true, !PAIR> io(sm, lane, g.w, plane + static_cast<int64_t>(g.y) * pitch + g.x, pitch, ftile, g.w, plane,
+                  plane + static_cast<int64_t>(f.height - 1) * pitch + f.plane_w[g.plane]);
   uint32_t vmax = 0, sym = 0;
   std::conditional_t<WIDE, WaveWide, WavePacked> st;
   auto begin = [&] {
@@ -555,12 +554,11 @@ __device__ void enc_wave_tile(const FrameDesc& f, const TileGeo& g, int32_t step
 
 template <bool MED, bool WIDE, bool PAIR>
 __device__ void enc_wave_any(const FrameDesc& f, const TileGeo& g, int32_t step, uint32_t magic,
-                             uint16_t* __restrict__ ftile, WaveSm* sms, int warp, int lane, bool rowwise,
-                             int32_t& bad) {
+                             uint16_t* __restrict__ ftile, WaveSm* sms, int warp, int lane, int32_t& bad) {
   if (f.src_pitch[g.plane] & 1)
-    enc_wave_tile<MED, WIDE, false, PAIR>(f, g, step, magic, ftile, sms, warp, lane, rowwise, bad);
+    enc_wave_tile<MED, WIDE, false, PAIR>(f, g, step, magic, ftile, sms, warp, lane, bad);
   else
-    enc_wave_tile<MED, WIDE, true, PAIR>(f, g, step, magic, ftile, sms, warp, lane, rowwise, bad);
+    enc_wave_tile<MED, WIDE, true, PAIR>(f, g, step, magic, ftile, sms, warp, lane, bad);
 }
 
 template <bool PAIR>
@@ -575,7 +573,6 @@ enc_predict_wave_kernel(const FrameDesc* __restrict__ frames, FrameState* __rest
   WaveSm* sms = reinterpret_cast<WaveSm*>(smem_raw);
   // tiles by place first, then from the queue (as dec_reconstruct_wave_kernel)
   const int64_t takers = static_cast<int64_t>(gridDim.x) * (PAIR ? kWarpsPerCta / 2 : kWarpsPerCta);
-  const bool rowwise = total_tiles > takers;
   for (int64_t t = static_cast<int64_t>(PAIR ? warp >> 1 : warp) * gridDim.x + blockIdx.x; t < total_tiles;) {
     const int64_t mine = t;
     if (PAIR) {
@@ -597,11 +594,11 @@ enc_predict_wave_kernel(const FrameDesc* __restrict__ frames, FrameState* __rest
     int32_t bad = 0;
     const bool wide = f.bit_depth > 12;
     if (st.use_med) {
-      if (wide) enc_wave_any<true, true, PAIR>(f, g, step, magic, ftile, sms, warp, lane, rowwise, bad);
-      else enc_wave_any<true, false, PAIR>(f, g, step, magic, ftile, sms, warp, lane, rowwise, bad);
+      if (wide) enc_wave_any<true, true, PAIR>(f, g, step, magic, ftile, sms, warp, lane, bad);
+      else enc_wave_any<true, false, PAIR>(f, g, step, magic, ftile, sms, warp, lane, bad);
     } else {
-      if (wide) enc_wave_any<false, true, PAIR>(f, g, step, magic, ftile, sms, warp, lane, rowwise, bad);
-      else enc_wave_any<false, false, PAIR>(f, g, step, magic, ftile, sms, warp, lane, rowwise, bad);
+      if (wide) enc_wave_any<false, true, PAIR>(f, g, step, magic, ftile, sms, warp, lane, bad);
+      else enc_wave_any<false, false, PAIR>(f, g, step, magic, ftile, sms, warp, lane, bad);
     }
     if (__any_sync(kFull, bad) && lane == 0) set_status(&st.status, 1);
   }

@@ -78,7 +78,8 @@ __device__ __forceinline__ uint32_t pair2(int32_t v) { return static_cast<uint32
 // global memory are copied as they lie, so a row's first chunk may hold up to
 // seven samples left of the tile, cleared by fix_edge().  CHECK: a chunk may
 // reach outside [lo, hi), the memory that may be read.
-template <bool CHECK>
+// ROWS: how rows that are not aligned alike are stored (see store_whole).
+template <bool CHECK, bool ROWS>
 struct WaveIo {
   static constexpr int kShift = 3;  // rows eight apart: columns 1 << kShift apart
   static_assert(4 * kSkew == 1 << kShift, "skew of eight rows");
@@ -96,7 +97,6 @@ struct WaveIo {
   int a_in, a_step;  // alignment (samples modulo 8) of row 0, and its change per row
   int store_mode;    // 0: single samples, 1: pairs, 2: 16-byte chunks
   bool ragged;       // rows have partial chunks
-  const bool rowwise;  // how modes 0 and 1 store (flush)
   // chunk role: chunk lj of rows lr, lr + 8, ...; c_first: the column of chunk
   // lj of row lr in window 0
   int lr, lj, c_first;
@@ -111,9 +111,9 @@ struct WaveIo {
   __device__ int off_of(int row) const { return (align_of(row) - skew(row)) & 7; }
 
   __device__ WaveIo(WaveSm& sm_, int lane_, int W_, const uint16_t* in_, int64_t in_pitch_, uint16_t* out_,
-                    int64_t out_pitch_, const uint16_t* lo_, const uint16_t* hi_, bool rowwise_)
+                    int64_t out_pitch_, const uint16_t* lo_, const uint16_t* hi_)
       : sm(sm_), lane(lane_), W(W_), in(in_), in_pitch(in_pitch_), out(out_), out_pitch(out_pitch_), lo(lo_),
-        hi(hi_), rowwise(rowwise_) {
+        hi(hi_) {
     a_in = static_cast<int>(reinterpret_cast<uintptr_t>(in) >> 1) & 7;
     a_step = static_cast<int>(in_pitch & 7);
     const int d_in = static_cast<int>(reinterpret_cast<uintptr_t>(out) >> 1) & 7;
@@ -226,8 +226,8 @@ struct WaveIo {
   // and output rows are aligned alike, else four or eight.  Those take a quarter
   // of the instructions of storing row by row, but touch every 32-byte sector
   // eight or sixteen times: the better way while a lone warp's instructions
-  // decide (a tile a warp at most: 43 us for an odd 1437x811 frame, 90 row by
-  // row), the worse one when the GPU is full (4 1921x1081 rgb10 frames in 64x64
+  // decide (warp pairs: 43 us for an odd 1437x811 frame, 90 row by row), the
+  // worse one when the GPU is full (4 1921x1081 rgb10 frames in 64x64
   // tiles, whole decode: 382 us, 326 us row by row).
   __device__ void store_whole(uint16_t* dst, const uint4 v) const {
     if (store_mode == 2) {
@@ -274,7 +274,7 @@ struct WaveIo {
   }
   // Positions 0..31 of window b, all rows, to the output.
   __device__ void flush(int b) {
-    if (rowwise && store_mode != 2) {
+    if (ROWS && store_mode != 2) {
       if (store_mode == 1) flush_rows<uint32_t>(b);
       else flush_rows<uint16_t>(b);
       return;
@@ -284,7 +284,7 @@ struct WaveIo {
     const uint4* src = sm.win[b & 1] + kWinChunks * lr + lj;
     // rows whose chunk lies in the tile as a whole
     const uint32_t whole = bit_range((c + 8 - W + (1 << kShift) - 1) >> kShift, min(c >> kShift, row_top));
-    if (store_mode == 2) {
+    if (ROWS || store_mode == 2) {
 #pragma unroll
       for (int i = 0; i < 8; ++i)
         if (whole & (1u << i)) *reinterpret_cast<uint4*>(dst + i * out_hop) = src[kWinHop * i];
@@ -391,8 +391,8 @@ __device__ __forceinline__ void wave_pair_sync(int warp) {
 
 // Sweeps a tile: begin() at each of the warp's bands, block(b) for its blocks,
 // end() after the last, by one warp or a pair.
-template <bool PAIR, bool CHECK, typename Begin, typename Block, typename End>
-__device__ __forceinline__ void wave_sweep(WaveIo<CHECK>& io, int height, int warp, Begin begin, Block block, End end) {
+template <bool PAIR, typename Io, typename Begin, typename Block, typename End>
+__device__ __forceinline__ void wave_sweep(Io& io, int height, int warp, Begin begin, Block block, End end) {
   if constexpr (!PAIR) {
     for (int y = 0; y < height; y += kBandRows, io.next_band()) {
       io.band(height - y);

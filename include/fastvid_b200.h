@@ -88,31 +88,24 @@ int fvb_get_wavefront_block(void);
  * even and odd 32-row bands in lock-step, the second warp two blocks behind,
  * handing each band's last row over in shared memory (tiles of one band or
  * under 66 columns stay on one warp).  0 restores the default (1).
- * Process-wide, read at each launch; no output depends on it. */
+ * Batches whose folded symbols are u16 always sweep a tile with one warp, two
+ * rows a lane.  Process-wide, read at each launch; no output depends on it. */
 int fvb_set_tile_warps(int warps);
 int fvb_get_tile_warps(void);
-/* Whether decode batches of 64 shards or more run dec_other (Rice,
+/* Whether decode batches of 4096 shards or more run dec_other (Rice,
  * zero-run and block-pack shards) on a side stream beside dec_rans (1, the
  * default) or after it on the caller's stream (0).  No reference
  * counterpart; process-wide, read at each launch; no output depends on it
  * (the autotuner's knob). */
 int fvb_set_decode_overlap(int on);
 int fvb_get_decode_overlap(void);
-/* How the rANS encoder fetches ahead of its state chain (no reference
- * counterpart, whose lanes load as they go, cuda/csrc/encode.cu:398-418): 0
- * loads 16 symbols and then their table entries before each 16 steps; 8 or
- * 16 runs a software pipeline over blocks of that many steps, the symbols
- * two blocks and the table entries one block ahead; -1 (the default) picks
- * per launch: the 8-step pipeline when the launch has at most 4 CTAs per SM
- * (a single frame: its lanes' load latency is exposed), the one-stage fetch
- * otherwise (it holds fewer registers).  Process-wide, read at each launch;
- * no output depends on it (the autotuner's knob). */
+/* A fetch scheme for the rANS encoder (0, 8, 16 or -1): accepted and reported
+ * back for callers that set it.  The encoder has one scheme -- symbols loaded
+ * sixteen steps and more ahead of the state chain, table entries four -- so
+ * the value has no effect. */
 int fvb_set_rans_pipeline(int steps);
 int fvb_get_rans_pipeline(void);
-/* The same choice for the encoder passes after the first, which re-encode
- * only the frames the frame policy retries (gray10 MED, gray16 step
- * refinement): few shards, so the pass is one lane's chain of dependent
- * steps long whatever the load, and fetching further ahead pays. */
+/* The same for the encoder passes after the first. */
 int fvb_set_rans_pipeline_tail(int steps);
 int fvb_get_rans_pipeline_tail(void);
 /* While profiling is on (per calling thread), every launch is bracketed by
