@@ -39,7 +39,7 @@ __host__ __device__ constexpr int64_t fold_padded(int64_t samples) {
 constexpr int kMaxRecordBytes = 3 + 32 + (kShardSymbols * 17 + 7) / 8;
 
 // rANS scratch per shard (encoder): symbol table for the 511 symbols (two
-// words each: freq<<16|cum and floor(2^32/freq)), the serialised table, and
+// words each, see rans_packed), the serialised table, and
 // four byte lanes written back to front.
 constexpr int kRansTableWords = 1024;
 constexpr int kRansSerialBytes = 1024;

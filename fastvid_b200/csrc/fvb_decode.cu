@@ -2,9 +2,9 @@
 //
 //   dec_parse        : thread-per-tile directory + shard-header walk
 //                      (reference decode.cu:131-220)
-//   dec_shards       : warp-per-shard entropy decode of every mode with every
-//                      rejection rule of the reference (decode.cu:222-550)
-//   dec_reconstruct  : warp-per-tile register wavefront, the mirror of
+//   dec_rans_tables, dec_rans, dec_other : entropy decode of every mode with
+//                      every rejection rule of the reference (decode.cu:222-550)
+//   dec_reconstruct  : warp-per-tile (or warp-pair) wavefront, the mirror of
 //                      enc_predict (decode.cu:552-606)
 //   dec_reconstruct_serial : one thread per tile, raster order
 //                      (decode.cu:608-656; the predictor="serial" diagnostic)

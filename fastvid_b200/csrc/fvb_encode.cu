@@ -1,15 +1,16 @@
 // fvb_encode.cu -- sm_100a encoder kernels for the fastvid intra codec.
 //
 // Pipeline (one launch each, all frames of a batch at once):
-//   enc_predict  : warp-per-tile register wavefront: predictor + quantizer +
-//                  reconstruction + zigzag (reference encode.cu:128-193)
+//   enc_predict  : warp-per-tile (or warp-pair) wavefront: predictor, quantizer,
+//                  reconstruction, zigzag (reference encode.cu:128-193);
+//                  enc_lossless for frames of step 1, without a wavefront
 //   enc_analyze  : warp-per-shard cost model: Rice k search, zero-run, block
 //                  pack, rANS histogram + 12-bit normalisation + table bytes
 //                  (encode.cu:195-317, 319-392)
 //   enc_rans     : thread-per-lane interleaved rANS (encode.cu:398-418)
-//   enc_scan     : CTA-per-frame mode choice, record offsets, directory,
-//                  header and the gray10/gray16 frame policy
-//                  (encode.cu:420-430, 812-904)
+//   enc_scan     : CTA-per-frame record offsets, directory, header and the
+//                  gray10/gray16 frame policy (encode.cu:812-904); the mode
+//                  choice (encode.cu:420-430) is enc_rans's
 //   enc_emit     : warp-per-shard record assembly in shared memory and one
 //                  aligned copy-out (encode.cu:488-682)
 // Nothing here traps; every failure is a status word.

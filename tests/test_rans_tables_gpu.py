@@ -1,0 +1,50 @@
+"""rANS shards over the sizes of their tables -- up to 36 symbols (entries in
+shared memory), up to 170 (bucket table in the record), up to 255 (built by the
+decoder), values of eight bits and wider, values above the encoder's local
+table -- and over few shards (tables of all slots) and many: lossless frames
+come back exactly, and small ones equal the oracle's streams byte for byte."""
+
+import numpy as np
+import pytest
+import torch
+
+import fastvid_b200
+import oracle
+from fastvid_b200.batch import BatchCodec
+
+pytestmark = pytest.mark.gpu
+
+# spread of the residuals, about a third of the distinct symbols
+SPREADS = (0, 2, 10, 17, 40, 55, 80, 84)
+
+
+def _planes(width, height, depth, spread, seed, device):
+    """Planes whose prediction residuals lie within +-spread: random samples in
+    a band of width spread (the gradient of such samples stays in the band)."""
+    gen = torch.Generator(device="cpu")
+    gen.manual_seed(seed)
+    mid = 1 << (depth - 1)
+    return tuple((torch.randint(0, spread + 1, (height, width), generator=gen) + mid).to(torch.int32).to(torch.uint16)
+                 .to(device) for _ in range(3))
+
+
+@pytest.mark.parametrize("spread", SPREADS)
+def test_small_frames_match_the_oracle(cuda, spread):
+    for depth in (8, 12, 16):
+        planes = _planes(101, 83, depth, spread, 7 * spread + depth, cuda)
+        kw = dict(layout="rgb444", bit_depth=depth, quality=100, tile_size=(64, 64))
+        stream = fastvid_b200.encode(planes, **kw)
+        assert bytes(stream.cpu().numpy()) == oracle.encode(tuple(p.cpu().numpy() for p in planes), **kw)
+        for a, b in zip(fastvid_b200.decode(stream), planes):
+            assert np.array_equal(a.cpu().numpy(), b.cpu().numpy())
+
+
+@pytest.mark.parametrize("depth", (12, 16))
+def test_many_shards_of_all_table_sizes(cuda, depth):
+    """2,300 shards and more: whole warps of one table size, mixed warps, ragged shards."""
+    frames = [_planes(901, 507, depth, s, 100 + s, cuda) for s in SPREADS]
+    codec = BatchCodec(cuda)
+    streams = codec.encode(frames, layout="rgb444", bit_depth=depth, quality=100, tile_size=(128, 96))
+    for frame, planes in zip(frames, codec.decode(streams)):
+        for a, b in zip(planes, frame):
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16))
