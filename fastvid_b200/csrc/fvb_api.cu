@@ -683,13 +683,18 @@ std::atomic<int> g_rans_pipeline{-1};
 std::atomic<int> g_rans_pipeline_tail{-1};
 std::atomic<int> g_tile_warps{kDefaultTileWarps};
 
-// Whether the u16 wavefronts sweep a tile by warp pairs: as long as every tile
-// then has a pair of its own (two in each of the default four CTAs an SM).  A
-// tile then takes three blocks more than one band instead of all its bands'
-// blocks: a 1080p frame in 256x128 tiles predicts in 47 us instead of 66 and
-// reconstructs in 30 instead of 38; with more tiles the pairs' idle slots cost
-// what the GPU would fill with other tiles.
-bool wave_pairs(int64_t tiles) { return tiles <= static_cast<int64_t>(device_sms()) * 8; }
+// Whether the u16 wavefronts sweep a tile by warp pairs: up to three tiles an
+// SM.  A tile then takes three blocks more than one band instead of all its
+// bands' blocks: a 1080p frame in 256x128 tiles predicts in 47 us instead of 66
+// and reconstructs in 30 instead of 38.  With more tiles a pair no longer has
+// the SM's store path to itself, and the pairs store unaligned rows chunk by
+// chunk: 2979x1875 rgb16 (540 tiles of 256x128) predicts in 115 us by pairs and
+// 85 by single warps and reconstructs in 103 and 68; 16 799x445 rgb12 frames
+// (768 tiles) in 133 and 109, and 125 and 72.  Aligned rows would gain from
+// pairs up to eight tiles an SM (16 800x446 frames: 70 us and 80), which is the
+// smaller difference.
+constexpr int kPairTilesPerSm = 3;
+bool wave_pairs(int64_t tiles) { return tiles <= static_cast<int64_t>(device_sms()) * kPairTilesPerSm; }
 
 // Whether dec_rans runs on tables of all slots: as long as all shards are
 // resident at once that way (six CTAs of two shards on an SM, 94 us for the

@@ -376,8 +376,8 @@ struct WaveBlock {
   }
 };
 
-// A warp pair's sweep of a tile, for launches with fewer tiles than half the
-// GPU's warps: band j runs on warp j % 2, three blocks behind band j - 1, whose
+// A warp pair's sweep of a tile, for launches that leave most of the
+// GPU's warps idle: band j runs on warp j % 2, three blocks behind band j - 1, whose
 // last row has then reached the columns that the block reads (row 63 is two
 // blocks behind row 0), in lock-step at the pair's barrier after every block.  A
 // carry row is overwritten by the band after next, at least three blocks behind
