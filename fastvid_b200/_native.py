@@ -78,6 +78,7 @@ SIGNATURES = {
     "fvb_profile_end": ([c_p, c_p, c_i32], c_i32),
     "fvb_encode_plan": ([c_i64, c_i64, c_i32, c_i32, c_i32, c_i64, c_i64, c_i64, c_i64,
                          ctypes.POINTER(Frame), ctypes.POINTER(c_i64)], c_i32),
+    "fvb_tile_geometry": ([ctypes.POINTER(Frame), c_i64, ctypes.POINTER(c_i64)], c_i32),
     "fvb_encode_analyze": ([ctypes.POINTER(Frame), c_p, c_p, c_p, c_i64, c_p, ctypes.POINTER(c_i64)], c_i32),
     "fvb_encode_emit": ([ctypes.POINTER(Frame), c_p, c_i64, c_p, c_i64, c_p], c_i32),
     "fvb_decode_plan": ([c_p, c_i64, c_i64, ctypes.POINTER(Frame), ctypes.POINTER(c_i64)], c_i32),

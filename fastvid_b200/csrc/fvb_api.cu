@@ -179,7 +179,7 @@ void build_desc(const fvb_frame& fr, FrameDesc& d, int use_med) {
       const int64_t h = r ? d.last_h : fr.tile_h;
       d.shards_int[p][r] = static_cast<int32_t>(ceil_div(ptw * h, kShardSymbols));
       d.shards_last[p][r] = static_cast<int32_t>(ceil_div(wl * h, kShardSymbols));
-      d.fold_int[p][r] = static_cast<int32_t>(fold_padded(ptw * h));
+      d.fold_int[p][r] = fold_padded(ptw * h);
       const int64_t row = (txs - 1) * fold_padded(ptw * h) + fold_padded(wl * h);
       if (!r) d.fold_row[p] = row;
       fold += r ? row : (d.tiles_y - 1) * row;
@@ -876,6 +876,16 @@ int fvb_encode_plan(int64_t width, int64_t height, int layout, int bit_depth, in
   if (workspace_bytes) {
     *workspace_bytes = static_cast<int64_t>(enc_layout(totals_of(frame, 1)).total);
   }
+  return FVB_OK;
+}
+
+int fvb_tile_geometry(const fvb_frame* frame, int64_t tile, int64_t* geometry) {
+  if (!frame || !geometry || tile < 0 || tile >= frame->tiles) return fail(FVB_ERR_ARGUMENT, "no such tile");
+  FrameDesc d;
+  build_desc(*frame, d, 0);
+  const TileGeo g = tile_geo(d, tile);
+  const int64_t out[8] = {g.plane, g.x, g.y, g.w, g.h, g.sample_base, g.first_shard, g.shard_count};
+  std::memcpy(geometry, out, sizeof(out));
   return FVB_OK;
 }
 

@@ -72,7 +72,7 @@ struct FrameDesc {
   int64_t shard0[4];    // first shard of each plane
   int64_t fold0[3];       // folded index of each plane's first sample
   int64_t fold_row[3];    // folded samples of one full-height tile row
-  int32_t fold_int[3][2]; // folded samples of an interior tile [plane][last row?]
+  int64_t fold_int[3][2]; // folded samples of an interior tile [plane][last row?]; tiles may have 2^32 samples
   int64_t shards_row[3];      // shards in one full-height tile row
   int32_t shards_int[3][2];   // shards of an interior tile [plane][last row?]
   int32_t shards_last[3][2];  // shards of a last-column tile
@@ -165,8 +165,7 @@ __host__ __device__ inline TileGeo tile_geo(const FrameDesc& f, int64_t t) {
   g.y = ty * f.tile_h;
   g.w = last_col ? f.plane_w[p] - g.x : f.ptile_w[p];
   g.h = last_row ? f.last_h : f.tile_h;
-  g.sample_base = f.fold0[p] + static_cast<int64_t>(ty) * f.fold_row[p] +
-                  static_cast<int64_t>(tx) * f.fold_int[p][last_row];
+  g.sample_base = f.fold0[p] + ty * f.fold_row[p] + tx * f.fold_int[p][last_row];
   g.first_shard = f.shard0[p] + static_cast<int64_t>(ty) * f.shards_row[p] +
                   static_cast<int64_t>(tx) * f.shards_int[p][last_row];
   g.shard_count = last_col ? f.shards_last[p][last_row] : f.shards_int[p][last_row];

@@ -127,6 +127,12 @@ int fvb_encode_plan(int64_t width, int64_t height, int layout, int bit_depth, in
                     int64_t fps_num, int64_t fps_den, int64_t tile_w, int64_t tile_h,
                     fvb_frame* frame, int64_t* workspace_bytes);
 
+/* Placement of one tile of a planned frame, as the kernels compute it: plane,
+ * x, y, width, height, index of its first symbol in the workspace's symbol
+ * array (tiles in order, each padded to a multiple of eight), its first shard
+ * and its number of shards.  FVB_ERR_ARGUMENT for a tile the frame has not. */
+int fvb_tile_geometry(const fvb_frame* frame, int64_t tile, int64_t* geometry);
+
 /* Predicts, analyses and lays out the stream on `cuda_stream` (the frame
  * policy of encode.cu:812-847 runs on the device), then waits for the one
  * 96-byte result read and returns the exact stream length.  planes[p] are
