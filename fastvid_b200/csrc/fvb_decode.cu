@@ -729,6 +729,7 @@ dec_rans_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
     }
     cp_async_commit();
     cp_async_wait<0>();
+    __syncwarp();  // the four lanes of a shard read what each other copied or built; a vote orders no memory
     const bool all_local = __all_sync(kFull, local);
     if (live) {
       const uint16_t* values = reinterpret_cast<const uint16_t*>(t.data + RansTable::values_at(nsym));

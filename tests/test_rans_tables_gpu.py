@@ -10,6 +10,7 @@ import torch
 
 import fastvid_b200
 import oracle
+from fastvid_b200 import autotune
 from fastvid_b200.batch import BatchCodec
 
 pytestmark = pytest.mark.gpu
@@ -48,3 +49,27 @@ def test_many_shards_of_all_table_sizes(cuda, depth):
     for frame, planes in zip(frames, codec.decode(streams)):
         for a, b in zip(planes, frame):
             assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
+def test_warps_that_take_several_groups(cuda):
+    """One CTA an SM, about three groups of eight shards a warp: a table that
+    the four lanes build takes the place of one that they copied, and back."""
+    warps = 4 * torch.cuda.get_device_properties(cuda).multi_processor_count
+    rows = -(-3 * 8 * warps // (3 * 22)) * 64  # 22 shards of 64x64 samples a row of tiles, three planes
+    planes = []
+    for p in range(3):
+        gen = torch.Generator(device="cpu")
+        gen.manual_seed(p)
+        spread = torch.tensor([105, 2, 10, 80, 105, 17, 2, 55, 105]).repeat(1000)
+        tiles = torch.rand(rows // 64, 64, 22, 64, generator=gen)
+        tiles *= spread[:tiles.shape[0] * 22].view(-1, 1, 22, 1) + 1
+        planes.append(tiles.to(torch.int32).view(rows, 22 * 64).to(torch.uint16).to(cuda))
+    codec = BatchCodec(cuda)
+    streams = codec.encode([planes], layout="rgb444", bit_depth=12, quality=100, tile_size=(64, 64))
+    try:
+        autotune.set_launch({"dec_rans": 1})
+        decoded = codec.decode(streams)[0]
+    finally:
+        autotune.reset_launch()
+    for a, b in zip(decoded, planes):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
