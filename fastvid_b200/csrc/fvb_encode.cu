@@ -1605,6 +1605,7 @@ enc_rans_kernel(const FrameDesc* __restrict__ frames, const FrameState* __restri
     }
   cp_async_commit();
   cp_async_wait<0>();
+  __syncwarp();  // the four lanes of a shard look up entries that each other copied; a vote orders no memory
   const bool all_local = !__any_sync(kFull, top >= kEncLocal);
   const int count = live ? shards[s].count : -1;
   const int count0 = __shfl_sync(kFull, count, 0);  // by all lanes: not inside the condition

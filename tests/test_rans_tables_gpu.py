@@ -73,3 +73,21 @@ def test_warps_that_take_several_groups(cuda):
         autotune.reset_launch()
     for a, b in zip(decoded, planes):
         assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
+@pytest.mark.parametrize("depth", (12, 16))
+def test_neighbouring_shards_of_different_tables(cuda, depth):
+    """The eight shards of an encoder warp with a table of their own each,
+    within the local table and above it, some of them ragged."""
+    gen = torch.Generator(device="cpu")
+    gen.manual_seed(depth)
+    spread = torch.tensor([105, 2, 40, 10, 80, 0, 17, 55, 84]).repeat(8)[:64]
+    planes = []
+    for p in range(3):
+        tiles = torch.rand(8, 64, 8, 64, generator=gen) * (spread.roll(p).view(8, 1, 8, 1) + 1)
+        planes.append(tiles.to(torch.int32).view(512, 512)[:509, :507].numpy().astype(np.uint16))
+    kw = dict(layout="rgb444", bit_depth=depth, quality=100, tile_size=(64, 64))
+    stream = fastvid_b200.encode(tuple(torch.from_numpy(p.copy()).to(cuda) for p in planes), **kw)
+    assert bytes(stream.cpu().numpy()) == oracle.encode(tuple(np.ascontiguousarray(p) for p in planes), **kw)
+    for a, b in zip(fastvid_b200.decode(stream), planes):
+        assert np.array_equal(a.cpu().numpy(), b)
