@@ -1725,6 +1725,7 @@ enc_scan_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
   const int64_t payload = carry_s;
   // directory (encode.cu:886-902)
   uint8_t* pre = prefix + f.prefix_base;
+  int too_large = 0;
   for (int64_t t = threadIdx.x; t < f.ntiles; t += blockDim.x) {
     const TileGeo g = tile_geo(f, t);
     const int64_t off = fs[g.first_shard].offset;
@@ -1737,9 +1738,12 @@ enc_scan_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
                       static_cast<uint32_t>(g.x), static_cast<uint32_t>(g.y), static_cast<uint32_t>(g.w));
     e[1] = make_uint4(static_cast<uint32_t>(g.h), static_cast<uint32_t>(off),
                       static_cast<uint32_t>(static_cast<uint64_t>(off) >> 32), static_cast<uint32_t>(end - off));
-    if (end - off > 0xffffffffll) set_status(&st.status, kStatusInternal + 1);  // "tile payload is too large"
+    too_large |= end - off > 0xffffffffll;
   }
+  // thread 0 decides and reports after every thread's tiles are known
+  too_large = __syncthreads_or(too_large);
   if (threadIdx.x == 0) {
+    if (too_large) set_status(&st.status, kStatusInternal + 1);  // "tile payload is too large"
     // frame policy
     const int64_t N = f.nsamples;
     int next = 0;  // 0 done, 1 run again
