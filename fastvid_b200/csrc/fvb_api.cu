@@ -563,33 +563,56 @@ __global__ void read_header_kernel(const uint8_t* __restrict__ stream, uint8_t* 
   out[threadIdx.x] = stream[threadIdx.x];
 }
 
-// 64 bytes of page-locked memory, one block per host thread, that the
-// single-frame entry points' kernels write their results to (see host_mapped
-// for why; a copy to pageable memory also costs a staging copy).  The entry
-// points wait for the result, so a block serves one call at a time.
-struct PinnedResult {
+// 64 bytes of page-locked memory that the kernels of a single-frame call write
+// its results to (see host_mapped for why; a copy to pageable memory also costs
+// a staging copy).  The call waits for its kernels and hands the block on to
+// the next call, of any thread; there are as many blocks as there have been
+// calls at once, and none is freed before the process ends: cudaFreeHost would
+// wait for the device, and it ends another thread's stream capture.
+std::mutex g_result_mutex;
+int64_t* g_result_free = nullptr;  // blocks not in use, linked through their first word
+
+struct ResultBlock {
   int64_t* host = nullptr;
-  ~PinnedResult() {
-    if (host) cudaFreeHost(host);
+  bool in_flight = false;  // kernels may still write to the block: it is not handed on
+  ResultBlock() = default;
+  ResultBlock(const ResultBlock&) = delete;
+  ResultBlock& operator=(const ResultBlock&) = delete;
+  ~ResultBlock() {
+    if (!host || in_flight) return;
+    std::lock_guard<std::mutex> lock(g_result_mutex);
+    std::memcpy(host, &g_result_free, sizeof(g_result_free));
+    g_result_free = host;
+  }
+  int acquire() {
+    {
+      std::lock_guard<std::mutex> lock(g_result_mutex);
+      if (g_result_free) {
+        host = g_result_free;
+        std::memcpy(&g_result_free, host, sizeof(g_result_free));
+      }
+    }
+    if (!host) {
+      // another thread may be capturing its stream: this allocation is no part of it
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      FVB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      const cudaError_t e =
+          cudaHostAlloc(reinterpret_cast<void**>(&host), 64, cudaHostAllocPortable | cudaHostAllocMapped);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      if (e != cudaSuccess) {
+        host = nullptr;
+        return cuda_fail(e, "cudaHostAlloc");
+      }
+    }
+    in_flight = true;
+    return FVB_OK;
+  }
+  int wait(cudaStream_t stream) {
+    FVB_CUDA(cudaStreamSynchronize(stream));
+    in_flight = false;
+    return FVB_OK;
   }
 };
-int pinned_result(int64_t** out) {
-  thread_local PinnedResult r;
-  if (!r.host) {
-    // another thread may be capturing its stream: this allocation is no part of it
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    FVB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-    const cudaError_t e =
-        cudaHostAlloc(reinterpret_cast<void**>(&r.host), 64, cudaHostAllocPortable | cudaHostAllocMapped);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (e != cudaSuccess) {
-      r.host = nullptr;
-      return cuda_fail(e, "cudaHostAlloc");
-    }
-  }
-  *out = r.host;
-  return FVB_OK;
-}
 
 // Restores the caller's current device when an entry point returns: the
 // library launches on the device that owns the workspace and switches to it
@@ -1186,15 +1209,18 @@ int fvb_encode_analyze(const fvb_frame* frame, const uint16_t* const* planes, co
   const Totals t = totals_of(frame, 1);
   rc = encode_prepare(t, frame, 1, p3, q3, workspace, workspace_bytes, cuda_stream, true);
   if (rc) return rc;
-  int64_t* res = nullptr;
-  rc = pinned_result(&res);
+  ResultBlock block;
+  rc = block.acquire();
   if (rc) return rc;
-  rc = encode_enqueue(t, workspace, workspace_bytes, res, cuda_stream, true);
-  if (rc) {  // no kernel of this call may write the result block after it
-    cudaStreamSynchronize(static_cast<cudaStream_t>(cuda_stream));
-    return rc;
+  const int64_t* res = block.host;
+  rc = encode_enqueue(t, workspace, workspace_bytes, block.host, cuda_stream, true);
+  if (rc) {  // wait for what was launched, and report the first error
+    const std::string error = g_error;
+    block.wait(static_cast<cudaStream_t>(cuda_stream));
+    return fail(rc, error);
   }
-  FVB_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(cuda_stream)));
+  rc = block.wait(static_cast<cudaStream_t>(cuda_stream));
+  if (rc) return rc;
   if (res[0] != 0) return fail(static_cast<int>(res[0] < kStatusInternal ? res[0] : FVB_ERR_INTERNAL),
                                status_message_encode(res[0]));
   if (stream_len) *stream_len = res[1];
@@ -1270,17 +1296,21 @@ int fvb_read_header(const uint8_t* stream_bytes, uint8_t* header, void* cuda_str
   if (device < 0) return fail(FVB_ERR_ARGUMENT, "encoded stream must be device memory");
   int cur = -1;
   if (cudaGetDevice(&cur) != cudaSuccess || cur != device) FVB_CUDA(cudaSetDevice(device));
-  int64_t* res = nullptr;
-  const int rc = pinned_result(&res);
+  ResultBlock block;
+  int rc = block.acquire();
   if (rc) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   {
     LaunchScope scope_(K_RESULTS, stream);
-    read_header_kernel<<<1, kHeaderBytes, 0, stream>>>(stream_bytes, static_cast<uint8_t*>(host_mapped(res)));
+    // the block's address is the device's too (unified addressing); host_mapped
+    // would find none for it in a thread that has no context yet
+    read_header_kernel<<<1, kHeaderBytes, 0, stream>>>(stream_bytes, reinterpret_cast<uint8_t*>(block.host));
   }
-  FVB_LAUNCHED("read_header_kernel");
-  FVB_CUDA(cudaStreamSynchronize(stream));
-  std::memcpy(header, res, kHeaderBytes);
+  const cudaError_t launched = cudaGetLastError();
+  rc = block.wait(stream);
+  if (launched != cudaSuccess) return cuda_fail(launched, "read_header_kernel");
+  if (rc) return rc;
+  std::memcpy(header, block.host, kHeaderBytes);
   return FVB_OK;
 }
 
@@ -1539,15 +1569,18 @@ int fvb_decode(const fvb_frame* frame, const uint8_t* stream, int64_t stream_len
   const Totals t = totals_of(frame, 1);
   rc = decode_prepare(t, frame, 1, s1, l1, p3, q3, workspace, workspace_bytes, cuda_stream, true);
   if (rc) return rc;
-  int64_t* res = nullptr;
-  rc = pinned_result(&res);
+  ResultBlock block;
+  rc = block.acquire();
   if (rc) return rc;
-  rc = decode_enqueue(t, wavefront, workspace, workspace_bytes, res, cuda_stream, true, true);
-  if (rc) {  // no kernel of this call may write the result block after it
-    cudaStreamSynchronize(static_cast<cudaStream_t>(cuda_stream));
-    return rc;
+  const int64_t* res = block.host;
+  rc = decode_enqueue(t, wavefront, workspace, workspace_bytes, block.host, cuda_stream, true, true);
+  if (rc) {  // wait for what was launched, and report the first error
+    const std::string error = g_error;
+    block.wait(static_cast<cudaStream_t>(cuda_stream));
+    return fail(rc, error);
   }
-  FVB_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(cuda_stream)));
+  rc = block.wait(static_cast<cudaStream_t>(cuda_stream));
+  if (rc) return rc;
   if (res[0] != 0) {
     char buf[96];
     std::snprintf(buf, sizeof(buf), "malformed entropy payload (CUDA status %lld)", static_cast<long long>(res[0]));
