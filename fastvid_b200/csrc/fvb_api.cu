@@ -324,11 +324,10 @@ struct Totals {
   int64_t samples_p[kMaxPasses] = {0, 0, 0}, prefix_p[kMaxPasses] = {0, 0, 0};
 };
 
-// Folded samples of a frame: its samples with every tile padded.
-int64_t folded_samples(const fvb_frame& fr) {
-  FrameDesc d;
-  build_desc(fr, d, 0);
-  return d.nfold;
+// Room for the symbols of so many samples in so many tiles, each of which is
+// padded to kFoldAlign.
+size_t fold_room(int64_t samples, int64_t tiles) {
+  return static_cast<size_t>(samples) + (kFoldAlign - 1) * static_cast<size_t>(tiles);
 }
 
 Totals totals_of(const fvb_frame* frames, int n) {
@@ -338,8 +337,7 @@ Totals totals_of(const fvb_frame* frames, int n) {
     const fvb_frame& f = frames[i];
     t.tiles += f.tiles;
     t.shards += f.shards;
-    const int64_t folded = folded_samples(f);
-    t.samples += folded;
+    t.samples += f.samples;
     t.prefix += f.prefix_bytes;
     const int64_t ptw0 = f.tile_w;
     if (ptw0 > kFastMaxW) t.wide = true;
@@ -351,7 +349,7 @@ Totals totals_of(const fvb_frame* frames, int n) {
       ++t.frames_p[p];
       t.tiles_p[p] += f.tiles;
       t.shards_p[p] += f.shards;
-      t.samples_p[p] += folded;
+      t.samples_p[p] += f.samples;
       t.prefix_p[p] += f.prefix_bytes;
     }
   }
@@ -497,14 +495,14 @@ EncLayout enc_layout(const Totals& t) {
   w.results = take(16 * static_cast<size_t>(n));
   w.shards = take(sizeof(ShardInfo) * t.shards);
   w.sizes = take(sizeof(int32_t) * t.shards);
-  w.folded = take((t.fold16 ? 2 : 4) * static_cast<size_t>(t.samples));
+  w.folded = take((t.fold16 ? 2 : 4) * fold_room(t.samples, t.tiles));
   w.rans = take(static_cast<size_t>(kRansScratchBytes) * t.shards);
   w.prefix = take(static_cast<size_t>(t.prefix));
-  w.recon = take(t.wide ? 2 * static_cast<size_t>(t.samples) : 0);
+  w.recon = take(t.wide ? 2 * fold_room(t.samples, t.tiles) : 0);
   const bool later = t.passes > 1;
   w.shards_b = take(later ? sizeof(ShardInfo) * t.shards_p[1] : 0);
   w.sizes_b = take(later ? sizeof(int32_t) * t.shards_p[1] : 0);
-  w.folded_b = take(later ? (t.fold16 ? 2 : 4) * static_cast<size_t>(t.samples_p[1]) : 0);
+  w.folded_b = take(later ? (t.fold16 ? 2 : 4) * fold_room(t.samples_p[1], t.tiles_p[1]) : 0);
   w.rans_b = take(later ? static_cast<size_t>(kRansScratchBytes) * t.shards_p[1] : 0);
   w.prefix_b = take(later ? static_cast<size_t>(t.prefix_p[1]) : 0);
   w.total = o;
@@ -533,7 +531,7 @@ DecLayout dec_layout(const Totals& t) {
   w.shards = take(sizeof(ShardInfo) * t.shards);
   w.items = take(4 * 4 * static_cast<size_t>(t.shards));
   w.tables = take(dec_rans_table_bytes() * static_cast<size_t>(t.shards));
-  w.folded = take((t.fold16 ? 2 : 4) * static_cast<size_t>(t.samples));
+  w.folded = take((t.fold16 ? 2 : 4) * fold_room(t.samples, t.tiles));
   w.total = o;
   return w;
 }
