@@ -1699,16 +1699,18 @@ __global__ void dec_reconstruct_wide_kernel(const FrameDesc* __restrict__ frames
     const int64_t pitch = f.dst_pitch[g.plane];
     const int64_t fbase = f.sample_base + g.sample_base;
     const int32_t maxs = f.max_sample;
+    const bool med = f.use_med0 != 0;
+    const Deltas deltas(f, folded, fold16);
     for (int d = 0; d < g.w + g.h - 1; ++d) {
       const int y0 = max(0, d - g.w + 1), y1 = min(d, g.h - 1);
       for (int y = y0 + threadIdx.x; y <= y1; y += blockDim.x) {
         const int x = d - y;
         uint16_t* o = plane + static_cast<int64_t>(g.y + y) * pitch + g.x + x;
+        const int32_t dq = deltas[fbase + static_cast<int64_t>(y) * g.w + x];
         const int32_t l = x > 0 ? o[-1] : 0;
         const int32_t a = y > 0 ? o[-pitch] : 0;
         const int32_t ul = (x > 0 && y > 0) ? o[-pitch - 1] : 0;
-        const int32_t pred = f.use_med0 ? predict_med(l, a, ul) : predict_grad(l, a, ul, maxs);
-        const int32_t dq = delta_at(f, folded, fold16, fbase + static_cast<int64_t>(y) * g.w + x);
+        const int32_t pred = med ? predict_med(l, a, ul) : predict_grad(l, a, ul, maxs);
         *o = static_cast<uint16_t>(max(0, min(maxs, pred + dq)));
       }
       __syncthreads();
@@ -1734,6 +1736,7 @@ __global__ void dec_reconstruct_serial_kernel(const FrameDesc* __restrict__ fram
   const int64_t fbase = f.sample_base + g.sample_base;
   const int32_t maxs = f.max_sample;
   const bool med = f.use_med0 != 0;
+  const Deltas deltas(f, folded, fold16);
   for (int y = 0; y < g.h; ++y) {
     int32_t left = 0, ul = 0;
     uint16_t* orow = plane + static_cast<int64_t>(g.y + y) * pitch + g.x;
@@ -1741,7 +1744,7 @@ __global__ void dec_reconstruct_serial_kernel(const FrameDesc* __restrict__ fram
     for (int x = 0; x < g.w; ++x) {
       const int32_t a = y > 0 ? orow[x - pitch] : 0;
       const int32_t pred = med ? predict_med(left, a, ul) : predict_grad(left, a, ul, maxs);
-      const int32_t r = max(0, min(maxs, pred + delta_at(f, folded, fold16, frow + x)));
+      const int32_t r = max(0, min(maxs, pred + deltas[frow + x]));
       orow[x] = static_cast<uint16_t>(r);
       ul = a;
       left = r;
