@@ -861,8 +861,8 @@ struct RiceBody {
 // Reads codes from bit `pos` while they start before `lim`, in a lane that
 // ends at bit `end`: emit(quotient, remainder, index) for each.  Returns the
 // bit after the last code, or kRiceNone when no further code was found (`rest`
-// is then where the search began; `bad` is set when the lane ends within a
-// code).  The number of codes is added to n.
+// is then where the search began; `bad`, which emit may share, is set when the
+// lane ends within a code and never cleared).  The number of codes is added to n.
 template <typename Emit>
 __device__ __forceinline__ int rice_read(const RiceBody& body, int pos, int lim, int end, int k, int& n, int& rest,
                                          bool& bad, Emit emit) {
@@ -899,7 +899,7 @@ __device__ __forceinline__ int rice_read(const RiceBody& body, int pos, int lim,
     p += x ? __ffs(x) - 1 : 0;
     if (p + 1 + k > end) {  // no further one bit in the lane, or one whose code would run past it
       rest = pos;
-      bad = p < end;
+      bad |= p < end;
       return kRiceNone;
     }
     const int r = p + 1;

@@ -80,3 +80,25 @@ def test_rice_lanes(cuda, k, pattern):
                         _stream(v, k, depth, width, height, cut=1)):
                 _check(bad)
     assert accepted >= 6
+
+
+@pytest.mark.parametrize("k", (4, 8, 12))
+def test_values_above_the_range_are_rejected(cuda, k):
+    """One value at or just above the largest, near a lane's end: before the
+    padding of its last byte and elsewhere."""
+    rng = np.random.default_rng(k)
+    outcomes = set()
+    for depth in (8, 12):
+        top = 2 * ((1 << depth) - 1)
+        for width, height in ((64, 64), (61, 67), (40, 30), (33, 3), (5, 1), (1, 1)):
+            n = width * height
+            for back in (1, 2, 3, 4, 5, 9, 40, 200):
+                if back > n:
+                    continue
+                for above in (0, 1, 2):
+                    v = np.minimum(rng.integers(0, 3 << k, n), top)
+                    v[n - back] = top + above
+                    accepted = _check(_stream(v.astype(int).tolist(), k, depth, width, height))
+                    assert accepted == (above == 0)
+                    outcomes.add(accepted)
+    assert outcomes == {True, False}
