@@ -67,9 +67,10 @@ __device__ __forceinline__ T fold_value(uint32_t v, const FoldMap& m) {
   }
 }
 // The residuals times the step of a decoded frame's samples, for the kernels
-// that reconstruct sample by sample.  What it depends on is held here: read from
-// the frame's descriptor, each sample would wait for it, as the kernels store
-// between two samples (a 1080p yuv422 10-bit frame as one tile 7.9 ms, 5.6 so).
+// that reconstruct sample by sample and read neighbours back from the planes.
+// What they depend on is held here, and they are read by plain loads: read-only
+// loads made the same kernels slower by a third to twice (a 1080p yuv422 10-bit
+// frame as one tile 7.2 and 5.6 ms; 7.9 with the descriptor read per sample).
 struct Deltas {
   const void* folded;
   int32_t step;
@@ -77,8 +78,8 @@ struct Deltas {
   __device__ Deltas(const FrameDesc& f, const void* folded_, int fold16)
       : folded(folded_), step(f.step0), u16(fold16 != 0), products(fold16 && f.bit_depth <= 12) {}
   __device__ __forceinline__ int32_t operator[](int64_t i) const {
-    if (!u16) return unzigzag(__ldg(static_cast<const uint32_t*>(folded) + i)) * step;
-    const uint16_t v = __ldg(static_cast<const uint16_t*>(folded) + i);
+    if (!u16) return unzigzag(static_cast<const uint32_t*>(folded)[i]) * step;
+    const uint16_t v = static_cast<const uint16_t*>(folded)[i];
     return products ? static_cast<int16_t>(v) : unzigzag(v) * step;
   }
 };
