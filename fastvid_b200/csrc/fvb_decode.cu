@@ -37,8 +37,12 @@ __device__ __forceinline__ uint32_t rd32(const uint8_t* p) {
 __device__ __forceinline__ uint64_t rd64(const uint8_t* p) {
   return rd32(p) | (static_cast<uint64_t>(rd32(p + 4)) << 32);
 }
-__device__ __forceinline__ int list_of_mode(int mode) {
-  return mode == kModeOrder0 ? 0 : (mode >= 1 && mode <= 17) ? 1 : mode == 0 ? 2 : 3;
+constexpr int kRiceSmall = 1024;  // see rice_shard
+__device__ __forceinline__ int list_of(int mode, int count) {
+  return mode == kModeOrder0 ? 0 : (mode >= 1 && mode <= 17) ? (count > kRiceSmall ? 1 : 4) : mode == 0 ? 2 : 3;
+}
+__device__ __forceinline__ int64_t list_slot(int list, int64_t pos, int64_t total_shards) {
+  return list == 4 ? 2 * total_shards - 1 - pos : list * total_shards + pos;
 }
 }  // namespace
 
@@ -133,7 +137,7 @@ __global__ void dec_parse_kernel(const FrameDesc* __restrict__ frames, FrameStat
     const int lane = static_cast<int>(threadIdx.x & 31);
     for (int j = 0; j < g.shard_count; ++j) {
       const int64_t s = f.shard_base + g.first_shard + j;
-      const int list = list_of_mode(shards[s].mode);
+      const int list = list_of(shards[s].mode, shards[s].count);
       const unsigned active = __activemask();
       const unsigned peers = __match_any_sync(active, list);
       const int leader = __ffs(peers) - 1;
@@ -141,7 +145,7 @@ __global__ void dec_parse_kernel(const FrameDesc* __restrict__ frames, FrameStat
       if (lane == leader) base = atomicAdd(&lists->count[list], __popc(peers));
       base = __shfl_sync(peers, base, leader);
       const int pos = base + __popc(peers & ((1u << lane) - 1u));
-      list_items[static_cast<int64_t>(list) * total_shards + pos] = static_cast<int32_t>(s);
+      list_items[list_slot(list, pos, total_shards)] = static_cast<int32_t>(s);
     }
   }
 }
@@ -833,18 +837,50 @@ dec_rans_slots_kernel(const FrameDesc* __restrict__ frames, FrameState* __restri
 // (about 30 instructions and 180 cycles in a lone warp): one thread a lane
 // read 1,024 of them in series, 100 us for the smallest frame with Rice
 // shards; eight threads a lane (a warp per shard) took 28 us, 32 take 12 us.
-constexpr int kRiceThreads = 32;    // per Rice lane
+//
+// Small shards (kRiceSmall) go a warp each, eight threads a lane, when there are
+// more than CTAs: with a few codes a thread a CTA's barriers and its other lead-ins
+// cost more than the codes.  4 4K gray8 frames in 32x32 tiles (32,640 shards of
+// 1,024 symbols) take 131 us so and 216 a CTA each, in 16x16 tiles 275 and 746;
+// one 720p frame in 32x32 tiles (920 shards) 27 and 17, in 32x16 tiles (1,800) 23
+// and 21, in 16x16 tiles (3,600) 19 and 29.  Shards of 2,048 symbols do as well
+// either way.
 constexpr int kOtherWarps = 4;
-constexpr int kRiceStage = 8800;    // bytes of a body held in shared memory: above any that the encoder writes
+constexpr int kRiceStage = 8832;    // bytes of a body held in shared memory: above any that the encoder writes
+constexpr int kRiceWave = 148 * 12;  // CTAs on the GPU at once
 constexpr int kRiceNone = 0x7fffffff;
+
+// The threads that decode a shard together: a CTA, or one of its warps with a
+// quarter of the CTA's shared memory.
+template <int WARPS>
+struct RiceGroup {
+  static constexpr int kThreads = 32 * WARPS;
+  static constexpr int kParts = 8 * WARPS;  // threads per Rice lane
+  static constexpr int kStage = kRiceStage * WARPS / kOtherWarps;
+  static constexpr int kSymbols = kShardSymbols * WARPS / kOtherWarps;
+  static constexpr int kBodyWords = (kStage + 48) / 4;
+  static __device__ __forceinline__ void sync() {
+    if (WARPS == 1) __syncwarp();
+    else __syncthreads();
+  }
+  // whether any thread's is true; orders shared memory as sync() does
+  static __device__ __forceinline__ bool any(bool b) {
+    if (WARPS > 1) return __syncthreads_or(b);
+    __syncwarp();
+    return __any_sync(kFull, b);
+  }
+};
+static_assert(RiceGroup<1>::kSymbols >= kRiceSmall, "a small shard's symbols");
 
 template <typename FoldT>
 struct alignas(16) RiceSm {
-  uint32_t body[(kRiceStage + 48) / 4];
+  uint32_t body[kOtherWarps * RiceGroup<1>::kBodyWords];
   FoldT out[kShardSymbols];
-  int32_t stop[4 * kRiceThreads];
+  int32_t stop[32 * kOtherWarps];
   int32_t total[kOtherWarps][4];
 };
+static_assert(kOtherWarps * RiceGroup<1>::kBodyWords >= RiceGroup<kOtherWarps>::kBodyWords &&
+                  RiceGroup<1>::kBodyWords % 4 == 0, "staging");
 
 // Words of a body, in shared memory or (a longer one) in global memory, where
 // only words that hold a byte of it are read; words past the end are zero.
@@ -910,12 +946,16 @@ __device__ __forceinline__ int rice_read(const RiceBody& body, int pos, int lim,
   return pos;
 }
 
-// A Rice shard by the whole CTA; returns whether it is valid (every thread
-// the same).
-template <typename FoldT>
-__device__ bool rice_shard(const uint8_t* __restrict__ body, int blen, int n, int k, uint32_t maxf, const FoldMap& fm,
-                           FoldT* __restrict__ out, RiceSm<FoldT>& sm) {
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+// A Rice shard by thread t of a group (of a CTA's warp w, when the group is a
+// warp); returns whether it is valid (every thread the same).
+template <int WARPS, typename FoldT>
+__device__ bool rice_shard(int w, int t, const uint8_t* __restrict__ body, int blen, int n, int k, uint32_t maxf,
+                           const FoldMap& fm, FoldT* __restrict__ out, RiceSm<FoldT>& sm) {
+  using G = RiceGroup<WARPS>;
+  uint32_t* const stage = sm.body + w * G::kBodyWords;
+  FoldT* const sout = sm.out + w * G::kSymbols;
+  int32_t* const stops = sm.stop + w * G::kThreads;
+  const int warp = t >> 5, lane = t & 31;
   const int lc = min(4, n);
   const int table = (lc - 1) * 4;
   if (table > blen) return false;
@@ -925,22 +965,22 @@ __device__ bool rice_shard(const uint8_t* __restrict__ body, int blen, int n, in
   const uint8_t* from = body - head;
   const int bytes = head + blen;
   RiceBody rb;
-  rb.staged = bytes <= kRiceStage;
+  rb.staged = bytes <= G::kStage;
   rb.last = (bytes - 1) >> 2;
   if (rb.staged) {
-    for (int i = 16 * t; i < bytes + 32; i += 16 * 32 * kOtherWarps) {
-      const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(sm.body)) + i;
+    for (int i = 16 * t; i < bytes + 32; i += 16 * G::kThreads) {
+      const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(stage)) + i;
       const int have = max(0, min(16, bytes - i));  // the rest of the 16 bytes is zeroed
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(have ? from + i : from), "r"(have)
                    : "memory");
     }
     cp_async_commit();
-    rb.words = sm.body;
+    rb.words = stage;
   } else {
     rb.words = reinterpret_cast<const uint32_t*>(from);
   }
   cp_async_wait<0>();
-  __syncthreads();
+  G::sync();
   // thread: Rice lane rl, part `part` of its bits (bit positions from `from`)
   const int rl = t & 3, part = t >> 2;
   const bool live = rl < lc;
@@ -953,12 +993,12 @@ __device__ bool rice_shard(const uint8_t* __restrict__ body, int blen, int n, in
   }
   if (rl == lc - 1) len = blen - off;
   if (off > blen || len < 0 || len > blen - off) bad = live;
-  if (__syncthreads_or(bad)) return false;
+  if (G::any(bad)) return false;
   const int nl = live ? (n - rl + lc - 1) / lc : 0;  // codes of the lane
   const int begin = 8 * (head + static_cast<int>(off)), end = live ? begin + 8 * static_cast<int>(len) : begin;
   const int size = end - begin;
-  const int lo = begin + static_cast<int>(static_cast<int64_t>(size) * part / kRiceThreads);
-  const int lim = begin + static_cast<int>(static_cast<int64_t>(size) * (part + 1) / kRiceThreads);
+  const int lo = begin + static_cast<int>(static_cast<int64_t>(size) * part / G::kParts);
+  const int lim = begin + static_cast<int>(static_cast<int64_t>(size) * (part + 1) / G::kParts);
   auto skip = [](uint32_t, uint32_t, int) {};
   int start = begin, stop, count = 0, rest = begin;
   if (part) {
@@ -966,19 +1006,19 @@ __device__ bool rice_shard(const uint8_t* __restrict__ body, int blen, int n, in
     if (start == kRiceNone) start = lo;
   }
   bool reread = true;
-  for (int round = 0; round < kRiceThreads; ++round) {
+  for (int round = 0; round < G::kParts; ++round) {
     if (reread) {
       count = 0;
       bad = false;
       stop = start;
       if (start != kRiceNone) stop = rice_read(rb, start, lim, end, k, count, rest, bad, skip);
     }
-    sm.stop[t] = stop;
-    __syncthreads();
-    const int before = part ? sm.stop[t - 4] : start;
+    stops[t] = stop;
+    G::sync();
+    const int before = part ? stops[t - 4] : start;
     reread = before != start;
     start = before;
-    if (!__syncthreads_or(reread)) break;
+    if (!G::any(reread)) break;
   }
   int at = count;  // codes of the parts up to this one
 #pragma unroll
@@ -986,27 +1026,29 @@ __device__ bool rice_shard(const uint8_t* __restrict__ body, int blen, int n, in
     const int v = __shfl_up_sync(kFull, at, o);
     if (lane >= o) at += v;
   }
-  if (lane >= 28) sm.total[warp][rl] = at;
-  __syncthreads();
-  for (int w = 0; w < warp; ++w) at += sm.total[w][rl];
+  if constexpr (WARPS > 1) {
+    if (lane >= 28) sm.total[warp][rl] = at;
+    G::sync();
+    for (int v = 0; v < warp; ++v) at += sm.total[v][rl];
+  }
   // exactly the lane's codes, and fewer than eight bits left, all zero
   if (start != kRiceNone && stop == kRiceNone) bad |= end - rest > 7;
-  if (part == kRiceThreads - 1) bad |= at != nl;
+  if (part == G::kParts - 1) bad |= at != nl;
   at -= count;
-  if (__syncthreads_or(bad)) return false;
+  if (G::any(bad)) return false;
   if (start != kRiceNone) {
     int m = 0;
     rice_read(rb, start, lim, end, k, m, rest, bad, [&](uint32_t q, uint32_t r, int i) {
       const uint64_t v = (static_cast<uint64_t>(q) << k) + r;
       bad |= v > maxf;
-      sm.out[(at + i) * lc + rl] = fold_value<FoldT>(static_cast<uint32_t>(v), fm);
+      sout[(at + i) * lc + rl] = fold_value<FoldT>(static_cast<uint32_t>(v), fm);
     });
   }
-  if (__syncthreads_or(bad)) return false;
+  if (G::any(bad)) return false;
   constexpr int kPer = 16 / sizeof(FoldT);
   uint4* o4 = reinterpret_cast<uint4*>(out);  // shards start on 16-byte boundaries
-  for (int i = t; i < n / kPer; i += 32 * kOtherWarps) o4[i] = reinterpret_cast<const uint4*>(sm.out)[i];
-  for (int i = n / kPer * kPer + t; i < n; i += 32 * kOtherWarps) out[i] = sm.out[i];
+  for (int i = t; i < n / kPer; i += G::kThreads) o4[i] = reinterpret_cast<const uint4*>(sout)[i];
+  for (int i = n / kPer * kPer + t; i < n; i += G::kThreads) out[i] = sout[i];
   return true;
 }
 
@@ -1069,7 +1111,8 @@ struct OtherSm {
 
 size_t dec_other_smem(bool fold16) { return fold16 ? sizeof(OtherSm<uint16_t>) : sizeof(OtherSm<uint32_t>); }
 
-// A CTA takes a Rice shard, or four zero-run or block shards (one a warp).
+// A CTA takes a large Rice shard, or four small ones, zero-run or block shards
+// (one a warp).
 template <typename FoldT>
 __global__ void __launch_bounds__(32 * kOtherWarps)
 dec_other_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
@@ -1081,33 +1124,44 @@ dec_other_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   OtherSm<FoldT>& osm = *reinterpret_cast<OtherSm<FoldT>*>(smem_raw);
   OtherGroupSm& sm = osm.block[warp];
-  const int count1 = lists->count[1], count2 = lists->count[2], count3 = lists->count[3];
-  const int fours2 = (count2 + kOtherWarps - 1) / kOtherWarps, fours3 = (count3 + kOtherWarps - 1) / kOtherWarps;
+  // work items: the large Rice shards, the small ones, the others
+  const bool lone = lists->count[4] <= kRiceWave;  // small Rice shards go a CTA each, too
+  int ends[5], items[5] = {0, 1, 4, 2, 3};
+  ends[0] = 0;
+#pragma unroll
+  for (int i = 1; i < 5; ++i) {
+    const int n = lists->count[items[i]];
+    ends[i] = ends[i - 1] + (i == 1 || (i == 2 && lone) ? n : (n + kOtherWarps - 1) / kOtherWarps);
+  }
   for (;;) {
     __syncthreads();  // the CTA's last shard is done, its claim read
     if (threadIdx.x == 0) osm.claimed = atomicAdd(&lists->next_group, 1);
     __syncthreads();
     int g = osm.claimed;
-    if (g >= count1 + fours2 + fours3) break;
-    const int list = g < count1 ? 1 : g < count1 + fours2 ? 2 : 3;  // Rice, zero-run, block pack
-    if (list == 2) g = (g - count1) * kOtherWarps + warp;
-    if (list == 3) g = (g - count1 - fours2) * kOtherWarps + warp;
+    if (g >= ends[4]) break;
+    const int list = g < ends[1] ? 1 : g < ends[2] ? 4 : g < ends[3] ? 2 : 3;
+    const bool cta = list == 1 || (list == 4 && lone);
+    g -= list == 1 ? 0 : list == 4 ? ends[1] : list == 2 ? ends[2] : ends[3];
+    if (!cta) g = g * kOtherWarps + warp;
     if (g >= lists->count[list]) continue;
-    const ShardInfo& si = shards[list_items[static_cast<int64_t>(list) * total_shards + g]];
+    const ShardInfo& si = shards[list_items[list_slot(list, g, total_shards)]];
     const int fi = si.frame;
     // a failed parse may have left shard records unwritten.  (Only the parse
     // writes status 10 and 11; one set meanwhile by another shard must not
-    // split the CTA, so the CTA decides together.)
+    // split the CTA or the warp, so they decide together.)
     const int failed = state[fi].status != 0;
-    if (list == 1 ? __syncthreads_or(failed) : failed) continue;
+    if (cta ? __syncthreads_or(failed) : __any_sync(kFull, failed)) continue;
     const FrameDesc& f = frames[fi];
     const int mode = si.mode, n = si.count, blen = si.body;
     const uint8_t* body = f.stream + si.offset;
     FoldT* out = folded + si.sample_base;
     const uint32_t maxf = static_cast<uint32_t>(f.max_sample) * 2u;
     const FoldMap fm = fold_map(f, sizeof(FoldT) == 2);
-    if (list == 1) {
-      if (!rice_shard(body, blen, n, mode - 1, maxf, fm, out, osm.rice) && threadIdx.x == 0)
+    if (cta) {
+      if (!rice_shard<kOtherWarps>(0, threadIdx.x, body, blen, n, mode - 1, maxf, fm, out, osm.rice) && threadIdx.x == 0)
+        set_status(&state[fi].status, 2);
+    } else if (list == 4) {
+      if (!rice_shard<1>(warp, lane, body, blen, n, mode - 1, maxf, fm, out, osm.rice) && lane == 0)
         set_status(&state[fi].status, 2);
     } else if (list == 2) {
       if (!zero_run_warp(body, blen, n, maxf, fm, out, lane) && lane == 0) set_status(&state[fi].status, 1);

@@ -141,13 +141,15 @@ struct EmitHeads {
 void enc_emit_launch(bool fold16, int grid, size_t smem, cudaStream_t stream, const FrameState* state, EmitRegion a,
                      EmitRegion b, int64_t total_shards, EmitHeads heads, uint8_t* const* outs, uint8_t* only_out);
 cudaError_t enc_emit_set_smem(int bytes);
-// decoder: shards binned by mode (0 rANS, 1 Rice, 2 zero-run, 3 block pack);
-// counts from dims (entry 0)
+// decoder: shards binned by mode (0 rANS, 1 Rice, 2 zero-run, 3 block pack, 4
+// Rice shards of up to kRiceSmall symbols); counts from dims (entry 0).  A list's
+// items lie one after another from list * (shards of the batch) on, the small
+// Rice shards' downwards from the end of list 1's room.
 struct DecodeLists {
-  int32_t count[4];
+  int32_t count[5];
   int32_t next_group;       // dec_other work counter
   int32_t next_group_rans;  // dec_rans work counter
-  int32_t pad[2];
+  int32_t pad;
 };
 struct RansTable;
 __global__ void dec_parse_kernel(const FrameDesc* frames, FrameState* state, const BatchDims* dims,
