@@ -18,7 +18,7 @@ ROOT = PKG.parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libfastvid_b200.so"
 SOURCES = ["fvb_api.cu", "fvb_encode.cu", "fvb_decode.cu"]
-HEADERS = ["fvb_common.cuh", "fvb_kernels.cuh"]
+HEADERS = ["fvb_common.cuh", "fvb_kernels.cuh", "fvb_wave.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
