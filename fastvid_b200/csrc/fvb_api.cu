@@ -719,10 +719,26 @@ bool wave_pairs(int64_t tiles) { return tiles <= static_cast<int64_t>(device_sms
 
 // Whether dec_rans runs on tables of all slots: as long as all shards are
 // resident at once that way (six CTAs of two shards on an SM, 94 us for the
-// chain of a shard against 125 us with bucket tables, which take ten times as
-// many shards at once).
+// chain of a shard against 109 to 125 us with bucket tables, which take eight to
+// thirteen times as many shards at once).
 constexpr int kSlotCtasPerSm = 6;
 bool few_rans_shards(int64_t shards) { return shards <= static_cast<int64_t>(device_sms()) * kSlotCtasPerSm * 2; }
+
+// Whether dec_rans's bucket tables have room for the entries and values of any
+// shard that has such a table: as long as whole shards of all the samples are
+// resident at once that way (three CTAs on an SM; a bucket's capacity may be the
+// next step above), in no more than twice as many shards.  A wide shard's values,
+// read from its table record, hold up the warp at every store: three 2470x1265
+// yuv422-10 frames 146 us without room, 120 with (126 with values looked up symbol
+// by symbol); 9 1080p rgb10 frames 185 and 145; 8 1080p rgb12 frames of tables
+// above 36 symbols 385 and 149.  Past the bound the five CTAs on an SM that the
+// small tables leave room for are better: 14 1080p rgb10 frames 230 us without
+// room, 262 with.
+constexpr int kRoomyCtasPerSm = 3;
+bool roomy_rans_shards(int64_t shards, int64_t samples) {
+  const int64_t wave = static_cast<int64_t>(device_sms()) * kRoomyCtasPerSm * kWarpsPerCta * kGroupShards;
+  return shards <= 2 * wave && samples <= bucket_round(wave * kShardSymbols, 1);
+}
 
 int ctas(int kernel) {
   const int v = g_ctas[kernel].load(std::memory_order_relaxed);
@@ -1462,7 +1478,7 @@ int decode_enqueue(const Totals& t, int wavefront, void* workspace, int64_t work
     const bool few = few_rans_shards(t.shards);
     const int grid = few ? grid_for(t.shards, 2, kSlotCtasPerSm)
                          : grid_for(ceil_div(t.shards, kGroupShards), kWarpsPerCta, ctas(K_DEC_RANS));
-    dec_rans_launch(f16, few, grid, stream, frames_d, state, shards, lists, items, tables, folded);
+    dec_rans_launch(f16, few, roomy_rans_shards(t.shards, t.samples), grid, stream, frames_d, state, shards, lists, items, tables, folded);
   }
   FVB_LAUNCHED("dec_rans_kernel");
   {

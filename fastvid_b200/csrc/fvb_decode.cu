@@ -469,18 +469,22 @@ struct LaneRing {
 };
 
 // Shared memory of one dec_rans warp: eight shards' tables (bucket words, then
-// the entries of up to kLocalSymbols symbols; a shard with more reads its
-// entries from its table record) and the lanes' byte rings.
+// the entries of up to LOCAL symbols; a shard with more reads its entries from
+// its table record) and the lanes' byte rings; ROOMY: the symbols' values too.
 constexpr int kGroups = 8;  // shards per warp, four lanes each
-constexpr int kLocalSymbols = 36;  // five CTAs on an SM: 758 us for 16 4K rgb10 frames, 854 us with 64 and four
-constexpr int kTableWords = kBuckets + kLocalSymbols;
-
+template <bool ROOMY>
 struct alignas(16) RansWarpSm {
-  uint32_t table[kGroups][kTableWords];
+  // 36: five CTAs on an SM, 758 us for 16 4K rgb10 frames, 854 us with 64 and four
+  static constexpr int kSymbols = ROOMY ? 176 : 36;
+  static constexpr int kWords = kBuckets + kSymbols;
+  static constexpr int kValueWords = ROOMY ? kSymbols / 2 : 0;
+  uint32_t table[kGroups][kWords + kValueWords];
   uint4 rings[LaneRing<32>::kChunks][32];
 };
+static_assert(RansWarpSm<true>::kSymbols >= kBucketSymbols && (RansWarpSm<true>::kWords & 3) == 0, "local tables");
 
-size_t dec_rans_smem() { return sizeof(RansWarpSm) * kWarpsPerCta; }
+template <bool ROOMY>
+constexpr size_t dec_rans_smem() { return sizeof(RansWarpSm<ROOMY>) * kWarpsPerCta; }
 
 // Bucket table of a shard of more than kBucketSymbols symbols, by its four
 // lanes: lane l writes buckets 64l .. 64l + 63.
@@ -590,7 +594,7 @@ __device__ __forceinline__ uint32_t rans_four(const Lookup lookup, LaneRing<LANE
 // the four lanes, one byte each, are transposed among the lanes by two
 // shuffles, so each lane stores four consecutive symbols at once.
 template <typename FoldT, int LANES, typename Lookup>
-__device__ __forceinline__ void rans_decode_lane(const Lookup lookup, bool narrow, const uint16_t* __restrict__ values,
+__device__ __forceinline__ void rans_decode_lane(const Lookup lookup, bool narrow, const uint16_t* values,
                                                  LaneRing<LANES>& ring, FoldT* __restrict__ out, int n, int my_l,
                                                  unsigned group, uint32_t& x) {
   const uint32_t sel1 = my_l < 2 ? 0x5410u : 0x3276u, sel2 = (my_l & 1) ? 0x3715u : 0x6240u;
@@ -690,7 +694,8 @@ __device__ __forceinline__ void rans_decode_lane(const Lookup lookup, bool narro
 // bytes for every symbol's value and tables built by four lanes while the rest
 // of the warp waited; 861 us with the value in the entry, 16-byte transposed
 // stores and tables made once by dec_rans_tables; 750 us with 20 warps an SM.
-template <typename FoldT>
+// ROOMY is for launches that leave the SMs room (roomy_rans_shards).
+template <typename FoldT, bool ROOMY>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 dec_rans_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
                 const ShardInfo* __restrict__ shards, DecodeLists* __restrict__ lists,
@@ -698,7 +703,8 @@ dec_rans_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
                 FoldT* __restrict__ folded) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  RansWarpSm& sm = reinterpret_cast<RansWarpSm*>(smem_raw)[warp];
+  using Sm = RansWarpSm<ROOMY>;
+  Sm& sm = reinterpret_cast<Sm*>(smem_raw)[warp];
   const int j = lane >> 2, my_l = lane & 3;
   const unsigned group = 0xfu << (4 * j);
   const int count = lists->count[0];
@@ -711,7 +717,7 @@ dec_rans_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
     const bool live = p < count && tables[p].valid;
     const RansTable& t = tables[live ? p : p0];
     const int nsym = live ? t.nsym : 0;
-    const bool local = nsym <= kLocalSymbols;
+    const bool local = nsym <= Sm::kSymbols;
     LaneRing<32> ring;
     const ShardInfo* si = nullptr;
     const FrameDesc* f = nullptr;
@@ -727,6 +733,8 @@ dec_rans_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
       if (nsym <= kBucketSymbols) {
         const int chunks = (kBuckets + (local ? nsym : 0) + 3) / 4;  // the entries follow the buckets
         for (int i = my_l; i < chunks; i += 4) cp_async16(to + 4 * i, t.data + 4 * i);
+        if (ROOMY && !t.narrow)
+          for (int i = my_l; i < (nsym + 1) / 2; i += 4) cp_async4(to + Sm::kWords + i, t.data + RansTable::values_at(nsym) + i);
       } else {
         build_buckets(to, entries, nsym, my_l);
       }
@@ -742,8 +750,9 @@ dec_rans_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
       const int from = ring.at;
       const uint32_t* at = local ? sm.table[j] + kBuckets : entries;
       if (all_local)
-        rans_decode_lane<FoldT, 32>(BucketLookup{sm.table[j], sm.table[j] + kBuckets}, t.narrow, values, ring, out,
-                                    si->count, my_l, group, x);
+        rans_decode_lane<FoldT, 32>(BucketLookup{sm.table[j], sm.table[j] + kBuckets}, t.narrow,
+                                    ROOMY ? reinterpret_cast<const uint16_t*>(sm.table[j] + Sm::kWords) : values, ring,
+                                    out, si->count, my_l, group, x);
       else
         rans_decode_lane<FoldT, 32>(BucketLookup{sm.table[j], at}, t.narrow, values, ring, out, si->count, my_l,
                                     group, x);
@@ -756,7 +765,7 @@ dec_rans_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ s
 // Few shards: the chain of a step decides, not the number of lanes in flight.
 // A warp of its own takes two shards and spreads their tables over all 4096
 // slots (16 KB each), which leaves one lookup a step: a 1080p rgb10 frame of
-// 1,539 shards takes 94 us here, 125 us in dec_rans_kernel.
+// 1,539 shards takes 94 us here, 125 us in dec_rans_kernel's small tables.
 constexpr int kSlotGroups = 2;
 struct alignas(16) RansSlotSm {
   uint32_t slots[kSlotGroups][1 << kRansTableLog];
@@ -1676,32 +1685,39 @@ void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, bool pairs,
       frames, state, dims, static_cast<const uint32_t*>(folded), queue, results);
 }
 
-void dec_rans_launch(bool fold16, bool few, int grid, cudaStream_t stream, const FrameDesc* frames,
+void dec_rans_launch(bool fold16, bool few, bool roomy, int grid, cudaStream_t stream, const FrameDesc* frames,
                      FrameState* state, const ShardInfo* shards, DecodeLists* lists, const int32_t* list_items,
                      const RansTable* tables, void* folded) {
   const int threads = few ? 32 : kWarpsPerCta * 32;
-  const size_t smem = few ? dec_rans_slots_smem() : dec_rans_smem();
+  const size_t smem = few ? dec_rans_slots_smem() : roomy ? dec_rans_smem<true>() : dec_rans_smem<false>();
   if (fold16) {
-    auto k = few ? dec_rans_slots_kernel<uint16_t> : dec_rans_kernel<uint16_t>;
+    auto k = few     ? dec_rans_slots_kernel<uint16_t>
+             : roomy ? dec_rans_kernel<uint16_t, true>
+                     : dec_rans_kernel<uint16_t, false>;
     k<<<grid, threads, smem, stream>>>(frames, state, shards, lists, list_items, tables,
                                        static_cast<uint16_t*>(folded));
   } else {
-    auto k = few ? dec_rans_slots_kernel<uint32_t> : dec_rans_kernel<uint32_t>;
+    auto k = few     ? dec_rans_slots_kernel<uint32_t>
+             : roomy ? dec_rans_kernel<uint32_t, true>
+                     : dec_rans_kernel<uint32_t, false>;
     k<<<grid, threads, smem, stream>>>(frames, state, shards, lists, list_items, tables,
                                        static_cast<uint32_t*>(folded));
   }
 }
 
 cudaError_t dec_rans_set_smem() {
-  const int b = static_cast<int>(dec_rans_smem()), bs = static_cast<int>(dec_rans_slots_smem());
+  const int b = static_cast<int>(dec_rans_smem<false>()), br = static_cast<int>(dec_rans_smem<true>()),
+            bs = static_cast<int>(dec_rans_slots_smem());
   auto set = [](auto k, int bytes) {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     return e != cudaSuccess ? e
                             : cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
                                                    cudaSharedmemCarveoutMaxShared);
   };
-  cudaError_t e = set(dec_rans_kernel<uint16_t>, b);
-  if (e == cudaSuccess) e = set(dec_rans_kernel<uint32_t>, b);
+  cudaError_t e = set(dec_rans_kernel<uint16_t, false>, b);
+  if (e == cudaSuccess) e = set(dec_rans_kernel<uint32_t, false>, b);
+  if (e == cudaSuccess) e = set(dec_rans_kernel<uint16_t, true>, br);
+  if (e == cudaSuccess) e = set(dec_rans_kernel<uint32_t, true>, br);
   if (e == cudaSuccess) e = set(dec_rans_slots_kernel<uint16_t>, bs);
   if (e == cudaSuccess) e = set(dec_rans_slots_kernel<uint32_t>, bs);
   return e;

@@ -157,8 +157,9 @@ __global__ void dec_parse_kernel(const FrameDesc* frames, FrameState* state, con
 __global__ void dec_rans_tables_kernel(const FrameDesc* frames, FrameState* state, const ShardInfo* shards,
                                        const DecodeLists* lists, const int32_t* list_items, RansTable* tables,
                                        int fold16);
-// `few` shards: one warp for two shards, tables of all slots
-void dec_rans_launch(bool fold16, bool few, int grid, cudaStream_t stream, const FrameDesc* frames,
+// `few` shards: one warp for two shards, tables of all slots; `roomy`: entries
+// and values of up to 176 symbols in shared memory
+void dec_rans_launch(bool fold16, bool few, bool roomy, int grid, cudaStream_t stream, const FrameDesc* frames,
                      FrameState* state, const ShardInfo* shards, DecodeLists* lists, const int32_t* list_items,
                      const RansTable* tables, void* folded);
 cudaError_t dec_rans_set_smem();

@@ -91,3 +91,28 @@ def test_neighbouring_shards_of_different_tables(cuda, depth):
     assert bytes(stream.cpu().numpy()) == oracle.encode(tuple(np.ascontiguousarray(p) for p in planes), **kw)
     for a, b in zip(fastvid_b200.decode(stream), planes):
         assert np.array_equal(a.cpu().numpy(), b)
+
+
+def test_short_shards_of_all_table_sizes(cuda):
+    """More shards than dec_rans gives room for whole tables: tables within the
+    small local room, above it, and built by the decoder, narrow and wide."""
+    gen = torch.Generator(device="cpu")
+    gen.manual_seed(4)
+    rows, cols = 133, 72  # tiles of 32x16, three planes: 28,728 shards
+    spread = torch.tensor([120, 2, 10, 80, 115, 17, 0, 40, 120, 30, 7])
+    planes = []
+    for p in range(3):
+        tiles = torch.rand(rows, 16, cols, 32, generator=gen)
+        tiles *= spread[(torch.arange(rows * cols) + p) % len(spread)].view(rows, 1, cols, 1) + 1
+        planes.append(tiles.to(torch.int32).view(rows * 16, cols * 32).to(torch.uint16).to(cuda))
+    codec = BatchCodec(cuda)
+    streams = codec.encode([planes], layout="rgb444", bit_depth=12, quality=100, tile_size=(32, 16))
+    for a, b in zip(codec.decode(streams)[0], planes):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+    # and as the only frames of their kind (tables of all slots), in the oracle's bytes
+    part = tuple(p[:64, :160].contiguous() for p in planes)
+    kw = dict(layout="rgb444", bit_depth=12, quality=100, tile_size=(32, 16))
+    stream = fastvid_b200.encode(part, **kw)
+    assert bytes(stream.cpu().numpy()) == oracle.encode(tuple(p.cpu().numpy() for p in part), **kw)
+    for a, b in zip(fastvid_b200.decode(stream), part):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
