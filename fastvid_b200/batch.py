@@ -201,6 +201,7 @@ class BatchCodec:
         rates = _per_frame(frame_rate, n, "frame_rate")
         tiles = _per_frame(tile_size, n, "tile_size")
         plans, shapes, ptrs, pitches = [], [], [], []
+        held = []  # copies of planes that had to be made contiguous, until the encoder has read them
         for i, planes in enumerate(frames):
             lay = layouts[i]
             if lay is None:
@@ -223,6 +224,8 @@ class BatchCodec:
                 shape = self._enc_shape(frame)
                 if all(v is p for v, p in zip(views, planes)):  # no copy was needed: cacheable
                     self._plans[key] = (frame, pit, shape)
+                else:
+                    held.append(views)
             plans.append(frame)
             shapes.append(shape)
             for v in views:
