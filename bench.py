@@ -485,7 +485,7 @@ def run_reference_gpu(args, specs):
 
 # Algorithmic bytes per sample of each stage (encode: 2 B in + stream out;
 # decode: stream in + 2 B out).  A kernel is charged its stage's figure.
-ENC_KERNELS = {"enc_init", "enc_predict", "enc_predict_wide", "enc_analyze", "enc_rans", "enc_scan", "enc_prefix",
+ENC_KERNELS = {"enc_init", "enc_predict", "enc_predict_wide", "enc_analyze", "enc_rans", "enc_scan",
                "enc_emit", "enc_lossless"}
 
 

@@ -51,12 +51,12 @@ int cuda_fail(cudaError_t e, const char* where) {
 // by CUDA events on its own stream and the elapsed times are summed per
 // kernel when profiling ends.
 enum KernelId {
-  K_ENC_INIT, K_ENC_PREDICT, K_ENC_PREDICT_WIDE, K_ENC_ANALYZE, K_ENC_RANS, K_ENC_SCAN, K_ENC_PREFIX,
+  K_ENC_INIT, K_ENC_PREDICT, K_ENC_PREDICT_WIDE, K_ENC_ANALYZE, K_ENC_RANS, K_ENC_SCAN,
   K_ENC_EMIT, K_DEC_PARSE, K_DEC_SHARDS, K_DEC_RECON, K_DEC_RECON_WIDE, K_DEC_RECON_SERIAL, K_RESULTS,
   K_DEC_RANS, K_DEC_OTHER, K_ENC_LOSSLESS, K_COUNT
 };
 const char* const kKernelNames[K_COUNT] = {
-    "enc_init", "enc_predict", "enc_predict_wide", "enc_analyze", "enc_rans", "enc_scan", "enc_prefix",
+    "enc_init", "enc_predict", "enc_predict_wide", "enc_analyze", "enc_rans", "enc_scan",
     "enc_emit", "dec_parse", "dec_rans_tables", "dec_reconstruct", "dec_reconstruct_wide",
     "dec_reconstruct_serial", "results", "dec_rans", "dec_other", "enc_lossless"};
 constexpr int kGroupShards = 8;
@@ -692,7 +692,7 @@ int grid_for(int64_t items, int per_cta, int ctas_per_sm) {
 // it -- every such kernel takes its work from a queue or a grid-stride loop.
 constexpr int kDefaultCtas[K_COUNT] = {
     /*enc_init*/ 0, /*enc_predict*/ 4, /*enc_predict_wide*/ 8, /*enc_analyze*/ 6, /*enc_rans*/ 0,
-    /*enc_scan*/ 0, /*enc_prefix*/ 0, /*enc_emit*/ 8, /*dec_parse*/ 8, /*dec_rans_tables*/ 16,
+    /*enc_scan*/ 0, /*enc_emit*/ 8, /*dec_parse*/ 8, /*dec_rans_tables*/ 16,
     /*dec_reconstruct*/ 4, /*dec_reconstruct_wide*/ 8, /*dec_reconstruct_serial*/ 0, /*results*/ 0,
     /*dec_rans*/ 16, /*dec_other*/ 16, /*enc_lossless*/ 0};
 std::atomic<int> g_ctas[K_COUNT];

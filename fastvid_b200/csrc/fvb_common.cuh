@@ -172,17 +172,6 @@ __host__ __device__ inline TileGeo tile_geo(const FrameDesc& f, int64_t t) {
   return g;
 }
 
-// Locate the frame of a global index (frames sorted by base); n is small.
-__device__ inline int find_frame(const int64_t* bases, int n, int64_t idx) {
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (bases[mid] <= idx) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
-
 __device__ inline void set_status(int32_t* status, int32_t code) { atomicCAS(status, 0, code); }
 
 // Asynchronous global -> shared copies (cp.async, sm_80+), completed per

@@ -1249,23 +1249,22 @@ dec_other_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ 
 // 64-column ring, the reconstruction goes out through another and is flushed
 // to the output plane 32 columns at a time (decode.cu:552-606).
 
-template <typename FoldT>
 struct RecWarpSmem {
-  static constexpr int kFS = fold_stride<FoldT>();
-  FoldT fold[32 * kFS];             // folded-residual ring (skewed)
+  static constexpr int kFS = kFoldStride;
+  uint32_t fold[32 * kFS];             // folded-residual ring (skewed)
   uint16_t out[32 * kSrcStride];    // reconstruction ring (u16, skewed)
   uint16_t carry[kFastMaxW + 128];  // row above the band, column c at index c + 32
 };
 
 size_t dec_reconstruct_smem(bool fold16) {
-  return (fold16 ? sizeof(WaveSm) : sizeof(RecWarpSmem<uint32_t>)) * kWarpsPerCta;
+  return (fold16 ? sizeof(WaveSm) : sizeof(RecWarpSmem)) * kWarpsPerCta;
 }
 
-template <bool MED, bool STEP1, bool EDGE, int UNROLL, bool SPLIT, typename FoldT>
-__device__ __forceinline__ void rec_block(RecWarpSmem<FoldT>& sm, const uint16_t* carry_in, uint16_t* carry_out, int lane,
+template <bool MED, bool STEP1, bool EDGE, int UNROLL, bool SPLIT>
+__device__ __forceinline__ void rec_block(RecWarpSmem& sm, const uint16_t* carry_in, uint16_t* carry_out, int lane,
                                           int t0, int W, int32_t maxs, int32_t step, bool band0, int32_t& rec,
                                           int32_t& a_prev) {
-  const FoldT* frow = sm.fold + lane * RecWarpSmem<FoldT>::kFS + (t0 & 32);
+  const uint32_t* frow = sm.fold + lane * RecWarpSmem::kFS + (t0 & 32);
   uint16_t* orow = sm.out + lane * kSrcStride + (t0 & 32);
   const uint16_t* crow_in = carry_in + 32 - lane + t0;  // lane 0: column t0 + u
   // one warp per tile reads and writes the same row: one pointer
@@ -1298,35 +1297,35 @@ __device__ __forceinline__ void rec_block(RecWarpSmem<FoldT>& sm, const uint16_t
 // flushes the rest.  Lane 0 reads the row above the band from carry_in;
 // lane 31 writes the band's last row to carry_out (one warp per tile: the
 // same row, read before it is overwritten).
-template <bool MED, bool STEP1, int UNROLL, bool SPLIT, typename FoldT>
+template <bool MED, bool STEP1, int UNROLL, bool SPLIT>
 struct RecBand {
-  static constexpr int kFS = RecWarpSmem<FoldT>::kFS;
-  RecWarpSmem<FoldT>& sm;
+  static constexpr int kFS = RecWarpSmem::kFS;
+  RecWarpSmem& sm;
   int lane;
   uint16_t* __restrict__ plane;
   int64_t pitch;
   int W, H, x0, y0;
   int32_t maxs, step;
   int nchunks, nblocks;
-  const FoldT* __restrict__ ftile;
+  const uint32_t* __restrict__ ftile;
   int band_rows;
   bool band0;
   uint16_t* __restrict__ orows;
-  const FoldT* __restrict__ frows;
+  const uint32_t* __restrict__ frows;
   const uint16_t* carry_in;
   uint16_t* carry_out;
   int32_t rec, a_prev;
   uint32_t pf[32];
 
-  __device__ RecBand(const FrameDesc& f, const TileGeo& g, int32_t step_, const FoldT* ftile_,
-                     RecWarpSmem<FoldT>& sm_, int lane_)
+  __device__ RecBand(const FrameDesc& f, const TileGeo& g, int32_t step_, const uint32_t* ftile_,
+                     RecWarpSmem& sm_, int lane_)
       : sm(sm_), lane(lane_), plane(f.dst[g.plane]), pitch(f.dst_pitch[g.plane]), W(g.w), H(g.h), x0(g.x),
         y0(g.y), maxs(f.max_sample), step(step_), nchunks((g.w + 31) >> 5), nblocks((g.w + 31 + 31) >> 5),
         ftile(ftile_) {}
 
   __device__ void load_chunk(int k) {
     const int col = k * 32 + lane;
-    const FoldT* __restrict__ p = frows + col;
+    const uint32_t* __restrict__ p = frows + col;
     if (band_rows == 32 && col < W) {
 #pragma unroll
       for (int r = 0; r < 32; ++r) pf[r] = ldf(p + static_cast<int64_t>(r) * W);
@@ -1338,7 +1337,7 @@ struct RecBand {
   __device__ void store_chunk(int k) {
     const int pj = k * 32 + lane;
 #pragma unroll
-    for (int r = 0; r < 32; ++r) sm.fold[r * kFS + ((pj + r) & 63)] = static_cast<FoldT>(pf[r]);
+    for (int r = 0; r < 32; ++r) sm.fold[r * kFS + ((pj + r) & 63)] = pf[r];
   }
   __device__ void flush_chunk(int k) {
     const int col = k * 32 + lane;
@@ -1375,9 +1374,9 @@ struct RecBand {
     }
     const int t0 = blk * 32;
     if (t0 < 31 || t0 + 31 >= W)
-      rec_block<MED, STEP1, true, UNROLL, SPLIT, FoldT>(sm, carry_in, carry_out, lane, t0, W, maxs, step, band0, rec, a_prev);
+      rec_block<MED, STEP1, true, UNROLL, SPLIT>(sm, carry_in, carry_out, lane, t0, W, maxs, step, band0, rec, a_prev);
     else
-      rec_block<MED, STEP1, false, UNROLL, SPLIT, FoldT>(sm, carry_in, carry_out, lane, t0, W, maxs, step, band0, rec, a_prev);
+      rec_block<MED, STEP1, false, UNROLL, SPLIT>(sm, carry_in, carry_out, lane, t0, W, maxs, step, band0, rec, a_prev);
   }
   __device__ void end() {
     __syncwarp();
@@ -1391,9 +1390,9 @@ __device__ __forceinline__ void pair_sync(int pair) {
   asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
 }
 
-template <bool MED, bool STEP1, int UNROLL, bool PAIRS, typename FoldT>
-__device__ void rec_tile(const FrameDesc& f, const TileGeo& g, int32_t step, const FoldT* __restrict__ ftile,
-                         RecWarpSmem<FoldT>* smw, int warp, int lane) {
+template <bool MED, bool STEP1, int UNROLL, bool PAIRS>
+__device__ void rec_tile(const FrameDesc& f, const TileGeo& g, int32_t step, const uint32_t* __restrict__ ftile,
+                         RecWarpSmem* smw, int warp, int lane) {
   if constexpr (PAIRS) {
     if (pair_splits(g.w, g.h)) {
       // warp pair: even bands on the first warp, odd bands on the second two
@@ -1402,8 +1401,8 @@ __device__ void rec_tile(const FrameDesc& f, const TileGeo& g, int32_t step, con
       // other's.  Both warps take the same number of slots (a function of the
       // tile's size only).
       const int pw = warp & 1;
-      RecWarpSmem<FoldT>& sm = smw[warp];
-      RecBand<MED, STEP1, UNROLL, true, FoldT> rb(f, g, step, ftile, sm, lane);
+      RecWarpSmem& sm = smw[warp];
+      RecBand<MED, STEP1, UNROLL, true> rb(f, g, step, ftile, sm, lane);
       const int n = rb.nblocks, nbands = (g.h + 31) >> 5;
       const int own = pw ? (nbands / 2) * n : ((nbands + 1) / 2) * n;
       const int slots = max(((nbands + 1) / 2) * n, (nbands / 2) * n + 2);
@@ -1421,8 +1420,8 @@ __device__ void rec_tile(const FrameDesc& f, const TileGeo& g, int32_t step, con
     }
     if (warp & 1) return;  // too small to split: the pair's first warp alone
   }
-  RecWarpSmem<FoldT>& sm = smw[warp];
-  RecBand<MED, STEP1, UNROLL, false, FoldT> rb(f, g, step, ftile, sm, lane);
+  RecWarpSmem& sm = smw[warp];
+  RecBand<MED, STEP1, UNROLL, false> rb(f, g, step, ftile, sm, lane);
   for (int band = 0; band * 32 < g.h; ++band) {
     rb.begin(band, sm.carry, sm.carry);
     for (int blk = 0; blk < rb.nblocks; ++blk) rb.block(blk);
@@ -1446,10 +1445,10 @@ __device__ __forceinline__ void write_results(const FrameDesc* frames, const Fra
 // tile and both read it after the pair barrier (two alternating slots, so a
 // claim never overwrites a tile the other warp has yet to read); both then
 // make the same decisions from the same tile, so they meet at every barrier.
-template <int UNROLL, bool PAIRS, typename FoldT>
+template <int UNROLL, bool PAIRS>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, PAIRS ? 3 : 4)
 dec_reconstruct_kernel(const FrameDesc* __restrict__ frames, const FrameState* __restrict__ state,
-                       const BatchDims* __restrict__ dims, const FoldT* __restrict__ folded,
+                       const BatchDims* __restrict__ dims, const uint32_t* __restrict__ folded,
                        int* __restrict__ queue, int64_t* __restrict__ results) {
   static_assert(kWarpsPerCta % 2 == 0, "warp pairs");
   constexpr bool pairs = PAIRS;
@@ -1459,7 +1458,7 @@ dec_reconstruct_kernel(const FrameDesc* __restrict__ frames, const FrameState* _
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int64_t claimed[kWarpsPerCta / 2][2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  RecWarpSmem<FoldT>* smw = reinterpret_cast<RecWarpSmem<FoldT>*>(smem_raw);
+  RecWarpSmem* smw = reinterpret_cast<RecWarpSmem*>(smem_raw);
   for (int it = 0;; ++it) {
     int64_t t = 0;
     if (pairs) {
@@ -1476,13 +1475,13 @@ dec_reconstruct_kernel(const FrameDesc* __restrict__ frames, const FrameState* _
     if (state[fi].status != 0) continue;
     const TileGeo g = tile_geo(f, t - f.tile_base);
     if (g.w > kFastMaxW) continue;
-    const FoldT* ftile = folded + f.sample_base + g.sample_base;
+    const uint32_t* ftile = folded + f.sample_base + g.sample_base;
     if (f.use_med0) {
-      if (f.step0 == 1) rec_tile<true, true, UNROLL, PAIRS, FoldT>(f, g, 1, ftile, smw, warp, lane);
-      else rec_tile<true, false, UNROLL, PAIRS, FoldT>(f, g, f.step0, ftile, smw, warp, lane);
+      if (f.step0 == 1) rec_tile<true, true, UNROLL, PAIRS>(f, g, 1, ftile, smw, warp, lane);
+      else rec_tile<true, false, UNROLL, PAIRS>(f, g, f.step0, ftile, smw, warp, lane);
     } else {
-      if (f.step0 == 1) rec_tile<false, true, UNROLL, PAIRS, FoldT>(f, g, 1, ftile, smw, warp, lane);
-      else rec_tile<false, false, UNROLL, PAIRS, FoldT>(f, g, f.step0, ftile, smw, warp, lane);
+      if (f.step0 == 1) rec_tile<false, true, UNROLL, PAIRS>(f, g, 1, ftile, smw, warp, lane);
+      else rec_tile<false, false, UNROLL, PAIRS>(f, g, f.step0, ftile, smw, warp, lane);
     }
   }
 }
@@ -1651,9 +1650,9 @@ dec_reconstruct_wave_kernel(const FrameDesc* __restrict__ frames, const FrameSta
 // 8, 16 or 32 steps unrolled; identical planes), as are its warps per tile.
 cudaError_t dec_reconstruct_set_smem() {
   const int b32 = static_cast<int>(dec_reconstruct_smem(false)), b16 = static_cast<int>(dec_reconstruct_smem(true));
-  for (auto k : {dec_reconstruct_kernel<4, false, uint32_t>, dec_reconstruct_kernel<8, false, uint32_t>,
-                 dec_reconstruct_kernel<16, false, uint32_t>, dec_reconstruct_kernel<32, false, uint32_t>,
-                 dec_reconstruct_kernel<8, true, uint32_t>}) {
+  for (auto k : {dec_reconstruct_kernel<4, false>, dec_reconstruct_kernel<8, false>,
+                 dec_reconstruct_kernel<16, false>, dec_reconstruct_kernel<32, false>,
+                 dec_reconstruct_kernel<8, true>}) {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, b32);
     if (e != cudaSuccess) return e;
   }
@@ -1676,11 +1675,11 @@ void dec_reconstruct_launch(int unroll, int tile_warps, bool fold16, bool pairs,
     return;
   }
   // warp pairs run with the default wavefront block
-  auto k = tile_warps == 2 ? dec_reconstruct_kernel<8, true, uint32_t>
-           : unroll == 4   ? dec_reconstruct_kernel<4, false, uint32_t>
-           : unroll == 16  ? dec_reconstruct_kernel<16, false, uint32_t>
-           : unroll == 32  ? dec_reconstruct_kernel<32, false, uint32_t>
-                           : dec_reconstruct_kernel<8, false, uint32_t>;
+  auto k = tile_warps == 2 ? dec_reconstruct_kernel<8, true>
+           : unroll == 4   ? dec_reconstruct_kernel<4, false>
+           : unroll == 16  ? dec_reconstruct_kernel<16, false>
+           : unroll == 32  ? dec_reconstruct_kernel<32, false>
+                           : dec_reconstruct_kernel<8, false>;
   k<<<grid, kWarpsPerCta * 32, dec_reconstruct_smem(false), stream>>>(
       frames, state, dims, static_cast<const uint32_t*>(folded), queue, results);
 }

@@ -55,20 +55,19 @@ __device__ __forceinline__ int32_t div_step(uint32_t n, uint32_t magic) {
 // the instruction's immediate inside each unrolled 32-step block.  Blocks in
 // which every lane's column lies inside the tile run without predicates.
 
-template <typename FoldT>
 struct EncWarpSmem {
-  static constexpr int kFS = fold_stride<FoldT>();
+  static constexpr int kFS = kFoldStride;
   uint16_t src[32 * kSrcStride];    // source ring (u16, skewed)
-  FoldT fold[32 * kFS];             // folded-residual ring (skewed)
+  uint32_t fold[32 * kFS];             // folded-residual ring (skewed)
   uint16_t carry[kFastMaxW + 128];  // row above the band, column c at index c + 32
 };
 
-template <bool MED, bool EDGE, int UNROLL, bool SPLIT, typename FoldT>
-__device__ __forceinline__ void enc_block(EncWarpSmem<FoldT>& sm, const uint16_t* carry_in, uint16_t* carry_out, int lane,
+template <bool MED, bool EDGE, int UNROLL, bool SPLIT>
+__device__ __forceinline__ void enc_block(EncWarpSmem& sm, const uint16_t* carry_in, uint16_t* carry_out, int lane,
                                           int t0, int W, int32_t maxs, int32_t step, int32_t half, uint32_t magic,
                                           bool band0, int32_t& rec, int32_t& a_prev) {
   const uint16_t* srow = sm.src + lane * kSrcStride + (t0 & 32);
-  FoldT* frow = sm.fold + lane * EncWarpSmem<FoldT>::kFS + (t0 & 32);
+  uint32_t* frow = sm.fold + lane * EncWarpSmem::kFS + (t0 & 32);
   const uint16_t* crow_in = carry_in + 32 - lane + t0;  // lane 0: column t0 + u
   // one warp per tile reads and writes the same row: one pointer
   uint16_t* crow_out = SPLIT ? carry_out + 32 - lane + t0 : const_cast<uint16_t*>(crow_in);      // lane 31: column t0 + u - 31 (index (t - lane) + 32)
@@ -90,7 +89,7 @@ __device__ __forceinline__ void enc_block(EncWarpSmem<FoldT>& sm, const uint16_t
     } else {
       if (lane == 31) crow_out[u] = static_cast<uint16_t>(rn);
     }
-    frow[u] = static_cast<FoldT>(zigzag(q));
+    frow[u] = zigzag(q);
     a_prev = a;
     rec = rn;
   }
@@ -101,10 +100,10 @@ __device__ __forceinline__ void enc_block(EncWarpSmem<FoldT>& sm, const uint16_t
 // source chunks, block(k) runs wavefront block k (staging the chunk ahead
 // and flushing the folded residuals two chunks behind), end() flushes the
 // rest.  vmax tracks the largest source sample read (the depth check).
-template <bool MED, int UNROLL, bool SPLIT, typename FoldT>
+template <bool MED, int UNROLL, bool SPLIT>
 struct EncBand {
-  static constexpr int kFS = EncWarpSmem<FoldT>::kFS;
-  EncWarpSmem<FoldT>& sm;
+  static constexpr int kFS = EncWarpSmem::kFS;
+  EncWarpSmem& sm;
   int lane;
   const uint16_t* __restrict__ plane;
   int64_t pitch;
@@ -112,19 +111,19 @@ struct EncBand {
   int32_t maxs, step, half;
   uint32_t magic;
   int nchunks, nblocks;
-  FoldT* __restrict__ ftile;
+  uint32_t* __restrict__ ftile;
   uint32_t vmax = 0;
   int band_rows;
   bool band0;
   const uint16_t* __restrict__ rows;
-  FoldT* __restrict__ frows;
+  uint32_t* __restrict__ frows;
   const uint16_t* carry_in;
   uint16_t* carry_out;
   int32_t rec, a_prev;
   uint32_t pf[32];
 
-  __device__ EncBand(const FrameDesc& f, const TileGeo& g, int32_t step_, uint32_t magic_, FoldT* ftile_,
-                     EncWarpSmem<FoldT>& sm_, int lane_)
+  __device__ EncBand(const FrameDesc& f, const TileGeo& g, int32_t step_, uint32_t magic_, uint32_t* ftile_,
+                     EncWarpSmem& sm_, int lane_)
       : sm(sm_), lane(lane_), plane(f.src[g.plane]), pitch(f.src_pitch[g.plane]), W(g.w), H(g.h), x0(g.x), y0(g.y),
         maxs(f.max_sample), step(step_), half(step_ >> 1), magic(magic_), nchunks((g.w + 31) >> 5),
         nblocks((g.w + 31 + 31) >> 5), ftile(ftile_) {}
@@ -154,7 +153,7 @@ struct EncBand {
   __device__ void flush_chunk(int k) {
     const int col = k * 32 + lane;
     if (col < W) {
-      FoldT* __restrict__ q = frows + col;
+      uint32_t* __restrict__ q = frows + col;
       if (band_rows == 32) {
 #pragma unroll
         for (int r = 0; r < 32; ++r) q[static_cast<int64_t>(r) * W] = sm.fold[r * kFS + ((col + r) & 63)];
@@ -186,10 +185,10 @@ struct EncBand {
     }
     const int t0 = blk * 32;
     if (t0 < 31 || t0 + 31 >= W)
-      enc_block<MED, true, UNROLL, SPLIT, FoldT>(sm, carry_in, carry_out, lane, t0, W, maxs, step, half, magic, band0, rec,
+      enc_block<MED, true, UNROLL, SPLIT>(sm, carry_in, carry_out, lane, t0, W, maxs, step, half, magic, band0, rec,
                                           a_prev);
     else
-      enc_block<MED, false, UNROLL, SPLIT, FoldT>(sm, carry_in, carry_out, lane, t0, W, maxs, step, half, magic, band0, rec,
+      enc_block<MED, false, UNROLL, SPLIT>(sm, carry_in, carry_out, lane, t0, W, maxs, step, half, magic, band0, rec,
                                            a_prev);
   }
   __device__ void end() {
@@ -202,10 +201,10 @@ struct EncBand {
 // A tile by one warp: bands in order, one carry row (read by lane 0 before
 // lane 31 overwrites it).  Kept apart from EncBand: written as one loop nest
 // it needs no register spills.
-template <bool MED, int UNROLL, typename FoldT>
+template <bool MED, int UNROLL>
 __device__ void enc_tile_fast(const FrameDesc& f, const TileGeo& g, int32_t step, uint32_t magic,
-                              FoldT* __restrict__ folded_tile, EncWarpSmem<FoldT>& sm, int lane, int32_t& bad) {
-  constexpr int kFS = EncWarpSmem<FoldT>::kFS;
+                              uint32_t* __restrict__ folded_tile, EncWarpSmem& sm, int lane, int32_t& bad) {
+  constexpr int kFS = EncWarpSmem::kFS;
   const uint16_t* __restrict__ plane = f.src[g.plane];
   const int64_t pitch = f.src_pitch[g.plane];
   const int W = g.w, H = g.h;
@@ -217,7 +216,7 @@ __device__ void enc_tile_fast(const FrameDesc& f, const TileGeo& g, int32_t step
   for (int band = 0; band * 32 < H; ++band) {
     const int band_rows = min(32, H - band * 32);
     const uint16_t* __restrict__ rows = plane + static_cast<int64_t>(g.y + band * 32) * pitch + g.x;
-    FoldT* __restrict__ frows = folded_tile + static_cast<int64_t>(band * 32) * W;
+    uint32_t* __restrict__ frows = folded_tile + static_cast<int64_t>(band * 32) * W;
     uint32_t pf[32];
     auto load_chunk = [&](int k) {
       const int col = k * 32 + lane;
@@ -243,7 +242,7 @@ __device__ void enc_tile_fast(const FrameDesc& f, const TileGeo& g, int32_t step
     auto flush_chunk = [&](int k) {
       const int col = k * 32 + lane;
       if (col < W) {
-        FoldT* __restrict__ q = frows + col;
+        uint32_t* __restrict__ q = frows + col;
         if (band_rows == 32) {
 #pragma unroll
           for (int r = 0; r < 32; ++r) q[static_cast<int64_t>(r) * W] = sm.fold[r * kFS + ((col + r) & 63)];
@@ -268,10 +267,10 @@ __device__ void enc_tile_fast(const FrameDesc& f, const TileGeo& g, int32_t step
       const int t0 = blk * 32;
       const bool edge = t0 < 31 || t0 + 31 >= W;
       if (edge)
-        enc_block<MED, true, UNROLL, false, FoldT>(sm, sm.carry, sm.carry, lane, t0, W, maxs, step, half, magic, band0,
+        enc_block<MED, true, UNROLL, false>(sm, sm.carry, sm.carry, lane, t0, W, maxs, step, half, magic, band0,
                                                    rec, a_prev);
       else
-        enc_block<MED, false, UNROLL, false, FoldT>(sm, sm.carry, sm.carry, lane, t0, W, maxs, step, half, magic,
+        enc_block<MED, false, UNROLL, false>(sm, sm.carry, sm.carry, lane, t0, W, maxs, step, half, magic,
                                                     band0, rec, a_prev);
     }
     __syncwarp();
@@ -286,9 +285,9 @@ __device__ __forceinline__ void enc_pair_sync(int pair) {
   asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
 }
 
-template <bool MED, int UNROLL, bool PAIRS, typename FoldT>
+template <bool MED, int UNROLL, bool PAIRS>
 __device__ void enc_tile(const FrameDesc& f, const TileGeo& g, int32_t step, uint32_t magic,
-                         FoldT* __restrict__ folded_tile, EncWarpSmem<FoldT>* smw, int warp, int lane,
+                         uint32_t* __restrict__ folded_tile, EncWarpSmem* smw, int warp, int lane,
                          int32_t& bad) {
   if constexpr (PAIRS) {
     if (pair_splits(g.w, g.h)) {
@@ -296,8 +295,8 @@ __device__ void enc_tile(const FrameDesc& f, const TileGeo& g, int32_t step, uin
       // blocks behind, in lock-step at the pair barrier after every slot (the
       // schedule of dec_reconstruct)
       const int pw = warp & 1;
-      EncWarpSmem<FoldT>& sm = smw[warp];
-      EncBand<MED, UNROLL, true, FoldT> eb(f, g, step, magic, folded_tile, sm, lane);
+      EncWarpSmem& sm = smw[warp];
+      EncBand<MED, UNROLL, true> eb(f, g, step, magic, folded_tile, sm, lane);
       const int n = eb.nblocks, nbands = (g.h + 31) >> 5;
       const int own = pw ? (nbands / 2) * n : ((nbands + 1) / 2) * n;
       const int slots = max(((nbands + 1) / 2) * n, (nbands / 2) * n + 2);
@@ -316,7 +315,7 @@ __device__ void enc_tile(const FrameDesc& f, const TileGeo& g, int32_t step, uin
     }
     if (warp & 1) return;  // too small to split: the pair's first warp alone
   }
-  enc_tile_fast<MED, UNROLL, FoldT>(f, g, step, magic, folded_tile, smw[warp], lane, bad);
+  enc_tile_fast<MED, UNROLL>(f, g, step, magic, folded_tile, smw[warp], lane, bad);
 }
 
 // Shard records of a tile (encode.cu:753-759), written for every frame of the
@@ -340,11 +339,11 @@ __device__ __forceinline__ bool frame_lossless(const FrameDesc& f) { return f.st
 // Tiles come from a queue; with warp pairs the pair's first warp claims a
 // tile and both read it after the pair barrier (two alternating slots), and
 // both make the same decisions from it, so they meet at every barrier.
-template <int UNROLL, bool PAIRS, typename FoldT>
+template <int UNROLL, bool PAIRS>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, PAIRS ? 3 : 4)
 enc_predict_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict__ state,
                    const BatchDims* __restrict__ dims, int pass, ShardInfo* __restrict__ shards,
-                   FoldT* __restrict__ folded, int* __restrict__ queue) {
+                   uint32_t* __restrict__ folded, int* __restrict__ queue) {
   static_assert(kWarpsPerCta % 2 == 0, "warp pairs");
   constexpr bool pairs = PAIRS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -352,7 +351,7 @@ enc_predict_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict_
   const int nframes = dims->frames_p[pass];
   const int64_t total_tiles = dims->tiles_p[pass];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  EncWarpSmem<FoldT>* smw = reinterpret_cast<EncWarpSmem<FoldT>*>(smem_raw);
+  EncWarpSmem* smw = reinterpret_cast<EncWarpSmem*>(smem_raw);
   for (int it = 0;; ++it) {
     int64_t t = 0;
     if (pairs) {
@@ -375,11 +374,11 @@ enc_predict_kernel(const FrameDesc* __restrict__ frames, FrameState* __restrict_
     if (g.w > kFastMaxW) continue;  // wide tiles go through enc_predict_wide_kernel
     const int32_t step = st.step;
     const uint32_t magic = step > 1 ? static_cast<uint32_t>((0x100000000ull + step - 1) / step) : 0u;
-    FoldT* ftile = folded + f.sample_base + g.sample_base;
+    uint32_t* ftile = folded + f.sample_base + g.sample_base;
     int32_t bad = 0;
     const bool med = st.use_med != 0;
-    if (med) enc_tile<true, UNROLL, PAIRS, FoldT>(f, g, step, magic, ftile, smw, warp, lane, bad);
-    else enc_tile<false, UNROLL, PAIRS, FoldT>(f, g, step, magic, ftile, smw, warp, lane, bad);
+    if (med) enc_tile<true, UNROLL, PAIRS>(f, g, step, magic, ftile, smw, warp, lane, bad);
+    else enc_tile<false, UNROLL, PAIRS>(f, g, step, magic, ftile, smw, warp, lane, bad);
     if (__any_sync(kFull, bad) && lane == 0) set_status(&st.status, 1);
   }
 }
@@ -792,9 +791,9 @@ void enc_lossless_launch(bool fold16, int64_t tiles, int max_ctas, cudaStream_t 
 // as are its warps per tile: every choice computes the same bytes.
 cudaError_t enc_predict_set_smem() {
   const int b32 = static_cast<int>(enc_predict_smem(false)), b16 = static_cast<int>(enc_predict_smem(true));
-  for (auto k : {enc_predict_kernel<4, false, uint32_t>, enc_predict_kernel<8, false, uint32_t>,
-                 enc_predict_kernel<16, false, uint32_t>, enc_predict_kernel<32, false, uint32_t>,
-                 enc_predict_kernel<8, true, uint32_t>}) {
+  for (auto k : {enc_predict_kernel<4, false>, enc_predict_kernel<8, false>,
+                 enc_predict_kernel<16, false>, enc_predict_kernel<32, false>,
+                 enc_predict_kernel<8, true>}) {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, b32);
     if (e != cudaSuccess) return e;
   }
@@ -815,11 +814,11 @@ void enc_predict_launch(int unroll, int tile_warps, bool fold16, bool pairs, int
     return;
   }
   // warp pairs run with the default wavefront block
-  auto k = tile_warps == 2 ? enc_predict_kernel<8, true, uint32_t>
-           : unroll == 4   ? enc_predict_kernel<4, false, uint32_t>
-           : unroll == 16  ? enc_predict_kernel<16, false, uint32_t>
-           : unroll == 32  ? enc_predict_kernel<32, false, uint32_t>
-                           : enc_predict_kernel<8, false, uint32_t>;
+  auto k = tile_warps == 2 ? enc_predict_kernel<8, true>
+           : unroll == 4   ? enc_predict_kernel<4, false>
+           : unroll == 16  ? enc_predict_kernel<16, false>
+           : unroll == 32  ? enc_predict_kernel<32, false>
+                           : enc_predict_kernel<8, false>;
   k<<<grid, kWarpsPerCta * 32, enc_predict_smem(false), stream>>>(frames, state, dims, pass, shards,
                                                                   static_cast<uint32_t*>(folded), queue);
 }
@@ -1815,9 +1814,6 @@ __global__ void enc_init_kernel(const FrameDesc* __restrict__ frames, FrameState
   state[i] = s;
 }
 
-// Before each re-run pass: reset the tile queue.  (Frames whose policy is
-// finished keep active = 0 and are skipped by every kernel.)
-
 // ---------------------------------------------------------------------------
 // enc_emit: one warp per shard.  The record (mode byte, u16 body length,
 // body) is assembled in shared memory -- bit codes merged with shared
@@ -1835,7 +1831,7 @@ struct EmitWarpSmem {
 static_assert(sizeof(EmitWarpSmem) % 16 == 0, "record buffers must stay 16-byte aligned");
 
 size_t enc_predict_smem(bool fold16) {
-  return (fold16 ? sizeof(WaveSm) : sizeof(EncWarpSmem<uint32_t>)) * kWarpsPerCta;
+  return (fold16 ? sizeof(WaveSm) : sizeof(EncWarpSmem)) * kWarpsPerCta;
 }
 size_t enc_emit_smem() { return sizeof(EmitWarpSmem) * kWarpsPerCta; }
 

@@ -33,10 +33,6 @@ __host__ __device__ inline bool pair_splits(int w, int h) { return ((h + 31) >> 
 // 65535 by parity (fold_value), i.e. a residual of +32767 or -32768 steps,
 // which clamps to the same sample as the original since the step is >= 12.
 template <typename T>
-constexpr int fold_stride() {
-  return sizeof(T) == 2 ? kSrcStride : kFoldStride;
-}
-template <typename T>
 using FoldPiece = std::conditional_t<sizeof(T) == 2, uint2, uint4>;  // four symbols
 
 template <typename T>
