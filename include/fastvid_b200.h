@@ -71,25 +71,29 @@ const char* fvb_kernel_name(int kernel);
  * the knob the autotuner sets): its grid is capped at `ctas_per_sm` CTAs per
  * SM, 0 restoring the built-in default.  Process-wide, read at each launch;
  * no output depends on it.  FVB_ERR_ARGUMENT for a kernel without the knob
- * or a value outside 0..64. */
+ * or a value outside 0..64.  dec_rans's cap is for its form on bucket tables:
+ * batches of so few shards that all run at once on tables of all slots (1,776
+ * on B200) are launched whole. */
 int fvb_set_launch_ctas(int kernel, int ctas_per_sm);
 /* The cap in effect, or -1 for a kernel without the knob. */
 int fvb_get_launch_ctas(int kernel);
-/* Wavefront block of the predictor and reconstruction kernels (no
+/* Wavefront block of the predictor and reconstruction kernels of batches whose
+ * folded symbols are u32, i.e. that hold a lossless 16-bit frame (no
  * counterpart in the reference, whose predictor walks antidiagonals with a
  * barrier per step, cuda/csrc/encode.cu:150-192): each warp sweeps 32-row
  * bands in blocks of 32 steps, `steps` (4, 8, 16 or 32) of them unrolled;
- * 0 restores the default (8).  Process-wide, read at each launch; no output
- * depends on it (the autotuner's knob). */
+ * 0 restores the default (8).  u16 batches have one form.  Process-wide, read
+ * at each launch; no output depends on it (the autotuner's knob). */
 int fvb_set_wavefront_block(int steps);
 int fvb_get_wavefront_block(void);
 /* Warps per tile of the predictor and reconstruction kernels (no reference
  * counterpart; the autotuner's knob): 1, or 2 -- a warp pair sweeps a tile's
  * even and odd 32-row bands in lock-step, the second warp two blocks behind,
  * handing each band's last row over in shared memory (tiles of one band or
- * under 66 columns stay on one warp).  0 restores the default (1).
- * Batches whose folded symbols are u16 always sweep a tile with one warp, two
- * rows a lane.  Process-wide, read at each launch; no output depends on it. */
+ * under 66 columns stay on one warp).  0 restores the default (1).  For u32
+ * batches, as the block; u16 batches sweep a tile with a warp pair when they
+ * have up to three tiles an SM and with one warp otherwise, whatever the value.
+ * Process-wide, read at each launch; no output depends on it. */
 int fvb_set_tile_warps(int warps);
 int fvb_get_tile_warps(void);
 /* Whether decode batches of 4096 shards or more run dec_other (Rice,
