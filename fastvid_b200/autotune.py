@@ -7,11 +7,12 @@ Three kinds of knob, tuned by measurement and kept in a JSON table:
   decode warps... share an SM.  No output byte depends on it.  Chosen by
   coordinate descent over the kernels on the measured encode+decode time of a
   sample batch.
-* Wavefront block and warps per tile -- how many of the 32 steps of each
-  wavefront block the predictor and reconstruction warps unroll
-  (fvb_set_wavefront_block: 4, 8, 16 or 32), and whether one warp or a warp
-  pair sweeps a tile's bands (fvb_set_tile_warps: 1 or 2).  No output byte
-  depends on either; tuned before the launch caps.
+* Wavefront block and warps per tile of batches with u32 symbols (those that
+  hold a lossless 16-bit frame) -- how many of the 32 steps of each wavefront
+  block the predictor and reconstruction warps unroll (fvb_set_wavefront_block:
+  4, 8, 16 or 32), and whether one warp or a warp pair sweeps a tile's bands
+  (fvb_set_tile_warps: 1 or 2).  No output byte depends on either; tuned before
+  the launch caps, on the sample's 16-bit frames coded losslessly.
 * Tile geometry per frame format (layout, depth, width, height) -- the
   wavefront block each warp sweeps.  The tile size is written into the
   stream header, so it changes the bytes and the compression; the tuner takes
@@ -147,8 +148,9 @@ def set_rans_pipeline_tail(steps: int) -> None:
 
 
 def apply(table: dict) -> None:
-    """Set the table's launch geometry, wavefront block, warps per tile,
-    decode overlap and rANS encoder pipelines (process-wide)."""
+    """Set the table's launch geometry, wavefront block, warps per tile and
+    decode overlap (process-wide), and the rANS pipeline values, which the
+    library keeps without effect, if the table has any."""
     set_launch(table.get("launch", {}))
     set_wavefront_block(table.get("wavefront_block", 0))
     set_tile_warps(table.get("tile_warps", 0))
@@ -199,6 +201,14 @@ def tune_launch(codec, frames, params, knobs=LAUNCH_KNOBS, candidates=LAUNCH_CAN
     return best
 
 
+def wide_symbol_sample(specs) -> tuple[list[int], dict]:
+    """The frames of a sample, and the parameters, that make a batch with u32
+    symbols, which alone takes the wavefront block and the warps per tile: its
+    16-bit frames, lossless."""
+    idx = [i for i, s in enumerate(specs) if s["bit_depth"] == 16]
+    return idx, dict(layout=[specs[i]["layout"] for i in idx], bit_depth=16, quality=100)
+
+
 def tune_wavefront_block(codec, frames, params, candidates=WAVEFRONT_BLOCKS, reps: int = 3) -> tuple[int, dict]:
     """The wavefront block with the lowest measured batch time (the launch
     caps as currently set); returns it and every candidate's ms."""
@@ -208,20 +218,6 @@ def tune_wavefront_block(codec, frames, params, candidates=WAVEFRONT_BLOCKS, rep
         seen[steps] = _time_batch(codec, frames, params, reps)[0]
     best = min(seen, key=seen.get)
     set_wavefront_block(best)
-    return best, {str(k): round(v, 3) for k, v in seen.items()}
-
-
-def tune_rans_pipeline(codec, frames, params, reps: int = 3, tail: bool = False) -> tuple[int, dict]:
-    """The rANS encoder's fetch scheme (-1 automatic, 0, 8, 16) with the
-    lowest batch time, for the first encoder pass or (tail) the later ones;
-    the automatic choice wins ties."""
-    setter = set_rans_pipeline_tail if tail else set_rans_pipeline
-    seen = {}
-    for steps in (-1, 0, 8, 16):
-        setter(steps)
-        seen[steps] = _time_batch(codec, frames, params, reps)[0]
-    best = min(seen, key=seen.get)
-    setter(best)
     return best, {str(k): round(v, 3) for k, v in seen.items()}
 
 
@@ -294,10 +290,11 @@ def main(argv=None) -> int:
                   tile_size=[tuple(tiles[format_key(s["layout"], s["bit_depth"], s["width"], s["height"])])
                              for s in specs])
     base_ms = _time_batch(codec, frames, params, args.reps)[0]
-    block, block_ms = tune_wavefront_block(codec, frames, params, reps=args.reps)
-    warps, warps_ms = tune_tile_warps(codec, frames, params, reps=args.reps)
-    pipe, pipe_ms = tune_rans_pipeline(codec, frames, params, reps=args.reps)
-    pipe_tail, pipe_tail_ms = tune_rans_pipeline(codec, frames, params, reps=args.reps, tail=True)
+    wide, wide_params = wide_symbol_sample(specs)
+    wide_params["tile_size"] = [params["tile_size"][i] for i in wide]
+    wide = [frames[i] for i in wide]
+    block, block_ms = tune_wavefront_block(codec, wide, wide_params, reps=args.reps)
+    warps, warps_ms = tune_tile_warps(codec, wide, wide_params, reps=args.reps)
     launch = tune_launch(codec, frames, params, reps=args.reps)
     overlap, overlap_ms = tune_decode_overlap(codec, frames, params, reps=args.reps)
     tuned_ms = _time_batch(codec, frames, params, args.reps)[0]
@@ -305,8 +302,6 @@ def main(argv=None) -> int:
              "size_tolerance": args.size_tolerance, "tiles": tiles, "tile_measurements_ms_bytes": measured,
              "wavefront_block": block, "wavefront_block_ms": block_ms,
              "tile_warps": warps, "tile_warps_ms": warps_ms,
-             "rans_pipeline": pipe, "rans_pipeline_ms": pipe_ms,
-             "rans_pipeline_tail": pipe_tail, "rans_pipeline_tail_ms": pipe_tail_ms,
              "decode_overlap": overlap, "decode_overlap_ms": overlap_ms,
              "launch": launch, "launch_gain": {"default_ms": round(base_ms, 3), "tuned_ms": round(tuned_ms, 3)}}
     save(table, args.out)
