@@ -593,10 +593,15 @@ def main():
     # per-kernel times: eager steps, CUDA events around each launch
     eager.decode(eager.encode(dev_frames, layout=layouts, bit_depth=depths, quality=quals, tile_size=tiles))
     torch.cuda.synchronize()
+    # one kernel at a time: beside dec_rans, dec_other's time would be its wait
+    # for room on the SMs
+    overlap = autotune.decode_overlap()
+    autotune.set_decode_overlap(0)
     with _native.KernelProfile() as prof:
         for _ in range(args.steps):
             eager.decode(eager.encode(dev_frames, layout=layouts, bit_depth=depths, quality=quals, tile_size=tiles))
         torch.cuda.synchronize()
+    autotune.set_decode_overlap(overlap)
     enc_ms = sum(a.elapsed_time(b) for a, b, _ in ev) / args.steps
     dec_ms = sum(b.elapsed_time(c) for _, b, c in ev) / args.steps
     step_ms = max_over_ranks(enc_ms + dec_ms)
