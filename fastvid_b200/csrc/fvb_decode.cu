@@ -469,19 +469,21 @@ struct LaneRing {
 };
 
 // Shared memory of one dec_rans warp: eight shards' tables (bucket words, then
-// the entries of up to LOCAL symbols; a shard with more reads its entries from
-// its table record) and the lanes' byte rings; ROOMY: the symbols' values too.
+// the entries of up to kSymbols symbols; a shard with more reads its entries from
+// its table record) and the lanes' byte rings; ROOMY: the symbols' values too, of
+// any shard whose record has a bucket table.
 constexpr int kGroups = 8;  // shards per warp, four lanes each
 template <bool ROOMY>
 struct alignas(16) RansWarpSm {
   // 36: five CTAs on an SM, 758 us for 16 4K rgb10 frames, 854 us with 64 and four
-  static constexpr int kSymbols = ROOMY ? 176 : 36;
-  static constexpr int kWords = kBuckets + kSymbols;
-  static constexpr int kValueWords = ROOMY ? kSymbols / 2 : 0;
+  static constexpr int kSymbols = ROOMY ? kBucketSymbols : 36;
+  static constexpr int kWords = (kBuckets + kSymbols + 3) / 4 * 4;  // copied by 16 bytes
+  static constexpr int kValueWords = ROOMY ? (kSymbols + 7) / 8 * 4 : 0;
   uint32_t table[kGroups][kWords + kValueWords];
   uint4 rings[LaneRing<32>::kChunks][32];
 };
-static_assert(RansWarpSm<true>::kSymbols >= kBucketSymbols && (RansWarpSm<true>::kWords & 3) == 0, "local tables");
+static_assert(RansWarpSm<true>::kSymbols <= kBucketSymbols && RansWarpSm<false>::kSymbols <= kBucketSymbols,
+              "entries are copied with the bucket words");
 
 template <bool ROOMY>
 constexpr size_t dec_rans_smem() { return sizeof(RansWarpSm<ROOMY>) * kWarpsPerCta; }

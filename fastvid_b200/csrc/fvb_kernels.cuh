@@ -154,7 +154,7 @@ __global__ void dec_rans_tables_kernel(const FrameDesc* frames, FrameState* stat
                                        const DecodeLists* lists, const int32_t* list_items, RansTable* tables,
                                        int fold16);
 // `few` shards: one warp for two shards, tables of all slots; `roomy`: entries
-// and values of up to 176 symbols in shared memory
+// and values of up to 170 symbols in shared memory
 void dec_rans_launch(bool fold16, bool few, bool roomy, int grid, cudaStream_t stream, const FrameDesc* frames,
                      FrameState* state, const ShardInfo* shards, DecodeLists* lists, const int32_t* list_items,
                      const RansTable* tables, void* folded);

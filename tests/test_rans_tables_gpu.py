@@ -116,3 +116,30 @@ def test_short_shards_of_all_table_sizes(cuda):
     assert bytes(stream.cpu().numpy()) == oracle.encode(tuple(p.cpu().numpy() for p in part), **kw)
     for a, b in zip(fastvid_b200.decode(stream), part):
         assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
+@pytest.mark.parametrize("tiles", ((24, 28), (5, 9)))
+def test_tables_around_the_bucket_limit(cuda, tiles):
+    """Tables of some 160 to 185 symbols, in many shards and in few: with more
+    than 170 the decoder builds the bucket table itself."""
+    gen = torch.Generator(device="cpu")
+    gen.manual_seed(11)
+    rows, cols = tiles
+    spread = torch.arange(81, 95).repeat(rows * cols)
+    planes = []
+    for p in range(3):
+        t = torch.rand(rows, 64, cols, 64, generator=gen) * (spread[p:p + rows * cols].view(rows, 1, cols, 1) + 1)
+        planes.append(t.to(torch.int32).view(rows * 64, cols * 64).to(torch.uint16).to(cuda))
+    kw = dict(layout="rgb444", bit_depth=12, quality=100, tile_size=(64, 64))
+    codec = BatchCodec(cuda)
+    stream = codec.encode([planes], **kw)[0]
+    for a, b in zip(codec.decode([stream])[0], planes):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+    # the streams do hold tables on both sides of the limit
+    data = stream.cpu().numpy()
+    counts = set()
+    for t in range(int.from_bytes(data[28:32].tobytes(), "little")):
+        off = int.from_bytes(data[52 + 32 * t:60 + 32 * t].tobytes(), "little")
+        if data[off] == 19:
+            counts.add((int(data[off + 4]) & 127) + (int(data[off + 5]) << 7 if data[off + 4] & 128 else 0))
+    assert any(c <= 170 for c in counts) and any(170 < c <= 176 for c in counts) and any(c > 176 for c in counts)
